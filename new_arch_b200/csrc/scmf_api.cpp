@@ -81,8 +81,7 @@ scmf_status regrid(scmf_system* s) {
     CK(cudaMemsetAsync((char*)s->d_sys + offsetof(SysDev, cur), 0, sizeof(uint32_t), s->stream));
     LaunchShape sh = s->plan.move_shape();
     sh.blocks = 0;
-    CKL(launch_sweep(kGridOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh,
-                     s->plan.d_acc, s->stream));
+    CKL(launch_sweep(kGridOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh, s->stream));
     s->counts_stale = false;
     return SCMF_OK;
 }
@@ -387,6 +386,8 @@ static scmf_status create_system(const scmf_spec* spec, bool is_shard, int shard
     h.counts[0] = s->counts[0];
     h.counts[1] = s->counts[1];
     h.omega = s->omega;
+    fill_sweep_constants(&h);
+    s->sweep = h.sweep;
     if (cudaMemcpyAsync(s->chain_id, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(s->d_sys, &h, sizeof h, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemsetAsync(s->x, 0, nbp * 4, st) != cudaSuccess || cudaMemsetAsync(s->y, 0, nbp * 4, st) != cudaSuccess ||
@@ -613,8 +614,7 @@ scmf_status scmf_smc_move(scmf_system* s, int32_t n) {
     if (!s || n < 0) return fail(SCMF_E_INVALID, "bad argument");
     const LaunchShape sh = s->plan.move_shape();
     for (int i = 0; i < n; ++i) {
-        CKL(launch_sweep(kMoveOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh,
-                         s->plan.d_acc, s->stream));
+        CKL(launch_sweep(kMoveOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh, s->stream));
         RET(s->plan.enqueue_close(kCloseMove | kCloseAdvance, s->stream));
     }
     if (n > 0) s->counts_stale = true;  // like the reference, counts wait for reset_density_fields
@@ -919,8 +919,9 @@ static void snap_free(Snapshot* sn, cudaStream_t st) {
 }
 
 // Project-written autotuner: times a small grid of (threads per move CTA,
-// chains per tile, persistent CTAs) and then (cells per field tile) on the
-// batch's own systems, restoring their state after every trial.
+// chains per tile, persistent CTAs), where the general move kernel runs, and
+// then (cells per field tile) on the batch's own systems, restoring their state
+// after every trial.
 scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
     if (!b || sweeps < 1) return fail(SCMF_E_INVALID, "bad arguments");
     RET(batch_sync_members(b));
@@ -952,39 +953,37 @@ scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
     float best_ms = 1e30f;
     b->trials.clear();
     if (!rc) {
-        const int tile_beads[] = {1024, 2048, 4096, 8192};
-        const int threads[] = {64, 128, 256};
-        const int persist[] = {0, sm_count() * 4};
-        for (int tb : tile_beads)
-            for (int th : threads)
-                for (int pc : persist) {
-                    if (rc) break;
-                    scmf_tune t = b->plan.tune;
-                    t.chains_per_tile = 0;
-                    t.beads_per_tile = tb;
-                    t.threads_move = th;
-                    t.persistent_ctas = pc;
-                    float ms = 0;
-                    rc = trial(t, &ms);
-                    if (!rc) b->trials.push_back({t, ms});
-                    if (!rc && ms < best_ms) {
-                        best_ms = ms;
-                        best = t;
-                    }
-                }
-        const int cells[] = {2048, 8192, 32768};
-        scmf_tune base = best;
-        for (int c : cells) {
-            if (rc) break;
-            scmf_tune t = base;
-            t.cells_per_tile = c;
+        const auto tried = [&](const scmf_tune& t) {
             float ms = 0;
             rc = trial(t, &ms);
-            if (!rc) b->trials.push_back({t, ms});
-            if (!rc && ms < best_ms) {
+            if (rc) return;
+            b->trials.push_back({t, ms});
+            if (ms < best_ms) {
                 best_ms = ms;
                 best = t;
             }
+        };
+        if (b->plan.n_warp > 0) {
+            tried(b->plan.tune);  // linear chains: the move kernel sizes its own tiles
+        } else {
+            for (int tb : {1024, 2048, 4096, 8192})
+                for (int th : {64, 128, 256})
+                    for (int pc : {0, sm_count() * 4}) {
+                        if (rc) break;
+                        scmf_tune t = b->plan.tune;
+                        t.chains_per_tile = 0;
+                        t.beads_per_tile = tb;
+                        t.threads_move = th;
+                        t.persistent_ctas = pc;
+                        tried(t);
+                    }
+        }
+        const scmf_tune base = best;
+        for (int c : {2048, 8192, 32768}) {
+            if (rc) break;
+            scmf_tune t = base;
+            t.cells_per_tile = c;
+            tried(t);
         }
     }
     for (auto& sn : snaps) snap_free(&sn, b->stream);

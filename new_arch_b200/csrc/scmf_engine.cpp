@@ -9,6 +9,7 @@
 // host round trip, optionally replayed from a CUDA graph; the step counter,
 // the counts double buffer and the statistics live on the device.
 #include "scmf_engine.h"
+#include "scmf_screen_table.h"
 
 #include <cmath>
 #include <cstdarg>
@@ -216,25 +217,27 @@ void field_coefficients(int n, const double* xn, int nref, int hamiltonian, floa
         }
 }
 
-// 0: every axis a power of two (the move kernels may compile only the mask
-// fold), 1: some axis is not.
-int flat_threads_for(int tpc, int threads_move) {
-    // lcm(tpc, 32): a block of that many threads holds whole chains with no idle lane
-    int a = tpc, b = 32;
-    while (b) {
-        const int r = a % b;
-        a = b;
-        b = r;
+// Constants of the move kernel's screen (ScreenDev), rounded towards passing a
+// trial.  Off where they leave the range in which the bounds there hold, and
+// where proposals are small enough that most trials would pass: with x = A 4k,
+// 4k the c of an inner bead, |v|^2 has (x^2 + 1) / (2 x) times the mean of the
+// limit's |f|^2 term, so screened trials pass often below x of about 2.
+static ScreenDev screen_constants(const SysDev& d) {
+    ScreenDev s{};
+    const double eta = 0x1p-6, K = (1.0 + eta) * (1.0 + 0x1p-10), delta = SCMF_SCREEN_DELTA;
+    const double A = d.A, R = d.R, unit = 0x1p30;
+    s.on = A > 0.0 && A * (double)d.cdeg[2] >= kScreenFromAc;
+    const auto up = [](double v) { return std::nextafterf((float)v, INFINITY); };
+    s.add = up((1.0 + 1.0 / eta) * 3.0 * delta * delta * unit * unit);
+    s.u = up(4.0 / A);
+    for (int g = 1; g <= 2; ++g) {
+        const double c = d.cdeg[g], a = (A - 1.0 / c) / R, b = K / (c * c * R * R);
+        for (const double v : {A, R, c, (double)d.ac4deg[g], b})
+            if (!(v > 1e-12 && v < 1e12)) s.on = 0;
+        s.a[g] = (float)(a * unit);
+        s.b[g] = up(b * unit * unit);
     }
-    const int l = tpc / a * 32;
-    return l <= 256 ? l : std::max(32, threads_move);
-}
-
-int fold_kind_of(const scmf_spec& s) {
-    const int dims[3] = {s.nx, s.ny, s.nz};
-    bool pow2 = true;
-    for (int n : dims) pow2 = pow2 && (n & (n - 1)) == 0;
-    return pow2 ? 0 : 1;
+    return s;
 }
 
 void fill_sysdev_constants(const scmf_spec& s, int64_t n_beads, SysDev* d) {
@@ -269,6 +272,51 @@ void fill_sysdev_constants(const scmf_spec& s, int64_t n_beads, SysDev* d) {
     d->seed_hi = (uint32_t)(s.p.seed >> 32);
 }
 
+void fill_sweep_constants(SysDev* d) {
+    SweepSys& w = d->sweep;
+    w.x = d->x;
+    w.y = d->y;
+    w.z = d->z;
+    w.omega = d->omega;
+    w.counts = d->counts[0];
+    w.n_cells = (uint32_t)d->n_cells;
+    w.k2 = d->k2;
+    w.A = d->A;
+    w.R = d->R;
+    const float inv[3] = {d->inv_dx, d->inv_dy, d->inv_dz};
+    const int n[3] = {d->nx, d->ny, d->nz};
+    bool pow2 = true, small = true;
+    for (int i = 0; i < 3; ++i) {
+        w.inv_d[i] = inv[i];
+        w.n[i] = n[i];
+        pow2 = pow2 && (n[i] & (n[i] - 1)) == 0;
+        small = small && n[i] >= 2 && n[i] <= 256;
+    }
+    w.fold = pow2 ? 0 : small ? 1 : 2;
+    for (int i = 0; i < 3 && w.fold == 1; ++i) {
+        w.fold_off[i] = fold_offset((uint32_t)n[i]);
+        w.fold_mag[i] = fold_magic_of((uint32_t)n[i]);
+    }
+    for (int g = 0; g < 3; ++g) {
+        w.cdeg[g] = d->cdeg[g];
+        w.ac4[g] = d->ac4deg[g];
+    }
+    w.seed_lo = d->seed_lo;
+    w.seed_hi = d->seed_hi;
+    w.count16 = d->count16;
+    w.screen = screen_constants(*d);
+    FieldSys& f = d->field;
+    f.counts = d->counts[0];
+    f.omega = d->omega;
+    f.n_cells = d->n_cells;
+    f.scale = d->scale;
+    f.n_types = d->n_types;
+    f.literal = d->hamiltonian == SCMF_HAM_LITERAL ? 1 : 0;
+    f.count16 = d->count16;
+    f.rule = d->field_rule;
+    for (int i = 0; i < kMaxTypes * kMaxTypes; ++i) f.cf[i] = d->cf[i];
+}
+
 scmf_tune default_tune() {
     scmf_tune t{};
     t.chains_per_tile = 0;
@@ -297,28 +345,111 @@ scmf_tune resolve_tune(const scmf_tune* t) {
 void DevPlan::release() {
     if (graph) cudaGraphExecDestroy(graph);
     if (graph_src) cudaGraphDestroy(graph_src);
-    if (side) {
-        cudaStreamSynchronize(side);
-        cudaStreamDestroy(side);
-    }
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    side = nullptr;
-    ev_fork = ev_join = nullptr;
-    void* ptrs[] = {d_move, d_field, d_close, d_acc, d_ef, d_eb, d_flat_list, d_warp_list};
+    void* ptrs[] = {d_move, d_field, d_close, d_warp, d_ef, d_eb, d_run};
     for (void* p : ptrs) dev_free(p, stream);
-    d_flat_list = nullptr;
-    d_warp_list = nullptr;
-    n_flat = n_warp = 0;
     graph = nullptr;
     graph_src = nullptr;
     d_move = nullptr;
     d_field = nullptr;
     d_close = nullptr;
-    d_acc = nullptr;
+    d_warp = nullptr;
+    d_run = nullptr;
     d_ef = nullptr;
     d_eb = nullptr;
-    n_move = n_field = n_sys = 0;
+    n_move = n_field = n_sys = n_warp = 0;
+}
+
+// The tiles of k_sweep_warp: whole chains of one architecture, as many chains in
+// each (SweepArch::per).  Every warp of the GPU gets the same number of tiles, of
+// sizes up to what its buffer holds and no smaller than a row of 32 bead pairs.
+// Empty for a plan that the kernel does not take.
+static std::vector<SweepArch> tile_ranges(const Plan& p, int* warp_beads) {
+    std::vector<SweepArch> out;
+    if (!p.linear || p.chains.empty() || p.max_length > kSweepBeadsLong || !p.cells32) return out;
+    const bool longer = p.max_length > kSweepBeads;
+    const int cap = longer ? kSweepBeadsLong : kSweepBeads;
+    *warp_beads = cap;
+    const int64_t warps = (int64_t)sm_count() * (longer ? kSweepWarpsLong : kSweepWarps);
+    int64_t beads = 0;
+    int most = cap;  // what a tile of every architecture can reach
+    for (const auto& c : p.chains) {
+        beads += (int64_t)c.length * c.n_chains;
+        most = std::min(most, cap / c.length * c.length);
+    }
+    const int64_t turns = std::max<int64_t>(1, (beads + warps * most - 1) / (warps * most));  // tiles of a warp
+    const auto per_tile = [&](const Plan::Chains& c, int64_t target) {
+        return (int)std::min<int64_t>(cap / c.length, std::max<int64_t>(1, (target + c.length - 1) / c.length));
+    };
+    int64_t target = std::max<int64_t>(64, (beads + warps * turns - 1) / (warps * turns));
+    for (; target < cap; target += std::max<int64_t>(1, target / 64)) {  // the last tile of each architecture is a part
+        int64_t n = 0;
+        for (const auto& c : p.chains) n += (c.n_chains + per_tile(c, target) - 1) / per_tile(c, target);
+        if (n <= warps * turns) break;
+    }
+    int first = 0;
+    for (const auto& c : p.chains) {
+        SweepArch r{c.arch, c.bead_base, first, per_tile(c, target), c.n_chains, c.length};
+        first += (c.n_chains + r.per - 1) / r.per;
+        out.push_back(r);
+    }
+    return out;
+}
+
+static int tiles_of(const std::vector<SweepArch>& ranges) {
+    return ranges.empty() ? 0 : ranges.back().first + (ranges.back().n_chains + ranges.back().per - 1) / ranges.back().per;
+}
+
+static std::vector<WarpTile> tile_list(const Plan& p, const std::vector<SweepArch>& ranges) {
+    std::vector<WarpTile> out;
+    out.reserve((size_t)tiles_of(ranges));
+    for (size_t k = 0; k < ranges.size(); ++k) {
+        const SweepArch& r = ranges[k];
+        for (int i = 0; i < r.n_chains; i += r.per) {
+            const int n = std::min(r.per, r.n_chains - i);
+            out.push_back({p.chains[k].sys, r.arch, r.bead_base + (int64_t)i * r.length, (uint32_t)i, n, n * r.length, r.length});
+        }
+    }
+    return out;
+}
+
+// The tables of k_run as one buffer, its pointers still offsets: field tiles of a
+// warp each, so that the warps of the launch share the cells evenly.
+static std::vector<char> run_tables(const Plan& p, int n_warp, int warp_beads, RunArgs* run) {
+    const int sms = sm_count(), most = warp_beads > kSweepBeads ? kSweepWarpsLong : kSweepWarps;
+    const int grid = std::min(n_warp, sms), warps = grid * std::min(most, (n_warp + grid - 1) / grid);  // as launched
+    int64_t cells = 0;
+    for (const auto& c : p.cells) cells += c.second;
+    // whole rows of four cells a lane, or of one where that leaves warps idle
+    const int64_t row = cells >= 128 * (int64_t)warps ? 128 : 32;
+    const int64_t turns = std::max<int64_t>(1, (cells + 4096 * (int64_t)warps - 1) / (4096 * (int64_t)warps));
+    const int64_t per = ((cells + warps * turns - 1) / (warps * turns) + row - 1) / row * row;
+    std::vector<RunSystem> systems;
+    std::vector<FieldTile> field;
+    for (const auto& c : p.cells) {
+        RunSystem rs{c.first, (int32_t)field.size(), 0};
+        for (int64_t i = 0; i < c.second; i += per) {
+            FieldTile t{};
+            t.sys = c.first;
+            t.cell0 = i;
+            t.n_cells = (int32_t)std::min(per, c.second - i);
+            field.push_back(t);
+        }
+        rs.field_count = (int32_t)field.size() - rs.field_first;
+        systems.push_back(rs);
+    }
+    const size_t at_field = round_up(64 + systems.size() * sizeof(RunSystem), 64);
+    const size_t at_ef = round_up(at_field + field.size() * sizeof(FieldTile), 64);
+    std::vector<char> image(at_ef + field.size() * sizeof(double), 0);  // the barrier's count first
+    std::memcpy(image.data() + 64, systems.data(), systems.size() * sizeof(RunSystem));
+    std::memcpy(image.data() + at_field, field.data(), field.size() * sizeof(FieldTile));
+    *run = RunArgs{};
+    run->barrier = nullptr;
+    run->systems = (const RunSystem*)(size_t)64;
+    run->field = (const FieldTile*)at_field;
+    run->ef_part = (double*)at_ef;
+    run->n_sys = (int)systems.size();
+    run->n_field = (int)field.size();
+    return image;
 }
 
 scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) {
@@ -330,42 +461,49 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     max_tile_beads = p.max_tile_beads;
     max_length = p.max_length;
     n_types_uniform = p.n_types_uniform;
-    max_chains = p.max_chains;
-    linear = p.linear;
-    fold_kind = p.fold_kind;
-    flat_threads = p.flat_threads > 0 ? p.flat_threads : t.threads_move;
     one_seed = p.one_seed && !p.close.empty();
     one_seed_hi = p.one_seed_hi && !p.close.empty();
     seed = p.seed;
     n_sys = (int)p.close.size();
-    lean = n_sys == 1 && p.lean_ok && p.fold_kind == 0 && p.linear;
-    warp_even = p.warp_even && p.linear && p.max_length <= 64;
-    sc = p.sc;
-    std::vector<int32_t> fl, wl;
-    for (size_t i = 0; i < p.move.size(); ++i) (p.tile_flat[i] ? fl : wl).push_back((int32_t)i);
-    n_flat = (int)fl.size();
-    n_warp = (int)wl.size();
-    if (n_flat > 0 && n_warp > 0 && p.linear && p.max_length <= 64) {
-        CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+    warp_beads = 0;
+    const std::vector<SweepArch> ranges = tile_ranges(p, &warp_beads);
+    n_warp = tiles_of(ranges);
+    one = n_sys == 1 && ranges.size() <= kSweepMaxArch;
+    std::vector<WarpTile> wt;
+    if (one) {
+        system = p.close[0].sys;
+        n_arch = (int)ranges.size();
+        std::copy(ranges.begin(), ranges.end(), arch);
+    } else {
+        wt = tile_list(p, ranges);
     }
+    sweep = p.sweep;
+    once = p.position_bytes > kL2Bytes / 2;
+    beads = (int64_t)(p.position_bytes / 12);
     const size_t nm = std::max<size_t>(1, p.move.size()), nf = std::max<size_t>(1, p.field.size());
     scmf_status rc;
     if ((rc = dev_alloc((void**)&d_move, nm * sizeof(MoveTile), st)) ||
         (rc = dev_alloc((void**)&d_field, nf * sizeof(FieldTile), st)) ||
         (rc = dev_alloc((void**)&d_close, std::max<size_t>(1, p.close.size()) * sizeof(SysClose), st)) ||
-        (rc = dev_alloc((void**)&d_acc, nm * kMaxWarps * sizeof(unsigned), st)) ||
-        (rc = dev_alloc((void**)&d_ef, nf * sizeof(double), st)) || (rc = dev_alloc((void**)&d_eb, nm * sizeof(double), st)) ||
-        (rc = dev_alloc((void**)&d_flat_list, std::max<size_t>(1, fl.size()) * sizeof(int32_t), st)) ||
-        (rc = dev_alloc((void**)&d_warp_list, std::max<size_t>(1, wl.size()) * sizeof(int32_t), st)))
+        (rc = dev_alloc((void**)&d_warp, std::max<size_t>(1, wt.size()) * sizeof(WarpTile), st)) ||
+        (rc = dev_alloc((void**)&d_ef, nf * sizeof(double), st)) || (rc = dev_alloc((void**)&d_eb, nm * sizeof(double), st)))
         return rc;
-    if (!fl.empty()) CK(cudaMemcpyAsync(d_flat_list, fl.data(), fl.size() * 4, cudaMemcpyHostToDevice, st));
-    if (!wl.empty()) CK(cudaMemcpyAsync(d_warp_list, wl.data(), wl.size() * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(d_acc, 0, nm * kMaxWarps * sizeof(unsigned), st));
+    if (!wt.empty()) CK(cudaMemcpyAsync(d_warp, wt.data(), wt.size() * sizeof(WarpTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_move, p.move.data(), p.move.size() * sizeof(MoveTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_field, p.field.data(), p.field.size() * sizeof(FieldTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_close, p.close.data(), p.close.size() * sizeof(SysClose), cudaMemcpyHostToDevice, st));
+    std::vector<char> run_image;
+    const bool longer = warp_beads > kSweepBeads;
+    if (n_warp > 0 && n_warp <= sm_count() * (longer ? kSweepWarpsLong : kSweepWarps)) {  // a tile a warp
+        run_image = run_tables(p, n_warp, warp_beads, &run);
+        if ((rc = dev_alloc(&d_run, run_image.size(), st))) return rc;
+        CK(cudaMemcpyAsync(d_run, run_image.data(), run_image.size(), cudaMemcpyHostToDevice, st));
+        const auto at = [&](const void* offset) { return (char*)d_run + (size_t)offset; };
+        run.systems = (const RunSystem*)at(run.systems);
+        run.field = (const FieldTile*)at(run.field);
+        run.ef_part = (double*)at(run.ef_part);
+        run.barrier = (unsigned long long*)at(run.barrier);
+    }
     // the host vectors may go away after return: wait for the (pageable) copies
     CK(cudaStreamSynchronize(st));
     return SCMF_OK;
@@ -376,19 +514,17 @@ LaunchShape DevPlan::move_shape() const {
     sh.blocks = tune.persistent_ctas > 0 ? std::min(tune.persistent_ctas, n_move) : 0;
     sh.threads = tune.threads_move;
     sh.n_types = n_types_uniform;
-    sh.linear = linear ? 1 : 0;
-    sh.max_chains = max_chains;
-    sh.flat_list = d_flat_list;
-    sh.n_flat = n_flat;
-    sh.warp_list = d_warp_list;
-    sh.n_warp = n_warp;
-    sh.fold = fold_kind;
-    sh.flat_threads = flat_threads;
     sh.keyed = one_seed ? kKeysBoth : (one_seed_hi ? kKeysHigh : kKeysNone);
     sh.keys = philox_schedule((uint32_t)seed, (uint32_t)(seed >> 32));
-    sh.lean = lean && one_seed && n_flat == 0 ? 1 : 0;
-    sh.warp_even = warp_even ? 1 : 0;
-    sh.sc = sc;
+    sh.warp_tiles = d_warp;
+    sh.n_warp_tiles = n_warp;
+    sh.warp_beads = warp_beads;
+    sh.one = one ? 1 : 0;
+    sh.system = system;
+    sh.n_arch = one ? n_arch : 0;
+    for (int i = 0; i < sh.n_arch; ++i) sh.arch[i] = arch[i];
+    sh.once = once ? 1 : 0;
+    sh.sweep = sweep;
     return sh;
 }
 
@@ -397,12 +533,11 @@ LaunchShape DevPlan::field_shape() const {
     sh.blocks = tune.persistent_ctas > 0 ? std::min(tune.persistent_ctas, n_field) : 0;
     sh.threads = tune.threads_field;
     sh.n_types = n_types_uniform;
-    sh.linear = linear ? 1 : 0;
     return sh;
 }
 
 scmf_status DevPlan::enqueue_close(int mode, cudaStream_t st) const {
-    CKL(launch_close(d_close, n_sys, d_acc, warps_per_tile(), d_ef, d_eb, mode, st));
+    CKL(launch_close(d_close, n_sys, d_ef, d_eb, mode, st));
     return SCMF_OK;
 }
 
@@ -412,19 +547,7 @@ scmf_status DevPlan::enqueue_sweep(cudaStream_t st) const {
 }
 
 scmf_status DevPlan::enqueue_move(cudaStream_t st) const {
-    if (side && n_warp > 0 && n_flat > 0) {
-        LaunchShape warp = move_shape(), flat = move_shape();
-        warp.part = 1;
-        flat.part = 2;
-        CK(cudaEventRecord(ev_fork, st));
-        CK(cudaStreamWaitEvent(side, ev_fork, 0));
-        CKL(launch_sweep(kMoveGrid, d_move, n_move, max_tile_beads, max_length, flat, d_acc, side));
-        CK(cudaEventRecord(ev_join, side));
-        CKL(launch_sweep(kMoveGrid, d_move, n_move, max_tile_beads, max_length, warp, d_acc, st));
-        CK(cudaStreamWaitEvent(st, ev_join, 0));
-    } else {
-        CKL(launch_sweep(kMoveGrid, d_move, n_move, max_tile_beads, max_length, move_shape(), d_acc, st));
-    }
+    CKL(launch_sweep(kMoveGrid, d_move, n_move, max_tile_beads, max_length, move_shape(), st));
     return SCMF_OK;
 }
 
@@ -435,6 +558,15 @@ scmf_status DevPlan::enqueue_field(cudaStream_t st) const {
 
 scmf_status DevPlan::run_sweeps(cudaStream_t st, int n) {
     if (n <= 0) return SCMF_OK;
+    if (d_run) {
+        // some milliseconds a launch, so that other work on the GPU gets its turn
+        const LaunchShape sh = move_shape();
+        for (RunArgs r = run; n > 0; n -= r.n_sweeps) {
+            r.n_sweeps = std::min(n, 1024);
+            CKL(launch_run(sh, r, st));
+        }
+        return SCMF_OK;
+    }
     if (tune.use_graph) {
         if (!graph) {
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -477,50 +609,12 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     const int64_t target_small = std::max<int64_t>(1, n_beads / (4 * sms));
     const size_t first_tile = p->move.size();
     const size_t first_field = p->field.size();
-    p->fold_kind = std::max(p->fold_kind, fold_kind_of(spec));
-    // the lean kernel indexes beads and cells (times types) with 32-bit integers
-    p->lean_ok = p->lean_ok && n_beads < (1ll << 31) && (int64_t)n_cells * spec.n_types < (1ll << 31);
+    p->cells32 = p->cells32 && n_cells * spec.n_types < (1ll << 31);
+    p->position_bytes += (size_t)n_beads * 12;
+    p->cells.push_back({d_sys, n_cells});
     if (p->close.empty()) {
         p->seed = spec.p.seed;
-        SysDev h{};
-        fill_sysdev_constants(spec, n_beads, &h);
-        SysConsts& c = p->sc;
-        c.x = x;
-        c.y = y;
-        c.z = z;
-        c.chain_id = chain_id;
-        c.omega = omega;
-        c.n_cells = h.n_cells;
-        c.k2 = h.k2;
-        c.A = h.A;
-        c.R = h.R;
-        c.inv_dx = h.inv_dx;
-        c.inv_dy = h.inv_dy;
-        c.inv_dz = h.inv_dz;
-        c.nx = h.nx;
-        c.ny = h.ny;
-        c.nz = h.nz;
-        for (int g = 0; g < 3; ++g) {
-            c.cdeg[g] = h.cdeg[g];
-            c.ac4deg[g] = h.ac4deg[g];
-        }
-        c.sys = d_sys;
-        c.n_arch = 0;
-        for (size_t a = 0; a < archs.size(); ++a) {
-            if (archs[a].n_chains == 0) continue;
-            if (c.n_arch == kLeanMaxArch) {
-                p->lean_ok = false;
-                break;
-            }
-            LeanArch& la = c.arch[c.n_arch++];
-            la.types = h_arch[a].types;
-            la.length = archs[a].length;
-            la.n_chains = archs[a].n_chains;
-            la.chain0 = archs[a].chain_base;
-            la.bead0 = (int32_t)archs[a].bead_base;
-            la.rng0 = archs[a].rng_base;  // chain_id[chain_base + c] = rng_base + c (storage order is never permuted)
-            la.pad = 0;
-        }
+        p->sweep = sweep;
     } else {
         if (p->seed != spec.p.seed) p->one_seed = false;
         if ((p->seed >> 32) != (spec.p.seed >> 32)) p->one_seed_hi = false;
@@ -528,20 +622,12 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     for (size_t a = 0; a < archs.size(); ++a) {
         const ArchHost& A = archs[a];
         if (A.n_chains == 0) continue;
-        const bool explicit_cpt = t.beads_per_tile <= 0 && t.chains_per_tile > 0;
         int cpt = t.beads_per_tile > 0 ? std::max(1, t.beads_per_tile / A.length) : t.chains_per_tile;
         if (cpt <= 0) {
             const int64_t target = std::min<int64_t>(4096, std::max<int64_t>(A.length, target_small));
             cpt = (int)std::max<int64_t>(1, target / A.length);
-        }
-        if (!explicit_cpt && A.linear && A.length <= 64) {
-            // whole iterations of the register kernel: a CTA moves cpi chains per
-            // iteration, and a tile that is not a multiple of cpi ends on a mostly
-            // idle one (measured 2.5 % on the large system)
-            const int tpc = (A.length + 1) / 2;
-            const int threads = 32 % tpc ? flat_threads_for(tpc, t.threads_move) : std::max(32, t.threads_move);
-            const int cpi = 32 % tpc ? std::max(1, threads / tpc) : (32 / tpc) * (threads / 32);
-            cpt = std::max(cpi, (cpt + cpi / 2) / cpi * cpi);
+            // a few hundred beads at least, so that small systems do not fall into tiles of single chains
+            if (A.linear && A.length <= 64) cpt = std::max(cpt, 256 / A.length);
         }
         cpt = std::max(1, std::min(cpt, kMaxTileBeads / A.length));
         for (int c = 0; c < A.n_chains; c += cpt) {
@@ -554,23 +640,10 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
             mt.n_tiles_sys = 0;
             mt.arch_index = (int32_t)a;
             p->move.push_back(mt);
-            const bool flat = A.linear && A.length <= 64 && 32 % ((A.length + 1) / 2) != 0;
-            p->tile_flat.push_back(flat ? 1 : 0);
-            if (flat) {
-                const int ft = flat_threads_for((A.length + 1) / 2, t.threads_move);
-                p->flat_threads = p->flat_threads == 0 || p->flat_threads == ft ? ft : -1;  // -1: archs disagree
-            }
             p->max_tile_beads = std::max(p->max_tile_beads, mt.n_chains * A.length);
-            p->max_chains = std::max(p->max_chains, mt.n_chains);
         }
         p->max_length = std::max(p->max_length, A.length);
-        p->lean_ok = p->lean_ok && A.linear && A.length % 2 == 0 && A.length <= 64 && 32 % (A.length / 2) == 0;
-        // the multi-system lean kernel reads bead pairs as float2: every warp-wise
-        // architecture must have an even length and start at an even bead (an
-        // odd-length architecture with an odd chain count before it would shift
-        // it by one); otherwise the register kernel, which checks, runs them
-        if (A.linear && A.length <= 64 && 32 % ((A.length + 1) / 2) == 0)
-            p->warp_even = p->warp_even && A.length % 2 == 0 && A.bead_base % 2 == 0;
+        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.chain_base, (int)a, A.bead_base});
         p->max_deg = std::max(p->max_deg, A.max_deg);
         p->linear = p->linear && A.linear;
     }

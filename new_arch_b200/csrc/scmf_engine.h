@@ -55,11 +55,8 @@ scmf_status prepare_archs(const scmf_spec& s, std::vector<ArchHost>* out, int64_
 uint32_t magic_for(uint32_t n);
 size_t system_device_bytes(const scmf_spec& s);
 void fill_sysdev_constants(const scmf_spec& s, int64_t n_beads, SysDev* d);
-int fold_kind_of(const scmf_spec& s);  // 0: every grid axis a power of two, 1: otherwise
-// Block size for chains of ceil(L/2) = tpc threads laid across warps:
-// lcm(tpc, 32) when it is at most 256 (no idle lane), else threads_move.
-int flat_threads_for(int tpc, int threads_move);
-
+// d->sweep from the rest of d (buffers and constants).
+void fill_sweep_constants(SysDev* d);
 // Work decomposition of one or many systems for one launch shape.
 struct Plan {
     std::vector<MoveTile> move;
@@ -69,57 +66,57 @@ struct Plan {
     int max_length = 0;
     int n_types_uniform = 0;
     int max_deg = 0;
-    int max_chains = 0;   // most chains in one move tile
+    size_t position_bytes = 0;  // of all systems
+    SweepSys sweep{};           // of the first system
     bool linear = true;
-    int fold_kind = 0;  // largest fold_kind_of() of the systems
-    int flat_threads = 0;  // block size of the block-wide move launch (0: none yet, -1: archs disagree)
-    std::vector<uint8_t> tile_flat;  // per move tile: chains run across warps (32 % ceil(L/2) != 0)
+    bool cells32 = true;  // cells times types below 2^31 in every system
+    // the chains of every architecture, for the warp tiles of k_sweep_warp
+    struct Chains {
+        SysDev* sys;
+        const ArchDev* arch;
+        int length, n_chains, chain_base, arch_index;
+        int64_t bead_base;
+    };
+    std::vector<Chains> chains;
+    std::vector<std::pair<SysDev*, int64_t>> cells;  // of every system, for the field tiles of k_run
     uint64_t seed = 0;      // the systems' seed when they all share one
     bool one_seed = true;   // every system appended so far has `seed`
     bool one_seed_hi = true;  // ... or at least its upper 32 bits
-    bool lean_ok = true;      // every architecture so far fits the lean move kernel
-    bool warp_even = true;    // every warp-wise linear architecture so far has an even length
-    SysConsts sc{};           // move constants of the first system appended
 };
 
 struct DevPlan {
     MoveTile* d_move = nullptr;
     FieldTile* d_field = nullptr;
     SysClose* d_close = nullptr;
-    unsigned* d_acc = nullptr;   // accept count per (move tile, warp)
+    // k_run: its systems, field tiles, partial energies and barrier, in one buffer
+    void* d_run = nullptr;
+    RunArgs run{};
+    int64_t beads = 0;           // of all systems
+    // one system of few architectures: its constants and tile ranges (no list)
+    bool one = false;
+    SysDev* system = nullptr;
+    SweepSys sweep{};
+    int n_arch = 0;
+    SweepArch arch[kSweepMaxArch] = {};
+    bool once = false;           // the positions are more than L2 holds
+    WarpTile* d_warp = nullptr;  // tiles of k_sweep_warp (linear plans; see warp_tiles)
     double* d_ef = nullptr;      // field energy per field tile
     double* d_eb = nullptr;      // bond energy per move tile
-    int n_move = 0, n_field = 0, n_sys = 0;
-    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0, max_chains = 0;
-    bool linear = false;
-    int32_t* d_flat_list = nullptr;  // tile indices for the block-wide register kernel
-    int32_t* d_warp_list = nullptr;  // tile indices for the warp-wise register kernel
-    int n_flat = 0, n_warp = 0;
-    int fold_kind = 0;
-    int flat_threads = 0;
+    int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;
+    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0, warp_beads = 0;
     bool one_seed = false;     // every system of the plan has `seed`: move launches take its key schedule
     bool one_seed_hi = false;  // they share its upper 32 bits: the second key word's schedule
     uint64_t seed = 0;
-    bool lean = false;  // one system that fits the lean move kernel (LaunchShape::lean)
-    bool warp_even = false;  // LaunchShape::warp_even
-    SysConsts sc{};
     scmf_tune tune{};
     cudaGraphExec_t graph = nullptr;
     cudaGraph_t graph_src = nullptr;
     cudaStream_t stream = nullptr;  // allocations of the plan are ordered on it
-    // plans with both warp-wise and flat tiles run the two move launches side
-    // by side (fork on ev_fork, join on ev_join) so neither waits for the
-    // other's last partial wave
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     void release();
     scmf_status upload(const Plan& p, const scmf_tune& t, cudaStream_t st);
     LaunchShape move_shape() const;
     LaunchShape field_shape() const;
-    int warps_per_tile() const { return tune.threads_move / 32; }
-    // one fused sweep (move+grid, field, close) enqueued on `st`: the move
-    // launches (two side by side when the plan has both tile kinds), then the
-    // field launch whose last tile per system closes the sweep
+    // one fused sweep enqueued on `st`: the move launch, then the field launch
+    // whose last tile per system closes the sweep
     scmf_status enqueue_sweep(cudaStream_t st) const;
     scmf_status enqueue_move(cudaStream_t st) const;
     scmf_status enqueue_field(cudaStream_t st) const;
@@ -154,6 +151,7 @@ struct scmf_system {
     uint32_t* chain_id = nullptr;
     uint32_t* counts[2] = {nullptr, nullptr};
     float* omega = nullptr;
+    scmf::SweepSys sweep{};  // as in *d_sys
     scmf::SysDev* d_sys = nullptr;
     scmf::ArchDev* d_arch = nullptr;
     void* d_arch_blob = nullptr;

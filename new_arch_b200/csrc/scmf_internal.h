@@ -53,13 +53,70 @@ struct ArchDev {
     int32_t color_off[kMaxColors + 1];
     uint32_t color_magic[kMaxColors];  // ceil(2^32 / n_in_colour): i / n == umulhi(i, magic)
     uint32_t len_magic;          // ceil(2^32 / length)
-    uint32_t tpc_magic;          // magic of ceil(length / 2): threads per chain in k_sweep_reg
+    uint32_t tpc_magic;          // magic of ceil(length / 2): bead pairs per chain
     int32_t n_chains;
     int32_t chain_base;          // first storage slot of this architecture in the system
     int32_t rng_base;            // random-stream id of its first chain: chain_base, or for a chain
                                  // shard the id that chain has in the whole system
     int64_t bead_base;           // first bead of this architecture in the system arrays
     float init_sigma;
+};
+
+// The screen of k_sweep_warp: constants of the test that proves a trial
+// rejected before its exact normals, energy and omega are formed.
+//
+// With d = A f + R n the displacement and c = 2k deg, the energy that the trial
+// kernels evaluate is, up to rounding,
+//   dE_bond = (A c / 4)(c |d|^2 - 2 f.d) = (A c^2 R^2 / 4)|v|^2 - (A / 4)|f|^2,
+//   v = n + ((A - 1/c) / R) f,
+// and a trial is rejected when dE_bond >= span + L, span the largest fall of
+// omega (SysDev::omega_span) and L >= -log u, because then dE = fl(fl(w_new -
+// w_old) + dE_bond) >= max(0, -log u).  The screen has f exactly and n, hence v,
+// to within delta in each component (SCMF_SCREEN_DELTA), and |v'|^2 <= (1 + eta)
+// |v|^2 + (1 + 1/eta) 3 delta^2 for the v' it forms, so it rejects when
+//   |v'|^2 > b (|f|^2 + (4 / A)(span + L)) + add
+// with b = K / (c R)^2, K = (1 + eta)(1 + 2^-10), add = (1 + 1/eta) 3 delta^2
+// and eta = 2^-6.  The 2^-10 and 2^-18 added to span + L cover every rounding on
+// both sides (each a few 2^-24 of the terms bounded here).  v' is formed 2^30
+// times as large and b, add 2^60 times, so that where a force is large enough to
+// overflow the exact energy the right side is infinite and the trial passes.
+// a and b are indexed by the bead's bonds.
+struct ScreenDev {
+    float a[3], b[3];  // a = (A - 1/c) / R
+    float u;           // 4 / A
+    float add;
+    int32_t on;  // 0: every trial is resolved (see screen_constants)
+    int32_t pad;
+};
+
+// What the move kernel of linear chains reads of a system, fixed for its life.
+struct SweepSys {
+    float *x, *y, *z;
+    const float* omega;
+    uint32_t* counts;           // counts[0], which is always the current grid
+    uint32_t n_cells;           // n_cells * n_types < 2^31
+    float k2, A, R;
+    float inv_d[3];
+    int32_t n[3];
+    int32_t fold;               // 0: every axis a power of two; 1: every axis of 2 to 256 cells; 2: others
+    int32_t fold_off[3];        // fold_magic's
+    uint32_t fold_mag[3];
+    float cdeg[3], ac4[3];      // c = 2k deg and A c / 4
+    uint32_t seed_lo, seed_hi;
+    int32_t count16;
+    ScreenDev screen;
+};
+
+// What the field step of k_run reads of a system.
+struct FieldSys {
+    const uint32_t* counts;
+    float* omega;
+    unsigned long long* avg;      // the averaging state as the launch finds it
+    int64_t n_cells;
+    float scale;
+    int32_t n_types, literal, count16, rule;
+    uint32_t avg_every;
+    float cf[kMaxTypes * kMaxTypes];
 };
 
 struct SysDev {
@@ -115,6 +172,12 @@ struct SysDev {
     uint32_t om_max_key, om_min_key;
     float omega_span;
     uint32_t pad3;
+    // the same in a launch of many sweeps (k_run): largest and smallest key of the
+    // field step of each sweep, by its number mod 3
+    uint32_t om_keys[3][2];
+    unsigned long long slot_last[kSlots];  // k_run: accepted moves of its last sweep
+    SweepSys sweep;
+    FieldSys field;
     // the statistics of the last sweep in the public layout, written by
     // k_stats_out for asynchronous reads (scmf_step_stats_async)
     scmf_stats stats_out;
@@ -129,6 +192,15 @@ struct MoveTile {
     int64_t bead0;        // first bead (system arrays)
     int32_t n_tiles_sys;  // move tiles of this system in the launch
     int32_t arch_index;   // architecture of the tile within its system
+};
+
+// Work item of k_sweep_warp: a run of whole chains of one linear architecture.
+struct WarpTile {
+    SysDev* sys;
+    const ArchDev* arch;
+    int64_t bead0;      // first bead (system arrays)
+    uint32_t chain;     // first chain, counted in its architecture
+    int32_t n_chains, n_beads, length;
 };
 
 // Work item of the field kernel: a run of cells of one system.
@@ -169,6 +241,13 @@ struct SysClose {
 };
 
 // Launchers (scmf_kernels.cu).  Every pointer is device memory.
+// fold_magic's offset and multiplier for an axis of n cells, 2 <= n <= 256.
+inline int32_t fold_offset(uint32_t n) {
+    const uint32_t bias = n * (((1u << 22) + n - 1) / n);  // a multiple of n, at least 2^22
+    return (int32_t)(0x4B400000u - bias);
+}
+inline uint32_t fold_magic_of(uint32_t n) { return (uint32_t)(((1ull << 32) + n - 1) / n); }
+
 // Round keys of Philox4x32-10 for one 64-bit key: round r XORs in
 // (k0 + r * 0x9E3779B9, k1 + r * 0xBB67AE85) (mod 2^32).  Passed to a kernel
 // by value, the schedule sits in the parameter constant bank, so each round's
@@ -188,70 +267,74 @@ inline PhiloxKeys philox_schedule(uint32_t k0, uint32_t k1) {
     return s;
 }
 
+// The tiles of one architecture in a launch of one system: tile first + i has its
+// chains i * per ... (i + 1) * per.
+struct SweepArch {
+    const ArchDev* arch;
+    int64_t bead_base;
+    int32_t first, per, n_chains, length;
+};
+constexpr int kSweepMaxArch = 4;
+
 enum KeyMode { kKeysNone = 0, kKeysHigh = 1, kKeysBoth = 2 };
-
-// Move constants of the one system of a launch, passed by value so that the
-// single-system move kernel reads them from the parameter constant bank
-// (instruction operands) instead of loading them from SysDev into registers.
-// Fixed for the life of the system: device buffers and spec constants.
-// One architecture of the system the lean move kernel moves: linear chains of
-// an even length with length / 2 dividing 32.
-struct LeanArch {
-    const uint8_t* types;  // [length], monomer type per bead
-    int32_t length;
-    int32_t n_chains;
-    int32_t chain0;        // first chain (index into chain_id)
-    int32_t bead0;         // first bead
-    int32_t rng0;          // random-stream id of the first chain (chain_id[chain0 + c] = rng0 + c)
-    int32_t pad;
-};
-constexpr int kLeanMaxArch = 4;
-
-struct SysConsts {
-    float* x;
-    float* y;
-    float* z;
-    const uint32_t* chain_id;
-    const float* omega;
-    int64_t n_cells;
-    float k2, A, R, inv_dx, inv_dy, inv_dz;
-    int32_t nx, ny, nz, pad;
-    float cdeg[3], ac4deg[3];  // c = 2k deg and A c / 4 for 0, 1, 2 bonds
-    SysDev* sys;
-    int32_t n_arch, pad2;
-    LeanArch arch[kLeanMaxArch];
-};
 
 struct LaunchShape {
     int blocks;    // 0 = one CTA per tile
     int threads;
     int smem;      // unused by the launchers (they size shared memory themselves)
     int n_types;   // field kernel: monomer types shared by all systems, 0 = mixed
-    int linear;    // sweep kernel: every architecture is a linear chain
-    int max_chains;  // sweep kernel: most chains in one tile
-    // sweep kernel, linear chains of at most 64 beads: tiles whose ceil(L/2)
-    // does not divide 32 (chains laid across warps) and the others, as lists
-    // of tile indices; n_flat == 0 means every tile is a warp tile
-    const int32_t* flat_list;
-    int n_flat;
-    const int32_t* warp_list;
-    int n_warp;
-    int part;        // 0: every tile; 1: warp tiles only; 2: flat tiles only
-    int fold;        // 0: every system's grid axes are powers of two (mask-only fold)
-    int flat_threads;  // block size of the block-wide launch (0: threads)
     // sweep kernel: kKeysBoth when every system of the launch has the seed of
     // `keys`, kKeysHigh when they share its upper 32 bits, else kKeysNone
     int keyed;
     PhiloxKeys keys;
-    // the launch moves one system (constants `sc`) whose architectures are all
-    // linear chains of an even length L <= 64 with L/2 dividing 32, on a grid of
-    // power-of-two axes, with fewer than 2^31 beads: the lean move kernel runs
-    int lean;
-    SysConsts sc;
-    // every architecture whose chains fill warps exactly (ceil(L/2) divides 32)
-    // has an even length: those tiles run k_sweep_leanm
-    int warp_even;
+    // every architecture of the launch is a linear chain that fits a warp's
+    // tile: the tiles of k_sweep_warp and the beads that a tile may hold
+    const WarpTile* warp_tiles;
+    int n_warp_tiles, warp_beads;
+    int one;            // the launch has one system: `system`, with the constants `sweep` and n_arch tile ranges
+    int once;           // the positions are more than L2 holds
+    SysDev* system;
+    SweepSys sweep;
+    int n_arch;
+    SweepArch arch[kSweepMaxArch];
 };
+
+// A system of a k_run launch and its field tiles.
+struct RunSystem {
+    SysDev* sys;
+    int32_t field_first, field_count;
+};
+
+// What k_run needs besides SweepArgs.
+struct RunArgs {
+    const RunSystem* systems;
+    const FieldTile* field;       // a warp's work each
+    double* ef_part;              // field energy of every field tile after the last sweep
+    unsigned long long* barrier;  // the grid barrier's count
+    int n_sys, n_field, n_sweeps, pad;
+};
+
+// Parameters of k_sweep_warp.
+struct SweepArgs {
+    const WarpTile* tiles;
+    int n_tiles, move_counts, once, pad;
+    PhiloxKeys keys;
+    // one system
+    SysDev* system;
+    SweepSys sys;
+    int n_arch;
+    SweepArch arch[kSweepMaxArch];
+};
+
+// Warps of a k_sweep_warp CTA (one CTA per SM) and the beads of a warp's tile
+// that shared memory then leaves room for; half as many warps, and longer tiles,
+// where a chain is longer than that.
+constexpr size_t kL2Bytes = 126u << 20;
+constexpr int kSweepWarps = 16;
+constexpr int kSweepWarpsLong = 8;
+constexpr int kSweepBeads = 960;
+constexpr int kSweepBeadsLong = 1984;
+constexpr float kScreenFromAc = 2.0f;  // A 4k from which the screen runs
 
 // Streaming multiprocessors of the current device (read once per device; 148
 // on a B200), for grid and tile sizing.
@@ -266,14 +349,16 @@ int launch_copy_counts(const SysDev* d_sys, uint32_t* dst, int64_t n_words, void
 // the field kernel writes one energy per tile into ef_part, the bond-energy
 // kernel one per move tile into eb_part; k_close sums and publishes them.
 int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int max_tile_beads, int max_length,
-                 LaunchShape shape, unsigned* acc_part, void* stream);
+                 const LaunchShape& shape, void* stream);
 // close_mode != 0: the last field tile of every system closes it in the same
 // launch (what k_close does with that mode), so a sweep is two launches.
+// n_sweeps whole sweeps of a plan whose chains are all linear (shape.warp_tiles)
+// in one cooperative launch.
+int launch_run(const LaunchShape& shape, const RunArgs& run, void* stream);
 int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_tiles, LaunchShape shape,
                  double* ef_part, int close_mode, void* stream);
 int launch_bond_energy(const MoveTile* tiles, int n_tiles, LaunchShape shape, double* eb_part, void* stream);
-int launch_close(const SysClose* list, int n_sys, const unsigned* acc_part, int warps_per_tile,
-                 const double* ef_part, const double* eb_part, int mode, void* stream);
+int launch_close(const SysClose* list, int n_sys, const double* ef_part, const double* eb_part, int mode, void* stream);
 int launch_aos_to_soa(const float* aos, SysDev* sys, const ArchDev* arch, int n_arch, int64_t n_beads,
                       void* stream);
 // Storage beads [i0, i1) from AoS positions (storage order = chain order: the

@@ -1,19 +1,13 @@
 // sm_100a kernels of the SCMF engine.
 //
 //   k_init_coords   random-walk chains (device_function.cu:140-207)
-//   k_sweep_reg     one MC sweep of linear chains of up to 64 beads, positions
-//                   in registers (a thread per bead pair): odd/even half-sweeps
-//                   of smart-MC trials (device_function.cu:444-454, 509-799),
-//                   moving one cell count for each accepted move that leaves
-//                   its cell, so counts stay the grid of the positions
-//                   (device_function.cu:471-508); or, in kGridOnly, a gridding
-//                   pass from scratch
-//   k_sweep_lean    the same sweep for one system of even-length chains on a
-//                   power-of-two grid, constants in the parameter bank
-//   k_sweep_leanm   its structure for many systems / any grid (even lengths)
-//   k_sweep_linear  the same for longer linear chains, staged per warp in
-//                   shared memory
+//   k_sweep_warp    one MC sweep of linear chains (scmf_sweep.cuh): odd/even
+//                   half-sweeps of smart-MC trials (device_function.cu:444-454,
+//                   509-799), moving one cell count for each accepted move that
+//                   leaves its cell, so counts stay the grid of the positions
+//                   (device_function.cu:471-508)
 //   k_sweep         the same for any bond graph (graph-colour half-sweeps)
+//   k_grid          counts of the current positions from scratch
 //   k_field<fused>  counts -> omega (SCMF0, device_function.cu:373-412) with the
 //                   field-energy reduction; in the fused step the block that
 //                   finishes a system's last tile closes the sweep (step,
@@ -34,20 +28,18 @@
 #include "scmf_internal.h"
 #include "scmf_math.cuh"
 #include "scmf_normal_table.h"
+#include "scmf_screen_table.h"
 
 namespace scmf {
 
 // The inverse normal CDF table of normal_of, read-only in global memory.
 __device__ __align__(16) const float g_normal_tab[SCMF_NORMAL_SEGS * 4] = {SCMF_NORMAL_TABLE_DATA};
 
-__device__ __forceinline__ const float4* normal_table() { return reinterpret_cast<const float4*>(g_normal_tab); }
+// The screen's piecewise-linear table (scmf_sweep.cuh).
+__device__ __align__(16) const float g_screen_tab[SCMF_SCREEN_SEGS * 2] = {SCMF_SCREEN_TABLE_DATA};
 
-// Copies the table into a block's shared memory (all threads of the block
-// call it; a barrier follows).
-__device__ __forceinline__ void load_normal_table(float4* s_tab) {
-    for (int i = threadIdx.x; i < SCMF_NORMAL_SEGS; i += blockDim.x) s_tab[i] = __ldg(normal_table() + i);
-    __syncthreads();
-}
+__device__ __forceinline__ const float2* screen_table() { return reinterpret_cast<const float2*>(g_screen_tab); }
+__device__ __forceinline__ const float4* normal_table() { return reinterpret_cast<const float4*>(g_normal_tab); }
 
 // i / n via a multiply-high by magic = ceil(2^32 / n) (exact while i * n < 2^32).
 __device__ __forceinline__ uint32_t div_magic(uint32_t i, uint32_t magic, int n) {
@@ -119,12 +111,10 @@ __device__ __forceinline__ void load_fold(MoveConsts& c, const SysDev* S) {
 // the same n, which the constant cache broadcasts.
 __constant__ int2 c_fold[257];
 
-// FOLD = 0: every system of the launch has power-of-two axes, so only the
-// mask fold is compiled in; FOLD = -1 picks the fold per system at run time.
-template <int FOLD = -1>
+// Cell index of a position; the system's grid picks the fold.
 __device__ __forceinline__ int cell_of(const MoveConsts& c, float x, float y, float z) {
     int ix, iy, iz;
-    if (FOLD == 0 || c.pow2) {
+    if (c.pow2) {
         ix = fold_pow2(x, c.inv_dx, c.nx - 1);
         iy = fold_pow2(y, c.inv_dy, c.ny - 1);
         iz = fold_pow2(z, c.inv_dz, c.nz - 1);
@@ -170,7 +160,6 @@ __device__ __forceinline__ bool maybe_accepted(float deb, float span, float lf) 
 // f - c d).  Same FP32 expression (explicit fma) as the oracle's move_bead().
 // Returns whether the move is accepted; (px,py,pz) is the proposed position
 // and cell_old / cell_new the cells of the old and proposed positions.
-template <int FOLD = -1>
 __device__ __forceinline__ bool trial_f(const MoveConsts& c, float x, float y, float z, float fx, float fy, float fz,
                                         float cc, float ac4, float n0, float n1, float n2, uint32_t aw,
                                         const float* __restrict__ w_t, float& px, float& py, float& pz, int& cell_old,
@@ -193,8 +182,8 @@ __device__ __forceinline__ bool trial_f(const MoveConsts& c, float x, float y, f
     bool acc = false;
     int c_old = 0, c_new = 0;
     if (maybe_accepted(deb, c.span, log_lower(u01(aw)))) {
-        c_old = cell_of<FOLD>(c, x, y, z);
-        c_new = cell_of<FOLD>(c, px, py, pz);
+        c_old = cell_of(c, x, y, z);
+        c_new = cell_of(c, px, py, pz);
         const float dE = __fadd_rn(__fsub_rn(__ldg(w_t + c_new), __ldg(w_t + c_old)), deb);
         if (dE < 0.0f)
             acc = true;
@@ -208,7 +197,7 @@ __device__ __forceinline__ bool trial_f(const MoveConsts& c, float x, float y, f
 
 // One smart-MC trial (device_function.cu:637-717, 562-588, 444-454) of a bead
 // at (x,y,z) with deg bonded neighbours q[0..deg) in ascending bead order.
-template <int MAXDEG, int FOLD = -1>
+template <int MAXDEG>
 __device__ __forceinline__ bool trial(const MoveConsts& c, float x, float y, float z, const float* qx,
                                       const float* qy, const float* qz, int deg, float cc, float ac4, float n0,
                                       float n1, float n2, uint32_t aw, const float* __restrict__ w_t, float& px,
@@ -217,7 +206,7 @@ __device__ __forceinline__ bool trial(const MoveConsts& c, float x, float y, flo
 #pragma unroll
     for (int d = 0; d < MAXDEG; ++d)
         if (d < deg) add_bond(c.k2, x, y, z, qx[d], qy[d], qz[d], fx, fy, fz);
-    return trial_f<FOLD>(c, x, y, z, fx, fy, fz, cc, ac4, n0, n1, n2, aw, w_t, px, py, pz, cell_old, cell_new);
+    return trial_f(c, x, y, z, fx, fy, fz, cc, ac4, n0, n1, n2, aw, w_t, px, py, pz, cell_old, cell_new);
 }
 
 // Counts are kept as the grid of the current positions: a fused sweep moves
@@ -271,17 +260,13 @@ size_t sweep_smem_bytes(int max_tile_beads, int max_length) {
 }
 
 // One MC sweep over tiles of whole chains staged in shared memory.
-//   MODE kMoveOnly / kMoveGrid / kGridOnly: moves; moves keeping counts[cur]
-//   the grid of the positions (accepted moves that change cell move a count);
-//   counts of the current positions added into counts[cur] (a cleared buffer).
-//   LINEAR: every architecture of the launch is a linear chain (bonds i-i+1,
-//   even beads colour 0, odd beads colour 1); neighbours are computed, not looked up.
+//   MODE kMoveOnly / kMoveGrid: moves; moves keeping counts[cur] the grid of
+//   the positions (accepted moves that change cell move a count).
 //   Two 256-thread CTAs per SM leave it 128 registers and no spill (at 64 it
 //   spilled ~400 B per thread and moved combs 12 % slower).
-template <int MODE, bool LINEAR, int KEYS>
+template <int MODE, int KEYS>
 __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ tiles, int n_tiles,
-                                                   int max_tile_beads, int max_length, unsigned* __restrict__ acc_part,
-                                                   const PhiloxKeys keys) {
+                                                   int max_tile_beads, int max_length, const PhiloxKeys keys) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* sx = reinterpret_cast<float*>(smem_raw);
     float* sy = sx + max_tile_beads;
@@ -290,12 +275,11 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
     BeadInfo* sinfo = reinterpret_cast<BeadInfo*>(smem_raw + off);
     off = (off + (size_t)max_length * sizeof(BeadInfo) + 15) & ~(size_t)15;
     uint16_t* scol = reinterpret_cast<uint16_t*>(smem_raw + off);
-    uint8_t* stype = reinterpret_cast<uint8_t*>(sinfo);  // LINEAR: types only
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x) {
         const MoveTile t = tiles[ti];
         SysDev* S = t.sys;
-        if (MODE != kGridOnly && S->step >= S->stop_step) continue;  // block-uniform
+        if (S->step >= S->stop_step) continue;  // block-uniform
         const ArchDev* Ap = t.arch;
         const int L = Ap->length;
         const int nb = t.n_chains * L;
@@ -307,14 +291,9 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
         c.k = S->k; c.k2 = S->k2; c.A = S->A; c.R = S->R;
         c.inv_dx = S->inv_dx; c.inv_dy = S->inv_dy; c.inv_dz = S->inv_dz;
         load_fold(c, S);
-        const uint32_t len_magic = Ap->len_magic;
         for (int i = tid; i < L; i += T) {
-            if (LINEAR) {
-                stype[i] = Ap->beads[i].type;
-            } else {
-                sinfo[i] = Ap->beads[i];
-                scol[i] = Ap->color_beads[i];
-            }
+            sinfo[i] = Ap->beads[i];
+            scol[i] = Ap->color_beads[i];
         }
         float* gx = S->x + t.bead0;
         float* gy = S->y + t.bead0;
@@ -339,7 +318,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
         }
         __syncthreads();
 
-        if (MODE != kGridOnly) {
+        {
             const uint32_t step = S->step + 1u;
             const uint32_t k0 = S->seed_lo, k1 = S->seed_hi;
             const uint32_t* __restrict__ cid = S->chain_id + t.chain0;
@@ -356,44 +335,26 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
                 for (int j = tid; j < items; j += T) {
                     const int cl = (int)div_magic((uint32_t)j, mg, ncol);
                     const int base = cl * L;
-                    float qx[LINEAR ? 2 : kMaxDeg], qy[LINEAR ? 2 : kMaxDeg], qz[LINEAR ? 2 : kMaxDeg];
+                    float qx[kMaxDeg], qy[kMaxDeg], qz[kMaxDeg];
                     int b, deg, type;
-                    if (LINEAR) {
-                        b = 2 * (j - cl * ncol) + col;
-                        type = stype[b];
-                        deg = 0;
-                        if (b > 0) {
-                            qx[0] = sx[base + b - 1];
-                            qy[0] = sy[base + b - 1];
-                            qz[0] = sz[base + b - 1];
-                            deg = 1;
-                        }
-                        if (b + 1 < L) {
-                            qx[deg] = sx[base + b + 1];
-                            qy[deg] = sy[base + b + 1];
-                            qz[deg] = sz[base + b + 1];
-                            ++deg;
-                        }
-                    } else {
-                        b = scol[Ap->color_off[col] + (j - cl * ncol)];
-                        const BeadInfo bi = sinfo[b];
-                        type = bi.type;
-                        deg = bi.deg;
+                    b = scol[Ap->color_off[col] + (j - cl * ncol)];
+                    const BeadInfo bi = sinfo[b];
+                    type = bi.type;
+                    deg = bi.deg;
 #pragma unroll
-                        for (int d = 0; d < kMaxDeg; ++d) {
-                            if (d < deg) {
-                                const int q = base + bi.nbr[d];
-                                qx[d] = sx[q];
-                                qy[d] = sy[q];
-                                qz[d] = sz[q];
-                            }
+                    for (int d = 0; d < kMaxDeg; ++d) {
+                        if (d < deg) {
+                            const int q = base + bi.nbr[d];
+                            qx[d] = sx[q];
+                            qy[d] = sy[q];
+                            qz[d] = sz[q];
                         }
                     }
                     float n0, n1, n2;
                     const uint32_t aw = bead_normals<KEYS>(__ldg(cid + cl), b, step, k0, k1, keys, n0, n1, n2);
                     float px, py, pz;
                     int c_old, c_new;
-                    const bool acc = trial<LINEAR ? 2 : kMaxDeg>(c, sx[base + b], sy[base + b], sz[base + b], qx, qy,
+                    const bool acc = trial<kMaxDeg>(c, sx[base + b], sy[base + b], sz[base + b], qx, qy,
                                                                  qz, deg, deg == 2 ? cc2 : S->cdeg[deg],
                                                                  deg == 2 ? ac42 : S->ac4deg[deg], n0, n1, n2, aw,
                                                                  omega + (int64_t)type * NC, px, py, pz, c_old, c_new);
@@ -411,23 +372,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
             if (lane == 0 && nacc) atomicAdd(&S->slot_acc[(ti * kMaxWarps + warp) % kSlots], (unsigned long long)nacc);
         }
 
-        if (MODE == kGridOnly) {
-            uint32_t* cnt = S->counts[S->cur];
-            const int64_t NC = S->n_cells;
-            const bool c16 = S->count16 != 0;
-            for (int i = tid; i < nb; i += T) {
-                const int cl = (int)div_magic((uint32_t)i, len_magic, L);
-                const int b = i - cl * L;
-                const int type = LINEAR ? stype[b] : sinfo[b].type;
-                const int64_t idx = (int64_t)type * NC + cell_of(c, sx[i], sy[i], sz[i]);
-                if (c16)
-                    atomicAdd(cnt + (idx >> 1), 1u << ((idx & 1) * 16));
-                else
-                    atomicAdd(cnt + idx, 1u);
-            }
-        }
-
-        if (MODE != kGridOnly) {
+        {
             if (vec) {
                 float4* vx = reinterpret_cast<float4*>(gx);
                 float4* vy = reinterpret_cast<float4*>(gy);
@@ -449,724 +394,37 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
     }
 }
 
-// Linear chains, one warp per run of whole chains.  Each warp stages its
-// chains in its own slice of shared memory in a parity-split layout (for chain
-// cl: even beads at cl*L + b/2, odd beads at cl*L + h0 + b/2, h0 = ceil(L/2)),
-// so the lanes of a half-sweep read consecutive words, and the warp needs no
-// block barrier: load, even half-sweep, odd half-sweep, store, separated by
-// __syncwarp.  Results are identical to k_sweep (same trial, same keys).
-// Three 256-thread CTAs per SM leave it 80 registers and no spill (at 64 it
-// spilled ~100 B per thread and moved chains of 128 beads 12 % slower).
-template <int MODE, int KEYS>
-__global__ void __launch_bounds__(256, 3) k_sweep_linear(const MoveTile* __restrict__ tiles,
-                                                          const int32_t* __restrict__ list, int n_list,
-                                                          int warp_beads, unsigned* __restrict__ acc_part,
-                                                          const PhiloxKeys keys) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    // per warp: x, y, z of its chains (parity-split)
-    float* sx = reinterpret_cast<float*>(smem_raw) + (size_t)warp * 3 * warp_beads;
-    float* sy = sx + warp_beads;
-    float* sz = sy + warp_beads;
-    for (int li = blockIdx.x; li < n_list; li += gridDim.x) {
-        const int ti = list ? __ldg(list + li) : li;
+// Counts of the current positions added into counts[cur] (a cleared buffer),
+// over the tiles of the launch (device_function.cu:471-508).
+__global__ void __launch_bounds__(256) k_grid(const MoveTile* __restrict__ tiles, int n_tiles) {
+    for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x) {
         const MoveTile t = tiles[ti];
         SysDev* S = t.sys;
-        if (MODE != kGridOnly && S->step >= S->stop_step) continue;
         const ArchDev* Ap = t.arch;
         const int L = Ap->length;
-        const int h0 = (L + 1) >> 1;
-        const int cpw = (t.n_chains + nwarps - 1) / nwarps;
-        const int c_begin = warp * cpw;
-        const int nch = min(cpw, t.n_chains - c_begin);
-        if (nch <= 0) {
-            continue;
-        }
-        const int nb = nch * L;
-        if (nb > warp_beads) {
-            if (lane == 0) atomicOr(&S->error_word, 2u);
-            continue;
-        }
+        const int nb = t.n_chains * L;
         MoveConsts c;
-        c.k = S->k; c.k2 = S->k2; c.A = S->A; c.R = S->R;
         c.inv_dx = S->inv_dx; c.inv_dy = S->inv_dy; c.inv_dz = S->inv_dz;
         load_fold(c, S);
-        const uint32_t len_magic = Ap->len_magic;
-        const int64_t g0 = t.bead0 + (int64_t)c_begin * L;
-        float* gx = S->x + g0;
-        float* gy = S->y + g0;
-        float* gz = S->z + g0;
-        for (int i = lane; i < nb; i += 32) {
-            const int cl = (int)div_magic((uint32_t)i, len_magic, L);
-            const int b = i - cl * L;
-            const int slot = cl * L + (b & 1) * h0 + (b >> 1);
-            sx[slot] = __ldcs(gx + i);
-            sy[slot] = __ldcs(gy + i);
-            sz[slot] = __ldcs(gz + i);
-        }
+        const float* X = S->x + t.bead0;
+        const float* Y = S->y + t.bead0;
+        const float* Z = S->z + t.bead0;
+        uint32_t* cnt = S->counts[S->cur];
+        const int64_t NC = S->n_cells;
+        const bool c16 = S->count16 != 0;
         const uint8_t* __restrict__ types = Ap->types;
-        const int64_t NC = S->n_cells;
-        uint32_t* cnt = S->counts[S->cur];
-        const bool c16 = S->count16 != 0;
-        __syncwarp();
-        if (MODE != kGridOnly) {
-            const uint32_t step = S->step + 1u;
-            const uint32_t k0 = S->seed_lo, k1 = S->seed_hi;
-            const uint32_t my_cid = lane < nch ? __ldg(S->chain_id + t.chain0 + c_begin + lane) : 0u;
-            const float* __restrict__ omega = S->omega;
-            const float cc1 = S->cdeg[1], ac41 = S->ac4deg[1], cc2 = S->cdeg[2], ac42 = S->ac4deg[2];
-            unsigned nacc = 0;
-#pragma unroll 1
-            for (int col = 0; col < 2; ++col) {
-                const int half = col == 0 ? h0 : (L >> 1);
-                const uint32_t mg = Ap->color_magic[col];
-                const int items = nch * half;
-                const int own = col * h0, other = (1 - col) * h0;
-                // lanes of one iteration share the loop bound: every lane runs the
-                // shuffle below, inactive ones on a dummy item
-                for (int j0 = 0; j0 < items; j0 += 32) {
-                    const int j = j0 + lane;
-                    const bool act = j < items;
-                    const int jj = act ? j : 0;
-                    const int cl = (int)div_magic((uint32_t)jj, mg, half);
-                    const uint32_t gc = __shfl_sync(0xffffffffu, my_cid, cl & 31);
-                    if (!act) continue;
-                    const int k = jj - cl * half;
-                    const int b = 2 * k + col;
-                    const int base = cl * L;
-                    const int me = base + own + k;
-                    float qx[2], qy[2], qz[2];
-                    int deg = 0;
-                    if (b > 0) {
-                        const int q = base + other + k - 1 + col;
-                        qx[0] = sx[q];
-                        qy[0] = sy[q];
-                        qz[0] = sz[q];
-                        deg = 1;
-                    }
-                    if (b + 1 < L) {
-                        const int q = base + other + k + col;
-                        qx[deg] = sx[q];
-                        qy[deg] = sy[q];
-                        qz[deg] = sz[q];
-                        ++deg;
-                    }
-                    const int type = __ldg(types + b);
-                    float n0, n1, n2;
-                    const uint32_t aw = bead_normals<KEYS>(gc, b, step, k0, k1, keys, n0, n1, n2);
-                    float px, py, pz;
-                    int c_old, c_new;
-                    const bool acc = trial<2>(c, sx[me], sy[me], sz[me], qx, qy, qz, deg, deg == 2 ? cc2 : cc1,
-                                              deg == 2 ? ac42 : ac41, n0, n1, n2, aw, omega + (int64_t)type * NC, px,
-                                              py, pz, c_old, c_new);
-                    if (acc) {
-                        sx[me] = px;
-                        sy[me] = py;
-                        sz[me] = pz;
-                    }
-                    nacc += acc ? 1u : 0u;
-                    if (MODE == kMoveGrid && acc && c_new != c_old) count_move(cnt, c16, (int64_t)type * NC, c_old, c_new);
-                }
-                __syncwarp();
-            }
-            nacc = warp_sum(nacc);
-            if (lane == 0 && nacc) atomicAdd(&S->slot_acc[(ti * kMaxWarps + warp) % kSlots], (unsigned long long)nacc);
-        }
-        if (MODE == kGridOnly) {
-            for (int i = lane; i < nb; i += 32) {
-                const int cl = (int)div_magic((uint32_t)i, len_magic, L);
-                const int b = i - cl * L;
-                const int slot = cl * L + (b & 1) * h0 + (b >> 1);
-                const int64_t idx = (int64_t)__ldg(types + b) * NC + cell_of(c, sx[slot], sy[slot], sz[slot]);
-                if (c16)
-                    atomicAdd(cnt + (idx >> 1), 1u << ((idx & 1) * 16));
-                else
-                    atomicAdd(cnt + idx, 1u);
-            }
-        } else {
-            for (int i = lane; i < nb; i += 32) {
-                const int cl = (int)div_magic((uint32_t)i, len_magic, L);
-                const int b = i - cl * L;
-                const int slot = cl * L + (b & 1) * h0 + (b >> 1);
-                __stcs(gx + i, sx[slot]);
-                __stcs(gy + i, sy[slot]);
-                __stcs(gz + i, sz[slot]);
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// Linear chains of at most 64 beads, positions in registers.  Each thread owns
-// the bead pair (2t, 2t+1) of one chain (ceil(L/2) threads per chain).  Even
-// half-sweep: bead 2t moves against 2t-1 (the odd bead of lane-1, by shuffle)
-// and 2t+1 (its own); odd half-sweep: bead 2t+1 moves against 2t (its own,
-// already moved) and 2t+2 (the even bead of lane+1).  When ceil(L/2) divides
-// 32, each warp holds whole chains: no shared memory, no block barrier.
-// Otherwise (L = 48: 24 threads per chain would idle a quarter of every warp)
-// the block holds as many whole chains as fit in all its threads, chains run
-// across warp boundaries: a warp's first even bead reads its left neighbour
-// from global memory (not yet moved, not yet stored), its last odd bead gets
-// the moved right neighbour through shared memory after one block barrier per
-// iteration; every chain still moves all its even beads before any odd bead.  Tiles are read and written with
-// coalesced float2 accesses.  Same trial and keys as k_sweep.
-// Register cap per instance.  80 (six 128-thread CTAs, 24 warps per SM) is
-// what the general instances need without spilling; the instances that read
-// their Philox round keys from the parameter bank fit in 72 without spilling,
-// which gives seven CTAs (28 warps) per SM (large system 0.661 -> 0.621 ms,
-// batched mix +4.4 %).  At 64 (32 warps) they spill 20-36 B.
-constexpr int reg_cap(bool flat, int fold, int keys) {
-    return (keys == kKeysBoth || (keys == kKeysHigh && fold != 0 && !flat)) ? 72 : 80;
-}
-
-template <int MODE, bool ANY_FLAT, int FOLD, int KEYS>
-__global__ void __maxnreg__(reg_cap(ANY_FLAT, FOLD, KEYS)) k_sweep_reg(const MoveTile* __restrict__ tiles,
-                                                                        const int32_t* __restrict__ list, int n_list,
-                                                                        unsigned* __restrict__ acc_part,
-                                                                        const PhiloxKeys keys) {
-    // even bead of each warp's lane 0 after its move, double-buffered by
-    // iteration parity: with one barrier per iteration a warp may write the
-    // next iteration's slot while its left neighbour still reads this one
-    __shared__ float s_first_even[2][kMaxWarps][3];
-    __shared__ float4 s_ntab[SCMF_NORMAL_SEGS];
-    if (MODE != kGridOnly) load_normal_table(s_ntab);
-    // Every instance computes the odd bead's Philox block together with the
-    // even bead's (two independent chains of rounds to interleave).  The keyed
-    // instances, whose Philox key lives (at least half) in the parameter bank,
-    // also add the even bead's bond forces one at a time (no local array); the
-    // others spill that way and keep the two-entry array.  All give the same bits.
-    constexpr bool kLean = KEYS != kKeysNone;
-    int parity = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int li = blockIdx.x; li < n_list; li += gridDim.x) {
-        const int ti = list ? __ldg(list + li) : li;  // tile index in the plan
-        const MoveTile t = tiles[ti];
-        SysDev* S = t.sys;
-        if (MODE != kGridOnly && S->step >= S->stop_step) continue;  // block-uniform
-        const ArchDev* Ap = t.arch;
-        const int L = Ap->length;
-        const int tpc = (L + 1) >> 1;                        // threads per chain
-        const bool flat = ANY_FLAT && (32 % tpc) != 0;       // chains run across warps (block-uniform)
-        const int slot = flat ? (int)threadIdx.x : lane;     // pair slot in the block / in the warp
-        const int cpw = flat ? (int)blockDim.x / tpc : 32 / tpc;  // chains per block / per warp iteration
-        const int cs = (int)div_magic((uint32_t)slot, Ap->tpc_magic, tpc);
-        const int tt = slot - cs * tpc;                      // pair index in the chain
-        const int be = 2 * tt, bo = 2 * tt + 1;
-        MoveConsts c;
-        c.k = S->k; c.k2 = S->k2; c.A = S->A; c.R = S->R;
-        c.inv_dx = S->inv_dx; c.inv_dy = S->inv_dy; c.inv_dz = S->inv_dz;
-        load_fold(c, S);
-        const int64_t NC = S->n_cells;
-        // counts pointer and width: read here for gridding, and again at each (rare)
-        // count move of the move modes, so that no register holds them across a sweep
-        uint32_t* cnt = S->counts[S->cur];
-        const bool c16 = S->count16 != 0;
-        const float* __restrict__ omega = S->omega;
-        const uint32_t step = S->step + 1u;
-        const uint32_t k0 = S->seed_lo, k1 = S->seed_hi;
-        const float cc1 = S->cdeg[1], ac41 = S->ac4deg[1], cc2 = S->cdeg[2], ac42 = S->ac4deg[2];
-        const int type_e = cs < cpw ? __ldg(Ap->types + min(be, L - 1)) : 0;
-        const int type_o = cs < cpw && bo < L ? __ldg(Ap->types + bo) : 0;
-        const bool pair_aligned = ((t.bead0 & 1) == 0) && ((L & 1) == 0);
-        unsigned nacc = 0;
-        for (int cbase = flat ? 0 : warp * cpw; cbase < t.n_chains; cbase += flat ? cpw : nwarps * cpw) {
-            const int chain = cbase + cs;
-            const bool live = cs < cpw && chain < t.n_chains;
-            const bool has_o = live && bo < L;
-            const int64_t g = t.bead0 + (int64_t)chain * L + be;
-            float xe = 0.0f, ye = 0.0f, ze = 0.0f, xo = 0.0f, yo = 0.0f, zo = 0.0f;
-            uint32_t gc = 0u;
-            if (live) {
-                if (pair_aligned) {
-                    const float2 vx = __ldcs(reinterpret_cast<const float2*>(S->x + g));
-                    const float2 vy = __ldcs(reinterpret_cast<const float2*>(S->y + g));
-                    const float2 vz = __ldcs(reinterpret_cast<const float2*>(S->z + g));
-                    xe = vx.x; xo = vx.y;
-                    ye = vy.x; yo = vy.y;
-                    ze = vz.x; zo = vz.y;
-                } else {
-                    xe = __ldcs(S->x + g);
-                    ye = __ldcs(S->y + g);
-                    ze = __ldcs(S->z + g);
-                    if (has_o) {
-                        xo = __ldcs(S->x + g + 1);
-                        yo = __ldcs(S->y + g + 1);
-                        zo = __ldcs(S->z + g + 1);
-                    }
-                }
-                gc = __ldg(S->chain_id + t.chain0 + chain);
-            }
-            if (MODE == kGridOnly) {
-                if (live) {
-                    const int64_t ie = (int64_t)type_e * NC + cell_of<FOLD>(c, xe, ye, ze);
-                    if (c16) atomicAdd(cnt + (ie >> 1), 1u << ((ie & 1) * 16)); else atomicAdd(cnt + ie, 1u);
-                }
-                if (has_o) {
-                    const int64_t io = (int64_t)type_o * NC + cell_of<FOLD>(c, xo, yo, zo);
-                    if (c16) atomicAdd(cnt + (io >> 1), 1u << ((io & 1) * 16)); else atomicAdd(cnt + io, 1u);
-                }
-                continue;
-            }
-            uint4 wo = make_uint4(0u, 0u, 0u, 0u);  // the odd bead's Philox block
-            // even half-sweep
-            {
-                float lx = __shfl_up_sync(0xffffffffu, xo, 1);
-                float ly = __shfl_up_sync(0xffffffffu, yo, 1);
-                float lz = __shfl_up_sync(0xffffffffu, zo, 1);
-                if (flat && lane == 0 && warp > 0 && live && tt > 0) {
-                    // the previous warp's last odd bead, not yet moved: positions of this
-                    // iteration are stored only after the barrier below, so global memory
-                    // still holds its start-of-sweep value (read through L2)
-                    lx = __ldcg(S->x + g - 1);
-                    ly = __ldcg(S->y + g - 1);
-                    lz = __ldcg(S->z + g - 1);
-                }
-                if (live) {
-                    // neighbours in ascending bead order: 2t-1 (if any), then 2t+1 (if any),
-                    // one at a time (kLean) or through a two-entry array (in a 24 B stack
-                    // frame; the other instances spill 16-32 B without it).  Same fma sequence.
-                    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-                    float qx[2], qy[2], qz[2];
-                    int deg = 0;
-                    if (kLean) {
-                        if (tt > 0) add_bond(c.k2, xe, ye, ze, lx, ly, lz, fx, fy, fz);
-                        if (has_o) add_bond(c.k2, xe, ye, ze, xo, yo, zo, fx, fy, fz);
-                        deg = (tt > 0 ? 1 : 0) + (has_o ? 1 : 0);
-                    } else {
-                        if (tt > 0) { qx[0] = lx; qy[0] = ly; qz[0] = lz; deg = 1; }
-                        if (has_o) { qx[deg] = xo; qy[deg] = yo; qz[deg] = zo; ++deg; }
-                    }
-                    const uint4 w = philox_block<KEYS>(make_uint4(gc, (uint32_t)be, step, 0u), k0, k1, keys);
-                    wo = philox_block<KEYS>(make_uint4(gc, (uint32_t)bo, step, 0u), k0, k1, keys);
-                    float n0, n1, n2;
-                    normals3(w, s_ntab, n0, n1, n2);
-                    float px, py, pz;
-                    int c_old, c_new;
-                    const float cc = deg == 2 ? cc2 : (deg == 1 ? cc1 : 0.0f);
-                    const float ac4 = deg == 2 ? ac42 : (deg == 1 ? ac41 : 0.0f);
-                    const float* w_e = omega + (int64_t)type_e * NC;
-                    const bool acc = kLean ? trial_f<FOLD>(c, xe, ye, ze, fx, fy, fz, cc, ac4, n0, n1, n2,
-                                                           accept_word(w), w_e, px, py, pz, c_old, c_new)
-                                           : trial<2, FOLD>(c, xe, ye, ze, qx, qy, qz, deg, cc, ac4, n0, n1, n2,
-                                                            accept_word(w), w_e, px, py, pz, c_old, c_new);
-                    if (acc) { xe = px; ye = py; ze = pz; }
-                    nacc += acc ? 1u : 0u;
-                    if (MODE == kMoveGrid && acc && c_new != c_old)
-                        count_move(S->counts[S->cur], S->count16 != 0, (int64_t)type_e * NC, c_old, c_new);
-                }
-            }
-            // odd half-sweep
-            {
-                float rx = __shfl_down_sync(0xffffffffu, xe, 1);
-                float ry = __shfl_down_sync(0xffffffffu, ye, 1);
-                float rz = __shfl_down_sync(0xffffffffu, ze, 1);
-                if (flat) {
-                    if (lane == 0) {
-                        s_first_even[parity][warp][0] = xe;
-                        s_first_even[parity][warp][1] = ye;
-                        s_first_even[parity][warp][2] = ze;
-                    }
-                    __syncthreads();
-                    if (lane == 31 && warp + 1 < nwarps) {
-                        rx = s_first_even[parity][warp + 1][0];
-                        ry = s_first_even[parity][warp + 1][1];
-                        rz = s_first_even[parity][warp + 1][2];
-                    }
-                    parity ^= 1;
-                }
-                if (has_o) {
-                    float qx[2], qy[2], qz[2];
-                    qx[0] = xe; qy[0] = ye; qz[0] = ze;
-                    int deg = 1;
-                    if (bo + 1 < L) { qx[1] = rx; qy[1] = ry; qz[1] = rz; deg = 2; }
-                    float n0, n1, n2;
-                    normals3(wo, s_ntab, n0, n1, n2);
-                    float px, py, pz;
-                    int c_old, c_new;
-                    const bool acc = trial<2, FOLD>(c, xo, yo, zo, qx, qy, qz, deg, deg == 2 ? cc2 : cc1,
-                                              deg == 2 ? ac42 : ac41, n0, n1, n2, accept_word(wo),
-                                              omega + (int64_t)type_o * NC, px, py, pz, c_old, c_new);
-                    if (acc) { xo = px; yo = py; zo = pz; }
-                    nacc += acc ? 1u : 0u;
-                    if (MODE == kMoveGrid && acc && c_new != c_old)
-                        count_move(S->counts[S->cur], S->count16 != 0, (int64_t)type_o * NC, c_old, c_new);
-                }
-            }
-            if (live) {
-                if (pair_aligned) {
-                    __stcs(reinterpret_cast<float2*>(S->x + g), make_float2(xe, xo));
-                    __stcs(reinterpret_cast<float2*>(S->y + g), make_float2(ye, yo));
-                    __stcs(reinterpret_cast<float2*>(S->z + g), make_float2(ze, zo));
-                } else {
-                    __stcs(S->x + g, xe);
-                    __stcs(S->y + g, ye);
-                    __stcs(S->z + g, ze);
-                    if (has_o) {
-                        __stcs(S->x + g + 1, xo);
-                        __stcs(S->y + g + 1, yo);
-                        __stcs(S->z + g + 1, zo);
-                    }
-                }
-            }
-        }
-        if (MODE != kGridOnly) {
-            nacc = warp_sum(nacc);
-            if (lane == 0 && nacc) atomicAdd(&S->slot_acc[(ti * kMaxWarps + warp) % kSlots], (unsigned long long)nacc);
+        const uint32_t len_magic = Ap->len_magic;
+        for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+            const int b = i - (int)div_magic((uint32_t)i, len_magic, L) * L;
+            const int64_t idx = (int64_t)__ldg(types + b) * NC + cell_of(c, X[i], Y[i], Z[i]);
+            if (c16)
+                atomicAdd(cnt + (idx >> 1), 1u << ((idx & 1) * 16));
+            else
+                atomicAdd(cnt + idx, 1u);
         }
     }
 }
 
-// Lean move kernel for launches of one system whose architectures are linear
-// chains of an even length L <= 64 with L/2 dividing 32, on a grid of
-// power-of-two axes (LaunchShape::lean; the large system and the blend are
-// such launches).  Same sweep, trials and random numbers as k_sweep_reg, with
-// less work per trial:
-//  * the system's constants (positions, omega, chain ids, k, A, R, cell
-//    inverses, grid, per-degree c and A c / 4, the architectures' chain and
-//    bead ranges) come from the parameter bank (SysConsts), the Philox round
-//    keys too;
-//  * every pair has an odd bead, so the even/odd branches go away; a missing
-//    bond neighbour at a chain end is replaced by the bead itself, whose term
-//    fma(+0, 2k, f) leaves the force bit for bit as if it were skipped (the
-//    force starts at +0 and can only be -0 from a -0 sum, which RN never
-//    gives here);
-//  * lanes beyond an architecture's last chain (a partial last group) repeat
-//    that chain and store nothing, so every lane runs the same code;
-//  * the Metropolis logarithm and the count moves sit under warp-uniform
-//    branches (__any_sync); the outcome of every trial is unchanged;
-//  * a trial whose bonded energy change alone exceeds what the omega span
-//    and its uniform allow is rejected before the cell folds and the omega
-//    gathers (maybe_accepted), which about half of the warps then skip.
-// Persistent: one CTA of kLeanThreads (28 warps, 72 registers each: the SM's
-// whole register file) per SM.  Each warp strides over the groups of 32/(L/2)
-// chains of every architecture, so no tile tail is left, and loads the next
-// group's pairs while it moves the current one.  The CTA keeps kLeanCopies
-// copies of the normal table in shared memory, entry-interleaved, and lane l
-// reads copy l % 8: the eight lanes of one 16-byte shared-memory phase then
-// always read eight different bank groups (with one copy, random segments made
-// 2.3 wavefronts of every phase).  Bead and cell indices are 32-bit (the plan
-// checks the sizes).
-constexpr int kLeanThreads = 896;
-constexpr int kLeanCopies = 8;
-constexpr size_t kLeanSmem = (size_t)SCMF_NORMAL_SEGS * kLeanCopies * sizeof(float4);
-
-
-// One trial of the bead at (x, y, z) with bond force f, updated in place when
-// accepted (lanes with live false never move): the proposal, its cells and
-// the omega reads are formed only in warps where some lane passes the span
-// bound.  Returns whether the move was accepted.
-__device__ __forceinline__ bool trial_lean(const MoveConsts& c, float& x, float& y, float& z, float fx, float fy,
-                                           float fz, float cc, float ac4, float n0, float n1, float n2, uint32_t aw,
-                                           float span, bool live, const float* __restrict__ w_t, int& cell_old,
-                                           int& cell_new) {
-    const float A = c.A, R = c.R;
-    const float dx = __fmaf_rn(A, fx, __fmul_rn(R, n0));
-    const float dy = __fmaf_rn(A, fy, __fmul_rn(R, n1));
-    const float dz = __fmaf_rn(A, fz, __fmul_rn(R, n2));
-    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-    const float fd = __fmaf_rn(fx, dx, __fmaf_rn(fy, dy, __fmul_rn(fz, dz)));
-    const float deb = __fmul_rn(ac4, __fmaf_rn(cc, d2, __fmul_rn(-2.0f, fd)));
-    const float u = u01(aw);
-    bool acc = false;
-    cell_old = cell_new = 0;
-    if (__any_sync(0xffffffffu, maybe_accepted(deb, span, log_lower(u)))) {
-        const float px = __fadd_rn(x, dx), py = __fadd_rn(y, dy), pz = __fadd_rn(z, dz);
-        cell_old = cell_of<0>(c, x, y, z);
-        cell_new = cell_of<0>(c, px, py, pz);
-        const float dE = __fadd_rn(__fsub_rn(__ldg(w_t + cell_new), __ldg(w_t + cell_old)), deb);
-        // accept if dE < 0; else if log(u) < -dE (log_lower decides without the
-        // logarithm for all but a few trials in a thousand; dE >= 17 fails
-        // -dE > log_lower(u) >= -16, so no separate bound is needed)
-        acc = dE < 0.0f;
-        const bool near = !acc && -dE > log_lower(u);
-        if (__any_sync(0xffffffffu, near)) acc = acc || (near && log_f(u) < -dE);
-        acc = acc && live;
-        if (acc) {
-            x = px;
-            y = py;
-            z = pz;
-        }
-    }
-    return acc;
-}
-
-template <int MODE>
-__global__ void __maxnreg__(72) k_sweep_lean(const PhiloxKeys keys, const SysConsts sc) {
-    extern __shared__ float4 s_ntab_lean[];  // [SCMF_NORMAL_SEGS][kLeanCopies]
-    for (int i = threadIdx.x; i < SCMF_NORMAL_SEGS * kLeanCopies; i += blockDim.x)
-        s_ntab_lean[i] = __ldg(normal_table() + i / kLeanCopies);
-    __syncthreads();
-    SysDev* S = sc.sys;
-    if (S->step >= S->stop_step) return;  // grid-uniform
-    const uint32_t step = S->step + 1u;
-    const float span = S->omega_span;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + warp;  // this warp among all
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    const float4* tab = s_ntab_lean + (lane & (kLeanCopies - 1));
-    MoveConsts c;
-    c.k = 0.0f;
-    c.k2 = sc.k2;
-    c.A = sc.A;
-    c.R = sc.R;
-    c.inv_dx = sc.inv_dx;
-    c.inv_dy = sc.inv_dy;
-    c.inv_dz = sc.inv_dz;
-    c.nx = sc.nx;
-    c.ny = sc.ny;
-    c.nz = sc.nz;
-    c.pow2 = true;
-    c.small = false;
-    unsigned nacc = 0;
-    for (int a = 0; a < sc.n_arch; ++a) {
-        const int L = sc.arch[a].length;
-        const int lg = __ffs(L >> 1) - 1;                         // log2(L/2): L/2 divides 32
-        const int tpc = 1 << lg;                                  // threads per chain
-        const int cs = lane >> lg;                                // chain slot in the warp
-        const int tt = lane & (tpc - 1);                          // pair index in the chain
-        const int cpw = 32 >> lg;                                 // chains per group
-        const int be = 2 * tt, bo = be + 1;
-        const bool first = tt == 0, last = tt == tpc - 1;         // chain ends: one bond
-        const float cc_e = first ? sc.cdeg[1] : sc.cdeg[2], ac4_e = first ? sc.ac4deg[1] : sc.ac4deg[2];
-        const float cc_o = last ? sc.cdeg[1] : sc.cdeg[2], ac4_o = last ? sc.ac4deg[1] : sc.ac4deg[2];
-        const int toff_e = (int)__ldg(sc.arch[a].types + be) * (int)sc.n_cells;
-        const int toff_o = (int)__ldg(sc.arch[a].types + bo) * (int)sc.n_cells;
-        // a chain end's missing bond: the shuffles below return the lane's own
-        // bead there, and these zero spring constants make its term +-0
-        const float k2_l = first ? 0.0f : sc.k2, k2_r = last ? 0.0f : sc.k2;
-        const int nch = sc.arch[a].n_chains;
-        const int bead0 = sc.arch[a].bead0;
-        const uint32_t rng0 = (uint32_t)sc.arch[a].rng0;
-        const int groups = (nch + cpw - 1) >> (5 - lg);
-        // the pairs and chain id of the warp's next group are loaded one group
-        // ahead, so the DRAM latency overlaps this group's trials
-        float2 nvx = make_float2(0.0f, 0.0f), nvy = nvx, nvz = nvx;
-        auto fetch = [&](int grp) {
-            const int ch = min(grp * cpw + cs, nch - 1);
-            const int gn = bead0 + ch * L + be;
-            nvx = __ldcs(reinterpret_cast<const float2*>(sc.x + gn));
-            nvy = __ldcs(reinterpret_cast<const float2*>(sc.y + gn));
-            nvz = __ldcs(reinterpret_cast<const float2*>(sc.z + gn));
-        };
-        if (gw < groups) fetch(gw);
-        for (int grp = gw; grp < groups; grp += nw) {  // warp-uniform bounds
-            const int chain = grp * cpw + cs;
-            const bool live = chain < nch;
-            const int chc = live ? chain : nch - 1;
-            const int g = bead0 + chc * L + be;
-            const float2 vx = nvx, vy = nvy, vz = nvz;
-            const uint32_t gc = rng0 + (uint32_t)chc;  // storage order is the stream order
-            if (grp + nw < groups) fetch(grp + nw);
-            float xe = vx.x, xo = vx.y, ye = vy.x, yo = vy.y, ze = vz.x, zo = vz.y;
-            // even bead 2t: bonds to 2t-1 (lane - 1's odd bead; the bead itself at the chain start) and 2t+1
-            const float lx = __shfl_up_sync(0xffffffffu, xo, 1, tpc);
-            const float ly = __shfl_up_sync(0xffffffffu, yo, 1, tpc);
-            const float lz = __shfl_up_sync(0xffffffffu, zo, 1, tpc);
-            const uint4 w = philox4x32_10(make_uint4(gc, (uint32_t)be, step, 0u), keys);
-            const uint4 wo = philox4x32_10(make_uint4(gc, (uint32_t)bo, step, 0u), keys);
-            float n0, n1, n2;
-            normals3<kLeanCopies>(w, tab, n0, n1, n2);
-            bool acc_e, mv_e;
-            int ce_old, ce_new;
-            {
-                float fx = __fmaf_rn(__fsub_rn(lx, xe), k2_l, 0.0f);
-                float fy = __fmaf_rn(__fsub_rn(ly, ye), k2_l, 0.0f);
-                float fz = __fmaf_rn(__fsub_rn(lz, ze), k2_l, 0.0f);
-                add_bond(c.k2, xe, ye, ze, xo, yo, zo, fx, fy, fz);
-                acc_e = trial_lean(c, xe, ye, ze, fx, fy, fz, cc_e, ac4_e, n0, n1, n2, accept_word(w), span, live,
-                                   sc.omega + toff_e, ce_old, ce_new);
-                mv_e = acc_e && ce_new != ce_old;
-            }
-            // odd bead 2t+1: bonds to 2t (moved) and 2t+2 (lane + 1's moved even bead; the bead itself at the end)
-            const float rx = __shfl_down_sync(0xffffffffu, xe, 1, tpc);
-            const float ry = __shfl_down_sync(0xffffffffu, ye, 1, tpc);
-            const float rz = __shfl_down_sync(0xffffffffu, ze, 1, tpc);
-            normals3<kLeanCopies>(wo, tab, n0, n1, n2);
-            bool acc_o, mv_o;
-            int co_old, co_new;
-            {
-                float fx = __fmaf_rn(__fsub_rn(xe, xo), c.k2, 0.0f);
-                float fy = __fmaf_rn(__fsub_rn(ye, yo), c.k2, 0.0f);
-                float fz = __fmaf_rn(__fsub_rn(ze, zo), c.k2, 0.0f);
-                add_bond(k2_r, xo, yo, zo, rx, ry, rz, fx, fy, fz);
-                acc_o = trial_lean(c, xo, yo, zo, fx, fy, fz, cc_o, ac4_o, n0, n1, n2, accept_word(wo), span, live,
-                                   sc.omega + toff_o, co_old, co_new);
-                mv_o = acc_o && co_new != co_old;
-            }
-            nacc += (acc_e ? 1u : 0u) + (acc_o ? 1u : 0u);
-            if (MODE == kMoveGrid && __any_sync(0xffffffffu, mv_e || mv_o)) {
-                uint32_t* cnt = S->counts[S->cur];
-                const bool c16 = S->count16 != 0;
-                if (mv_e) count_move(cnt, c16, toff_e, ce_old, ce_new);
-                if (mv_o) count_move(cnt, c16, toff_o, co_old, co_new);
-            }
-            if (live) {
-                __stcs(reinterpret_cast<float2*>(sc.x + g), make_float2(xe, xo));
-                __stcs(reinterpret_cast<float2*>(sc.y + g), make_float2(ye, yo));
-                __stcs(reinterpret_cast<float2*>(sc.z + g), make_float2(ze, zo));
-            }
-        }
-    }
-    nacc = warp_sum(nacc);
-    if (lane == 0 && nacc) atomicAdd(&S->slot_acc[gw % kSlots], (unsigned long long)nacc);
-}
-
-// The lean kernel's structure for launches of many systems (batches, served
-// rounds) and for single systems that k_sweep_lean does not take: linear chains
-// whose ceil(L/2) divides 32 with L even (LaunchShape::warp_even), any grid (FOLD
-// 0: every axis a power of two; -1: the fold is chosen per system) and any key
-// mode.  Each tile's system constants come from its SysDev into registers; at
-// 96 registers (no spill) the 256-system mix ran 7.39e10 bead-moves/s against
-// 7.00e10 with k_sweep_reg (80-88 registers spilled and lost).
-template <int FOLD>
-__device__ __forceinline__ bool trial_leanm(const MoveConsts& c, float& x, float& y, float& z, float fx, float fy,
-                                           float fz, float cc, float ac4, float n0, float n1, float n2, uint32_t aw,
-                                           float span, bool live, const float* __restrict__ w_t, int& cell_old,
-                                           int& cell_new) {
-    const float A = c.A, R = c.R;
-    const float dx = __fmaf_rn(A, fx, __fmul_rn(R, n0));
-    const float dy = __fmaf_rn(A, fy, __fmul_rn(R, n1));
-    const float dz = __fmaf_rn(A, fz, __fmul_rn(R, n2));
-    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-    const float fd = __fmaf_rn(fx, dx, __fmaf_rn(fy, dy, __fmul_rn(fz, dz)));
-    const float deb = __fmul_rn(ac4, __fmaf_rn(cc, d2, __fmul_rn(-2.0f, fd)));
-    const float u = u01(aw);
-    bool acc = false;
-    cell_old = cell_new = 0;
-    // the omega span rejects most trials before the folds and gathers (see trial_lean)
-    if (__any_sync(0xffffffffu, maybe_accepted(deb, span, log_lower(u)))) {
-        const float px = __fadd_rn(x, dx), py = __fadd_rn(y, dy), pz = __fadd_rn(z, dz);
-        cell_old = cell_of<FOLD>(c, x, y, z);
-        cell_new = cell_of<FOLD>(c, px, py, pz);
-        const float dE = __fadd_rn(__fsub_rn(__ldg(w_t + cell_new), __ldg(w_t + cell_old)), deb);
-        acc = dE < 0.0f;
-        const bool near = !acc && -dE > log_lower(u);
-        if (__any_sync(0xffffffffu, near)) acc = acc || (near && log_f(u) < -dE);
-        acc = acc && live;
-        if (acc) {
-            x = px;
-            y = py;
-            z = pz;
-        }
-    }
-    return acc;
-}
-
-template <int MODE, int FOLD, int KEYS>
-__global__ void __maxnreg__(96) k_sweep_leanm(const MoveTile* __restrict__ tiles, const int32_t* __restrict__ list, int n_list,
-                                             const PhiloxKeys keys) {
-    __shared__ float4 s_ntab[SCMF_NORMAL_SEGS];
-    load_normal_table(s_ntab);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int li = blockIdx.x; li < n_list; li += gridDim.x) {
-        const int ti = list ? __ldg(list + li) : li;
-        const MoveTile t = tiles[ti];
-        SysDev* S = t.sys;
-        if (S->step >= S->stop_step) continue;  // block-uniform
-        const uint32_t step = S->step + 1u;
-        MoveConsts c;
-        c.k = S->k; c.k2 = S->k2; c.A = S->A; c.R = S->R;
-        c.inv_dx = S->inv_dx; c.inv_dy = S->inv_dy; c.inv_dz = S->inv_dz;
-        load_fold(c, S);
-        const uint32_t k0 = S->seed_lo, k1 = S->seed_hi;
-        float* const PX = S->x;
-        float* const PY = S->y;
-        float* const PZ = S->z;
-        const float* const OM = S->omega;
-        const float span = S->omega_span;
-        const int NCi = (int)S->n_cells;
-        const ArchDev* Ap = t.arch;
-        const int L = Ap->length;
-        const int tpc = L >> 1;                                   // threads per chain, divides 32
-        const int cs = (int)div_magic((uint32_t)lane, Ap->tpc_magic, tpc);
-        const int tt = lane - cs * tpc;                           // pair index in the chain
-        const int cpw = 32 / tpc;                                 // chains per warp iteration
-        const int be = 2 * tt, bo = be + 1;
-        const bool first = tt == 0, last = tt == tpc - 1;         // chain ends: one bond
-        const float cc_e = first ? S->cdeg[1] : S->cdeg[2], ac4_e = first ? S->ac4deg[1] : S->ac4deg[2];
-        const float cc_o = last ? S->cdeg[1] : S->cdeg[2], ac4_o = last ? S->ac4deg[1] : S->ac4deg[2];
-        const int toff_e = (int)__ldg(Ap->types + be) * NCi;
-        const int toff_o = (int)__ldg(Ap->types + bo) * NCi;
-        // a chain end's missing bond: the shuffles below return the lane's own
-        // bead there, and these zero spring constants make its term +-0
-        const float k2_l = first ? 0.0f : c.k2, k2_r = last ? 0.0f : c.k2;
-        // random-stream id of the tile's first chain (storage order is the stream order)
-        const uint32_t rng0 = (uint32_t)(Ap->rng_base + (t.chain0 - Ap->chain_base));
-        const int nch = t.n_chains;
-        const int stride = nwarps * cpw;
-        unsigned nacc = 0;
-        // the pair and chain id of the next iteration are loaded one iteration
-        // ahead, so the DRAM latency overlaps this iteration's trials
-        float2 nvx = make_float2(0.0f, 0.0f), nvy = nvx, nvz = nvx;
-        auto fetch = [&](int cb) {
-            const int ch = min(cb + cs, nch - 1);
-            const int gn = (int)t.bead0 + ch * L + be;
-            nvx = __ldcs(reinterpret_cast<const float2*>(PX + gn));
-            nvy = __ldcs(reinterpret_cast<const float2*>(PY + gn));
-            nvz = __ldcs(reinterpret_cast<const float2*>(PZ + gn));
-        };
-        if (warp * cpw < nch) fetch(warp * cpw);
-        for (int cbase = warp * cpw; cbase < nch; cbase += stride) {  // warp-uniform bounds
-            const int chain = cbase + cs;
-            const bool live = chain < nch;
-            const int chc = live ? chain : nch - 1;
-            const int g = (int)t.bead0 + chc * L + be;
-            const float2 vx = nvx, vy = nvy, vz = nvz;
-            const uint32_t gc = rng0 + (uint32_t)chc;
-            if (cbase + stride < nch) fetch(cbase + stride);
-            float xe = vx.x, xo = vx.y, ye = vy.x, yo = vy.y, ze = vz.x, zo = vz.y;
-            // even bead 2t: bonds to 2t-1 (lane - 1's odd bead; the bead itself at the chain start) and 2t+1
-            const float lx = __shfl_up_sync(0xffffffffu, xo, 1, tpc);
-            const float ly = __shfl_up_sync(0xffffffffu, yo, 1, tpc);
-            const float lz = __shfl_up_sync(0xffffffffu, zo, 1, tpc);
-            const uint4 w = philox_block<KEYS>(make_uint4(gc, (uint32_t)be, step, 0u), k0, k1, keys);
-            const uint4 wo = philox_block<KEYS>(make_uint4(gc, (uint32_t)bo, step, 0u), k0, k1, keys);
-            float n0, n1, n2;
-            normals3(w, s_ntab, n0, n1, n2);
-            bool acc_e, mv_e;
-            int ce_old, ce_new;
-            {
-                float fx = __fmaf_rn(__fsub_rn(lx, xe), k2_l, 0.0f);
-                float fy = __fmaf_rn(__fsub_rn(ly, ye), k2_l, 0.0f);
-                float fz = __fmaf_rn(__fsub_rn(lz, ze), k2_l, 0.0f);
-                add_bond(c.k2, xe, ye, ze, xo, yo, zo, fx, fy, fz);
-                acc_e = trial_leanm<FOLD>(c, xe, ye, ze, fx, fy, fz, cc_e, ac4_e, n0, n1, n2, accept_word(w), span,
-                                          live, OM + toff_e, ce_old, ce_new);
-                mv_e = acc_e && ce_new != ce_old;
-            }
-            // odd bead 2t+1: bonds to 2t (moved) and 2t+2 (lane + 1's moved even bead; the bead itself at the end)
-            const float rx = __shfl_down_sync(0xffffffffu, xe, 1, tpc);
-            const float ry = __shfl_down_sync(0xffffffffu, ye, 1, tpc);
-            const float rz = __shfl_down_sync(0xffffffffu, ze, 1, tpc);
-            normals3(wo, s_ntab, n0, n1, n2);
-            bool acc_o, mv_o;
-            int co_old, co_new;
-            {
-                float fx = __fmaf_rn(__fsub_rn(xe, xo), c.k2, 0.0f);
-                float fy = __fmaf_rn(__fsub_rn(ye, yo), c.k2, 0.0f);
-                float fz = __fmaf_rn(__fsub_rn(ze, zo), c.k2, 0.0f);
-                add_bond(k2_r, xo, yo, zo, rx, ry, rz, fx, fy, fz);
-                acc_o = trial_leanm<FOLD>(c, xo, yo, zo, fx, fy, fz, cc_o, ac4_o, n0, n1, n2, accept_word(wo), span,
-                                          live, OM + toff_o, co_old, co_new);
-                mv_o = acc_o && co_new != co_old;
-            }
-            nacc += (acc_e ? 1u : 0u) + (acc_o ? 1u : 0u);
-            if (MODE == kMoveGrid && __any_sync(0xffffffffu, mv_e || mv_o)) {
-                uint32_t* cnt = S->counts[S->cur];
-                const bool c16 = S->count16 != 0;
-                if (mv_e) count_move(cnt, c16, toff_e, ce_old, ce_new);
-                if (mv_o) count_move(cnt, c16, toff_o, co_old, co_new);
-            }
-            if (live) {
-                __stcs(reinterpret_cast<float2*>(PX + g), make_float2(xe, xo));
-                __stcs(reinterpret_cast<float2*>(PY + g), make_float2(ye, yo));
-                __stcs(reinterpret_cast<float2*>(PZ + g), make_float2(ze, zo));
-            }
-        }
-        nacc = warp_sum(nacc);
-        if (lane == 0 && nacc) atomicAdd(&S->slot_acc[(ti * kMaxWarps + warp) % kSlots], (unsigned long long)nacc);
-    }
-}
 
 // ------------------------------------------------------------------ field
 
@@ -1211,8 +469,9 @@ __device__ __forceinline__ double omega_of_cell(int nt, const uint32_t* cnt, flo
     return ef;
 }
 
-// Scalar path: one cell (any count width, any alignment).
-template <int NT, bool FUSED>
+// Scalar path: one cell (any count width, any alignment).  FROM_L2: counts and
+// omega change in the course of the launch, so they are not read through L1.
+template <int NT, bool FROM_L2>
 __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, float scale, bool lit, bool upd,
                                              bool c16, const uint32_t* src32, float* W, const float* cf,
                                              unsigned long long* avg, float& wmax, float& wmin) {
@@ -1224,8 +483,14 @@ __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, fl
 #pragma unroll
     for (int u = 0; u < M; ++u) {
         if (u < nt) {
-            cnt[u] = c16 ? (uint32_t)src16[u * NC + cell] : src32[u * NC + cell];
-            if (!upd) w[u] = W[u * NC + cell];
+            const int64_t i = u * NC + cell;
+            if (FROM_L2) {
+                cnt[u] = c16 ? (uint32_t)__ldcg(src16 + i) : __ldcg(src32 + i);
+                if (!upd) w[u] = __ldcg(W + i);
+            } else {
+                cnt[u] = c16 ? (uint32_t)src16[i] : src32[i];
+                if (!upd) w[u] = W[i];
+            }
             if (avg) avg[u * NC + cell] += cnt[u];
         }
     }
@@ -1243,7 +508,7 @@ __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, fl
 
 // Vector path: four consecutive cells with 16-byte loads and stores (32-bit
 // counts, n_cells and the tile start multiples of 4).
-template <int NT, bool FUSED>
+template <int NT, bool FROM_L2>
 __device__ __forceinline__ double field_cells4(int64_t cell, int64_t NC, float scale, bool lit, bool upd,
                                                const uint32_t* src32, float* W, const float* cf,
                                                unsigned long long* avg, float& wmax, float& wmin) {
@@ -1251,8 +516,10 @@ __device__ __forceinline__ double field_cells4(int64_t cell, int64_t NC, float s
     float4 wv[NT];
 #pragma unroll
     for (int u = 0; u < NT; ++u) {
-        cv[u] = *reinterpret_cast<const uint4*>(src32 + u * NC + cell);
-        if (!upd) wv[u] = *reinterpret_cast<const float4*>(W + u * NC + cell);
+        const uint4* const c = reinterpret_cast<const uint4*>(src32 + u * NC + cell);
+        const float4* const w = reinterpret_cast<const float4*>(W + u * NC + cell);
+        cv[u] = FROM_L2 ? __ldcg(c) : *c;
+        if (!upd) wv[u] = FROM_L2 ? __ldcg(w) : *w;
     }
     if (avg) {
 #pragma unroll
@@ -1292,6 +559,22 @@ __device__ __forceinline__ double field_cells4(int64_t cell, int64_t NC, float s
     }
     return ef;
 }
+
+// Order-preserving integer key of a non-NaN float (for atomicMax / atomicMin)
+// and its inverse.
+__device__ __forceinline__ uint32_t ord_key(float f) {
+    const uint32_t b = __float_as_uint(f);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float ord_val(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
+}
+
+}  // namespace scmf
+
+#include "scmf_sweep.cuh"
+
+namespace scmf {
 
 // Closes one system after a launch (one block): sums the accept slots and the
 // energy partials part[0 .. count) in an order fixed by the block size, and
@@ -1338,16 +621,6 @@ __device__ void close_system(SysDev* S, const double* part, int count, int mode,
     __syncthreads();
 }
 
-// Order-preserving integer key of a non-NaN float (for atomicMax / atomicMin)
-// and its inverse.
-__device__ __forceinline__ uint32_t ord_key(float f) {
-    const uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float ord_val(uint32_t k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
 template <bool FUSED, int NT>
 __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ tiles, int n_tiles, int force_update,
                                                 double* __restrict__ ef_part, int close_mode) {
@@ -1380,10 +653,10 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
         const int64_t end = t.cell0 + t.n_cells;
         if (NT > 0 && !c16 && (NC & 3) == 0 && (t.cell0 & 3) == 0 && (t.n_cells & 3) == 0) {
             for (int64_t cell = t.cell0 + 4 * tid; cell < end; cell += 4 * T)
-                ef += field_cells4<(NT > 0 ? NT : 1), FUSED>(cell, NC, scale, lit, upd, src32, W, cf, avg, wmax, wmin);
+                ef += field_cells4<(NT > 0 ? NT : 1), false>(cell, NC, scale, lit, upd, src32, W, cf, avg, wmax, wmin);
         } else {
             for (int64_t cell = t.cell0 + tid; cell < end; cell += T)
-                ef += field_cell<NT, FUSED>(n, cell, NC, scale, lit, upd, c16, src32, W, cf, avg, wmax, wmin);
+                ef += field_cell<NT, false>(n, cell, NC, scale, lit, upd, c16, src32, W, cf, avg, wmax, wmin);
         }
         ef = warp_sum(ef);
 #pragma unroll
@@ -1438,7 +711,6 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
 // Closes a launch for every system of the plan (one block per system): the
 // sums of close_system over each system's tile ranges.
 __global__ void __launch_bounds__(256) k_close(const SysClose* __restrict__ list, int n_sys,
-                                                const unsigned* __restrict__ acc_part, int warps_per_tile,
                                                 const double* __restrict__ ef_part, const double* __restrict__ eb_part,
                                                 int mode) {
     __shared__ unsigned long long s_a[32];
@@ -1752,13 +1024,15 @@ int launch_init_coords(SysDev* d_sys, const ArchDev* d_arch, int n_arch, int n_c
     return (int)cudaGetLastError();
 }
 
-// Opt the sweep kernels in to the largest dynamic shared memory once, outside
-// any stream capture (called when a system is created).
-template <int MODE, int KEYS>
-static cudaError_t allow_smem(int bytes) {
-    cudaError_t e = cudaFuncSetAttribute(k_sweep<MODE, false, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_sweep_linear<MODE, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+template <bool ONE, int KEYS>
+static cudaError_t opt_in_warp() {
+    const auto opt_in = [](const void* f, int bytes) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    cudaError_t e = opt_in((const void*)k_sweep_warp<ONE, false, KEYS>, SweepLayout<false>::kBytes);
+    if (e == cudaSuccess) e = opt_in((const void*)k_sweep_warp<ONE, true, KEYS>, SweepLayout<true>::kBytes);
+    if (e == cudaSuccess) e = opt_in((const void*)k_run<ONE, false, KEYS>, SweepLayout<false>::kBytes);
+    if (e == cudaSuccess) e = opt_in((const void*)k_run<ONE, true, KEYS>, SweepLayout<true>::kBytes);
     return e;
 }
 
@@ -1772,125 +1046,102 @@ int configure_kernels() {
     std::lock_guard<std::mutex> g(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return 0;
     int2 fold_tab[257] = {};
-    for (uint32_t n = 2; n <= 256; ++n) {
-        const uint32_t bias = n * (((1u << 22) + n - 1) / n);  // a multiple of n, at least 2^22
-        fold_tab[n] = make_int2((int)(0x4B400000u - bias), (int)(uint32_t)(((1ull << 32) + n - 1) / n));
-    }
+    for (int n = 2; n <= 256; ++n) fold_tab[n] = make_int2(fold_offset(n), (int)fold_magic_of(n));
     cudaError_t ef = cudaMemcpyToSymbol(c_fold, fold_tab, sizeof fold_tab);
     if (ef != cudaSuccess) return (int)ef;
-    ef = cudaFuncSetAttribute(k_sweep_lean<kMoveOnly>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeanSmem);
-    if (ef == cudaSuccess)
-        ef = cudaFuncSetAttribute(k_sweep_lean<kMoveGrid>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeanSmem);
-    if (ef != cudaSuccess) return (int)ef;
+    // opt the sweep kernels in to the largest dynamic shared memory, outside any stream capture
     const int bytes = (int)sweep_smem_bytes(kMaxTileBeads, kMaxLength);
-    cudaError_t e = cudaSuccess;
-    for (int keys = kKeysNone; keys <= kKeysBoth && e == cudaSuccess; ++keys) {
-        if (keys == kKeysNone) {
-            e = allow_smem<kGridOnly, kKeysNone>(bytes);
-            if (e == cudaSuccess) e = allow_smem<kMoveOnly, kKeysNone>(bytes);
-            if (e == cudaSuccess) e = allow_smem<kMoveGrid, kKeysNone>(bytes);
-        } else if (keys == kKeysHigh) {
-            e = allow_smem<kMoveOnly, kKeysHigh>(bytes);
-            if (e == cudaSuccess) e = allow_smem<kMoveGrid, kKeysHigh>(bytes);
-        } else {
-            e = allow_smem<kMoveOnly, kKeysBoth>(bytes);
-            if (e == cudaSuccess) e = allow_smem<kMoveGrid, kKeysBoth>(bytes);
-        }
-    }
+    const auto opt_in = [](const void* f, int n) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+    };
+    const void* const general[] = {(const void*)k_sweep<kMoveOnly, kKeysNone>, (const void*)k_sweep<kMoveGrid, kKeysNone>,
+                                   (const void*)k_sweep<kMoveOnly, kKeysHigh>, (const void*)k_sweep<kMoveGrid, kKeysHigh>,
+                                   (const void*)k_sweep<kMoveOnly, kKeysBoth>, (const void*)k_sweep<kMoveGrid, kKeysBoth>};
+    cudaError_t e = opt_in_warp<true, kKeysBoth>();
+    if (e == cudaSuccess) e = opt_in_warp<false, kKeysHigh>();
+    if (e == cudaSuccess) e = opt_in_warp<false, kKeysNone>();
+    for (const void* f : general)
+        if (e == cudaSuccess) e = opt_in(f, bytes);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return (int)e;
 }
 
-template <int MODE, bool FLAT>
-static void launch_reg(const LaunchShape& sh, int blocks, int threads, cudaStream_t st, const MoveTile* tiles,
-                       const int32_t* list, int n, unsigned* acc) {
-    const int keys = MODE == kGridOnly ? kKeysNone : sh.keyed;
-    if constexpr (MODE != kGridOnly && !FLAT) {
-        if (sh.lean && keys == kKeysBoth && sh.fold == 0 && !list) {
-            k_sweep_lean<MODE><<<sm_count(), kLeanThreads, kLeanSmem, st>>>(sh.keys, sh.sc);
-            return;
-        }
-        if (sh.warp_even) {
-            if (keys == kKeysBoth) {
-                if (sh.fold == 0) k_sweep_leanm<MODE, 0, kKeysBoth><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-                else k_sweep_leanm<MODE, -1, kKeysBoth><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-            } else if (keys == kKeysHigh) {
-                if (sh.fold == 0) k_sweep_leanm<MODE, 0, kKeysHigh><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-                else k_sweep_leanm<MODE, -1, kKeysHigh><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-            } else {
-                if (sh.fold == 0) k_sweep_leanm<MODE, 0, kKeysNone><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-                else k_sweep_leanm<MODE, -1, kKeysNone><<<blocks, threads, 0, st>>>(tiles, list, n, sh.keys);
-            }
-            return;
-        }
-    }
-    if (keys == kKeysBoth) {
-        if (sh.fold == 0)
-            k_sweep_reg<MODE, FLAT, 0, kKeysBoth><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-        else
-            k_sweep_reg<MODE, FLAT, -1, kKeysBoth><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-    } else if (keys == kKeysHigh) {
-        if (sh.fold == 0)
-            k_sweep_reg<MODE, FLAT, 0, kKeysHigh><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-        else
-            k_sweep_reg<MODE, FLAT, -1, kKeysHigh><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-    } else {
-        if (sh.fold == 0)
-            k_sweep_reg<MODE, FLAT, 0, kKeysNone><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-        else
-            k_sweep_reg<MODE, FLAT, -1, kKeysNone><<<blocks, threads, 0, st>>>(tiles, list, n, acc, sh.keys);
-    }
-}
-
 template <int MODE>
-static int launch_sweep_t(const MoveTile* tiles, int n_tiles, int mtb, int ml, LaunchShape sh, unsigned* acc,
-                          cudaStream_t st) {
-    if (mtb > kMaxTileBeads || ml > kMaxLength || sh.threads > 256 || sh.threads < 32) return (int)cudaErrorInvalidValue;
-    const int blocks = sh.blocks > 0 ? sh.blocks : n_tiles;
-    const int keys = MODE == kGridOnly ? kKeysNone : sh.keyed;
-    if (sh.linear && ml <= 64) {
-        // tiles whose chains fill warps exactly run the barrier-free kernel,
-        // the others (sh.flat_list) the block-wide one: one launch each
-        const int n_warp = sh.n_flat > 0 ? sh.n_warp : n_tiles;
-        const int32_t* warp_list = sh.n_flat > 0 ? sh.warp_list : nullptr;
-        if (n_warp > 0 && sh.part != 2)
-            launch_reg<MODE, false>(sh, sh.blocks > 0 ? min(sh.blocks, n_warp) : n_warp, sh.threads, st, tiles,
-                                    warp_list, n_warp, acc);
-        if (sh.n_flat > 0 && sh.part != 1)
-            launch_reg<MODE, true>(sh, sh.blocks > 0 ? min(sh.blocks, sh.n_flat) : sh.n_flat,
-                                   sh.flat_threads > 0 ? sh.flat_threads : sh.threads, st, tiles, sh.flat_list,
-                                   sh.n_flat, acc);
-    } else if (sh.linear) {
-        // per-warp slice: ceil(chains per tile / warps) chains of the longest length
-        const int nw = sh.threads / 32;
-        const int wb = ((sh.max_chains + nw - 1) / nw) * ml;
-        const size_t smem = (size_t)nw * 3 * wb * sizeof(float);
-        if (smem > sweep_smem_bytes(kMaxTileBeads, kMaxLength)) return (int)cudaErrorInvalidValue;
-        if (keys == kKeysBoth)
-            k_sweep_linear<MODE, kKeysBoth><<<blocks, sh.threads, smem, st>>>(tiles, nullptr, n_tiles, wb, acc, sh.keys);
-        else if (keys == kKeysHigh)
-            k_sweep_linear<MODE, kKeysHigh><<<blocks, sh.threads, smem, st>>>(tiles, nullptr, n_tiles, wb, acc, sh.keys);
-        else
-            k_sweep_linear<MODE, kKeysNone><<<blocks, sh.threads, smem, st>>>(tiles, nullptr, n_tiles, wb, acc, sh.keys);
-    } else {
-        const size_t smem = sweep_smem_bytes(mtb, ml);
-        if (keys == kKeysBoth)
-            k_sweep<MODE, false, kKeysBoth><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, acc, sh.keys);
-        else if (keys == kKeysHigh)
-            k_sweep<MODE, false, kKeysHigh><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, acc, sh.keys);
-        else
-            k_sweep<MODE, false, kKeysNone><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, acc, sh.keys);
-    }
-    return (int)cudaGetLastError();
+static void launch_general(const MoveTile* tiles, int n_tiles, int blocks, int mtb, int ml, const LaunchShape& sh,
+                           cudaStream_t st) {
+    const size_t smem = sweep_smem_bytes(mtb, ml);
+    if (sh.keyed == kKeysBoth)
+        k_sweep<MODE, kKeysBoth><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, sh.keys);
+    else if (sh.keyed == kKeysHigh)
+        k_sweep<MODE, kKeysHigh><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, sh.keys);
+    else
+        k_sweep<MODE, kKeysNone><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, sh.keys);
 }
 
-int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int mtb, int ml, LaunchShape sh, unsigned* acc_part,
-                 void* stream) {
+// The launch of a plan's warp tiles: k_sweep_warp, or k_run when `run` is given.
+template <bool ONE, bool LONG, int KEYS>
+static cudaError_t launch_warp(const SweepArgs& a, const RunArgs* run, cudaStream_t st) {
+    using Lay = SweepLayout<LONG>;
+    const int sms = sm_count(), grid = a.n_tiles < sms ? a.n_tiles : sms;
+    const int per_sm = (a.n_tiles + grid - 1) / grid, nw = per_sm < Lay::kWarps ? per_sm : Lay::kWarps;
+    const int smem = kSweepTabBytes + nw * (int)sizeof(typename Lay::Warp) + kSlack;
+    if (!run) {
+        k_sweep_warp<ONE, LONG, KEYS><<<grid, 32 * nw, smem, st>>>(a);
+        return cudaGetLastError();
+    }
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;  // the blocks wait for one another
+    at.val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(32u * (unsigned)nw);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_run<ONE, LONG, KEYS>, a, *run);
+}
+
+template <bool ONE, int KEYS>
+static cudaError_t launch_warp(const SweepArgs& a, int beads, const RunArgs* run, cudaStream_t st) {
+    return beads > kSweepBeads ? launch_warp<ONE, true, KEYS>(a, run, st) : launch_warp<ONE, false, KEYS>(a, run, st);
+}
+
+static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const RunArgs* run, cudaStream_t st) {
+    SweepArgs a{};
+    a.tiles = sh.warp_tiles;
+    a.n_tiles = sh.n_warp_tiles;
+    a.move_counts = move_counts;
+    a.once = sh.once;
+    a.keys = sh.keys;
+    a.system = sh.system;
+    a.sys = sh.sweep;
+    a.n_arch = sh.n_arch;
+    for (int i = 0; i < sh.n_arch; ++i) a.arch[i] = sh.arch[i];
+    if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.warp_beads, run, st);
+    if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.warp_beads, run, st);
+    return launch_warp<false, kKeysNone>(a, sh.warp_beads, run, st);
+}
+
+int launch_run(const LaunchShape& sh, const RunArgs& run, void* stream) {
+    return (int)launch_warp(sh, true, &run, (cudaStream_t)stream);
+}
+
+int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int mtb, int ml, const LaunchShape& sh, void* stream) {
     if (n_tiles <= 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if (mode == kMoveOnly) return launch_sweep_t<kMoveOnly>(tiles, n_tiles, mtb, ml, sh, acc_part, st);
-    if (mode == kMoveGrid) return launch_sweep_t<kMoveGrid>(tiles, n_tiles, mtb, ml, sh, acc_part, st);
-    return launch_sweep_t<kGridOnly>(tiles, n_tiles, mtb, ml, sh, acc_part, st);
+    if (mtb > kMaxTileBeads || ml > kMaxLength || sh.threads > 256 || sh.threads < 32) return (int)cudaErrorInvalidValue;
+    const int blocks = sh.blocks > 0 ? sh.blocks : n_tiles;
+    if (mode == kGridOnly) {
+        k_grid<<<blocks, sh.threads, 0, st>>>(tiles, n_tiles);
+    } else if (sh.n_warp_tiles > 0) {
+        return (int)launch_warp(sh, mode == kMoveGrid, nullptr, st);
+    } else if (mode == kMoveOnly) {
+        launch_general<kMoveOnly>(tiles, n_tiles, blocks, mtb, ml, sh, st);
+    } else {
+        launch_general<kMoveGrid>(tiles, n_tiles, blocks, mtb, ml, sh, st);
+    }
+    return (int)cudaGetLastError();
 }
 
 template <bool FUSED>
@@ -1925,11 +1176,9 @@ int launch_bond_energy(const MoveTile* tiles, int n_tiles, LaunchShape sh, doubl
     return (int)cudaGetLastError();
 }
 
-int launch_close(const SysClose* list, int n_sys, const unsigned* acc_part, int warps_per_tile, const double* ef_part,
-                 const double* eb_part, int mode, void* stream) {
+int launch_close(const SysClose* list, int n_sys, const double* ef_part, const double* eb_part, int mode, void* stream) {
     if (n_sys <= 0) return 0;
-    k_close<<<n_sys < 1024 ? n_sys : 1024, 256, 0, (cudaStream_t)stream>>>(list, n_sys, acc_part, warps_per_tile,
-                                                                             ef_part, eb_part, mode);
+    k_close<<<n_sys < 1024 ? n_sys : 1024, 256, 0, (cudaStream_t)stream>>>(list, n_sys, ef_part, eb_part, mode);
     return (int)cudaGetLastError();
 }
 

@@ -357,8 +357,7 @@ scmf_status scmf_validate(scmf_system* s, scmf_validation* out) {
     CK(cudaMemcpyAsync((char*)s->d_sys + offsetof(SysDev, cur), &other, 4, cudaMemcpyHostToDevice, s->stream));
     LaunchShape sh = s->plan.move_shape();
     sh.blocks = 0;
-    CKL(launch_sweep(kGridOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh,
-                     s->plan.d_acc, s->stream));
+    CKL(launch_sweep(kGridOnly, s->plan.d_move, s->plan.n_move, s->plan.max_tile_beads, s->plan.max_length, sh, s->stream));
     CK(cudaMemcpyAsync((char*)s->d_sys + offsetof(SysDev, cur), &cur, 4, cudaMemcpyHostToDevice, s->stream));
     CKL(launch_validate_positions(s->d_sys, s->n_beads, s->d_check, s->stream));
     CKL(launch_validate_cells(s->d_sys, s->counts[cur], s->counts[other], (int64_t)(cb / 4),

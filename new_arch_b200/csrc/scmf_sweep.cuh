@@ -1,0 +1,950 @@
+// The move of linear chains: k_sweep_warp (one sweep's move of any systems) and
+// k_run (many whole sweeps of systems that fit on the chip); included by
+// scmf_kernels.cu.
+//
+// What a sweep costs is arithmetic: every trial needs its Philox block (twenty
+// 32 x 32 -> 64 bit products, four cycles of a scheduler's multiplier each),
+// three normals, a force and an energy, about 200 warp instructions in all, while
+// its bytes take a third of that time.  Where proposals overshoot (A 4k of
+// several, the synthetic workloads: one trial in two hundred accepted) nearly all
+// of this proves a rejection that a coarser computation can prove too.  So a
+// sweep is split:
+//
+//  * screen: every trial is proposed with its own Philox block but with normals
+//    from a small piecewise-linear table, and rejected when the energy that
+//    even the table's error leaves cannot pass the Metropolis test whatever
+//    omega holds (ScreenDev has the inequality).  The even and the odd bead of a
+//    pair run side by side, as the halves of packed f32x2 operations, and share
+//    the first Philox rounds.  The loop takes 141 cycles of a scheduler per
+//    warp of trials, half of them Philox's, from four warps a scheduler on
+//    (16, 24, 28 and 32 warps an SM measure the same).
+//  * resolve: the trials left over (2.8 % in the large system) are gathered into
+//    a list of the warp and made exactly, a full warp at a time: exact normals,
+//    energy, cells, omega, Metropolis, with the words of the general kernel.
+//    Even beads first; every odd neighbour of an even bead that moved, whose
+//    screen saw the old position, is added to the odd beads' list.
+//
+// A system whose proposals mostly pass (ScreenDev::on 0: the reference's own
+// units) skips the screen and resolves every trial.  Either way positions and
+// counts are the ones that the oracle gives, bit for bit.
+//
+// Each warp has tiles of its own (up to kSweepBeads beads in its part of shared
+// memory) and waits for no other warp.  Measured against this on the large system
+// (51.2M beads, 0.326 ms): warps that only screen beside warps that only resolve
+// 0.375 ms (an exact trial waits for positions, table and omega, but mostly it
+// takes its share of the same pipes); the trials of several tiles resolved
+// together from global memory 0.344 ms; 20 warps with smaller tiles 0.324 ms.
+// The kernels before it (a thread per bead pair in registers, every trial exact)
+// took 0.379 ms, and 0.051 ms for 2.0M beads in chains of 33 where this takes
+// 0.025 ms.
+#pragma once
+#include <stddef.h>
+
+#include <type_traits>
+
+#include "scmf_screen_table.h"
+
+namespace scmf {
+
+// ---------------------------------------------------------- packed fp32 pairs
+// Two rounded-to-nearest FP32 operations in one instruction (sm_100).  The
+// same bits as the scalar operations on each half.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// ------------------------------------------------------ bulk copies, barriers
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return done != 0u;
+}
+// Waits for a phase of a barrier of this CTA; false after about two seconds
+// (never in a sound run).
+constexpr long long kWaitClocks = 4000000000ll;
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    do {
+        if (mbar_try(bar, parity)) return true;
+    } while (clock64() - t0 < kWaitClocks);
+    return false;
+}
+// A bulk copy from global memory whose lines leave L2 before others where
+// `once` is set: positions that are read once a sweep, when they are more than L2
+// holds, would push omega and the counts out.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, bool once) {
+    uint64_t policy;
+    if (once)
+        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    else
+        asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+        : "memory");
+}
+// Orders this thread's earlier accesses before later bulk copies.
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// ------------------------------------------------------------------- layout
+constexpr int kScreenCopies = 16;
+constexpr int kListLen = 128;
+constexpr int kSlack = 256;  // the lanes past a tile's last pair read up to 64 words past its buffer
+constexpr int kTilePad = 12;  // 4 words before the tile, its offset of up to 3, and 2 read past its last pair
+// The screen table follows the exact normal table: kScreenCopies lane-
+// interleaved copies (lane l reads copy l mod 16: the half warps of an 8-byte
+// read then meet no bank twice).
+constexpr int kScreenTabAt = SCMF_NORMAL_SEGS * (int)sizeof(float4);
+constexpr int kSweepTabBytes = kScreenTabAt + SCMF_SCREEN_SEGS * kScreenCopies * (int)sizeof(float2);
+
+// A CTA's warps and what each has in shared memory.  LONG: for chains longer
+// than kSweepBeads.
+template <bool LONG>
+struct SweepLayout {
+    static constexpr int kWarps = LONG ? kSweepWarpsLong : kSweepWarps;
+    static constexpr int kBeads = LONG ? kSweepBeadsLong : kSweepBeads;
+    static constexpr int kStride = kBeads + kTilePad;  // from x to y to z
+    struct Warp {
+        uint64_t full;         // barrier: the tile has arrived
+        uint64_t pad;
+        uint32_t moved[32];    // odd beads next to an even bead that moved: a bit for each row, a word for each lane
+        uint16_t list[kListLen];
+        SweepSys sys;          // of the tile's system, where a launch has several
+        FieldSys field;        // of the system of the warp's field tile (k_run)
+        alignas(16) float pos[3 * kStride];
+    };
+    static constexpr int kBytes = kSweepTabBytes + kWarps * (int)sizeof(Warp) + kSlack;
+    static_assert(kBeads <= 2048, "a row of 32 bead pairs is a bit of a lane's mask");
+    static_assert(kSweepTabBytes % 16 == 0 && sizeof(Warp) % 16 == 0 && offsetof(Warp, pos) % 16 == 0 && kStride % 4 == 0,
+                  "16-byte copies");
+    static_assert(kBytes <= 227 * 1024, "shared memory of an SM");
+};
+
+// ------------------------------------------------------------------- screen
+// A normal of word w to within SCMF_SCREEN_DELTA, times 2^30.  lane_at is the
+// byte offset of the lane's copy in an entry (bits 3 to 6).
+__device__ __forceinline__ float screen_normal(uint32_t w, uint32_t lane_at) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const float f = __uint2float_rn(w + w + 1u);
+    const uint32_t at = ((__float_as_uint(f) >> 14) & 0xFFFFFF80u) | lane_at;  // (bits >> 21) * 16 copies * 8 bytes
+    const float2 c = *reinterpret_cast<const float2*>(smem_raw + (kScreenTabAt - (127 << 2) * kScreenCopies * 8) + at);
+    const float z = __fmaf_rn(c.y, f, c.x);
+    return __uint_as_float(__float_as_uint(z) ^ (w & 0x80000000u));
+}
+__device__ __forceinline__ uint32_t screen_lane() { return (uint32_t)(threadIdx.x & (kScreenCopies - 1)) * 8u; }
+
+// log2 of a value that lies below the uniform of word w (u01 drops the low
+// nine bits of w; the conversion and the subtraction round by at most 2^-25
+// each): -inf or NaN for the smallest uniforms, which then pass the screen.
+__device__ __forceinline__ float log2_below_u(uint32_t w) {
+    const float u = __fmaf_rn(__uint2float_rn(w), -0x1p-32f, 0x1.fffffcp-1f);
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
+    return l;
+}
+
+// The Philox blocks of the two beads of a pair, with the work that they share
+// (the chain and step words) done once: (chain, b, step, 0) and (chain, b + 1,
+// step, 0).  PairHead is what depends on the beads and the step alone.
+struct PairHead {
+    uint32_t y1;                  // low word of M1 * step
+    uint64_t p0e, p0o;            // M0 * x of round 1, for the even and the odd bead
+};
+template <int KEYS>
+__device__ __forceinline__ PairHead pair_head(uint32_t b, uint32_t step, uint32_t k0, const PhiloxKeys& ks) {
+    const uint64_t m1s = (uint64_t)0xCD9E8D57u * step;
+    const uint32_t hi = (uint32_t)(m1s >> 32) ^ (KEYS == kKeysBoth ? ks.k[0] : k0);
+    PairHead h;
+    h.y1 = (uint32_t)m1s;
+    h.p0e = (uint64_t)0xD2511F53u * (hi ^ b);
+    h.p0o = (uint64_t)0xD2511F53u * (hi ^ (b + 1u));
+    return h;
+}
+template <int KEYS>
+__device__ __forceinline__ void pair_blocks(uint32_t chain, const PairHead& h, uint32_t k0, uint32_t k1,
+                                            const PhiloxKeys& ks, uint4& we, uint4& wo) {
+    // the key words of round r (KeyMode: from the schedule, or advanced here)
+    const auto key0 = [&](int r) { return KEYS == kKeysBoth ? ks.k[2 * r] : k0; };
+    const auto key1 = [&](int r) { return KEYS != kKeysNone ? ks.k[2 * r + 1] : k1; };
+    const auto next = [&] {
+        if (KEYS != kKeysBoth) k0 += 0x9E3779B9u;
+        if (KEYS == kKeysNone) k1 += 0xBB67AE85u;
+    };
+    const uint64_t a = (uint64_t)0xD2511F53u * chain;                                   // round 1
+    const uint64_t q = (uint64_t)0xCD9E8D57u * ((uint32_t)(a >> 32) ^ key1(0));         // round 2
+    next();
+    const uint32_t x2 = (uint32_t)(q >> 32) ^ h.y1 ^ key0(1);
+    we.z = (uint32_t)(h.p0e >> 32) ^ (uint32_t)a ^ key1(1);
+    wo.z = (uint32_t)(h.p0o >> 32) ^ (uint32_t)a ^ key1(1);
+    next();
+    const uint64_t c = (uint64_t)0xD2511F53u * x2;                                      // round 3
+    const uint64_t de = (uint64_t)0xCD9E8D57u * we.z, d_o = (uint64_t)0xCD9E8D57u * wo.z;
+    we = make_uint4((uint32_t)(de >> 32) ^ (uint32_t)q ^ key0(2), (uint32_t)de,
+                    (uint32_t)(c >> 32) ^ (uint32_t)h.p0e ^ key1(2), (uint32_t)c);
+    wo = make_uint4((uint32_t)(d_o >> 32) ^ (uint32_t)q ^ key0(2), (uint32_t)d_o,
+                    (uint32_t)(c >> 32) ^ (uint32_t)h.p0o ^ key1(2), (uint32_t)c);
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+        next();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint4& w = i ? wo : we;
+            const uint64_t p0 = (uint64_t)0xD2511F53u * w.x, p1 = (uint64_t)0xCD9E8D57u * w.z;
+            w = make_uint4((uint32_t)(p1 >> 32) ^ w.y ^ key0(r), (uint32_t)p1,
+                           (uint32_t)(p0 >> 32) ^ w.w ^ key1(r), (uint32_t)p0);
+        }
+    }
+}
+
+// Constants of a pair's two trials (even bead, odd bead).
+struct PairConsts {
+    f32x2 k2l, k2r;  // spring constants of the left and right bond, 0 where there is none; the odd bead's left
+                     // one is negated (its difference is the even bead's right one)
+    f32x2 a, b;      // ScreenDev's a and b
+    // keeps the values in registers through the loop that follows
+    __device__ __forceinline__ void pin() { asm volatile("" : "+l"(k2l), "+l"(k2r), "+l"(a), "+l"(b)); }
+};
+// What a warp keeps of the system and architecture that it is at.
+struct SweepConsts {
+    int L, h;                       // beads and pairs (ceil(L / 2)) of a chain
+    uint32_t h_magic;               // div_magic of h
+    uint32_t step, k0, k1;          // the sweep being made, the seed
+    float k2, a1, a2, b1, b2, add;  // ScreenDev's, for beads of one and two bonds
+    float u0, u1;                   // (4 / A)(span + 2^-18) and -(4 / A) ln 2: span + L of ScreenDev times 4 / A
+    PairConsts pc;                  // KIND 0: the lane's
+    PairHead head;
+};
+// first: the even bead starts its chain; single: it also ends it (no odd bead); last: the odd bead ends it.
+__device__ __forceinline__ PairConsts pair_consts(const SweepConsts& s, bool first, bool single, bool last) {
+    const bool e1 = first || single;
+    PairConsts c;
+    c.k2l = pack2(first ? 0.0f : s.k2, -s.k2);
+    c.k2r = pack2(single ? 0.0f : s.k2, last ? 0.0f : s.k2);
+    c.a = pack2(e1 ? s.a1 : s.a2, last ? s.a1 : s.a2);
+    c.b = pack2(e1 ? s.b1 : s.b2, last ? s.b1 : s.b2);
+    return c;
+}
+
+// The lane's pairs of a tile of `items` pairs: bit i for pair 32 i + lane.
+__device__ __forceinline__ uint32_t row_mask(int items) {
+    const int n = max(0, (items - (int)(threadIdx.x & 31) + 31) >> 5);
+    return n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u;
+}
+
+// Screens a tile: bit i of even (odd): the trial of the even (odd) bead of pair
+// 32 i + lane may be accepted.  X is the first bead's x.
+//   KIND 0: even L, h divides 32 (a lane's place in its chain never changes); 1:
+//   even L; 2: odd L, or a tile whose first bead is at an odd offset.
+template <int KIND, bool LONG, int KEYS>
+__device__ __forceinline__ void screen_tile(const SweepConsts& s, const float* X, uint32_t rng0, int n_chains,
+                                            const PhiloxKeys& keys, uint32_t tab, uint32_t& even_out, uint32_t& odd_out) {
+    using Lay = SweepLayout<LONG>;
+    const int lane = threadIdx.x & 31;
+    const int L = s.L, h = s.h, items = n_chains * h;
+    uint32_t bit = 1u, even = 0u, odd = 0u;
+    const uint32_t step = s.step, k0 = s.k0, k1 = s.k1, h_magic = s.h_magic;
+    const float u0 = s.u0, u1 = s.u1;
+    const f32x2 add = pack2(s.add, s.add);
+    PairConsts pc = s.pc;
+    PairHead head = s.head;
+    if (KIND == 0) pc.pin();
+    const float* P0 = X + 2 * lane;  // KIND 0: the lane's chain and place advance by constants
+    uint32_t gc0 = KIND == 0 ? rng0 + div_magic((uint32_t)lane, h_magic, h) : 0u;
+    const uint32_t gc_step = KIND == 0 ? 32u / (uint32_t)h : 0u;
+#pragma unroll 1
+    for (int j0 = 0; j0 < items; j0 += 32, bit += bit, P0 += 64, gc0 += gc_step) {
+        int j = j0 + lane;
+        if (KIND == 2) j = min(j, items - 1);
+        const int cl = KIND == 0 ? 0 : (int)div_magic((uint32_t)j, h_magic, h);
+        const int k = KIND == 0 ? 0 : j - cl * h;
+        const float* const PX = KIND == 2 ? X + (cl * L + 2 * k) : P0;
+        const uint32_t gc = KIND == 0 ? gc0 : rng0 + (uint32_t)cl;
+        const bool single = KIND == 2 && 2 * k + 1 >= L;  // the pair has no odd bead
+        if (KIND != 0) {
+            pc = pair_consts(s, k == 0, single, KIND == 2 ? 2 * k + 2 >= L : k == h - 1);
+            head = pair_head<KEYS>(2u * (uint32_t)k, step, k0, keys);
+        }
+        f32x2 f[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float* P = PX + a * Lay::kStride;
+            float e, o;
+            if (KIND == 2) {
+                e = P[0];
+                o = P[1];
+            } else {
+                const float2 v = *reinterpret_cast<const float2*>(P);
+                e = v.x;
+                o = v.y;
+            }
+            // the forces of the trial kernels, left bond then right bond; the
+            // odd bead's left difference is the even bead's right one negated
+            const float d = __fsub_rn(o, e), dl = __fsub_rn(P[-1], e), dr = __fsub_rn(P[2], o);
+            f[a] = fma2(pack2(d, dr), pc.k2r, mul2(pack2(dl, d), pc.k2l));
+        }
+        uint4 we, wo;
+        pair_blocks<KEYS>(gc, head, k0, k1, keys, we, wo);
+        const f32x2 vx = fma2(f[0], pc.a, pack2(screen_normal(we.x, tab), screen_normal(wo.x, tab)));
+        const f32x2 vy = fma2(f[1], pc.a, pack2(screen_normal(we.y, tab), screen_normal(wo.y, tab)));
+        const f32x2 vz = fma2(f[2], pc.a, pack2(screen_normal(we.z, tab), screen_normal(wo.z, tab)));
+        const f32x2 q = fma2(vx, vx, fma2(vy, vy, mul2(vz, vz)));
+        const f32x2 u = pack2(__fmaf_rn(log2_below_u(accept_word(we)), u1, u0), __fmaf_rn(log2_below_u(accept_word(wo)), u1, u0));
+        const f32x2 lim = fma2(pc.b, fma2(f[0], f[0], fma2(f[1], f[1], fma2(f[2], f[2], u))), add);
+        float qe, qo, le, lo;
+        unpack2(q, qe, qo);
+        unpack2(lim, le, lo);
+        if (!(qe > le)) even += bit;  // NaN passes
+        if (!(qo > lo) && !single) odd += bit;
+    }
+    const uint32_t valid = row_mask(items);
+    even_out = even & valid;
+    odd_out = odd & valid;
+}
+
+// The cell of a position.
+__device__ __forceinline__ int cell_index(const SweepSys& c, float x, float y, float z) {
+    int ix, iy, iz;
+    if (c.fold == 0) {
+        ix = fold_pow2(x, c.inv_d[0], c.n[0] - 1);
+        iy = fold_pow2(y, c.inv_d[1], c.n[1] - 1);
+        iz = fold_pow2(z, c.inv_d[2], c.n[2] - 1);
+    } else if (c.fold == 1) {
+        ix = fold_magic(x, c.inv_d[0], c.n[0], c.fold_off[0], c.fold_mag[0]);
+        iy = fold_magic(y, c.inv_d[1], c.n[1], c.fold_off[1], c.fold_mag[1]);
+        iz = fold_magic(z, c.inv_d[2], c.n[2], c.fold_off[2], c.fold_mag[2]);
+    } else {
+        ix = fold(x, c.inv_d[0], c.n[0]);
+        iy = fold(y, c.inv_d[1], c.n[1]);
+        iz = fold(z, c.inv_d[2], c.n[2]);
+    }
+    return ix + c.n[0] * (iy + c.n[1] * iz);
+}
+
+// What the exact trials of a tile need besides the system.
+struct TileRef {
+    float* X;                // the first bead's x in the buffer
+    int64_t bead0;           // its index in the system
+    uint32_t rng0;           // random-stream id of the first chain
+    int items;               // bead pairs
+    const uint8_t* types;
+    float span;
+    bool move_counts;
+};
+
+// The exact trials of the beads of parity par of N pairs a lane (pair[i], where
+// act[i]), with trial_f's expressions.  A move updates the tile and the positions
+// in global memory, moves a count if it leaves its cell, and marks the odd beads
+// next to it, whose screen saw the old position.  Returns the lane's moves.  The
+// N trials of a lane are independent: without branches between them their chains
+// (Philox, table, omega) run side by side.
+template <int N, bool LONG, int KEYS>
+__device__ __forceinline__ unsigned exact_trials(const SweepSys& c, const SweepConsts& s, const TileRef& t, uint32_t* moved,
+                                                 const PhiloxKeys& keys, const float4* ntab, int par, const int (&pair)[N],
+                                                 bool (&act)[N]) {
+    constexpr int kStride = SweepLayout<LONG>::kStride;
+    int p[N], b[N], c_old[N], c_new[N];
+    uint32_t typ[N];
+    float x[N], y[N], z[N], dx[N], dy[N], dz[N], deb[N], u[N], lo[N];
+    bool may[N];
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int cl = (int)div_magic((uint32_t)pair[i], s.h_magic, s.h);
+        int bead = 2 * (pair[i] - cl * s.h) + par;
+        act[i] = act[i] && bead < s.L;
+        bead = act[i] ? bead : 0;
+        b[i] = bead;
+        p[i] = cl * s.L + bead;
+        typ[i] = (uint32_t)__ldg(t.types + bead) * c.n_cells;
+        const bool has_l = bead > 0, has_r = bead + 1 < s.L;
+        const int l = has_l ? -1 : 0, r = has_r ? 1 : 0;  // a missing bond: the bead itself, and no spring
+        const float* const Q = t.X + p[i];
+        x[i] = Q[0];
+        y[i] = Q[kStride];
+        z[i] = Q[2 * kStride];
+        const uint4 w = philox_block<KEYS>(make_uint4(t.rng0 + (uint32_t)cl, (uint32_t)bead, s.step, 0u), s.k0, s.k1, keys);
+        float n0, n1, n2;
+        normals3(w, ntab, n0, n1, n2);
+        const float kl = has_l ? c.k2 : 0.0f, kr = has_r ? c.k2 : 0.0f;
+        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+        add_bond(kl, x[i], y[i], z[i], Q[l], Q[l + kStride], Q[l + 2 * kStride], fx, fy, fz);
+        add_bond(kr, x[i], y[i], z[i], Q[r], Q[r + kStride], Q[r + 2 * kStride], fx, fy, fz);
+        const int deg = (has_l ? 1 : 0) + (has_r ? 1 : 0);
+        const float cc = deg == 2 ? c.cdeg[2] : deg == 1 ? c.cdeg[1] : 0.0f;
+        const float ac4 = deg == 2 ? c.ac4[2] : deg == 1 ? c.ac4[1] : 0.0f;
+        dx[i] = __fmaf_rn(c.A, fx, __fmul_rn(c.R, n0));
+        dy[i] = __fmaf_rn(c.A, fy, __fmul_rn(c.R, n1));
+        dz[i] = __fmaf_rn(c.A, fz, __fmul_rn(c.R, n2));
+        const float d2 = __fmaf_rn(dx[i], dx[i], __fmaf_rn(dy[i], dy[i], __fmul_rn(dz[i], dz[i])));
+        const float fd = __fmaf_rn(fx, dx[i], __fmaf_rn(fy, dy[i], __fmul_rn(fz, dz[i])));
+        deb[i] = __fmul_rn(ac4, __fmaf_rn(cc, d2, __fmul_rn(-2.0f, fd)));
+        u[i] = u01(accept_word(w));
+        lo[i] = log_lower(u[i]);
+        may[i] = act[i] && maybe_accepted(deb[i], t.span, lo[i]);
+        any = any || may[i];
+    }
+    unsigned nacc = 0;
+    if (any) {
+        float w_old[N], w_new[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            c_old[i] = cell_index(c, x[i], y[i], z[i]);
+            c_new[i] = cell_index(c, __fadd_rn(x[i], dx[i]), __fadd_rn(y[i], dy[i]), __fadd_rn(z[i], dz[i]));
+            w_old[i] = __ldcg(c.omega + (typ[i] + c_old[i]));
+            w_new[i] = __ldcg(c.omega + (typ[i] + c_new[i]));
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float dE = __fadd_rn(__fsub_rn(w_new[i], w_old[i]), deb[i]);
+            // log_lower decides without the logarithm for all but a few trials (trial_f)
+            if (!(may[i] && (dE < 0.0f || (-dE > lo[i] && log_f(u[i]) < -dE)))) continue;
+            float* const Q = t.X + p[i];
+            const int64_t g = t.bead0 + p[i];
+            Q[0] = c.x[g] = __fadd_rn(x[i], dx[i]);
+            Q[kStride] = c.y[g] = __fadd_rn(y[i], dy[i]);
+            Q[2 * kStride] = c.z[g] = __fadd_rn(z[i], dz[i]);
+            if (t.move_counts && c_new[i] != c_old[i]) count_move(c.counts, c.count16 != 0, typ[i], c_old[i], c_new[i]);
+            ++nacc;
+            if (par == 0) {
+                const int j = pair[i];
+                if (b[i] > 0) atomicOr(moved + ((j - 1) & 31), 1u << ((j - 1) >> 5));
+                if (b[i] + 1 < s.L) atomicOr(moved + (j & 31), 1u << (j >> 5));
+            }
+        }
+    }
+    return nacc;
+}
+
+// Makes the trials of a tile that the masks name (bit i of even / odd: the even
+// / odd bead of pair 32 i + lane).  Returns the lane's accepted moves.
+template <bool LONG, int KEYS>
+__device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<LONG>::Warp* wp, const SweepSys& c, const SweepConsts& s,
+                                                 const TileRef& t, const PhiloxKeys& keys, const float4* ntab, uint32_t even,
+                                                 uint32_t odd) {
+    const int lane = threadIdx.x & 31;
+    unsigned nacc = 0;
+    uint32_t mask = even;
+#pragma unroll 1
+    for (int par = 0; par < 2; ++par) {
+        if (par) {  // the odd neighbours of the even beads that moved
+            mask = odd | wp->moved[lane];
+            wp->moved[lane] = 0u;
+        }
+        const int own = __popc(mask);
+        int before = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, before, 31);
+        if (2 * total <= t.items && total <= kListLen) {  // the pairs, gathered into full warps
+            uint16_t* at = wp->list + (before - own);
+            for (uint32_t m = mask; m; m &= m - 1u) *at++ = (uint16_t)((__ffs(m) - 1) * 32 + lane);
+            __syncwarp();
+#pragma unroll 1
+            for (int r = lane; r < total; r += 32) {
+                const int pair[1] = {(int)wp->list[r]};
+                bool act[1] = {true};
+                nacc += exact_trials<1, LONG, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+            }
+        } else {  // row by row
+#pragma unroll 1
+            for (int r = 0; 32 * r < t.items; ++r) {
+                const int pair[1] = {min(32 * r + lane, t.items - 1)};
+                bool act[1] = {((mask >> r) & 1u) != 0u};
+                nacc += exact_trials<1, LONG, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+            }
+        }
+        __syncwarp();
+    }
+    return nacc;
+}
+
+// A warp of a move kernel: its tile, its shared memory and the constants of the
+// system and architecture it is at.  ONE: the launch has one system, whose
+// constants are parameters (instruction operands).
+template <bool ONE, bool LONG, int KEYS>
+struct Mover {
+    using Lay = SweepLayout<LONG>;
+    const SweepArgs& a;
+    typename Lay::Warp* const wp;
+    const float4* const ntab;
+    const int lane;
+    SweepConsts s;
+    SysDev* S = nullptr;
+    const ArchDev* A = nullptr;
+    const uint8_t* types = nullptr;
+    uint32_t rng_base = 0u, parity = 0u;
+    float span = 0.0f;
+    int mode = 0;  // 0: the system's sweeps are done; 1: resolve every trial; 2: screen
+
+    __device__ __forceinline__ Mover(const SweepArgs& args, unsigned char* smem)
+        : a(args),
+          wp(reinterpret_cast<typename Lay::Warp*>(smem + kSweepTabBytes) + (threadIdx.x >> 5)),
+          ntab(reinterpret_cast<const float4*>(smem)),
+          lane(threadIdx.x & 31) {}
+    __device__ __forceinline__ const SweepSys& sys() const { return ONE ? a.sys : wp->sys; }
+
+    // One lane: has the buffer filled with a tile, from the 16-byte boundary below it.
+    __device__ __forceinline__ void load(const WarpTile& t) {
+        const SweepSys& c = ONE ? a.sys : t.sys->sweep;
+        const uint32_t bar = smem_addr(&wp->full), dst = smem_addr(wp->pos + 4);
+        const int off = (int)(t.bead0 & 3);
+        const uint32_t bytes = (uint32_t)((off + t.n_beads + 3) & ~3) * 4u;
+        const int64_t g = t.bead0 - off;
+        mbar_expect(bar, 3u * bytes);
+        bulk_load(dst, c.x + g, bytes, bar, a.once != 0);
+        bulk_load(dst + 4u * Lay::kStride, c.y + g, bytes, bar, a.once != 0);
+        bulk_load(dst + 8u * Lay::kStride, c.z + g, bytes, bar, a.once != 0);
+    }
+
+    // All threads of the block: the tables, the warp's barrier, and its first tile on the way.
+    __device__ __forceinline__ void start(unsigned char* smem, const WarpTile& t, bool any) {
+        if (lane == 0) {
+            mbar_init(smem_addr(&wp->full));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            fence_async();
+            if (any) load(t);
+        }
+        wp->moved[lane] = 0u;
+        float4* tab = reinterpret_cast<float4*>(smem);
+        for (int i = threadIdx.x; i < SCMF_NORMAL_SEGS; i += blockDim.x) tab[i] = __ldg(normal_table() + i);
+        float2* screen = reinterpret_cast<float2*>(smem + kScreenTabAt);
+        if (!ONE || a.sys.screen.on)
+            for (int i = threadIdx.x; i < SCMF_SCREEN_SEGS * kScreenCopies; i += blockDim.x)
+                screen[i] = __ldg(screen_table() + i / kScreenCopies);
+        __syncthreads();
+    }
+
+    // Turns to a tile's architecture.  `done`: sweeps of its system made before
+    // this one; omega_span: its omega's.
+    __device__ __forceinline__ void turn_to(const WarpTile& t, uint32_t done, bool active, float omega_span) {
+        if (!ONE && t.sys != S) {
+            __syncwarp();
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(&t.sys->sweep);
+            for (int i = lane; i < (int)(sizeof(SweepSys) / 4); i += 32) reinterpret_cast<uint32_t*>(&wp->sys)[i] = src[i];
+            __syncwarp();
+        }
+        const SweepSys& c = sys();
+        S = t.sys;
+        A = t.arch;
+        types = A->types;
+        rng_base = (uint32_t)A->rng_base;
+        span = omega_span;
+        s.L = A->length;
+        s.h = (s.L + 1) >> 1;
+        s.h_magic = A->tpc_magic;
+        s.step = done + 1u;
+        s.k0 = c.seed_lo;
+        s.k1 = c.seed_hi;
+        s.k2 = c.k2;
+        s.a1 = c.screen.a[1];
+        s.a2 = c.screen.a[2];
+        s.b1 = c.screen.b[1];
+        s.b2 = c.screen.b[2];
+        s.add = c.screen.add;
+        s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
+        s.u1 = __fmul_rn(c.screen.u, -0x1.62e7p-1f);  // a little over ln 2
+        mode = !active ? 0 : c.screen.on && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
+        const int k = lane & (s.h - 1);
+        s.pc = pair_consts(s, k == 0, false, k == s.h - 1);
+        s.head = pair_head<KEYS>(2u * (uint32_t)k, s.step, s.k0, a.keys);
+    }
+
+    // The same tile's next sweep.
+    __device__ __forceinline__ void next_sweep(uint32_t done, bool active, float omega_span) {
+        const SweepSys& c = sys();
+        span = omega_span;
+        s.step = done + 1u;
+        s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
+        mode = active ? mode : 0;
+        s.head = pair_head<KEYS>(2u * (uint32_t)(lane & (s.h - 1)), s.step, s.k0, a.keys);
+    }
+
+    // Waits for the tile asked for; false (and the error word) if it does not come.
+    __device__ __forceinline__ bool arrived() {
+        const bool ok = mbar_wait(smem_addr(&wp->full), parity);
+        if (!ok && lane == 0) atomicOr(&S->error_word, 4u);
+        parity ^= 1u;
+        return ok;
+    }
+
+    // One sweep of the tile in the buffer.  Returns the lane's accepted moves.
+    __device__ __forceinline__ unsigned move(const WarpTile& t) {
+        const int off = (int)(t.bead0 & 3), items = t.n_chains * s.h;
+        const uint32_t rng0 = rng_base + t.chain, tab = screen_lane();
+        float* X = wp->pos + 4 + off;
+        uint32_t even = 0u, odd = 0u;
+        if (mode == 2) {
+            if ((s.L | off) & 1)
+                screen_tile<2, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+            else if (32 % s.h)
+                screen_tile<1, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+            else
+                screen_tile<0, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+        } else if (mode == 1) {
+            even = odd = row_mask(items);
+        }
+        const TileRef ref{X, t.bead0, rng0, items, types, span, a.move_counts != 0};
+        return resolve_tile<LONG, KEYS>(wp, sys(), s, ref, a.keys, ntab, even, odd);
+    }
+};
+
+// Tile i of a launch: from the list, or where the launch has one system by
+// counting (each architecture's chains in tiles of `per`).
+template <bool ONE>
+__device__ __forceinline__ WarpTile tile_at(const SweepArgs& a, int i) {
+    if (!ONE) return a.tiles[i];
+    int k = 0;
+    while (k + 1 < a.n_arch && i >= a.arch[k + 1].first) ++k;
+    const SweepArch& r = a.arch[k];
+    const int chain = (i - r.first) * r.per;
+    WarpTile t;
+    t.sys = a.system;
+    t.arch = r.arch;
+    t.bead0 = r.bead_base + (int64_t)chain * r.length;
+    t.chain = (uint32_t)chain;
+    t.n_chains = min(r.per, r.n_chains - chain);
+    t.n_beads = t.n_chains * r.length;
+    t.length = r.length;
+    return t;
+}
+
+// One move of the systems of a launch.  One CTA per SM; each warp strides over
+// the tiles (whole chains of one architecture, up to kSweepBeads beads), whose
+// positions come by bulk copies, the next tile's from the moment the current one
+// is done.  Beads that move are written back, and nothing else.
+//
+// Warps that make equal tiles in step would ask for their positions together and
+// then leave memory idle together.  Where a warp makes several tiles, it begins
+// with a quarter, a half, three quarters or all of its first one (by its place
+// among the four warps of its SM sub-partition) and ends with the rest: 0.322 ->
+// 0.313 ms on the large system.
+template <bool ONE, bool LONG, int KEYS>
+__global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1) k_sweep_warp(const __grid_constant__ SweepArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Mover<ONE, LONG, KEYS> m(a, smem_raw);
+    // consecutive tiles go to different SMs, so that few tiles spread over all of them
+    const int warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
+    const int first = warp * (int)gridDim.x + (int)blockIdx.x, stride = nwarps * (int)gridDim.x;
+    const int turns = first < a.n_tiles ? (a.n_tiles - first + stride - 1) / stride : 0;
+    WarpTile t{};
+    if (turns > 0) t = tile_at<ONE>(a, first);
+    const WarpTile whole = t;
+    const int begin = turns >= 4 ? max(1, t.n_chains * (4 * warp / nwarps + 1) / 4) : t.n_chains;  // chains of the first part
+    const int parts = turns + (begin < whole.n_chains ? 1 : 0);
+    t.n_chains = begin;
+    t.n_beads = begin * t.length;
+    m.start(smem_raw, t, turns > 0);
+#pragma unroll 1
+    for (int q = 0; q < parts; ++q) {
+        WarpTile next = whole;
+        if (q + 1 < turns) {
+            next = tile_at<ONE>(a, first + (q + 1) * stride);
+        } else {
+            next.chain += (uint32_t)begin;
+            next.bead0 += (int64_t)begin * next.length;
+            next.n_chains -= begin;
+            next.n_beads -= begin * next.length;
+        }
+        if (t.arch != m.A) m.turn_to(t, t.sys->step, t.sys->step < t.sys->stop_step, t.sys->omega_span);
+        if (!m.arrived()) return;
+        unsigned nacc = m.move(t);
+        fence_async();  // this lane's reads and writes of the buffer, before the next copies land
+        __syncwarp();
+        if (q + 1 < parts && m.lane == 0) m.load(next);
+        if (__any_sync(0xffffffffu, nacc)) {
+            nacc = warp_sum(nacc);
+            if (m.lane == 0) atomicAdd(&m.S->slot_acc[(first + q) % kSlots], (unsigned long long)nacc);
+        }
+        t = next;
+    }
+}
+
+// ------------------------------------------------------ many sweeps a launch
+// A barrier of all CTAs of a (cooperative) launch, on a count in global memory
+// that only grows, by one a CTA and barrier.
+struct GridBarrier {
+    unsigned long long* count;
+    unsigned long long target;  // thread 0's
+    // The count is a whole number of barriers until the last CTA comes to the first one.
+    __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {
+        if (threadIdx.x == 0) target = __ldcg(c) / gridDim.x * gridDim.x;
+    }
+    // False (to all threads of the CTA) after about two seconds.
+    __device__ __forceinline__ bool wait(int* s_ok) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            target += gridDim.x;
+            asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+            unsigned long long now;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
+            if (now < target) {
+                const long long t0 = clock64();
+                do {
+                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
+                } while (now < target && clock64() - t0 < kWaitClocks);
+            }
+            *s_ok = now >= target;
+        }
+        __syncthreads();
+        return *s_ok != 0;
+    }
+};
+
+// Whether sweep `step` ends with a field update (test.cpp:42).
+__device__ __forceinline__ bool updates_field(int rule, uint32_t step) { return rule == 1 || step % 10u != 0u; }
+
+// The omega span that the sweep after `done` sweeps uses, in a launch that
+// started at `base`: of the last field update, from the launch's slots (om_keys,
+// by the update's step mod 3) or, before its first one, the system's.
+__device__ __forceinline__ float span_after(const SysDev* S, int rule, uint32_t done, uint32_t base) {
+    const uint32_t at = updates_field(rule, done) ? done : done - 1u;
+    if (done == base || at == base) return __ldcg(&S->omega_span);
+    const uint32_t kx = __ldcg(&S->om_keys[at % 3u][0]), kn = __ldcg(&S->om_keys[at % 3u][1]);
+    const float span = kx >= kn ? __fsub_rn(ord_val(kx), ord_val(kn)) : INFINITY;
+    return span >= 0.0f ? span : INFINITY;  // NaN (inf - inf): no bound
+}
+
+// The warp's largest and smallest omega into a pair of ordered keys.
+__device__ __forceinline__ void fold_span(uint32_t* keys, float wmax, float wmin) {
+    const uint32_t kx = __reduce_max_sync(0xffffffffu, ord_key(wmax)), kn = __reduce_min_sync(0xffffffffu, ord_key(wmin));
+    if ((threadIdx.x & 31) == 0 && kx >= kn) {  // the warp saw a non-NaN omega
+        atomicMax(keys, kx);
+        atomicMin(keys + 1, kn);
+    }
+}
+
+// Closes a system after its sweeps of a launch (one block).
+__device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r, unsigned long long* s_acc, double* s_ef) {
+    SysDev* S = rs.sys;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t base = S->step, left = S->stop_step > base ? S->stop_step - base : 0u;
+    const uint32_t made = min((uint32_t)r.n_sweeps, left);
+    if (made) {  // block-uniform
+        unsigned long long all = 0, last = 0;
+        for (int i = tid; i < kSlots; i += blockDim.x) {
+            all += __ldcg(&S->slot_acc[i]);
+            last += __ldcg(&S->slot_last[i]);
+            S->slot_acc[i] = 0ull;
+            S->slot_last[i] = 0ull;
+        }
+        double f = 0.0;
+        for (int i = tid; i < rs.field_count; i += blockDim.x) f += __ldcg(r.ef_part + rs.field_first + i);
+        all = warp_sum(all);
+        last = warp_sum(last);
+        f = warp_sum(f);
+        if (lane == 0) {
+            s_acc[warp] = all;
+            s_acc[16 + warp] = last;
+            s_ef[warp] = f;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < nwarps; ++w) {
+                all += s_acc[w];
+                last += s_acc[16 + w];
+                f += s_ef[w];
+            }
+            const uint32_t step = base + made;
+            S->last_accepts = last;
+            S->total_accepts += all;
+            S->total_moves += (unsigned long long)made * (unsigned long long)S->n_beads;
+            S->e_field = f;
+            if (S->avg && S->avg_every) S->avg_samples += step / S->avg_every - base / S->avg_every;
+            S->omega_span = span_after(S, S->field_rule, step, base);
+            S->step = step;
+        }
+    }
+    __syncthreads();
+}
+
+// A warp's field step over one tile of cells: omega of the new counts, and the
+// averaging sample where the sweep takes one.  Returns the lane's field energy.
+__device__ __forceinline__ double field_tile(const FieldSys& f, int64_t cell0, int n_cells, bool upd, bool sample, float& wmax,
+                                             float& wmin) {
+    const int lane = threadIdx.x & 31, n = f.n_types;
+    const int64_t NC = f.n_cells, end = cell0 + n_cells;
+    const bool lit = f.literal != 0, c16 = f.count16 != 0;
+    unsigned long long* avg = sample ? f.avg : nullptr;
+    double ef = 0.0;
+    if (!c16 && n <= 3 && ((NC | cell0 | n_cells) & 3) == 0) {
+        for (int64_t cell = cell0 + 4 * lane; cell < end; cell += 128) {
+            if (n == 2)
+                ef += field_cells4<2, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
+            else if (n == 1)
+                ef += field_cells4<1, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
+            else
+                ef += field_cells4<3, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
+        }
+    } else {
+        for (int64_t cell = cell0 + lane; cell < end; cell += 32)
+            ef += field_cell<0, true>(n, cell, NC, f.scale, lit, upd, c16, f.counts, f.omega, f.cf, avg, wmax, wmin);
+    }
+    return ef;
+}
+
+// n_sweeps whole sweeps (move, field, statistics) of the systems of a launch in
+// one cooperative launch, where every warp has one tile at most: its positions
+// stay in shared memory from sweep to sweep, the tables and constants are set up
+// once, and two grid barriers a sweep take the place of two kernel launches.  A
+// sweep of such a system is mostly latency (launches, tables, descriptors, each
+// a dependent trip to L2).  A sweep in this form against two kernels replayed
+// from a graph: 32,000 beads 8.8 us against 18.6 us; 409,600 beads, unscreened,
+// 14.8 against 22.7 us; 2.0M beads in chains of 33 20.2 against 28.9 us.  (Before
+// the kernels of this file: 14.6, 20.7 and 55.4 us.)  A barrier takes 2 us.
+template <bool ONE, bool LONG, int KEYS>
+__global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
+    k_run(const __grid_constant__ SweepArgs a, const __grid_constant__ RunArgs r) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_ok;
+    __shared__ uint32_t s_keys[2];
+    __shared__ unsigned long long s_acc[32];
+    __shared__ double s_ef[16];
+    Mover<ONE, LONG, KEYS> m(a, smem_raw);
+    const int lane = m.lane, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int first = warp * (int)gridDim.x + (int)blockIdx.x, stride = nwarps * (int)gridDim.x;
+    const bool any = first < a.n_tiles;
+    GridBarrier barrier(r.barrier);
+    WarpTile t{};
+    if (any) t = tile_at<ONE>(a, first);
+    if (threadIdx.x < 2) s_keys[threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
+    for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {  // the slot of the launch's first field step
+        SysDev* S = r.systems[i].sys;
+        if (threadIdx.x < 2) S->om_keys[(S->step + 1u) % 3u][threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
+    }
+    m.start(smem_raw, t, any);
+    uint32_t base = 0u, stop = 0u;  // sweeps that the tile's system has made, and makes in all
+    int rule = 0;
+    if (any) {
+        base = t.sys->step;
+        stop = t.sys->stop_step;
+        rule = t.sys->field_rule;
+        m.turn_to(t, base, base < stop, t.sys->omega_span);
+        if (!m.arrived()) m.mode = 0;
+    }
+    // the warp's field tile (its first, where it has several) and that one's system
+    FieldSys* const fs = &m.wp->field;
+    FieldTile ft{};
+    if (first < r.n_field) ft = r.field[first];
+    uint32_t f_base = 0u, f_stop = 0u;
+    const auto at_system = [&](const SysDev* S) {
+        __syncwarp();
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(&S->field);
+        for (int i = lane; i < (int)(sizeof(FieldSys) / 4); i += 32) reinterpret_cast<uint32_t*>(fs)[i] = src[i];
+        if (lane == 0) {
+            fs->avg = S->avg;
+            fs->avg_every = S->avg_every;
+        }
+        f_base = S->step;
+        f_stop = S->stop_step;
+        __syncwarp();
+    };
+    if (first < r.n_field) at_system(ft.sys);
+    unsigned acc_all = 0, acc_last = 0;  // of all the launch's sweeps, of the system's last
+#pragma unroll 1
+    for (int sweep = 0; sweep < r.n_sweeps; ++sweep) {
+        if (any && m.mode) {
+            const uint32_t done = base + (uint32_t)sweep;
+            if (sweep) m.next_sweep(done, done < stop, span_after(m.S, rule, done, base));
+            if (m.mode) {
+                acc_last = m.move(t);
+                acc_all += acc_last;
+            }
+        }
+        if (!barrier.wait(&s_ok)) return;
+        float wmax = -INFINITY, wmin = INFINITY;
+#pragma unroll 1
+        for (int fi = first; fi < r.n_field; fi += stride) {
+            if (fi != first || r.n_field > stride) {
+                const SysDev* before = ft.sys;
+                ft = r.field[fi];
+                if (ft.sys != before) at_system(ft.sys);
+            }
+            const uint32_t step = f_base + (uint32_t)sweep + 1u;
+            if (step > f_stop) continue;
+            const bool upd = updates_field(fs->rule, step), last = sweep + 1 == r.n_sweeps || step == f_stop;
+            const bool sample = fs->avg && fs->avg_every && step % fs->avg_every == 0u;
+            if (!upd && !last && !sample) continue;  // nothing to write and nothing to report
+            if (!ONE) {
+                wmax = -INFINITY;
+                wmin = INFINITY;
+            }
+            double ef = field_tile(*fs, ft.cell0, ft.n_cells, upd, sample, wmax, wmin);
+            if (last) {
+                ef = warp_sum(ef);
+                if (lane == 0) r.ef_part[fi] = ef;
+            }
+            if (!upd)
+                wmax = -INFINITY, wmin = INFINITY;
+            else if (!ONE)
+                fold_span(ft.sys->om_keys[step % 3u], wmax, wmin);
+        }
+        if (ONE) {
+            fold_span(s_keys, wmax, wmin);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            if (ONE) {
+                const uint32_t step = base + (uint32_t)sweep + 1u;  // block-wide: thread 0's warp has a tile
+                if (s_keys[0]) {
+                    atomicMax(&m.S->om_keys[step % 3u][0], s_keys[0]);
+                    atomicMin(&m.S->om_keys[step % 3u][1], s_keys[1]);
+                }
+                s_keys[0] = 0u;
+                s_keys[1] = 0xFFFFFFFFu;
+                if (blockIdx.x == 0) {  // the slot of the next field step
+                    m.S->om_keys[(step + 1u) % 3u][0] = 0u;
+                    m.S->om_keys[(step + 1u) % 3u][1] = 0xFFFFFFFFu;
+                }
+            } else {
+                for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {
+                    SysDev* S = r.systems[i].sys;
+                    const uint32_t next = (S->step + (uint32_t)sweep + 2u) % 3u;
+                    S->om_keys[next][0] = 0u;
+                    S->om_keys[next][1] = 0xFFFFFFFFu;
+                }
+            }
+        }
+        if (sweep + 1 == r.n_sweeps && any) {
+            const unsigned all = warp_sum(acc_all), last = warp_sum(acc_last);
+            if (lane == 0) {
+                if (all) atomicAdd(&m.S->slot_acc[first % kSlots], (unsigned long long)all);
+                if (last) atomicAdd(&m.S->slot_last[first % kSlots], (unsigned long long)last);
+            }
+        }
+        if (!barrier.wait(&s_ok)) return;
+    }
+    // the statistics of every system, in a fixed order
+    for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) close_run(r.systems[i], r, s_acc, s_ef);
+}
+
+}  // namespace scmf

@@ -1275,8 +1275,8 @@ int launch_observables(const MoveTile* tiles, int n_tiles, const float* ref_xyz,
 // holds that array (kNoAllocMaxTiles doubles, 16 KiB) until the process exits.
 namespace scmf {
 
-constexpr int kNoAllocTileCells = 4096;
-constexpr int kNoAllocMaxTiles = 2048;  // n_cells <= 2048 * 4096 = 8,388,608
+constexpr int kNoAllocTileCells = 4096;  // cells of a tile at most
+constexpr int kNoAllocMaxTiles = 2048;   // n_cells <= 2048 * 4096 = 8,388,608
 
 static __device__ __align__(256) double g_noalloc_partials[kNoAllocMaxTiles];
 
@@ -1288,45 +1288,60 @@ struct FieldParams {
     float cf[kMaxTypes * kMaxTypes];
 };
 
-// One tile of kNoAllocTileCells cells per block: omega of every cell and the
-// tile's field energy sum_T omega_T n_T into partials[tile] (no atomics).
+// One tile of cells per block: omega of every cell and the tile's field energy
+// sum_T omega_T n_T into partials[tile] (no atomics).  Bound by memory: a
+// counts word in and an omega out per cell and type.  NT > 0 (1 to 4 types,
+// buffers on 16-byte boundaries, n_cells a multiple of 4): 16-byte loads and
+// stores, the type count and the coefficients known as operands; NT = 0: any
+// types and alignment, a cell at a time.  The tile is the smallest of 1,024, 2,048
+// and 4,096 cells that the partials' array covers, so that 2.1M cells are 2,048
+// blocks and every thread has its loads of all types in flight at once.  Two types
+// on 2,097,152 cells (33.5 MB): 26.6 us with a cell at a time and tiles of 4,096,
+// 6.6 us so, k_sum_partials included; 4,096 cells 12.7 and 3.0 us.
+template <int NT>
 __global__ void __launch_bounds__(256) k_field_noalloc(const uint32_t* __restrict__ counts, float* __restrict__ omega,
-                                                        FieldParams p, double* __restrict__ partials) {
-    __shared__ double s_ef[32];
-    __shared__ float cf[kMaxTypes * kMaxTypes];
-    const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < kMaxTypes * kMaxTypes; i += T) cf[i] = p.cf[i];
-    __syncthreads();
-    const int64_t c0 = (int64_t)blockIdx.x * kNoAllocTileCells;
-    const int64_t c1 = min(c0 + (int64_t)kNoAllocTileCells, p.n_cells);
+                                                        const __grid_constant__ FieldParams p, int tile_cells,
+                                                        double* __restrict__ partials) {
+    __shared__ double s_ef[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t c0 = (int64_t)blockIdx.x * tile_cells, c1 = min(c0 + (int64_t)tile_cells, p.n_cells);
     double ef = 0.0;
     float wmax = -INFINITY, wmin = INFINITY;  // not used: the caller's omega has no span slot
-    for (int64_t cell = c0 + tid; cell < c1; cell += T)
-        ef += field_cell<0, false>(p.n_types, cell, p.n_cells, p.scale, p.lit != 0, true, false, counts, omega, cf,
-                                   nullptr, wmax, wmin);
+    if constexpr (NT > 0) {
+        for (int64_t cell = c0 + 4 * tid; cell < c1; cell += 1024)
+            ef += field_cells4<NT, false>(cell, p.n_cells, p.scale, p.lit != 0, true, counts, omega, p.cf, nullptr, wmax, wmin);
+    } else {
+        for (int64_t cell = c0 + tid; cell < c1; cell += 256)
+            ef += field_cell<0, false>(p.n_types, cell, p.n_cells, p.scale, p.lit != 0, true, false, counts, omega, p.cf,
+                                       nullptr, wmax, wmin);
+    }
     ef = warp_sum(ef);
     if (lane == 0) s_ef[warp] = ef;
     __syncthreads();
     if (tid == 0) {
         double e = 0.0;
-        for (int w = 0; w < (T + 31) / 32; ++w) e += s_ef[w];
+        for (int w = 0; w < 8; ++w) e += s_ef[w];
         partials[blockIdx.x] = e;
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // k_sum_partials may be set up
 }
 
 // Sum of the tile partials in a fixed order (one block).
+// Launched as the field kernel's programmatic dependent: it waits here for that
+// kernel's end, so only its own start overlaps.
 __global__ void __launch_bounds__(256) k_sum_partials(const double* __restrict__ partials, int n,
                                                        double* __restrict__ out) {
-    __shared__ double s[256];
+    __shared__ double s_e[8];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     double e = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) e += partials[i];
-    s[threadIdx.x] = e;
+    for (int i = threadIdx.x; i < n; i += 256) e += __ldcg(partials + i);
+    e = warp_sum(e);
+    if ((threadIdx.x & 31) == 0) s_e[threadIdx.x >> 5] = e;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) e += s_e[w];
+        *out = e;
     }
-    if (threadIdx.x == 0) *out = s[0];
 }
 
 // The id of the calling thread's current CUDA context (0 when none is current
@@ -1413,11 +1428,30 @@ extern "C" scmf_status scmf_update_omega_noalloc(const uint32_t* d_counts, float
     p.n_types = n_types;
     p.lit = hamiltonian == SCMF_HAM_LITERAL;
     field_coefficients(n_types, xn, reference_nbeads, hamiltonian, p.cf);
-    const int tiles = (int)((n_cells + kNoAllocTileCells - 1) / kNoAllocTileCells);
+    int tile = 1024;
+    while (tile < kNoAllocTileCells && n_cells > (int64_t)kNoAllocMaxTiles * tile) tile *= 2;
+    const int tiles = (int)((n_cells + tile - 1) / tile);
+    const bool vec = n_types <= 4 && n_cells % 4 == 0 && (((uintptr_t)d_counts | (uintptr_t)d_omega) & 15) == 0;
     cudaStream_t st = (cudaStream_t)stream;
-    k_field_noalloc<<<tiles, 256, 0, st>>>(d_counts, d_omega, p, scratch);
-    k_sum_partials<<<1, 256, 0, st>>>(scratch, tiles, d_energy);
+    const auto k = !vec           ? k_field_noalloc<0>
+                   : n_types == 1 ? k_field_noalloc<1>
+                   : n_types == 2 ? k_field_noalloc<2>
+                   : n_types == 3 ? k_field_noalloc<3>
+                                  : k_field_noalloc<4>;
+    k<<<tiles, 256, 0, st>>>(d_counts, d_omega, p, tile, scratch);
     e = cudaGetLastError();
+    if (e == cudaSuccess) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, k_sum_partials, (const double*)scratch, tiles, d_energy);
+    }
     if (e != cudaSuccess) return fail(SCMF_E_CUDA, "launch: %s", cudaGetErrorString(e));
     return SCMF_OK;
 }

@@ -363,13 +363,13 @@ void DevPlan::release() {
 // each (SweepArch::per).  Every warp of the GPU gets the same number of tiles, of
 // sizes up to what its buffer holds and no smaller than a row of 32 bead pairs.
 // Empty for a plan that the kernel does not take.
-static std::vector<SweepArch> tile_ranges(const Plan& p, int* warp_beads) {
+static std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     std::vector<SweepArch> out;
-    if (!p.linear || p.chains.empty() || p.max_length > kSweepBeadsLong || !p.cells32) return out;
-    const bool longer = p.max_length > kSweepBeads;
-    const int cap = longer ? kSweepBeadsLong : kSweepBeads;
-    *warp_beads = cap;
-    const int64_t warps = (int64_t)sm_count() * (longer ? kSweepWarpsLong : kSweepWarps);
+    if (!p.linear || p.chains.empty() || p.max_length > kSweepForms[kFormLong].beads || !p.cells32) return out;
+    *form = p.screened ? kFormScreened : kFormUnscreened;
+    if (p.max_length > kSweepForms[*form].beads) *form = kFormLong;
+    const int cap = kSweepForms[*form].beads;
+    const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
     int64_t beads = 0;
     int most = cap;  // what a tile of every architecture can reach
     for (const auto& c : p.chains) {
@@ -414,8 +414,8 @@ static std::vector<WarpTile> tile_list(const Plan& p, const std::vector<SweepArc
 
 // The tables of k_run as one buffer, its pointers still offsets: field tiles of a
 // warp each, so that the warps of the launch share the cells evenly.
-static std::vector<char> run_tables(const Plan& p, int n_warp, int warp_beads, RunArgs* run) {
-    const int sms = sm_count(), most = warp_beads > kSweepBeads ? kSweepWarpsLong : kSweepWarps;
+static std::vector<char> run_tables(const Plan& p, int n_warp, int form, RunArgs* run) {
+    const int sms = sm_count(), most = kSweepForms[form].warps;
     const int grid = std::min(n_warp, sms), warps = grid * std::min(most, (n_warp + grid - 1) / grid);  // as launched
     int64_t cells = 0;
     for (const auto& c : p.cells) cells += c.second;
@@ -465,8 +465,8 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     one_seed_hi = p.one_seed_hi && !p.close.empty();
     seed = p.seed;
     n_sys = (int)p.close.size();
-    warp_beads = 0;
-    const std::vector<SweepArch> ranges = tile_ranges(p, &warp_beads);
+    form = kFormScreened;
+    const std::vector<SweepArch> ranges = tile_ranges(p, &form);
     n_warp = tiles_of(ranges);
     one = n_sys == 1 && ranges.size() <= kSweepMaxArch;
     std::vector<WarpTile> wt;
@@ -493,9 +493,8 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     CK(cudaMemcpyAsync(d_field, p.field.data(), p.field.size() * sizeof(FieldTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_close, p.close.data(), p.close.size() * sizeof(SysClose), cudaMemcpyHostToDevice, st));
     std::vector<char> run_image;
-    const bool longer = warp_beads > kSweepBeads;
-    if (n_warp > 0 && n_warp <= sm_count() * (longer ? kSweepWarpsLong : kSweepWarps)) {  // a tile a warp
-        run_image = run_tables(p, n_warp, warp_beads, &run);
+    if (n_warp > 0 && n_warp <= sm_count() * kSweepForms[form].warps) {  // a tile a warp
+        run_image = run_tables(p, n_warp, form, &run);
         if ((rc = dev_alloc(&d_run, run_image.size(), st))) return rc;
         CK(cudaMemcpyAsync(d_run, run_image.data(), run_image.size(), cudaMemcpyHostToDevice, st));
         const auto at = [&](const void* offset) { return (char*)d_run + (size_t)offset; };
@@ -518,7 +517,7 @@ LaunchShape DevPlan::move_shape() const {
     sh.keys = philox_schedule((uint32_t)seed, (uint32_t)(seed >> 32));
     sh.warp_tiles = d_warp;
     sh.n_warp_tiles = n_warp;
-    sh.warp_beads = warp_beads;
+    sh.form = form;
     sh.one = one ? 1 : 0;
     sh.system = system;
     sh.n_arch = one ? n_arch : 0;
@@ -612,6 +611,7 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     p->cells32 = p->cells32 && n_cells * spec.n_types < (1ll << 31);
     p->position_bytes += (size_t)n_beads * 12;
     p->cells.push_back({d_sys, n_cells});
+    p->screened = p->screened || sweep.screen.on;
     if (p->close.empty()) {
         p->seed = spec.p.seed;
         p->sweep = sweep;

@@ -70,6 +70,7 @@ struct Plan {
     SweepSys sweep{};           // of the first system
     bool linear = true;
     bool cells32 = true;  // cells times types below 2^31 in every system
+    bool screened = false;  // some system's moves are screened
     // the chains of every architecture, for the warp tiles of k_sweep_warp
     struct Chains {
         SysDev* sys;
@@ -103,7 +104,7 @@ struct DevPlan {
     double* d_ef = nullptr;      // field energy per field tile
     double* d_eb = nullptr;      // bond energy per move tile
     int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;
-    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0, warp_beads = 0;
+    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0, form = 0;
     bool one_seed = false;     // every system of the plan has `seed`: move launches take its key schedule
     bool one_seed_hi = false;  // they share its upper 32 bits: the second key word's schedule
     uint64_t seed = 0;

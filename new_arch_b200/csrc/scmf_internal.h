@@ -288,9 +288,10 @@ struct LaunchShape {
     int keyed;
     PhiloxKeys keys;
     // every architecture of the launch is a linear chain that fits a warp's
-    // tile: the tiles of k_sweep_warp and the beads that a tile may hold
+    // tile: the tiles of k_sweep_warp
     const WarpTile* warp_tiles;
-    int n_warp_tiles, warp_beads;
+    int n_warp_tiles;
+    int form;           // SweepFormId
     int one;            // the launch has one system: `system`, with the constants `sweep` and n_arch tile ranges
     int once;           // the positions are more than L2 holds
     SysDev* system;
@@ -326,14 +327,20 @@ struct SweepArgs {
     SweepArch arch[kSweepMaxArch];
 };
 
-// Warps of a k_sweep_warp CTA (one CTA per SM) and the beads of a warp's tile
-// that shared memory then leaves room for; half as many warps, and longer tiles,
-// where a chain is longer than that.
+// Forms of the move kernels of linear chains: the warps of a CTA (one CTA per SM)
+// and the beads of a warp's tile that shared memory then leaves room for.  Four
+// warps a scheduler keep the screen's pipes busy, and longer tiles fill the warps
+// of the resolve step better; half as many, with longer tiles still, where a chain
+// is longer than that.  Systems that are not screened have a form without the
+// screen's code, its table and the lists: 409,600 beads 13.1 us a sweep, 14.8 in
+// the screened form (and 13.9, 15.8, 17.7 with 12, 28 and 24 warps of an SM, the
+// last two short of registers).
+enum SweepFormId { kFormScreened = 0, kFormLong = 1, kFormUnscreened = 2 };
+struct SweepForm {
+    int warps, beads;
+};
+constexpr SweepForm kSweepForms[3] = {{16, 960}, {8, 1984}, {16, 960}};
 constexpr size_t kL2Bytes = 126u << 20;
-constexpr int kSweepWarps = 16;
-constexpr int kSweepWarpsLong = 8;
-constexpr int kSweepBeads = 960;
-constexpr int kSweepBeadsLong = 1984;
 constexpr float kScreenFromAc = 2.0f;  // A 4k from which the screen runs
 
 // Streaming multiprocessors of the current device (read once per device; 148

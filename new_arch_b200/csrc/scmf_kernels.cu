@@ -1024,15 +1024,20 @@ int launch_init_coords(SysDev* d_sys, const ArchDev* d_arch, int n_arch, int n_c
     return (int)cudaGetLastError();
 }
 
+template <bool ONE, int FORM, int KEYS>
+static cudaError_t opt_in_form() {
+    const auto opt_in = [](const void* f) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SweepLayout<FORM>::kBytes);
+    };
+    const cudaError_t e = opt_in((const void*)k_sweep_warp<ONE, FORM, KEYS>);
+    return e == cudaSuccess ? opt_in((const void*)k_run<ONE, FORM, KEYS>) : e;
+}
+
 template <bool ONE, int KEYS>
 static cudaError_t opt_in_warp() {
-    const auto opt_in = [](const void* f, int bytes) {
-        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    };
-    cudaError_t e = opt_in((const void*)k_sweep_warp<ONE, false, KEYS>, SweepLayout<false>::kBytes);
-    if (e == cudaSuccess) e = opt_in((const void*)k_sweep_warp<ONE, true, KEYS>, SweepLayout<true>::kBytes);
-    if (e == cudaSuccess) e = opt_in((const void*)k_run<ONE, false, KEYS>, SweepLayout<false>::kBytes);
-    if (e == cudaSuccess) e = opt_in((const void*)k_run<ONE, true, KEYS>, SweepLayout<true>::kBytes);
+    cudaError_t e = opt_in_form<ONE, kFormScreened, KEYS>();
+    if (e == cudaSuccess) e = opt_in_form<ONE, kFormLong, KEYS>();
+    if (e == cudaSuccess) e = opt_in_form<ONE, kFormUnscreened, KEYS>();
     return e;
 }
 
@@ -1079,14 +1084,14 @@ static void launch_general(const MoveTile* tiles, int n_tiles, int blocks, int m
 }
 
 // The launch of a plan's warp tiles: k_sweep_warp, or k_run when `run` is given.
-template <bool ONE, bool LONG, int KEYS>
-static cudaError_t launch_warp(const SweepArgs& a, const RunArgs* run, cudaStream_t st) {
-    using Lay = SweepLayout<LONG>;
+template <bool ONE, int FORM, int KEYS>
+static cudaError_t launch_form(const SweepArgs& a, const RunArgs* run, cudaStream_t st) {
+    using Lay = SweepLayout<FORM>;
     const int sms = sm_count(), grid = a.n_tiles < sms ? a.n_tiles : sms;
     const int per_sm = (a.n_tiles + grid - 1) / grid, nw = per_sm < Lay::kWarps ? per_sm : Lay::kWarps;
-    const int smem = kSweepTabBytes + nw * (int)sizeof(typename Lay::Warp) + kSlack;
+    const int smem = Lay::kTabBytes + nw * (int)sizeof(typename Lay::Warp) + kSlack;
     if (!run) {
-        k_sweep_warp<ONE, LONG, KEYS><<<grid, 32 * nw, smem, st>>>(a);
+        k_sweep_warp<ONE, FORM, KEYS><<<grid, 32 * nw, smem, st>>>(a);
         return cudaGetLastError();
     }
     cudaLaunchAttribute at{};
@@ -1099,12 +1104,14 @@ static cudaError_t launch_warp(const SweepArgs& a, const RunArgs* run, cudaStrea
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_run<ONE, LONG, KEYS>, a, *run);
+    return cudaLaunchKernelEx(&cfg, k_run<ONE, FORM, KEYS>, a, *run);
 }
 
 template <bool ONE, int KEYS>
-static cudaError_t launch_warp(const SweepArgs& a, int beads, const RunArgs* run, cudaStream_t st) {
-    return beads > kSweepBeads ? launch_warp<ONE, true, KEYS>(a, run, st) : launch_warp<ONE, false, KEYS>(a, run, st);
+static cudaError_t launch_warp(const SweepArgs& a, int form, const RunArgs* run, cudaStream_t st) {
+    if (form == kFormLong) return launch_form<ONE, kFormLong, KEYS>(a, run, st);
+    if (form == kFormUnscreened) return launch_form<ONE, kFormUnscreened, KEYS>(a, run, st);
+    return launch_form<ONE, kFormScreened, KEYS>(a, run, st);
 }
 
 static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const RunArgs* run, cudaStream_t st) {
@@ -1118,9 +1125,9 @@ static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const Ru
     a.sys = sh.sweep;
     a.n_arch = sh.n_arch;
     for (int i = 0; i < sh.n_arch; ++i) a.arch[i] = sh.arch[i];
-    if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.warp_beads, run, st);
-    if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.warp_beads, run, st);
-    return launch_warp<false, kKeysNone>(a, sh.warp_beads, run, st);
+    if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.form, run, st);
+    if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.form, run, st);
+    return launch_warp<false, kKeysNone>(a, sh.form, run, st);
 }
 
 int launch_run(const LaunchShape& sh, const RunArgs& run, void* stream) {

@@ -122,14 +122,15 @@ constexpr int kTilePad = 12;  // 4 words before the tile, its offset of up to 3,
 // interleaved copies (lane l reads copy l mod 16: the half warps of an 8-byte
 // read then meet no bank twice).
 constexpr int kScreenTabAt = SCMF_NORMAL_SEGS * (int)sizeof(float4);
-constexpr int kSweepTabBytes = kScreenTabAt + SCMF_SCREEN_SEGS * kScreenCopies * (int)sizeof(float2);
+constexpr int sweep_tab_bytes(int form) {
+    return kScreenTabAt + (form == kFormUnscreened ? 0 : SCMF_SCREEN_SEGS * kScreenCopies * (int)sizeof(float2));
+}
 
-// A CTA's warps and what each has in shared memory.  LONG: for chains longer
-// than kSweepBeads.
-template <bool LONG>
+// A CTA's warps and what each has in shared memory, for each SweepFormId.
+template <int FORM>
 struct SweepLayout {
-    static constexpr int kWarps = LONG ? kSweepWarpsLong : kSweepWarps;
-    static constexpr int kBeads = LONG ? kSweepBeadsLong : kSweepBeads;
+    static constexpr int kWarps = kSweepForms[FORM].warps;
+    static constexpr int kBeads = kSweepForms[FORM].beads;
     static constexpr int kStride = kBeads + kTilePad;  // from x to y to z
     struct Warp {
         uint64_t full;         // barrier: the tile has arrived
@@ -137,12 +138,22 @@ struct SweepLayout {
         uint32_t moved[32];    // odd beads next to an even bead that moved: a bit for each row, a word for each lane
         uint16_t list[kListLen];
         SweepSys sys;          // of the tile's system, where a launch has several
-        FieldSys field;        // of the system of the warp's field tile (k_run)
+        // k_run, which has registers for one phase of a sweep at a time: the warp's
+        // tile and its architecture, the sweeps that its system has made and makes
+        // in all, and the system of the warp's field tile
+        struct {
+            WarpTile tile;
+            const uint8_t* types;
+            uint32_t rng_base, h_magic, base, stop;
+            int32_t rule, active;
+        } run;
+        FieldSys field;
         alignas(16) float pos[3 * kStride];
     };
-    static constexpr int kBytes = kSweepTabBytes + kWarps * (int)sizeof(Warp) + kSlack;
+    static constexpr int kTabBytes = sweep_tab_bytes(FORM);
+    static constexpr int kBytes = kTabBytes + kWarps * (int)sizeof(Warp) + kSlack;
     static_assert(kBeads <= 2048, "a row of 32 bead pairs is a bit of a lane's mask");
-    static_assert(kSweepTabBytes % 16 == 0 && sizeof(Warp) % 16 == 0 && offsetof(Warp, pos) % 16 == 0 && kStride % 4 == 0,
+    static_assert(kTabBytes % 16 == 0 && sizeof(Warp) % 16 == 0 && offsetof(Warp, pos) % 16 == 0 && kStride % 4 == 0,
                   "16-byte copies");
     static_assert(kBytes <= 227 * 1024, "shared memory of an SM");
 };
@@ -262,10 +273,10 @@ __device__ __forceinline__ uint32_t row_mask(int items) {
 // 32 i + lane may be accepted.  X is the first bead's x.
 //   KIND 0: even L, h divides 32 (a lane's place in its chain never changes); 1:
 //   even L; 2: odd L, or a tile whose first bead is at an odd offset.
-template <int KIND, bool LONG, int KEYS>
+template <int KIND, int FORM, int KEYS>
 __device__ __forceinline__ void screen_tile(const SweepConsts& s, const float* X, uint32_t rng0, int n_chains,
                                             const PhiloxKeys& keys, uint32_t tab, uint32_t& even_out, uint32_t& odd_out) {
-    using Lay = SweepLayout<LONG>;
+    using Lay = SweepLayout<FORM>;
     const int lane = threadIdx.x & 31;
     const int L = s.L, h = s.h, items = n_chains * h;
     uint32_t bit = 1u, even = 0u, odd = 0u;
@@ -356,19 +367,20 @@ struct TileRef {
     const uint8_t* types;
     float span;
     bool move_counts;
+    bool write;              // moved beads go to global memory too (k_run: after the last sweep)
 };
 
 // The exact trials of the beads of parity par of N pairs a lane (pair[i], where
-// act[i]), with trial_f's expressions.  A move updates the tile and the positions
-// in global memory, moves a count if it leaves its cell, and marks the odd beads
+// act[i]), with trial_f's expressions.  A move updates the tile and, where asked,
+// the positions in global memory, moves a count if it leaves its cell, and marks the odd beads
 // next to it, whose screen saw the old position.  Returns the lane's moves.  The
 // N trials of a lane are independent: without branches between them their chains
 // (Philox, table, omega) run side by side.
-template <int N, bool LONG, int KEYS>
+template <int N, int FORM, int KEYS>
 __device__ __forceinline__ unsigned exact_trials(const SweepSys& c, const SweepConsts& s, const TileRef& t, uint32_t* moved,
                                                  const PhiloxKeys& keys, const float4* ntab, int par, const int (&pair)[N],
                                                  bool (&act)[N]) {
-    constexpr int kStride = SweepLayout<LONG>::kStride;
+    constexpr int kStride = SweepLayout<FORM>::kStride;
     int p[N], b[N], c_old[N], c_new[N];
     uint32_t typ[N];
     float x[N], y[N], z[N], dx[N], dy[N], dz[N], deb[N], u[N], lo[N];
@@ -427,12 +439,17 @@ __device__ __forceinline__ unsigned exact_trials(const SweepSys& c, const SweepC
             if (!(may[i] && (dE < 0.0f || (-dE > lo[i] && log_f(u[i]) < -dE)))) continue;
             float* const Q = t.X + p[i];
             const int64_t g = t.bead0 + p[i];
-            Q[0] = c.x[g] = __fadd_rn(x[i], dx[i]);
-            Q[kStride] = c.y[g] = __fadd_rn(y[i], dy[i]);
-            Q[2 * kStride] = c.z[g] = __fadd_rn(z[i], dz[i]);
+            Q[0] = __fadd_rn(x[i], dx[i]);
+            Q[kStride] = __fadd_rn(y[i], dy[i]);
+            Q[2 * kStride] = __fadd_rn(z[i], dz[i]);
+            if (t.write) {
+                c.x[g] = Q[0];
+                c.y[g] = Q[kStride];
+                c.z[g] = Q[2 * kStride];
+            }
             if (t.move_counts && c_new[i] != c_old[i]) count_move(c.counts, c.count16 != 0, typ[i], c_old[i], c_new[i]);
             ++nacc;
-            if (par == 0) {
+            if (FORM != kFormUnscreened && par == 0) {
                 const int j = pair[i];
                 if (b[i] > 0) atomicOr(moved + ((j - 1) & 31), 1u << ((j - 1) >> 5));
                 if (b[i] + 1 < s.L) atomicOr(moved + (j & 31), 1u << (j >> 5));
@@ -444,8 +461,8 @@ __device__ __forceinline__ unsigned exact_trials(const SweepSys& c, const SweepC
 
 // Makes the trials of a tile that the masks name (bit i of even / odd: the even
 // / odd bead of pair 32 i + lane).  Returns the lane's accepted moves.
-template <bool LONG, int KEYS>
-__device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<LONG>::Warp* wp, const SweepSys& c, const SweepConsts& s,
+template <int FORM, int KEYS>
+__device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<FORM>::Warp* wp, const SweepSys& c, const SweepConsts& s,
                                                  const TileRef& t, const PhiloxKeys& keys, const float4* ntab, uint32_t even,
                                                  uint32_t odd) {
     const int lane = threadIdx.x & 31;
@@ -453,9 +470,21 @@ __device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<LONG>::War
     uint32_t mask = even;
 #pragma unroll 1
     for (int par = 0; par < 2; ++par) {
-        if (par) {  // the odd neighbours of the even beads that moved
+        if (FORM == kFormUnscreened) {
+            mask = par ? odd : even;
+        } else if (par) {  // the odd neighbours of the even beads that moved
             mask = odd | wp->moved[lane];
             wp->moved[lane] = 0u;
+        }
+        if (FORM == kFormUnscreened) {  // every trial, row by row
+#pragma unroll 1
+            for (int r = 0; 32 * r < t.items; ++r) {
+                const int pair[1] = {min(32 * r + lane, t.items - 1)};
+                bool act[1] = {((mask >> r) & 1u) != 0u};
+                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+            }
+            __syncwarp();
+            continue;
         }
         const int own = __popc(mask);
         int before = own;
@@ -473,14 +502,14 @@ __device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<LONG>::War
             for (int r = lane; r < total; r += 32) {
                 const int pair[1] = {(int)wp->list[r]};
                 bool act[1] = {true};
-                nacc += exact_trials<1, LONG, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
             }
         } else {  // row by row
 #pragma unroll 1
             for (int r = 0; 32 * r < t.items; ++r) {
                 const int pair[1] = {min(32 * r + lane, t.items - 1)};
                 bool act[1] = {((mask >> r) & 1u) != 0u};
-                nacc += exact_trials<1, LONG, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
             }
         }
         __syncwarp();
@@ -491,9 +520,9 @@ __device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<LONG>::War
 // A warp of a move kernel: its tile, its shared memory and the constants of the
 // system and architecture it is at.  ONE: the launch has one system, whose
 // constants are parameters (instruction operands).
-template <bool ONE, bool LONG, int KEYS>
+template <bool ONE, int FORM, int KEYS>
 struct Mover {
-    using Lay = SweepLayout<LONG>;
+    using Lay = SweepLayout<FORM>;
     const SweepArgs& a;
     typename Lay::Warp* const wp;
     const float4* const ntab;
@@ -508,7 +537,7 @@ struct Mover {
 
     __device__ __forceinline__ Mover(const SweepArgs& args, unsigned char* smem)
         : a(args),
-          wp(reinterpret_cast<typename Lay::Warp*>(smem + kSweepTabBytes) + (threadIdx.x >> 5)),
+          wp(reinterpret_cast<typename Lay::Warp*>(smem + Lay::kTabBytes) + (threadIdx.x >> 5)),
           ntab(reinterpret_cast<const float4*>(smem)),
           lane(threadIdx.x & 31) {}
     __device__ __forceinline__ const SweepSys& sys() const { return ONE ? a.sys : wp->sys; }
@@ -538,7 +567,7 @@ struct Mover {
         float4* tab = reinterpret_cast<float4*>(smem);
         for (int i = threadIdx.x; i < SCMF_NORMAL_SEGS; i += blockDim.x) tab[i] = __ldg(normal_table() + i);
         float2* screen = reinterpret_cast<float2*>(smem + kScreenTabAt);
-        if (!ONE || a.sys.screen.on)
+        if (FORM != kFormUnscreened)
             for (int i = threadIdx.x; i < SCMF_SCREEN_SEGS * kScreenCopies; i += blockDim.x)
                 screen[i] = __ldg(screen_table() + i / kScreenCopies);
         __syncthreads();
@@ -553,15 +582,20 @@ struct Mover {
             for (int i = lane; i < (int)(sizeof(SweepSys) / 4); i += 32) reinterpret_cast<uint32_t*>(&wp->sys)[i] = src[i];
             __syncwarp();
         }
-        const SweepSys& c = sys();
         S = t.sys;
         A = t.arch;
         types = A->types;
         rng_base = (uint32_t)A->rng_base;
+        set(A->length, A->tpc_magic, done, active, omega_span);
+    }
+
+    // The constants of a sweep of chains of L beads.
+    __device__ __forceinline__ void set(int L, uint32_t h_magic, uint32_t done, bool active, float omega_span) {
+        const SweepSys& c = sys();
         span = omega_span;
-        s.L = A->length;
-        s.h = (s.L + 1) >> 1;
-        s.h_magic = A->tpc_magic;
+        s.L = L;
+        s.h = (L + 1) >> 1;
+        s.h_magic = h_magic;
         s.step = done + 1u;
         s.k0 = c.seed_lo;
         s.k1 = c.seed_hi;
@@ -573,20 +607,10 @@ struct Mover {
         s.add = c.screen.add;
         s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
         s.u1 = __fmul_rn(c.screen.u, -0x1.62e7p-1f);  // a little over ln 2
-        mode = !active ? 0 : c.screen.on && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
+        mode = !active ? 0 : FORM != kFormUnscreened && c.screen.on && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
         const int k = lane & (s.h - 1);
         s.pc = pair_consts(s, k == 0, false, k == s.h - 1);
         s.head = pair_head<KEYS>(2u * (uint32_t)k, s.step, s.k0, a.keys);
-    }
-
-    // The same tile's next sweep.
-    __device__ __forceinline__ void next_sweep(uint32_t done, bool active, float omega_span) {
-        const SweepSys& c = sys();
-        span = omega_span;
-        s.step = done + 1u;
-        s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
-        mode = active ? mode : 0;
-        s.head = pair_head<KEYS>(2u * (uint32_t)(lane & (s.h - 1)), s.step, s.k0, a.keys);
     }
 
     // Waits for the tile asked for; false (and the error word) if it does not come.
@@ -598,23 +622,23 @@ struct Mover {
     }
 
     // One sweep of the tile in the buffer.  Returns the lane's accepted moves.
-    __device__ __forceinline__ unsigned move(const WarpTile& t) {
+    __device__ __forceinline__ unsigned move(const WarpTile& t, bool write) {
         const int off = (int)(t.bead0 & 3), items = t.n_chains * s.h;
         const uint32_t rng0 = rng_base + t.chain, tab = screen_lane();
         float* X = wp->pos + 4 + off;
         uint32_t even = 0u, odd = 0u;
-        if (mode == 2) {
+        if (FORM != kFormUnscreened && mode == 2) {
             if ((s.L | off) & 1)
-                screen_tile<2, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+                screen_tile<2, FORM, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
             else if (32 % s.h)
-                screen_tile<1, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+                screen_tile<1, FORM, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
             else
-                screen_tile<0, LONG, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
+                screen_tile<0, FORM, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
         } else if (mode == 1) {
             even = odd = row_mask(items);
         }
-        const TileRef ref{X, t.bead0, rng0, items, types, span, a.move_counts != 0};
-        return resolve_tile<LONG, KEYS>(wp, sys(), s, ref, a.keys, ntab, even, odd);
+        const TileRef ref{X, t.bead0, rng0, items, types, span, a.move_counts != 0, write};
+        return resolve_tile<FORM, KEYS>(wp, sys(), s, ref, a.keys, ntab, even, odd);
     }
 };
 
@@ -648,10 +672,10 @@ __device__ __forceinline__ WarpTile tile_at(const SweepArgs& a, int i) {
 // with a quarter, a half, three quarters or all of its first one (by its place
 // among the four warps of its SM sub-partition) and ends with the rest: 0.322 ->
 // 0.313 ms on the large system.
-template <bool ONE, bool LONG, int KEYS>
-__global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1) k_sweep_warp(const __grid_constant__ SweepArgs a) {
+template <bool ONE, int FORM, int KEYS>
+__global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_warp(const __grid_constant__ SweepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Mover<ONE, LONG, KEYS> m(a, smem_raw);
+    Mover<ONE, FORM, KEYS> m(a, smem_raw);
     // consecutive tiles go to different SMs, so that few tiles spread over all of them
     const int warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
     const int first = warp * (int)gridDim.x + (int)blockIdx.x, stride = nwarps * (int)gridDim.x;
@@ -677,7 +701,7 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1) k_sweep_war
         }
         if (t.arch != m.A) m.turn_to(t, t.sys->step, t.sys->step < t.sys->stop_step, t.sys->omega_span);
         if (!m.arrived()) return;
-        unsigned nacc = m.move(t);
+        unsigned nacc = m.move(t, true);
         fence_async();  // this lane's reads and writes of the buffer, before the next copies land
         __syncwarp();
         if (q + 1 < parts && m.lane == 0) m.load(next);
@@ -764,14 +788,14 @@ __device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r,
         f = warp_sum(f);
         if (lane == 0) {
             s_acc[warp] = all;
-            s_acc[16 + warp] = last;
+            s_acc[32 + warp] = last;
             s_ef[warp] = f;
         }
         __syncthreads();
         if (tid == 0) {
             for (int w = 1; w < nwarps; ++w) {
                 all += s_acc[w];
-                last += s_acc[16 + w];
+                last += s_acc[32 + w];
                 f += s_ef[w];
             }
             const uint32_t step = base + made;
@@ -821,42 +845,51 @@ __device__ __forceinline__ double field_tile(const FieldSys& f, int64_t cell0, i
 // from a graph: 32,000 beads 8.8 us against 18.6 us; 409,600 beads, unscreened,
 // 14.8 against 22.7 us; 2.0M beads in chains of 33 20.2 against 28.9 us.  (Before
 // the kernels of this file: 14.6, 20.7 and 55.4 us.)  A barrier takes 2 us.
-template <bool ONE, bool LONG, int KEYS>
-__global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
+template <bool ONE, int FORM, int KEYS>
+__global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     k_run(const __grid_constant__ SweepArgs a, const __grid_constant__ RunArgs r) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_ok;
     __shared__ uint32_t s_keys[2];
-    __shared__ unsigned long long s_acc[32];
-    __shared__ double s_ef[16];
-    Mover<ONE, LONG, KEYS> m(a, smem_raw);
-    const int lane = m.lane, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int first = warp * (int)gridDim.x + (int)blockIdx.x, stride = nwarps * (int)gridDim.x;
+    __shared__ unsigned long long s_acc[64];
+    __shared__ double s_ef[32];
+    auto* const wp = reinterpret_cast<typename SweepLayout<FORM>::Warp*>(smem_raw + SweepLayout<FORM>::kTabBytes) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int first = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x, stride = (int)(blockDim.x >> 5) * (int)gridDim.x;
     const bool any = first < a.n_tiles;
     GridBarrier barrier(r.barrier);
-    WarpTile t{};
-    if (any) t = tile_at<ONE>(a, first);
     if (threadIdx.x < 2) s_keys[threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
     for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {  // the slot of the launch's first field step
         SysDev* S = r.systems[i].sys;
         if (threadIdx.x < 2) S->om_keys[(S->step + 1u) % 3u][threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
     }
-    m.start(smem_raw, t, any);
-    uint32_t base = 0u, stop = 0u;  // sweeps that the tile's system has made, and makes in all
-    int rule = 0;
-    if (any) {
-        base = t.sys->step;
-        stop = t.sys->stop_step;
-        rule = t.sys->field_rule;
-        m.turn_to(t, base, base < stop, t.sys->omega_span);
-        if (!m.arrived()) m.mode = 0;
+    {
+        Mover<ONE, FORM, KEYS> m(a, smem_raw);
+        WarpTile t{};
+        if (any) t = tile_at<ONE>(a, first);
+        m.start(smem_raw, t, any);
+        if (any) {
+            const uint32_t base = t.sys->step, stop = t.sys->stop_step;
+            m.turn_to(t, base, base < stop, 0.0f);
+            const bool here = m.arrived();
+            if (lane == 0) {
+                wp->run.tile = t;
+                wp->run.types = m.types;
+                wp->run.rng_base = m.rng_base;
+                wp->run.h_magic = m.s.h_magic;
+                wp->run.base = base;
+                wp->run.stop = stop;
+                wp->run.rule = t.sys->field_rule;
+                wp->run.active = here;
+            }
+            __syncwarp();
+        }
     }
     // the warp's field tile (its first, where it has several) and that one's system
-    FieldSys* const fs = &m.wp->field;
-    FieldTile ft{};
-    if (first < r.n_field) ft = r.field[first];
+    FieldSys* const fs = &wp->field;
     uint32_t f_base = 0u, f_stop = 0u;
-    const auto at_system = [&](const SysDev* S) {
+    SysDev* f_sys = nullptr;
+    const auto at_system = [&](SysDev* S) {
         __syncwarp();
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&S->field);
         for (int i = lane; i < (int)(sizeof(FieldSys) / 4); i += 32) reinterpret_cast<uint32_t*>(fs)[i] = src[i];
@@ -866,17 +899,29 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
         }
         f_base = S->step;
         f_stop = S->stop_step;
+        f_sys = S;
         __syncwarp();
     };
-    if (first < r.n_field) at_system(ft.sys);
+    int64_t cell0 = 0;
+    int n_cells = 0;
+    if (first < r.n_field) {
+        at_system(r.field[first].sys);
+        cell0 = r.field[first].cell0;
+        n_cells = r.field[first].n_cells;
+    }
     unsigned acc_all = 0, acc_last = 0;  // of all the launch's sweeps, of the system's last
 #pragma unroll 1
     for (int sweep = 0; sweep < r.n_sweeps; ++sweep) {
-        if (any && m.mode) {
-            const uint32_t done = base + (uint32_t)sweep;
-            if (sweep) m.next_sweep(done, done < stop, span_after(m.S, rule, done, base));
-            if (m.mode) {
-                acc_last = m.move(t);
+        if (any && wp->run.active) {
+            const uint32_t base = wp->run.base, done = base + (uint32_t)sweep;
+            if (done < wp->run.stop) {
+                Mover<ONE, FORM, KEYS> m(a, smem_raw);
+                const WarpTile& t = wp->run.tile;
+                m.S = t.sys;
+                m.types = wp->run.types;
+                m.rng_base = wp->run.rng_base;
+                m.set(t.length, wp->run.h_magic, done, true, span_after(t.sys, wp->run.rule, done, base));
+                acc_last = m.move(t, false);
                 acc_all += acc_last;
             }
         }
@@ -884,10 +929,10 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
         float wmax = -INFINITY, wmin = INFINITY;
 #pragma unroll 1
         for (int fi = first; fi < r.n_field; fi += stride) {
-            if (fi != first || r.n_field > stride) {
-                const SysDev* before = ft.sys;
-                ft = r.field[fi];
-                if (ft.sys != before) at_system(ft.sys);
+            if (r.n_field > stride) {  // several field tiles a warp
+                if (r.field[fi].sys != f_sys) at_system(r.field[fi].sys);
+                cell0 = r.field[fi].cell0;
+                n_cells = r.field[fi].n_cells;
             }
             const uint32_t step = f_base + (uint32_t)sweep + 1u;
             if (step > f_stop) continue;
@@ -898,7 +943,7 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
                 wmax = -INFINITY;
                 wmin = INFINITY;
             }
-            double ef = field_tile(*fs, ft.cell0, ft.n_cells, upd, sample, wmax, wmin);
+            double ef = field_tile(*fs, cell0, n_cells, upd, sample, wmax, wmin);
             if (last) {
                 ef = warp_sum(ef);
                 if (lane == 0) r.ef_part[fi] = ef;
@@ -906,7 +951,7 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
             if (!upd)
                 wmax = -INFINITY, wmin = INFINITY;
             else if (!ONE)
-                fold_span(ft.sys->om_keys[step % 3u], wmax, wmin);
+                fold_span(f_sys->om_keys[step % 3u], wmax, wmin);
         }
         if (ONE) {
             fold_span(s_keys, wmax, wmin);
@@ -914,16 +959,16 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
         }
         if (threadIdx.x == 0) {
             if (ONE) {
-                const uint32_t step = base + (uint32_t)sweep + 1u;  // block-wide: thread 0's warp has a tile
+                const uint32_t step = wp->run.base + (uint32_t)sweep + 1u;  // thread 0's warp has a tile
                 if (s_keys[0]) {
-                    atomicMax(&m.S->om_keys[step % 3u][0], s_keys[0]);
-                    atomicMin(&m.S->om_keys[step % 3u][1], s_keys[1]);
+                    atomicMax(&a.system->om_keys[step % 3u][0], s_keys[0]);
+                    atomicMin(&a.system->om_keys[step % 3u][1], s_keys[1]);
                 }
                 s_keys[0] = 0u;
                 s_keys[1] = 0xFFFFFFFFu;
                 if (blockIdx.x == 0) {  // the slot of the next field step
-                    m.S->om_keys[(step + 1u) % 3u][0] = 0u;
-                    m.S->om_keys[(step + 1u) % 3u][1] = 0xFFFFFFFFu;
+                    a.system->om_keys[(step + 1u) % 3u][0] = 0u;
+                    a.system->om_keys[(step + 1u) % 3u][1] = 0xFFFFFFFFu;
                 }
             } else {
                 for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {
@@ -937,11 +982,22 @@ __global__ void __launch_bounds__(SweepLayout<LONG>::kWarps * 32, 1)
         if (sweep + 1 == r.n_sweeps && any) {
             const unsigned all = warp_sum(acc_all), last = warp_sum(acc_last);
             if (lane == 0) {
-                if (all) atomicAdd(&m.S->slot_acc[first % kSlots], (unsigned long long)all);
-                if (last) atomicAdd(&m.S->slot_last[first % kSlots], (unsigned long long)last);
+                SysDev* S = wp->run.tile.sys;
+                if (all) atomicAdd(&S->slot_acc[first % kSlots], (unsigned long long)all);
+                if (last) atomicAdd(&S->slot_last[first % kSlots], (unsigned long long)last);
             }
         }
         if (!barrier.wait(&s_ok)) return;
+    }
+    if (any && wp->run.active) {  // the positions
+        const SweepSys& c = ONE ? a.sys : wp->sys;
+        const WarpTile& t = wp->run.tile;
+        const float* P = wp->pos + 4 + (int)(t.bead0 & 3);
+        for (int i = lane; i < t.n_beads; i += 32) {
+            c.x[t.bead0 + i] = P[i];
+            c.y[t.bead0 + i] = P[i + SweepLayout<FORM>::kStride];
+            c.z[t.bead0 + i] = P[i + 2 * SweepLayout<FORM>::kStride];
+        }
     }
     // the statistics of every system, in a fixed order
     for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) close_run(r.systems[i], r, s_acc, s_ef);

@@ -338,7 +338,9 @@ static scmf_status create_system(const scmf_spec* spec, bool is_shard, int shard
         return bail(rc);
     // architecture tables
     size_t blob = 0;
-    auto arch_bytes = [](int L) { return round_up((size_t)L * (sizeof(BeadInfo) + sizeof(uint16_t) + 1) + 16, 256); };
+    auto arch_bytes = [](int L) {
+        return round_up((size_t)L * (sizeof(GraphBead) + sizeof(BeadInfo) + sizeof(uint16_t) + 1) + 16, 256);
+    };
     for (const auto& a : s->archs) blob += arch_bytes(a.length);
     if ((rc = dalloc(&s->d_arch_blob, blob, &tot, st))) return bail(rc);
     s->device_bytes = tot;
@@ -346,9 +348,22 @@ static scmf_status create_system(const scmf_spec* spec, bool is_shard, int shard
     size_t off = 0;
     for (const auto& a : s->archs) {
         ArchDev d{};
-        std::memcpy(hblob.data() + off, a.beads.data(), a.length * sizeof(BeadInfo));
-        d.beads = (const BeadInfo*)((char*)s->d_arch_blob + off);
-        const size_t off2 = off + (size_t)a.length * sizeof(BeadInfo);
+        if (!a.linear && a.max_deg <= kGraphDeg) {
+            GraphBead* g = (GraphBead*)(hblob.data() + off);
+            for (const uint16_t bead : a.color_beads) {
+                const BeadInfo& bi = a.beads[bead];
+                g->bead = bead;
+                g->deg = bi.deg;
+                g->type = bi.type;
+                for (int k = 0; k < kGraphDeg; ++k) g->nbr[k] = k < bi.deg ? bi.nbr[k] : bead;
+                ++g;
+            }
+            d.graph = (const GraphBead*)((char*)s->d_arch_blob + off);
+        }
+        const size_t off1 = off + (size_t)a.length * sizeof(GraphBead);
+        std::memcpy(hblob.data() + off1, a.beads.data(), a.length * sizeof(BeadInfo));
+        d.beads = (const BeadInfo*)((char*)s->d_arch_blob + off1);
+        const size_t off2 = off1 + (size_t)a.length * sizeof(BeadInfo);
         std::memcpy(hblob.data() + off2, a.color_beads.data(), a.length * sizeof(uint16_t));
         d.color_beads = (const uint16_t*)((char*)s->d_arch_blob + off2);
         const size_t off3 = off2 + (size_t)a.length * sizeof(uint16_t);
@@ -357,10 +372,14 @@ static scmf_status create_system(const scmf_spec* spec, bool is_shard, int shard
         off += arch_bytes(a.length);
         d.length = a.length;
         d.n_colors = a.n_colors;
+        d.max_deg = a.max_deg;
         for (int c = 0; c <= a.n_colors; ++c) d.color_off[c] = a.color_off[c];
         for (int c = 0; c < a.n_colors; ++c) {
             const uint32_t nc = (uint32_t)(a.color_off[c + 1] - a.color_off[c]);
             d.color_magic[c] = magic_for(nc);
+            const uint32_t blocks = (nc + 63) / 64;
+            d.color_width[c] = (int32_t)((nc + blocks - 1) / blocks);
+            d.color_per[c] = 64 / d.color_width[c];
         }
         d.len_magic = magic_for((uint32_t)a.length);
         d.tpc_magic = magic_for((uint32_t)((a.length + 1) / 2));
@@ -972,7 +991,7 @@ scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
             }
         };
         if (b->plan.n_warp > 0) {
-            tried(b->plan.tune);  // linear chains: the move kernel sizes its own tiles
+            tried(b->plan.tune);  // the move kernel sizes its own tiles
         } else {
             for (int tb : {1024, 2048, 4096, 8192})
                 for (int th : {64, 128, 256})

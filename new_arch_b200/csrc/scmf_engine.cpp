@@ -193,7 +193,7 @@ size_t system_device_bytes(const scmf_spec& s) {
     for (const auto& a : s.archs) {
         beads += (int64_t)a.length * a.n_chains;
         chains += a.n_chains;
-        arch_bytes += round_up((size_t)a.length * (sizeof(BeadInfo) + 3) + 16, 256);
+        arch_bytes += round_up((size_t)a.length * (sizeof(BeadInfo) + 3 + sizeof(GraphBead)) + 16, 256);
     }
     const size_t cells = (size_t)s.nx * s.ny * s.nz * s.n_types;
     size_t b = 3 * round_up((size_t)(beads + 4) * 4, 256) + round_up((size_t)chains * 4, 256);
@@ -222,21 +222,28 @@ void field_coefficients(int n, const double* xn, int nref, int hamiltonian, floa
 // where proposals are small enough that most trials would pass: with x = A 4k,
 // 4k the c of an inner bead, |v|^2 has (x^2 + 1) / (2 x) times the mean of the
 // limit's |f|^2 term, so screened trials pass often below x of about 2.
+constexpr double kScreenEta = 0x1p-6, kScreenUnit = 0x1p30;
+static float rounded_up(double v) { return std::nextafterf((float)v, INFINITY); }
+
+// a and b for beads of g bonds; false where they are out of range.
+static bool screen_of(const SysDev& d, int g, float* a, float* b) {
+    const double K = (1.0 + kScreenEta) * (1.0 + 0x1p-10), A = d.A, R = d.R, c = d.cdeg[g];
+    const double bg = K / (c * c * R * R);
+    *a = (float)((A - 1.0 / c) / R * kScreenUnit);
+    *b = rounded_up(bg * kScreenUnit * kScreenUnit);
+    for (const double v : {A, R, c, (double)d.ac4deg[g], bg})
+        if (!(v > 1e-12 && v < 1e12)) return false;
+    return true;
+}
+
 static ScreenDev screen_constants(const SysDev& d) {
     ScreenDev s{};
-    const double eta = 0x1p-6, K = (1.0 + eta) * (1.0 + 0x1p-10), delta = SCMF_SCREEN_DELTA;
-    const double A = d.A, R = d.R, unit = 0x1p30;
+    const double delta = SCMF_SCREEN_DELTA, A = d.A;
     s.on = A > 0.0 && A * (double)d.cdeg[2] >= kScreenFromAc;
-    const auto up = [](double v) { return std::nextafterf((float)v, INFINITY); };
-    s.add = up((1.0 + 1.0 / eta) * 3.0 * delta * delta * unit * unit);
-    s.u = up(4.0 / A);
-    for (int g = 1; g <= 2; ++g) {
-        const double c = d.cdeg[g], a = (A - 1.0 / c) / R, b = K / (c * c * R * R);
-        for (const double v : {A, R, c, (double)d.ac4deg[g], b})
-            if (!(v > 1e-12 && v < 1e12)) s.on = 0;
-        s.a[g] = (float)(a * unit);
-        s.b[g] = up(b * unit * unit);
-    }
+    s.add = rounded_up((1.0 + 1.0 / kScreenEta) * 3.0 * delta * delta * kScreenUnit * kScreenUnit);
+    s.u = rounded_up(4.0 / A);
+    for (int g = 1; g <= 2; ++g)
+        if (!screen_of(d, g, &s.a[g], &s.b[g])) s.on = 0;
     return s;
 }
 
@@ -305,6 +312,12 @@ void fill_sweep_constants(SysDev* d) {
     w.seed_hi = d->seed_hi;
     w.count16 = d->count16;
     w.screen = screen_constants(*d);
+    d->by_deg[0] = make_float4(0.0f, INFINITY, 0.0f, 0.0f);  // no bond, nothing to screen by
+    for (int g = 1; g <= kGraphDeg; ++g) {
+        float a, b;
+        if (!screen_of(*d, g, &a, &b)) w.screen.on = 0;
+        d->by_deg[g] = make_float4(a, b, d->cdeg[g], d->ac4deg[g]);
+    }
     FieldSys& f = d->field;
     f.counts = d->counts[0];
     f.omega = d->omega;
@@ -365,9 +378,10 @@ void DevPlan::release() {
 // Empty for a plan that the kernel does not take.
 static std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     std::vector<SweepArch> out;
-    if (!p.linear || p.chains.empty() || p.max_length > kSweepForms[kFormLong].beads || !p.cells32) return out;
-    *form = p.screened ? kFormScreened : kFormUnscreened;
-    if (p.max_length > kSweepForms[*form].beads) *form = kFormLong;
+    if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return out;
+    *form = !p.linear ? kFormGraph : p.screened ? kFormScreened : kFormUnscreened;
+    if (p.linear && p.max_length > kSweepForms[*form].beads) *form = kFormLong;
+    if (p.max_length > kSweepForms[*form].beads) return out;
     const int cap = kSweepForms[*form].beads;
     const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
     int64_t beads = 0;

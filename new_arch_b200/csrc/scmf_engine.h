@@ -79,7 +79,7 @@ struct Plan {
     int max_deg = 0;
     size_t position_bytes = 0;  // of all systems
     SweepSys sweep{};           // of the first system
-    bool linear = true;
+    bool linear = true;   // every architecture is a linear chain
     bool cells32 = true;  // cells times types below 2^31 in every system
     bool screened = false;  // some system's moves are screened
     // the chains of every architecture, for the warp tiles of k_sweep_warp
@@ -111,7 +111,7 @@ struct DevPlan {
     int n_arch = 0;
     SweepArch arch[kSweepMaxArch] = {};
     bool once = false;           // the positions are more than L2 holds
-    WarpTile* d_warp = nullptr;  // tiles of k_sweep_warp (linear plans; see warp_tiles)
+    WarpTile* d_warp = nullptr;  // tiles of k_sweep_warp (see tile_ranges)
     double* d_ef = nullptr;      // field energy per field tile
     double* d_eb = nullptr;      // bond energy per move tile
     int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;

@@ -43,15 +43,30 @@ struct BeadInfo {
     uint16_t nbr[kMaxDeg];
 };
 
+// A bead of an architecture that is no linear chain, as the move kernel of warp
+// tiles reads it (in 16 bytes; the bonded beads in ascending order, the rest of
+// `nbr` the bead itself).
+constexpr int kGraphDeg = 6;
+struct alignas(16) GraphBead {
+    uint16_t bead;
+    uint8_t deg, type;
+    uint16_t nbr[kGraphDeg];
+};
+
 // One polymer architecture of one system.
 struct ArchDev {
     const BeadInfo* beads;       // [length]
     const uint16_t* color_beads; // [length], beads grouped by colour
     const uint8_t* types;        // [length], monomer type per bead
+    const GraphBead* graph;      // [length] in the order of color_beads; NULL for a linear chain
     int32_t length;
     int32_t n_colors;
+    int32_t max_deg;
     int32_t color_off[kMaxColors + 1];
     uint32_t color_magic[kMaxColors];  // ceil(2^32 / n_in_colour): i / n == umulhi(i, magic)
+    // graph: the screen's split of a colour, so that two rows of lanes have the same beads
+    // from one step to the next: blocks of `width` beads, of `per` chains a step
+    int32_t color_width[kMaxColors], color_per[kMaxColors];
     uint32_t len_magic;          // ceil(2^32 / length)
     uint32_t tpc_magic;          // magic of ceil(length / 2): bead pairs per chain
     int32_t n_chains;
@@ -89,7 +104,7 @@ struct ScreenDev {
     int32_t pad;
 };
 
-// What the move kernel of linear chains reads of a system, fixed for its life.
+// What the move kernel of warp tiles reads of a system, fixed for its life.
 struct SweepSys {
     float *x, *y, *z;
     const float* omega;
@@ -177,6 +192,7 @@ struct SysDev {
     uint32_t om_keys[3][2];
     unsigned long long slot_last[kSlots];  // k_run: accepted moves of its last sweep
     SweepSys sweep;
+    float4 by_deg[kGraphDeg + 1];  // of a bead with that many bonds: ScreenDev's a and b, c = 2k deg, A c / 4
     FieldSys field;
     // the statistics of the last sweep in the public layout, written by
     // k_stats_out for asynchronous reads (scmf_step_stats_async)
@@ -194,7 +210,7 @@ struct MoveTile {
     int32_t arch_index;   // architecture of the tile within its system
 };
 
-// Work item of k_sweep_warp: a run of whole chains of one linear architecture.
+// Work item of k_sweep_warp: a run of whole chains of one architecture.
 struct WarpTile {
     SysDev* sys;
     const ArchDev* arch;
@@ -287,8 +303,7 @@ struct LaunchShape {
     // `keys`, kKeysHigh when they share its upper 32 bits, else kKeysNone
     int keyed;
     PhiloxKeys keys;
-    // every architecture of the launch is a linear chain that fits a warp's
-    // tile: the tiles of k_sweep_warp
+    // every architecture of the launch fits a warp's tile: the tiles of k_sweep_warp
     const WarpTile* warp_tiles;
     int n_warp_tiles;
     int form;           // SweepFormId
@@ -327,7 +342,7 @@ struct SweepArgs {
     SweepArch arch[kSweepMaxArch];
 };
 
-// Forms of the move kernels of linear chains: the warps of a CTA (one CTA per SM)
+// Forms of the move kernels of warp tiles: the warps of a CTA (one CTA per SM)
 // and the beads of a warp's tile that shared memory then leaves room for.  Four
 // warps a scheduler keep the screen's pipes busy, and longer tiles fill the warps
 // of the resolve step better; half as many, with longer tiles still, where a chain
@@ -335,11 +350,15 @@ struct SweepArgs {
 // screen's code, its table and the lists: 409,600 beads 13.1 us a sweep, 14.8 in
 // the screened form (and 13.9, 15.8, 17.7 with 12, 28 and 24 warps of an SM, the
 // last two short of registers).
-enum SweepFormId { kFormScreened = 0, kFormLong = 1, kFormUnscreened = 2 };
+// Plans with other bond graphs than linear chains have a form with the code for
+// both, screened or not, and twelve warps: 2.0M beads in combs 25.1 us a sweep; with
+// sixteen 28.5 (the screen of arbitrary neighbours does not fit 128 registers beside
+// the exact trials), with eight 26.6.
+enum SweepFormId { kFormScreened = 0, kFormLong = 1, kFormUnscreened = 2, kFormGraph = 3 };
 struct SweepForm {
     int warps, beads;
 };
-constexpr SweepForm kSweepForms[3] = {{16, 960}, {8, 1984}, {16, 960}};
+constexpr SweepForm kSweepForms[4] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280}};
 constexpr size_t kL2Bytes = 126u << 20;
 constexpr float kScreenFromAc = 2.0f;  // A 4k from which the screen runs
 
@@ -359,7 +378,7 @@ int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int max_tile_bead
                  const LaunchShape& shape, void* stream);
 // close_mode != 0: the last field tile of every system closes it in the same
 // launch (what k_close does with that mode), so a sweep is two launches.
-// n_sweeps whole sweeps of a plan whose chains are all linear (shape.warp_tiles)
+// n_sweeps whole sweeps of a plan with warp tiles (shape.warp_tiles)
 // in one cooperative launch.
 int launch_run(const LaunchShape& shape, const RunArgs& run, void* stream);
 int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_tiles, LaunchShape shape,

@@ -259,7 +259,9 @@ size_t sweep_smem_bytes(int max_tile_beads, int max_length) {
     return (b + 15) & ~(size_t)15;
 }
 
-// One MC sweep over tiles of whole chains staged in shared memory.
+// One MC sweep over tiles of whole chains staged in shared memory: of plans that
+// k_sweep_warp does not take (a bead of more than six bonds, a chain longer than a
+// warp's tile, 2^31 cells times types), every trial made exactly.
 //   MODE kMoveOnly / kMoveGrid: moves; moves keeping counts[cur] the grid of
 //   the positions (accepted moves that change cell move a count).
 //   Two 256-thread CTAs per SM leave it 128 registers and no spill (at 64 it
@@ -1038,6 +1040,7 @@ static cudaError_t opt_in_warp() {
     cudaError_t e = opt_in_form<ONE, kFormScreened, KEYS>();
     if (e == cudaSuccess) e = opt_in_form<ONE, kFormLong, KEYS>();
     if (e == cudaSuccess) e = opt_in_form<ONE, kFormUnscreened, KEYS>();
+    if (e == cudaSuccess) e = opt_in_form<ONE, kFormGraph, KEYS>();
     return e;
 }
 
@@ -1111,6 +1114,7 @@ template <bool ONE, int KEYS>
 static cudaError_t launch_warp(const SweepArgs& a, int form, const RunArgs* run, cudaStream_t st) {
     if (form == kFormLong) return launch_form<ONE, kFormLong, KEYS>(a, run, st);
     if (form == kFormUnscreened) return launch_form<ONE, kFormUnscreened, KEYS>(a, run, st);
+    if (form == kFormGraph) return launch_form<ONE, kFormGraph, KEYS>(a, run, st);
     return launch_form<ONE, kFormScreened, KEYS>(a, run, st);
 }
 

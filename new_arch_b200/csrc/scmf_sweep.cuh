@@ -1,4 +1,4 @@
-// The move of linear chains: k_sweep_warp (one sweep's move of any systems) and
+// The move on warp tiles: k_sweep_warp (one sweep's move of any systems) and
 // k_run (many whole sweeps of systems that fit on the chip); included by
 // scmf_kernels.cu.
 //
@@ -138,6 +138,7 @@ struct SweepLayout {
         uint32_t moved[32];    // odd beads next to an even bead that moved: a bit for each row, a word for each lane
         uint16_t list[kListLen];
         SweepSys sys;          // of the tile's system, where a launch has several
+        float4 by_deg[FORM == kFormGraph ? kGraphDeg + 1 : 1];  // SysDev's
         // k_run, which has registers for one phase of a sweep at a time: the warp's
         // tile and its architecture, the sweeps that its system has made and makes
         // in all, and the system of the warp's field tile
@@ -370,93 +371,87 @@ struct TileRef {
     bool write;              // moved beads go to global memory too (k_run: after the last sweep)
 };
 
-// The exact trials of the beads of parity par of N pairs a lane (pair[i], where
-// act[i]), with trial_f's expressions.  A move updates the tile and, where asked,
-// the positions in global memory, moves a count if it leaves its cell, and marks the odd beads
-// next to it, whose screen saw the old position.  Returns the lane's moves.  The
-// N trials of a lane are independent: without branches between them their chains
-// (Philox, table, omega) run side by side.
-template <int N, int FORM, int KEYS>
-__device__ __forceinline__ unsigned exact_trials(const SweepSys& c, const SweepConsts& s, const TileRef& t, uint32_t* moved,
-                                                 const PhiloxKeys& keys, const float4* ntab, int par, const int (&pair)[N],
-                                                 bool (&act)[N]) {
+// What a trial is made of: its random stream, the bead (its place p in the
+// tile, its type's omega), the force on it, and c and A c / 4 of its bonds.
+struct Trial {
+    uint32_t chain, bead, typ;
+    int p;
+    float x, y, z, fx, fy, fz, cc, ac4;
+};
+
+// Makes a lane's trial exactly (where act), with trial_f's expressions.  A move
+// updates the tile and, where asked, the positions in global memory, and moves a
+// count if it leaves its cell.  Returns whether the bead moved.
+template <int FORM, int KEYS>
+__device__ __forceinline__ bool settle(const SweepSys& c, const SweepConsts& s, const TileRef& t, const PhiloxKeys& keys,
+                                       const float4* ntab, const Trial& b, bool act) {
     constexpr int kStride = SweepLayout<FORM>::kStride;
-    int p[N], b[N], c_old[N], c_new[N];
-    uint32_t typ[N];
-    float x[N], y[N], z[N], dx[N], dy[N], dz[N], deb[N], u[N], lo[N];
-    bool may[N];
-    bool any = false;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const int cl = (int)div_magic((uint32_t)pair[i], s.h_magic, s.h);
-        int bead = 2 * (pair[i] - cl * s.h) + par;
-        act[i] = act[i] && bead < s.L;
-        bead = act[i] ? bead : 0;
-        b[i] = bead;
-        p[i] = cl * s.L + bead;
-        typ[i] = (uint32_t)__ldg(t.types + bead) * c.n_cells;
-        const bool has_l = bead > 0, has_r = bead + 1 < s.L;
-        const int l = has_l ? -1 : 0, r = has_r ? 1 : 0;  // a missing bond: the bead itself, and no spring
-        const float* const Q = t.X + p[i];
-        x[i] = Q[0];
-        y[i] = Q[kStride];
-        z[i] = Q[2 * kStride];
-        const uint4 w = philox_block<KEYS>(make_uint4(t.rng0 + (uint32_t)cl, (uint32_t)bead, s.step, 0u), s.k0, s.k1, keys);
-        float n0, n1, n2;
-        normals3(w, ntab, n0, n1, n2);
-        const float kl = has_l ? c.k2 : 0.0f, kr = has_r ? c.k2 : 0.0f;
-        float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-        add_bond(kl, x[i], y[i], z[i], Q[l], Q[l + kStride], Q[l + 2 * kStride], fx, fy, fz);
-        add_bond(kr, x[i], y[i], z[i], Q[r], Q[r + kStride], Q[r + 2 * kStride], fx, fy, fz);
-        const int deg = (has_l ? 1 : 0) + (has_r ? 1 : 0);
-        const float cc = deg == 2 ? c.cdeg[2] : deg == 1 ? c.cdeg[1] : 0.0f;
-        const float ac4 = deg == 2 ? c.ac4[2] : deg == 1 ? c.ac4[1] : 0.0f;
-        dx[i] = __fmaf_rn(c.A, fx, __fmul_rn(c.R, n0));
-        dy[i] = __fmaf_rn(c.A, fy, __fmul_rn(c.R, n1));
-        dz[i] = __fmaf_rn(c.A, fz, __fmul_rn(c.R, n2));
-        const float d2 = __fmaf_rn(dx[i], dx[i], __fmaf_rn(dy[i], dy[i], __fmul_rn(dz[i], dz[i])));
-        const float fd = __fmaf_rn(fx, dx[i], __fmaf_rn(fy, dy[i], __fmul_rn(fz, dz[i])));
-        deb[i] = __fmul_rn(ac4, __fmaf_rn(cc, d2, __fmul_rn(-2.0f, fd)));
-        u[i] = u01(accept_word(w));
-        lo[i] = log_lower(u[i]);
-        may[i] = act[i] && maybe_accepted(deb[i], t.span, lo[i]);
-        any = any || may[i];
+    const uint4 w = philox_block<KEYS>(make_uint4(b.chain, b.bead, s.step, 0u), s.k0, s.k1, keys);
+    float n0, n1, n2;
+    normals3(w, ntab, n0, n1, n2);
+    const float dx = __fmaf_rn(c.A, b.fx, __fmul_rn(c.R, n0));
+    const float dy = __fmaf_rn(c.A, b.fy, __fmul_rn(c.R, n1));
+    const float dz = __fmaf_rn(c.A, b.fz, __fmul_rn(c.R, n2));
+    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+    const float fd = __fmaf_rn(b.fx, dx, __fmaf_rn(b.fy, dy, __fmul_rn(b.fz, dz)));
+    const float deb = __fmul_rn(b.ac4, __fmaf_rn(b.cc, d2, __fmul_rn(-2.0f, fd)));
+    const float u = u01(accept_word(w));
+    const float lo = log_lower(u);
+    if (!(act && maybe_accepted(deb, t.span, lo))) return false;
+    const float px = __fadd_rn(b.x, dx), py = __fadd_rn(b.y, dy), pz = __fadd_rn(b.z, dz);
+    const int c_old = cell_index(c, b.x, b.y, b.z), c_new = cell_index(c, px, py, pz);
+    const float w_old = __ldcg(c.omega + (b.typ + c_old)), w_new = __ldcg(c.omega + (b.typ + c_new));
+    const float dE = __fadd_rn(__fsub_rn(w_new, w_old), deb);
+    // log_lower decides without the logarithm for all but a few trials (trial_f)
+    if (!(dE < 0.0f || (-dE > lo && log_f(u) < -dE))) return false;
+    float* const Q = t.X + b.p;
+    Q[0] = px;
+    Q[kStride] = py;
+    Q[2 * kStride] = pz;
+    if (t.write) {
+        const int64_t g = t.bead0 + b.p;
+        c.x[g] = px;
+        c.y[g] = py;
+        c.z[g] = pz;
     }
-    unsigned nacc = 0;
-    if (any) {
-        float w_old[N], w_new[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            c_old[i] = cell_index(c, x[i], y[i], z[i]);
-            c_new[i] = cell_index(c, __fadd_rn(x[i], dx[i]), __fadd_rn(y[i], dy[i]), __fadd_rn(z[i], dz[i]));
-            w_old[i] = __ldcg(c.omega + (typ[i] + c_old[i]));
-            w_new[i] = __ldcg(c.omega + (typ[i] + c_new[i]));
-        }
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float dE = __fadd_rn(__fsub_rn(w_new[i], w_old[i]), deb[i]);
-            // log_lower decides without the logarithm for all but a few trials (trial_f)
-            if (!(may[i] && (dE < 0.0f || (-dE > lo[i] && log_f(u[i]) < -dE)))) continue;
-            float* const Q = t.X + p[i];
-            const int64_t g = t.bead0 + p[i];
-            Q[0] = __fadd_rn(x[i], dx[i]);
-            Q[kStride] = __fadd_rn(y[i], dy[i]);
-            Q[2 * kStride] = __fadd_rn(z[i], dz[i]);
-            if (t.write) {
-                c.x[g] = Q[0];
-                c.y[g] = Q[kStride];
-                c.z[g] = Q[2 * kStride];
-            }
-            if (t.move_counts && c_new[i] != c_old[i]) count_move(c.counts, c.count16 != 0, typ[i], c_old[i], c_new[i]);
-            ++nacc;
-            if (FORM != kFormUnscreened && par == 0) {
-                const int j = pair[i];
-                if (b[i] > 0) atomicOr(moved + ((j - 1) & 31), 1u << ((j - 1) >> 5));
-                if (b[i] + 1 < s.L) atomicOr(moved + (j & 31), 1u << (j >> 5));
-            }
-        }
+    if (t.move_counts && c_new != c_old) count_move(c.counts, c.count16 != 0, b.typ, c_old, c_new);
+    return true;
+}
+
+// The exact trial of the bead of parity par of a lane's pair (where act).  A bead
+// that moves marks the odd beads next to it, whose screen saw the old position.
+template <int FORM, int KEYS>
+__device__ __forceinline__ unsigned exact_trial(const SweepSys& c, const SweepConsts& s, const TileRef& t, uint32_t* moved,
+                                                const PhiloxKeys& keys, const float4* ntab, int par, int pair, bool act) {
+    constexpr int kStride = SweepLayout<FORM>::kStride;
+    const int cl = (int)div_magic((uint32_t)pair, s.h_magic, s.h);
+    int bead = 2 * (pair - cl * s.h) + par;
+    act = act && bead < s.L;
+    bead = act ? bead : 0;
+    Trial b;
+    b.chain = t.rng0 + (uint32_t)cl;
+    b.bead = (uint32_t)bead;
+    b.p = cl * s.L + bead;
+    b.typ = (uint32_t)__ldg(t.types + bead) * c.n_cells;
+    const bool has_l = bead > 0, has_r = bead + 1 < s.L;
+    const int l = has_l ? -1 : 0, r = has_r ? 1 : 0;  // a missing bond: the bead itself, and no spring
+    const float* const Q = t.X + b.p;
+    b.x = Q[0];
+    b.y = Q[kStride];
+    b.z = Q[2 * kStride];
+    const float kl = has_l ? c.k2 : 0.0f, kr = has_r ? c.k2 : 0.0f;
+    b.fx = b.fy = b.fz = 0.0f;
+    add_bond(kl, b.x, b.y, b.z, Q[l], Q[l + kStride], Q[l + 2 * kStride], b.fx, b.fy, b.fz);
+    add_bond(kr, b.x, b.y, b.z, Q[r], Q[r + kStride], Q[r + 2 * kStride], b.fx, b.fy, b.fz);
+    const int deg = (has_l ? 1 : 0) + (has_r ? 1 : 0);
+    b.cc = deg == 2 ? c.cdeg[2] : deg == 1 ? c.cdeg[1] : 0.0f;
+    b.ac4 = deg == 2 ? c.ac4[2] : deg == 1 ? c.ac4[1] : 0.0f;
+    if (!settle<FORM, KEYS>(c, s, t, keys, ntab, b, act)) return 0u;
+    if (FORM != kFormUnscreened && par == 0) {
+        if (bead > 0) atomicOr(moved + ((pair - 1) & 31), 1u << ((pair - 1) >> 5));
+        if (bead + 1 < s.L) atomicOr(moved + (pair & 31), 1u << (pair >> 5));
     }
-    return nacc;
+    return 1u;
 }
 
 // Makes the trials of a tile that the masks name (bit i of even / odd: the even
@@ -479,9 +474,8 @@ __device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<FORM>::War
         if (FORM == kFormUnscreened) {  // every trial, row by row
 #pragma unroll 1
             for (int r = 0; 32 * r < t.items; ++r) {
-                const int pair[1] = {min(32 * r + lane, t.items - 1)};
-                bool act[1] = {((mask >> r) & 1u) != 0u};
-                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+                nacc += exact_trial<FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, min(32 * r + lane, t.items - 1),
+                                                ((mask >> r) & 1u) != 0u);
             }
             __syncwarp();
             continue;
@@ -500,19 +494,205 @@ __device__ __forceinline__ unsigned resolve_tile(typename SweepLayout<FORM>::War
             __syncwarp();
 #pragma unroll 1
             for (int r = lane; r < total; r += 32) {
-                const int pair[1] = {(int)wp->list[r]};
-                bool act[1] = {true};
-                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+                nacc += exact_trial<FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, (int)wp->list[r], true);
             }
         } else {  // row by row
 #pragma unroll 1
             for (int r = 0; 32 * r < t.items; ++r) {
-                const int pair[1] = {min(32 * r + lane, t.items - 1)};
-                bool act[1] = {((mask >> r) & 1u) != 0u};
-                nacc += exact_trials<1, FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, pair, act);
+                nacc += exact_trial<FORM, KEYS>(c, s, t, wp->moved, keys, ntab, par, min(32 * r + lane, t.items - 1),
+                                                ((mask >> r) & 1u) != 0u);
             }
         }
         __syncwarp();
+    }
+    return nacc;
+}
+
+// --------------------------------------------------------- other bond graphs
+// A bead's GraphBead.
+struct GraphRec {
+    uint4 v;
+    __device__ __forceinline__ uint32_t bead() const { return v.x & 0xFFFFu; }
+    __device__ __forceinline__ int deg() const { return (int)((v.x >> 16) & 0xFFu); }
+    __device__ __forceinline__ uint32_t type() const { return v.x >> 24; }
+    __device__ __forceinline__ int nbr(int d) const {
+        const uint32_t w = d < 2 ? v.y : d < 4 ? v.z : v.w;
+        return (int)(d & 1 ? w >> 16 : w & 0xFFFFu);
+    }
+};
+__device__ __forceinline__ GraphRec graph_rec(const GraphBead* beads, int k) {
+    return GraphRec{__ldg(reinterpret_cast<const uint4*>(beads) + k)};
+}
+
+// The Philox block of bead b of a chain: pair_blocks for one bead (p0 = M0 * x of
+// round 1, which the bead and the step give).
+template <int KEYS>
+__device__ __forceinline__ uint4 bead_block(uint32_t chain, uint32_t y1, uint64_t p0, uint32_t k0, uint32_t k1,
+                                            const PhiloxKeys& ks) {
+    const auto key0 = [&](int r) { return KEYS == kKeysBoth ? ks.k[2 * r] : k0; };
+    const auto key1 = [&](int r) { return KEYS != kKeysNone ? ks.k[2 * r + 1] : k1; };
+    const auto next = [&] {
+        if (KEYS != kKeysBoth) k0 += 0x9E3779B9u;
+        if (KEYS == kKeysNone) k1 += 0xBB67AE85u;
+    };
+    const uint64_t a = (uint64_t)0xD2511F53u * chain;                            // round 1
+    const uint64_t q = (uint64_t)0xCD9E8D57u * ((uint32_t)(a >> 32) ^ key1(0));  // round 2
+    next();
+    uint4 w = make_uint4((uint32_t)(q >> 32) ^ y1 ^ key0(1), (uint32_t)q, (uint32_t)(p0 >> 32) ^ (uint32_t)a ^ key1(1),
+                         (uint32_t)p0);
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        next();
+        const uint64_t m0 = (uint64_t)0xD2511F53u * w.x, m1 = (uint64_t)0xCD9E8D57u * w.z;
+        w = make_uint4((uint32_t)(m1 >> 32) ^ w.y ^ key0(r), (uint32_t)m1, (uint32_t)(m0 >> 32) ^ w.w ^ key1(r), (uint32_t)m0);
+    }
+    return w;
+}
+
+// One sweep of a tile of chains of any bond graph, colour by colour: beads of one
+// colour have no bond with each other, so a colour's trials are screened, gathered
+// and made exactly before the next colour's are looked at, and no screen sees a
+// position that moves.  Without the screen every trial is made.  Returns the
+// lane's accepted moves.
+//
+// The screen takes 64 trials a step, two a lane, as the halves of f32x2
+// operations.  A lane keeps its two beads from step to step while the chains
+// advance (ArchDev::color_width beads of color_per chains a step: at least half of
+// the lanes, and 60 of 64 for twenty beads of a colour): the bead's record, its
+// neighbours' places and its part of the Philox rounds are set up once a block.
+// DEG: the most bonds of a bead (a loop of bonds that ends early would keep the
+// compiler from placing loads and Philox rounds side by side).
+//
+// 2.0M beads in combs of 40 (a backbone of 24, eight side chains of two): 25.1 us a
+// sweep in k_run, where k_sweep (a block a tile, every trial exact) took 77.6.  Of
+// these 6 us are barriers and the field, 5 the exact trials (5.8 % of all: the ends
+// of the side chains have one bond and pass the screen five times as often), the
+// rest the screen, whose twelve scattered reads of shared memory a trial cost it
+// twice the linear one's time.  One row of trials a step 29.1 us, with the places
+// computed anew each step 31; a bit mask a lane instead of the list 25.6.
+template <int DEG, int FORM, int KEYS>
+__device__ __forceinline__ unsigned graph_tile(typename SweepLayout<FORM>::Warp* wp, const SweepSys& c, const SweepConsts& s,
+                                               const TileRef& t, int n_chains, const ArchDev* A, bool screened,
+                                               const PhiloxKeys& keys, const float4* ntab) {
+    constexpr int kStride = SweepLayout<FORM>::kStride;
+    const int lane = threadIdx.x & 31;
+    const uint32_t tab = screen_lane();
+    const int n_colors = A->n_colors;
+    unsigned nacc = 0;
+#pragma unroll 1
+    for (int k = 0; k < n_colors; ++k) {
+        const GraphBead* const beads = A->graph + A->color_off[k];
+        const int n = A->color_off[k + 1] - A->color_off[k], width = A->color_width[k], per = A->color_per[k];
+        const uint32_t magic = A->color_magic[k];
+        int slot0 = 0, c0 = 0;
+#pragma unroll 1
+        do {
+            int have = 0;
+            if (!screened) {
+                have = n_chains * n;
+                slot0 = n;
+            }
+#pragma unroll 1
+            while (slot0 < n) {
+                const float* Q[2];
+                int nbr[2][DEG], chain[2], item[2];
+                float2 ab[2];
+                uint64_t p0[2];
+                const uint64_t m1s = (uint64_t)0xCD9E8D57u * s.step;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int at = lane + 32 * i, ci = at / width, slot = slot0 + at - ci * width;
+                    const bool ok = ci < per && slot < n;
+                    const GraphRec rec = graph_rec(beads, ok ? slot : 0);
+                    chain[i] = ok ? c0 + ci : n_chains;  // none
+                    item[i] = chain[i] * n + slot;
+                    Q[i] = t.X + (chain[i] * s.L + (int)rec.bead());
+                    ab[i] = *reinterpret_cast<const float2*>(&wp->by_deg[rec.deg()]);
+#pragma unroll
+                    for (int d = 0; d < DEG; ++d) nbr[i][d] = rec.nbr(d) - (int)rec.bead();
+                    p0[i] = (uint64_t)0xD2511F53u * ((uint32_t)(m1s >> 32) ^ (KEYS == kKeysBoth ? keys.k[0] : s.k0) ^ rec.bead());
+                }
+                const f32x2 a2 = pack2(ab[0].x, ab[1].x), b2 = pack2(ab[0].y, ab[1].y), add = pack2(s.add, s.add);
+                const f32x2 k2 = pack2(c.k2, c.k2), zero = pack2(0.0f, 0.0f);
+                // full steps; a lane past the last chain looks at the tile's first bead
+#pragma unroll 1
+                for (; c0 < n_chains && have <= kListLen - 64; c0 += per) {
+                    f32x2 f[3] = {zero, zero, zero};
+                    const float *P[2], *O[2];
+                    bool in[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        in[i] = chain[i] < n_chains;
+                        P[i] = in[i] ? Q[i] : t.X;
+                    }
+                    const float x[2] = {P[0][0], P[1][0]}, y[2] = {P[0][kStride], P[1][kStride]},
+                                z[2] = {P[0][2 * kStride], P[1][2 * kStride]};
+#pragma unroll
+                    for (int d = 0; d < DEG; ++d) {  // a missing bond is one with the bead itself
+                        O[0] = in[0] ? P[0] + nbr[0][d] : t.X;
+                        O[1] = in[1] ? P[1] + nbr[1][d] : t.X;
+                        f[0] = fma2(pack2(__fsub_rn(O[0][0], x[0]), __fsub_rn(O[1][0], x[1])), k2, f[0]);
+                        f[1] = fma2(pack2(__fsub_rn(O[0][kStride], y[0]), __fsub_rn(O[1][kStride], y[1])), k2, f[1]);
+                        f[2] = fma2(pack2(__fsub_rn(O[0][2 * kStride], z[0]), __fsub_rn(O[1][2 * kStride], z[1])), k2, f[2]);
+                    }
+                    uint4 w[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        w[i] = bead_block<KEYS>(t.rng0 + (uint32_t)chain[i], (uint32_t)m1s, p0[i], s.k0, s.k1, keys);
+                    const f32x2 vx = fma2(f[0], a2, pack2(screen_normal(w[0].x, tab), screen_normal(w[1].x, tab)));
+                    const f32x2 vy = fma2(f[1], a2, pack2(screen_normal(w[0].y, tab), screen_normal(w[1].y, tab)));
+                    const f32x2 vz = fma2(f[2], a2, pack2(screen_normal(w[0].z, tab), screen_normal(w[1].z, tab)));
+                    const f32x2 q = fma2(vx, vx, fma2(vy, vy, mul2(vz, vz)));
+                    const f32x2 u = pack2(__fmaf_rn(log2_below_u(accept_word(w[0])), s.u1, s.u0),
+                                          __fmaf_rn(log2_below_u(accept_word(w[1])), s.u1, s.u0));
+                    const f32x2 lim = fma2(b2, fma2(f[0], f[0], fma2(f[1], f[1], fma2(f[2], f[2], u))), add);
+                    float qi[2], li[2];
+                    unpack2(q, qi[0], qi[1]);
+                    unpack2(lim, li[0], li[1]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const bool pass = !(qi[i] > li[i]) && in[i];  // NaN passes
+                        const uint32_t who = __ballot_sync(0xffffffffu, pass);
+                        if (pass) wp->list[have + __popc(who & ((1u << lane) - 1u))] = (uint16_t)item[i];
+                        have += __popc(who);
+                        chain[i] += per;
+                        item[i] += per * n;
+                        Q[i] += per * s.L;
+                    }
+                }
+                if (c0 < n_chains) break;  // the list is full
+                c0 = 0;
+                slot0 += width;
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int r = lane; r < have; r += 32) {
+                const int j = screened ? (int)wp->list[r] : r;
+                const int cl = (int)div_magic((uint32_t)j, magic, n);
+                const GraphRec rec = graph_rec(beads, j - cl * n);
+                const float2 ca = *(reinterpret_cast<const float2*>(&wp->by_deg[rec.deg()]) + 1);
+                const float* const first = t.X + cl * s.L;
+                const float* const Q = first + rec.bead();
+                Trial b;
+                b.x = Q[0];
+                b.y = Q[kStride];
+                b.z = Q[2 * kStride];
+                b.fx = b.fy = b.fz = 0.0f;
+#pragma unroll
+                for (int d = 0; d < DEG; ++d) {
+                    const float* const O = first + rec.nbr(d);
+                    add_bond(c.k2, b.x, b.y, b.z, O[0], O[kStride], O[2 * kStride], b.fx, b.fy, b.fz);
+                }
+                b.chain = t.rng0 + (uint32_t)cl;
+                b.bead = rec.bead();
+                b.typ = rec.type() * c.n_cells;
+                b.p = cl * s.L + (int)rec.bead();
+                b.cc = ca.x;
+                b.ac4 = ca.y;
+                nacc += settle<FORM, KEYS>(c, s, t, keys, ntab, b, true) ? 1u : 0u;
+            }
+            __syncwarp();
+        } while (slot0 < n);
     }
     return nacc;
 }
@@ -582,6 +762,11 @@ struct Mover {
             for (int i = lane; i < (int)(sizeof(SweepSys) / 4); i += 32) reinterpret_cast<uint32_t*>(&wp->sys)[i] = src[i];
             __syncwarp();
         }
+        if (FORM == kFormGraph && t.sys != S) {
+            __syncwarp();
+            if (lane <= kGraphDeg) wp->by_deg[lane] = t.sys->by_deg[lane];
+            __syncwarp();
+        }
         S = t.sys;
         A = t.arch;
         types = A->types;
@@ -626,6 +811,12 @@ struct Mover {
         const int off = (int)(t.bead0 & 3), items = t.n_chains * s.h;
         const uint32_t rng0 = rng_base + t.chain, tab = screen_lane();
         float* X = wp->pos + 4 + off;
+        if (FORM == kFormGraph && A->graph) {
+            const TileRef ref{X, t.bead0, rng0, 0, nullptr, span, a.move_counts != 0, write};
+            if (mode == 0) return 0u;
+            return A->max_deg <= 3 ? graph_tile<3, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab)
+                                   : graph_tile<kGraphDeg, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab);
+        }
         uint32_t even = 0u, odd = 0u;
         if (FORM != kFormUnscreened && mode == 2) {
             if ((s.L | off) & 1)
@@ -918,6 +1109,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 Mover<ONE, FORM, KEYS> m(a, smem_raw);
                 const WarpTile& t = wp->run.tile;
                 m.S = t.sys;
+                m.A = t.arch;
                 m.types = wp->run.types;
                 m.rng_base = wp->run.rng_base;
                 m.set(t.length, wp->run.h_magic, done, true, span_after(t.sys, wp->run.rule, done, base));

@@ -435,9 +435,11 @@ __global__ void __launch_bounds__(256) k_grid(const MoveTile* __restrict__ tiles
 // phi_S = n_S * scale, tot = sum_S phi_S (S ascending), then
 // SCMF0: w_T = (tot - 1) cf_TT + sum_{S != T} cf_TS (phi_T - phi_S)
 // literal: w_T = (tot - 1) cf_TT + sum_{S != T} cf_TS phi_S.
+// Returns the cell's field energy, or 0 without `energy` (its conversions to FP64
+// take longer than all the rest).
 template <int NT>
 __device__ __forceinline__ double omega_of_cell(int nt, const uint32_t* cnt, float scale, bool lit, bool upd, float* w,
-                                                const float* cf) {
+                                                const float* cf, bool energy = true) {
     constexpr int M = NT > 0 ? NT : kMaxTypes;
     float phi[M];
     float tot = 0.0f;
@@ -465,7 +467,7 @@ __device__ __forceinline__ double omega_of_cell(int nt, const uint32_t* cnt, flo
                 }
                 w[t] = v;
             }
-            ef += (double)w[t] * (double)cnt[t];
+            if (energy) ef += (double)w[t] * (double)cnt[t];
         }
     }
     return ef;
@@ -476,7 +478,8 @@ __device__ __forceinline__ double omega_of_cell(int nt, const uint32_t* cnt, flo
 template <int NT, bool FROM_L2>
 __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, float scale, bool lit, bool upd,
                                              bool c16, const uint32_t* src32, float* W, const float* cf,
-                                             unsigned long long* avg, float& wmax, float& wmin) {
+                                             unsigned long long* avg, float& wmax, float& wmin,
+                                             bool energy = true) {
     constexpr int M = NT > 0 ? NT : kMaxTypes;
     const int nt = NT > 0 ? NT : n;
     const uint16_t* src16 = reinterpret_cast<const uint16_t*>(src32);
@@ -496,7 +499,7 @@ __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, fl
             if (avg) avg[u * NC + cell] += cnt[u];
         }
     }
-    const double ef = omega_of_cell<NT>(nt, cnt, scale, lit, upd, w, cf);
+    const double ef = omega_of_cell<NT>(nt, cnt, scale, lit, upd, w, cf, energy);
 #pragma unroll
     for (int t = 0; t < M; ++t) {
         if (t < nt && upd) W[t * NC + cell] = w[t];
@@ -513,7 +516,8 @@ __device__ __forceinline__ double field_cell(int n, int64_t cell, int64_t NC, fl
 template <int NT, bool FROM_L2>
 __device__ __forceinline__ double field_cells4(int64_t cell, int64_t NC, float scale, bool lit, bool upd,
                                                const uint32_t* src32, float* W, const float* cf,
-                                               unsigned long long* avg, float& wmax, float& wmin) {
+                                               unsigned long long* avg, float& wmax, float& wmin,
+                                               bool energy = true) {
     uint4 cv[NT];
     float4 wv[NT];
 #pragma unroll
@@ -544,7 +548,7 @@ __device__ __forceinline__ double field_cells4(int64_t cell, int64_t NC, float s
             cnt[u] = l == 0 ? cv[u].x : l == 1 ? cv[u].y : l == 2 ? cv[u].z : cv[u].w;
             w[u] = l == 0 ? wv[u].x : l == 1 ? wv[u].y : l == 2 ? wv[u].z : wv[u].w;
         }
-        ef += omega_of_cell<NT>(NT, cnt, scale, lit, upd, w, cf);
+        ef += omega_of_cell<NT>(NT, cnt, scale, lit, upd, w, cf, energy);
 #pragma unroll
         for (int u = 0; u < NT; ++u) {
             wmax = fmaxf(wmax, w[u]);

@@ -141,12 +141,16 @@ struct SweepLayout {
         float4 by_deg[FORM == kFormGraph ? kGraphDeg + 1 : 1];  // SysDev's
         // k_run, which has registers for one phase of a sweep at a time: the warp's
         // tile and its architecture, the sweeps that its system has made and makes
-        // in all, and the system of the warp's field tile
+        // in all, and the warp's field tile and its system
         struct {
             WarpTile tile;
             const uint8_t* types;
             uint32_t rng_base, h_magic, base, stop;
             int32_t rule, active;
+            SysDev* f_sys;
+            int64_t cell0;
+            int32_t n_cells;
+            uint32_t f_base, f_stop;
         } run;
         FieldSys field;
         alignas(16) float pos[3 * kStride];
@@ -806,18 +810,14 @@ struct Mover {
         return ok;
     }
 
-    // One sweep of the tile in the buffer.  Returns the lane's accepted moves.
-    __device__ __forceinline__ unsigned move(const WarpTile& t, bool write) {
-        const int off = (int)(t.bead0 & 3), items = t.n_chains * s.h;
+    __device__ __forceinline__ bool graph() const { return FORM == kFormGraph && A->graph; }
+
+    // The trials of the tile in the buffer that may be accepted (screen_tile's masks).
+    __device__ __forceinline__ void screen(const WarpTile& t, uint32_t& even, uint32_t& odd) {
+        const int off = (int)(t.bead0 & 3);
         const uint32_t rng0 = rng_base + t.chain, tab = screen_lane();
-        float* X = wp->pos + 4 + off;
-        if (FORM == kFormGraph && A->graph) {
-            const TileRef ref{X, t.bead0, rng0, 0, nullptr, span, a.move_counts != 0, write};
-            if (mode == 0) return 0u;
-            return A->max_deg <= 3 ? graph_tile<3, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab)
-                                   : graph_tile<kGraphDeg, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab);
-        }
-        uint32_t even = 0u, odd = 0u;
+        const float* X = wp->pos + 4 + off;
+        even = odd = 0u;
         if (FORM != kFormUnscreened && mode == 2) {
             if ((s.L | off) & 1)
                 screen_tile<2, FORM, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
@@ -826,10 +826,25 @@ struct Mover {
             else
                 screen_tile<0, FORM, KEYS>(s, X, rng0, t.n_chains, a.keys, tab, even, odd);
         } else if (mode == 1) {
-            even = odd = row_mask(items);
+            even = odd = row_mask(t.n_chains * s.h);
         }
-        const TileRef ref{X, t.bead0, rng0, items, types, span, a.move_counts != 0, write};
+    }
+    // Makes them.  Returns the lane's accepted moves.
+    __device__ __forceinline__ unsigned resolve(const WarpTile& t, uint32_t even, uint32_t odd, bool write) {
+        TileRef ref{wp->pos + 4 + (int)(t.bead0 & 3), t.bead0, rng_base + t.chain, t.n_chains * s.h, types, span,
+                    a.move_counts != 0, write};
+        if (graph()) {
+            if (mode == 0) return 0u;
+            return A->max_deg <= 3 ? graph_tile<3, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab)
+                                   : graph_tile<kGraphDeg, FORM, KEYS>(wp, sys(), s, ref, t.n_chains, A, mode == 2, a.keys, ntab);
+        }
         return resolve_tile<FORM, KEYS>(wp, sys(), s, ref, a.keys, ntab, even, odd);
+    }
+    // One sweep of the tile.
+    __device__ __forceinline__ unsigned move(const WarpTile& t, bool write) {
+        uint32_t even = 0u, odd = 0u;
+        if (!graph()) screen(t, even, odd);
+        return resolve(t, even, odd, write);
     }
 };
 
@@ -914,12 +929,18 @@ struct GridBarrier {
     __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {
         if (threadIdx.x == 0) target = __ldcg(c) / gridDim.x * gridDim.x;
     }
-    // False (to all threads of the CTA) after about two seconds.
-    __device__ __forceinline__ bool wait(int* s_ok) {
+    __device__ __forceinline__ void arrive() {
         __syncthreads();
         if (threadIdx.x == 0) {
             target += gridDim.x;
             asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+        }
+    }
+    // False (to all threads of the CTA) after about two seconds.  Thread 0 calls
+    // `then` before the others go on.
+    template <typename Then>
+    __device__ __forceinline__ bool wait(int* s_ok, const Then& then) {
+        if (threadIdx.x == 0) {
             unsigned long long now;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
             if (now < target) {
@@ -929,6 +950,7 @@ struct GridBarrier {
                 } while (now < target && clock64() - t0 < kWaitClocks);
             }
             *s_ok = now >= target;
+            then();
         }
         __syncthreads();
         return *s_ok != 0;
@@ -937,6 +959,11 @@ struct GridBarrier {
 
 // Whether sweep `step` ends with a field update (test.cpp:42).
 __device__ __forceinline__ bool updates_field(int rule, uint32_t step) { return rule == 1 || step % 10u != 0u; }
+
+// The screen of the next sweep runs before its omega is known, for spans up to
+// this times the last one (the span moves by the omega of a bead or two in a few
+// cells); with more, the sweep is screened again.
+constexpr float kSpanAhead = 1.125f;
 
 // The omega span that the sweep after `done` sweeps uses, in a launch that
 // started at `base`: of the last field update, from the launch's slots (om_keys,
@@ -1002,29 +1029,34 @@ __device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r,
     __syncthreads();
 }
 
-// A warp's field step over one tile of cells: omega of the new counts, and the
-// averaging sample where the sweep takes one.  Returns the lane's field energy.
-__device__ __forceinline__ double field_tile(const FieldSys& f, int64_t cell0, int n_cells, bool upd, bool sample, float& wmax,
-                                             float& wmin) {
-    const int lane = threadIdx.x & 31, n = f.n_types;
+// A warp's field step over one tile of cells of N types (0: any number): omega
+// of the new counts, and the averaging sample where the sweep takes one.  Returns
+// the lane's field energy, where it is asked for.
+template <int N>
+__device__ __forceinline__ double field_tile_of(const FieldSys& f, int64_t cell0, int n_cells, bool upd, unsigned long long* avg,
+                                                bool energy, float& wmax, float& wmin) {
+    const int lane = threadIdx.x & 31;
     const int64_t NC = f.n_cells, end = cell0 + n_cells;
     const bool lit = f.literal != 0, c16 = f.count16 != 0;
-    unsigned long long* avg = sample ? f.avg : nullptr;
     double ef = 0.0;
-    if (!c16 && n <= 3 && ((NC | cell0 | n_cells) & 3) == 0) {
-        for (int64_t cell = cell0 + 4 * lane; cell < end; cell += 128) {
-            if (n == 2)
-                ef += field_cells4<2, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
-            else if (n == 1)
-                ef += field_cells4<1, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
-            else
-                ef += field_cells4<3, true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin);
-        }
+    if (N > 0 && !c16 && ((NC | cell0 | n_cells) & 3) == 0 && n_cells > 32) {
+        for (int64_t cell = cell0 + 4 * lane; cell < end; cell += 128)
+            ef += field_cells4<(N > 0 ? N : 1), true>(cell, NC, f.scale, lit, upd, f.counts, f.omega, f.cf, avg, wmax, wmin, energy);
     } else {
         for (int64_t cell = cell0 + lane; cell < end; cell += 32)
-            ef += field_cell<0, true>(n, cell, NC, f.scale, lit, upd, c16, f.counts, f.omega, f.cf, avg, wmax, wmin);
+            ef += field_cell<N, true>(f.n_types, cell, NC, f.scale, lit, upd, c16, f.counts, f.omega, f.cf, avg, wmax, wmin, energy);
     }
     return ef;
+}
+__device__ __forceinline__ double field_tile(const FieldSys& f, int64_t cell0, int n_cells, bool upd, bool sample, bool energy,
+                                             float& wmax, float& wmin) {
+    unsigned long long* avg = sample ? f.avg : nullptr;
+    switch (f.n_types) {
+        case 1: return field_tile_of<1>(f, cell0, n_cells, upd, avg, energy, wmax, wmin);
+        case 2: return field_tile_of<2>(f, cell0, n_cells, upd, avg, energy, wmax, wmin);
+        case 3: return field_tile_of<3>(f, cell0, n_cells, upd, avg, energy, wmax, wmin);
+        default: return field_tile_of<0>(f, cell0, n_cells, upd, avg, energy, wmax, wmin);
+    }
 }
 
 // n_sweeps whole sweeps (move, field, statistics) of the systems of a launch in
@@ -1033,14 +1065,25 @@ __device__ __forceinline__ double field_tile(const FieldSys& f, int64_t cell0, i
 // once, and two grid barriers a sweep take the place of two kernel launches.  A
 // sweep of such a system is mostly latency (launches, tables, descriptors, each
 // a dependent trip to L2).  A sweep in this form against two kernels replayed
-// from a graph: 32,000 beads 8.8 us against 18.6 us; 409,600 beads, unscreened,
-// 14.8 against 22.7 us; 2.0M beads in chains of 33 20.2 against 28.9 us.  (Before
-// the kernels of this file: 14.6, 20.7 and 55.4 us.)  A barrier takes 2 us.
+// from a graph: 32,000 beads 7.1 us against 18.6 us; 409,600 beads, unscreened,
+// 12.5 against 22.7 us; 2.0M beads in chains of 33 18.8 against 28.9 us.  (Before
+// the kernels of this file: 14.6, 20.7 and 55.4 us.)
+//
+// A screen needs nothing of the sweep before but the positions of its own tile and a
+// bound on omega's span.  So the next sweep's screen runs between arriving at the
+// barrier after the move and waiting there, with a span that is an eighth larger
+// than the last one; the exact trials, after the field step, use the true one, and
+// a sweep whose span is more than that is screened again.  Of the 7.1 us of 32,000
+// beads the exact trials take 2.2, the screen 0.8, the field 1.5 and the barriers
+// the rest (1.3 each at the least: arrival and a look at the count are a trip to L2
+// each).  Screening after the field step took 8.2, with the field step's energy summed
+// every sweep and each warp reading the span for itself 8.5.
 template <bool ONE, int FORM, int KEYS>
 __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     k_run(const __grid_constant__ SweepArgs a, const __grid_constant__ RunArgs r) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_ok;
+    __shared__ float s_span;  // one system's, of the sweep to come
     __shared__ uint32_t s_keys[2];
     __shared__ unsigned long long s_acc[64];
     __shared__ double s_ef[32];
@@ -1049,6 +1092,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     const int first = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x, stride = (int)(blockDim.x >> 5) * (int)gridDim.x;
     const bool any = first < a.n_tiles;
     GridBarrier barrier(r.barrier);
+    if (ONE && threadIdx.x == 0) s_span = a.system->omega_span;
     if (threadIdx.x < 2) s_keys[threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
     for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {  // the slot of the launch's first field step
         SysDev* S = r.systems[i].sys;
@@ -1078,55 +1122,66 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     }
     // the warp's field tile (its first, where it has several) and that one's system
     FieldSys* const fs = &wp->field;
-    uint32_t f_base = 0u, f_stop = 0u;
-    SysDev* f_sys = nullptr;
-    const auto at_system = [&](SysDev* S) {
+    const auto at_field = [&](const FieldTile& t) {
         __syncwarp();
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&S->field);
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(&t.sys->field);
         for (int i = lane; i < (int)(sizeof(FieldSys) / 4); i += 32) reinterpret_cast<uint32_t*>(fs)[i] = src[i];
         if (lane == 0) {
-            fs->avg = S->avg;
-            fs->avg_every = S->avg_every;
+            fs->avg = t.sys->avg;
+            fs->avg_every = t.sys->avg_every;
+            wp->run.f_sys = t.sys;
+            wp->run.cell0 = t.cell0;
+            wp->run.n_cells = t.n_cells;
+            wp->run.f_base = t.sys->step;
+            wp->run.f_stop = t.sys->stop_step;
         }
-        f_base = S->step;
-        f_stop = S->stop_step;
-        f_sys = S;
         __syncwarp();
     };
-    int64_t cell0 = 0;
-    int n_cells = 0;
-    if (first < r.n_field) {
-        at_system(r.field[first].sys);
-        cell0 = r.field[first].cell0;
-        n_cells = r.field[first].n_cells;
-    }
+    if (first < r.n_field) at_field(r.field[first]);
     unsigned acc_all = 0, acc_last = 0;  // of all the launch's sweeps, of the system's last
+    uint32_t even = 0u, odd = 0u;        // the screen of the sweep to come, where it has been made,
+    float screened_to = -INFINITY;       // which holds for spans up to this
+    float span_now = INFINITY;           // the last sweep's span
 #pragma unroll 1
     for (int sweep = 0; sweep < r.n_sweeps; ++sweep) {
-        if (any && wp->run.active) {
-            const uint32_t base = wp->run.base, done = base + (uint32_t)sweep;
-            if (done < wp->run.stop) {
-                Mover<ONE, FORM, KEYS> m(a, smem_raw);
-                const WarpTile& t = wp->run.tile;
-                m.S = t.sys;
-                m.A = t.arch;
-                m.types = wp->run.types;
-                m.rng_base = wp->run.rng_base;
-                m.set(t.length, wp->run.h_magic, done, true, span_after(t.sys, wp->run.rule, done, base));
-                acc_last = m.move(t, false);
+        // pass 0: this sweep's move; pass 1: the screen of the next one, between arriving at the barrier and waiting
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass) barrier.arrive();
+            if (!any || !wp->run.active || (pass && sweep + 1 == r.n_sweeps)) continue;
+            const uint32_t base = wp->run.base, done = base + (uint32_t)(sweep + pass);
+            if (done >= wp->run.stop) continue;
+            Mover<ONE, FORM, KEYS> m(a, smem_raw);
+            const WarpTile& t = wp->run.tile;
+            m.S = t.sys;
+            m.A = t.arch;
+            m.types = wp->run.types;
+            m.rng_base = wp->run.rng_base;
+            float span;
+            if (pass == 0) {
+                span = ONE ? s_span : span_after(t.sys, wp->run.rule, done, base);
+            } else {
+                span = __fmul_rn(span_now, kSpanAhead);
+                if (FORM == kFormUnscreened || !(span < INFINITY)) continue;
+            }
+            m.set(t.length, wp->run.h_magic, done, true, span);
+            const bool ahead = m.mode == 2 && !m.graph();  // a system whose screen may run ahead
+            if (pass == 0 ? !m.graph() && !(span <= screened_to) : ahead) m.screen(t, even, odd);
+            if (pass == 0) {
+                acc_last = m.resolve(t, even, odd, false);
                 acc_all += acc_last;
+                span_now = span;
+                screened_to = -INFINITY;
+            } else if (ahead) {
+                screened_to = span;
             }
         }
-        if (!barrier.wait(&s_ok)) return;
+        if (!barrier.wait(&s_ok, [] {})) return;
         float wmax = -INFINITY, wmin = INFINITY;
 #pragma unroll 1
         for (int fi = first; fi < r.n_field; fi += stride) {
-            if (r.n_field > stride) {  // several field tiles a warp
-                if (r.field[fi].sys != f_sys) at_system(r.field[fi].sys);
-                cell0 = r.field[fi].cell0;
-                n_cells = r.field[fi].n_cells;
-            }
-            const uint32_t step = f_base + (uint32_t)sweep + 1u;
+            if (r.n_field > stride) at_field(r.field[fi]);  // several field tiles a warp
+            const uint32_t step = wp->run.f_base + (uint32_t)sweep + 1u, f_stop = wp->run.f_stop;
             if (step > f_stop) continue;
             const bool upd = updates_field(fs->rule, step), last = sweep + 1 == r.n_sweeps || step == f_stop;
             const bool sample = fs->avg && fs->avg_every && step % fs->avg_every == 0u;
@@ -1135,7 +1190,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 wmax = -INFINITY;
                 wmin = INFINITY;
             }
-            double ef = field_tile(*fs, cell0, n_cells, upd, sample, wmax, wmin);
+            double ef = field_tile(*fs, wp->run.cell0, wp->run.n_cells, upd, sample, last, wmax, wmin);
             if (last) {
                 ef = warp_sum(ef);
                 if (lane == 0) r.ef_part[fi] = ef;
@@ -1143,7 +1198,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
             if (!upd)
                 wmax = -INFINITY, wmin = INFINITY;
             else if (!ONE)
-                fold_span(f_sys->om_keys[step % 3u], wmax, wmin);
+                fold_span(wp->run.f_sys->om_keys[step % 3u], wmax, wmin);
         }
         if (ONE) {
             fold_span(s_keys, wmax, wmin);
@@ -1179,7 +1234,11 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 if (last) atomicAdd(&S->slot_last[first % kSlots], (unsigned long long)last);
             }
         }
-        if (!barrier.wait(&s_ok)) return;
+        barrier.arrive();
+        const bool ok = barrier.wait(&s_ok, [&] {
+            if (ONE) s_span = span_after(a.system, wp->run.rule, wp->run.base + (uint32_t)sweep + 1u, wp->run.base);
+        });
+        if (!ok) return;
     }
     if (any && wp->run.active) {  // the positions
         const SweepSys& c = ONE ? a.sys : wp->sys;

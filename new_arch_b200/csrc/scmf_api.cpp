@@ -56,6 +56,7 @@ void free_system(scmf_system* s) {
         cudaStreamSynchronize(s->stream);
         cudaStreamDestroy(s->stream);
     }
+    if (s->counted) stage_system_gone();
     delete s;
 }
 
@@ -420,6 +421,8 @@ static scmf_status create_system(const scmf_spec* spec, bool is_shard, int shard
     const scmf_tune t = default_tune();
     // upload() waits for the stream, so the host staging above may go out of scope
     if ((rc = s->append_plan(t, &p)) || (rc = s->plan.upload(p, t, st))) return bail(rc);
+    stage_system_made();
+    s->counted = true;
     *out = s;
     return SCMF_OK;
 }
@@ -528,14 +531,30 @@ static scmf_status upload_chunked(scmf_system* s, const float* xyz) {
     CK(cudaEventRecord(s->chunk_ev[0], s->stream));
     CK(cudaStreamWaitEvent(s->copy_stream, s->chunk_ev[0], 0));
     const int64_t n = s->n_beads, per = (n + kChunks - 1) / kChunks;
-    for (int k = 0; k < kChunks; ++k) {
-        const int64_t i0 = std::min<int64_t>(n, k * per), i1 = std::min<int64_t>(n, i0 + per);
-        if (i1 <= i0) break;
-        CK(cudaMemcpyAsync(s->d_aos + 3 * i0, xyz + 3 * i0, (size_t)(i1 - i0) * 3 * sizeof(float),
-                           cudaMemcpyHostToDevice, s->copy_stream));
-        CK(cudaEventRecord(s->chunk_ev[k], s->copy_stream));
-        CK(cudaStreamWaitEvent(s->stream, s->chunk_ev[k], 0));
-        CKL(launch_aos_chunk(s->d_aos, s->d_sys, s->d_arch, (int)s->archs.size(), i0, i1, s->stream));
+    int k = 0;
+    // converts the chunks whose positions the copy stream has been asked for
+    const auto convert = [&](size_t bytes) -> scmf_status {
+        for (; k < kChunks; ++k) {
+            const int64_t i0 = std::min<int64_t>(n, k * per), i1 = std::min<int64_t>(n, i0 + per);
+            if ((size_t)i1 * 3 * sizeof(float) > bytes) break;
+            if (i1 <= i0) continue;
+            CK(cudaEventRecord(s->chunk_ev[k], s->copy_stream));
+            CK(cudaStreamWaitEvent(s->stream, s->chunk_ev[k], 0));
+            CKL(launch_aos_chunk(s->d_aos, s->d_sys, s->d_arch, (int)s->archs.size(), i0, i1, s->stream));
+        }
+        return SCMF_OK;
+    };
+    scmf_status rc;
+    if (copy_to_device_staged(s->d_aos, xyz, (size_t)n * 3 * sizeof(float), s->copy_stream, convert, &rc)) {
+        RET(rc);
+    } else {
+        for (int c = 0; c < kChunks; ++c) {
+            const int64_t i0 = std::min<int64_t>(n, c * per), i1 = std::min<int64_t>(n, i0 + per);
+            if (i1 <= i0) break;
+            CK(cudaMemcpyAsync(s->d_aos + 3 * i0, xyz + 3 * i0, (size_t)(i1 - i0) * 3 * sizeof(float),
+                               cudaMemcpyHostToDevice, s->copy_stream));
+            RET(convert((size_t)i1 * 3 * sizeof(float)));
+        }
     }
     s->counts_stale = false;
     return SCMF_OK;
@@ -558,9 +577,7 @@ scmf_status scmf_get_coords(const scmf_system* cs, float* xyz, size_t n) {
     if (n != (size_t)s->n_beads * 3) return fail(SCMF_E_INVALID, "expected %lld floats, got %zu", (long long)s->n_beads * 3, n);
     RET(ensure_aos(s));
     CKL(launch_soa_to_aos(s->d_aos, s->d_sys, s->d_arch, (int)s->archs.size(), s->n_beads, s->stream));
-    CK(cudaMemcpyAsync(xyz, s->d_aos, n * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    return SCMF_OK;
+    return copy_to_host(xyz, s->d_aos, n * sizeof(float), s->stream);
 }
 
 scmf_status scmf_set_step(scmf_system* s, uint64_t step) {
@@ -668,29 +685,20 @@ scmf_status scmf_get_counts(const scmf_system* cs, uint32_t* out, size_t n) {
     if (!s || !out) return fail(SCMF_E_INVALID, "NULL argument");
     const size_t want = (size_t)s->n_cells * s->spec.n_types;
     if (n != want) return fail(SCMF_E_INVALID, "expected %zu counts, got %zu", want, n);
-    SysDev d;
-    RET(fetch_sysdev(s, &d));
-    if (s->spec.p.count_bits == 16) {
-        if (!s->d_u32) {
-            size_t dummy = 0;
-            RET(dalloc(&s->d_u32, want * 4, &dummy, s->stream));
-        }
-        CKL(launch_unpack_counts16(s->d_sys, s->d_u32, (int64_t)want, s->stream));
-        CK(cudaMemcpyAsync(out, s->d_u32, want * 4, cudaMemcpyDeviceToHost, s->stream));
-    } else {
-        CK(cudaMemcpyAsync(out, s->counts[d.cur & 1u], want * 4, cudaMemcpyDeviceToHost, s->stream));
+    if (s->spec.p.count_bits != 16) return copy_to_host(out, s->counts[0], want * 4, s->stream);  // the current grid
+    if (!s->d_u32) {
+        size_t dummy = 0;
+        RET(dalloc(&s->d_u32, want * 4, &dummy, s->stream));
     }
-    CK(cudaStreamSynchronize(s->stream));
-    return SCMF_OK;
+    CKL(launch_unpack_counts16(s->d_sys, s->d_u32, (int64_t)want, s->stream));
+    return copy_to_host(out, s->d_u32, want * 4, s->stream);
 }
 
 scmf_status scmf_get_omega(const scmf_system* s, float* out, size_t n) {
     if (!s || !out) return fail(SCMF_E_INVALID, "NULL argument");
     const size_t want = (size_t)s->n_cells * s->spec.n_types;
     if (n != want) return fail(SCMF_E_INVALID, "expected %zu values, got %zu", want, n);
-    CK(cudaMemcpyAsync(out, s->omega, want * 4, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-    return SCMF_OK;
+    return copy_to_host(out, s->omega, want * 4, s->stream);
 }
 
 scmf_status scmf_set_omega(scmf_system* s, const float* in, size_t n) {

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 #include <utility>
 #include <vector>
@@ -44,6 +45,16 @@ struct ArchHost {
     int color_off[kMaxColors + 1] = {};
 };
 
+// Copies between the device and the caller's host memory (scmf_stage.cpp): large
+// ones to and from pageable memory through a pinned buffer and several threads.
+// copy_to_host waits for the stream and the copy.  copy_to_device_staged makes
+// the copy if it is one of those (else false), calling `enqueued` after every
+// piece with the bytes that the stream's copies so far cover, and waits for it.
+scmf_status copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
+bool copy_to_device_staged(void* dev, const void* host, size_t bytes, cudaStream_t st,
+                           const std::function<scmf_status(size_t)>& enqueued, scmf_status* rc);
+void stage_system_made();  // a system's life: the buffer is freed with the last one
+void stage_system_gone();
 // Stream-ordered device memory (cudaMallocAsync / cudaFreeAsync on the
 // device's default pool, kept cached): creating and destroying systems and
 // plans never synchronises the device.
@@ -134,6 +145,7 @@ struct scmf_system {
     scmf_spec spec;  // for a chain shard: the shard's own chain counts
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    bool counted = false;  // in stage_system_made()
     int device = 0;
     int64_t n_beads = 0, n_cells = 0;
     // chain shard `shard` of `n_shards` (n_shards == 1: a whole system); n_beads_total

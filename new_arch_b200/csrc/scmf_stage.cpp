@@ -1,0 +1,189 @@
+// Large copies between the GPU and pageable host memory.
+//
+// The driver stages such a copy on one thread: 4.6 GB/s into memory whose pages
+// are new (an array that numpy has just made), where the link carries 55 GB/s.
+// Here several threads move the pieces between the caller's memory and a small
+// pinned buffer while the copy engine moves the others: 600 MB to the host in 26 ms
+// instead of 121 (eight threads on sixteen cores), from the host in 15 instead of
+// 53; 70 MB in 3.5 instead of 14.8 and in 3.1 instead of 5.3.  Below kStageFrom,
+// into memory that is pinned already, and while another copy holds the buffer, a
+// copy is the driver's: into memory that has been touched before it takes 0.46 ms
+// for 8 MB, where starting threads and pieces costs as much as it saves.
+//
+// The buffer (kPieces * kPieceBytes) is allocated at the first large copy, shared
+// by all systems of the process and freed with the last of them.
+#include <cstring>
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "scmf_engine.h"
+
+namespace scmf {
+
+#define CK(expr)                                                                                   \
+    do {                                                                                           \
+        cudaError_t e_ = (expr);                                                                   \
+        if (e_ != cudaSuccess) return fail(SCMF_E_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
+    } while (0)
+
+namespace {
+
+constexpr size_t kStageFrom = 64u << 20;  // from here the copy gains more than making the buffer costs
+constexpr size_t kPieceBytes = 1u << 20;
+constexpr int kPieces = 12;
+
+std::mutex g_mu;               // the buffer's user, and the two below
+char* g_buffer = nullptr;
+int g_systems = 0;             // systems alive
+
+bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// One staged copy: pieces 0 .. n-1 in order, piece k in slot k % kPieces.
+// state[k]: 0 not begun, 1 in the buffer (to the device) or asked for (to the
+// host), 2 asked for (to the device) or delivered (to the host).
+struct Transfer {
+    int device = 0, n = 0;
+    bool to_host = false;
+    char* host = nullptr;
+    char* dev = nullptr;
+    size_t bytes = 0;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done[kPieces] = {};  // the slot's last copy
+    std::vector<std::atomic<int>> state;
+    std::atomic<int> next{0};
+    std::atomic<int> error{0};  // cudaError_t
+
+    size_t size_of(int k) const { return std::min(kPieceBytes, bytes - (size_t)k * kPieceBytes); }
+    char* slot(int k) const { return g_buffer + (size_t)(k % kPieces) * kPieceBytes; }
+    // Waits for state[k] >= s; false when the copy has failed.
+    bool wait(int k, int s) {
+        while (state[k].load(std::memory_order_acquire) < s) {
+            if (error.load(std::memory_order_relaxed)) return false;
+            std::this_thread::yield();
+        }
+        return true;
+    }
+    bool ok(cudaError_t e) {
+        if (e != cudaSuccess) error.store((int)e);
+        return e == cudaSuccess;
+    }
+    void work() {
+        if (!ok(cudaSetDevice(device))) return;
+        for (;;) {
+            const int k = next.fetch_add(1);
+            if (k >= n || error.load()) return;
+            char* h = host + (size_t)k * kPieceBytes;
+            if (to_host) {
+                if (!wait(k, 1) || !ok(cudaEventSynchronize(done[k % kPieces]))) return;
+                std::memcpy(h, slot(k), size_of(k));
+                state[k].store(2, std::memory_order_release);
+            } else {
+                if (k >= kPieces && (!wait(k - kPieces, 2) || !ok(cudaEventSynchronize(done[k % kPieces])))) return;
+                std::memcpy(slot(k), h, size_of(k));
+                state[k].store(1, std::memory_order_release);
+            }
+        }
+    }
+};
+
+// False: not staged, nothing done.
+bool staged(void* dev, void* host, size_t bytes, bool to_host, cudaStream_t st,
+            const std::function<scmf_status(size_t)>& enqueued, scmf_status* rc) {
+    if (bytes < kStageFrom || !pageable(host)) return false;
+    if (to_host && cudaStreamSynchronize(st) != cudaSuccess) return false;  // no thread spins on earlier work
+    std::unique_lock<std::mutex> lock(g_mu, std::try_to_lock);
+    if (!lock.owns_lock()) return false;
+    if (!g_buffer && cudaHostAlloc((void**)&g_buffer, kPieces * kPieceBytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        g_buffer = nullptr;
+        return false;
+    }
+    Transfer t;
+    t.n = (int)((bytes + kPieceBytes - 1) / kPieceBytes);
+    t.to_host = to_host;
+    t.host = (char*)host;
+    t.dev = (char*)dev;
+    t.bytes = bytes;
+    t.stream = st;
+    std::vector<std::thread> threads;
+    bool ready = cudaGetDevice(&t.device) == cudaSuccess;
+    for (auto& e : t.done) ready = ready && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (ready) {
+        try {
+            t.state = std::vector<std::atomic<int>>((size_t)t.n);
+            const unsigned cores = std::thread::hardware_concurrency();
+            const int want = (int)std::max(2u, std::min(8u, cores / 2));
+            for (int i = 0; i < want; ++i) threads.emplace_back([&t] { t.work(); });
+        } catch (...) {
+            ready = !threads.empty();  // as many as there are
+        }
+    }
+    *rc = SCMF_OK;
+    for (int k = 0; ready && k < t.n && *rc == SCMF_OK; ++k) {
+        char* d = t.dev + (size_t)k * kPieceBytes;
+        if (to_host) {
+            if (k >= kPieces && !t.wait(k - kPieces, 2)) break;
+            if (!t.ok(cudaMemcpyAsync(t.slot(k), d, t.size_of(k), cudaMemcpyDeviceToHost, st))) break;
+        } else {
+            if (!t.wait(k, 1)) break;
+            if (!t.ok(cudaMemcpyAsync(d, t.slot(k), t.size_of(k), cudaMemcpyHostToDevice, st))) break;
+        }
+        if (!t.ok(cudaEventRecord(t.done[k % kPieces], st))) break;
+        t.state[k].store(to_host ? 1 : 2, std::memory_order_release);
+        if (enqueued) {
+            *rc = enqueued((size_t)k * kPieceBytes + t.size_of(k));
+            if (*rc != SCMF_OK) t.error.store((int)cudaErrorUnknown);
+        }
+    }
+    for (auto& th : threads) th.join();
+    const cudaError_t end = cudaStreamSynchronize(st);  // the buffer is free again
+    for (auto& e : t.done)
+        if (e) cudaEventDestroy(e);
+    if (!ready) {
+        cudaGetLastError();
+        return false;
+    }
+    if (*rc == SCMF_OK && (t.error.load() || end != cudaSuccess))
+        *rc = fail(SCMF_E_CUDA, "staged copy: %s", cudaGetErrorString(t.error.load() ? (cudaError_t)t.error.load() : end));
+    return true;
+}
+
+}  // namespace
+
+scmf_status copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st) {
+    scmf_status rc;
+    if (staged(const_cast<void*>(dev), host, bytes, true, st, nullptr, &rc)) return rc;
+    CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return SCMF_OK;
+}
+
+bool copy_to_device_staged(void* dev, const void* host, size_t bytes, cudaStream_t st,
+                           const std::function<scmf_status(size_t)>& enqueued, scmf_status* rc) {
+    return staged(dev, const_cast<void*>(host), bytes, false, st, enqueued, rc);
+}
+
+void stage_system_made() {
+    std::lock_guard<std::mutex> g(g_mu);
+    ++g_systems;
+}
+
+void stage_system_gone() {
+    std::lock_guard<std::mutex> g(g_mu);
+    if (--g_systems == 0 && g_buffer) {
+        cudaFreeHost(g_buffer);
+        g_buffer = nullptr;
+    }
+}
+
+}  // namespace scmf

@@ -129,7 +129,7 @@ struct DevPlan {
     LaunchShape field_shape() const;
     // one fused sweep enqueued on `st`: the move launch, then the field launch
     // whose last tile per system closes the sweep
-    scmf_status enqueue_sweep(cudaStream_t st) const;
+    scmf_status enqueue_sweep(cudaStream_t st, bool last) const;
     scmf_status enqueue_move(cudaStream_t st) const;
     scmf_status enqueue_field(cudaStream_t st) const;
     scmf_status enqueue_close(int mode, cudaStream_t st) const;

@@ -235,7 +235,8 @@ enum SweepMode : int { kMoveOnly = 0, kMoveGrid = 1, kGridOnly = 2 };
 enum CloseMode : int {
     kCloseMove = 1, kCloseField = 2, kCloseBond = 4, kCloseAdvance = 16,
     kCloseAverage = 32,  // count a time-averaged density sample when the sweep took one
-    kSweepClose = kCloseMove | kCloseField | kCloseAdvance | kCloseAverage
+    kSweepClose = kCloseMove | kCloseField | kCloseAdvance | kCloseAverage,
+    kSweepOn = kSweepClose & ~kCloseField  // of a sweep that another one follows in the same call
 };
 
 // Per-tile partial sums of the chain observables (k_observables), each over
@@ -309,6 +310,7 @@ struct LaunchShape {
     int form;           // SweepFormId
     int one;            // the launch has one system: `system`, with the constants `sweep` and n_arch tile ranges
     int once;           // the positions are more than L2 holds
+    int chained;        // the kernel before in the stream is this plan's: the launch may begin beside its last blocks
     SysDev* system;
     SweepSys sweep;
     int n_arch;

@@ -639,32 +639,42 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x) {
         const FieldTile t = tiles[ti];
         SysDev* S = t.sys;
-        if (FUSED && S->step >= S->stop_step) continue;  // block-uniform: the system's sweeps are done
         for (int i = tid; i < kMaxTypes * kMaxTypes; i += T) cf[i] = S->cf[i];
-        __syncthreads();
-        const uint32_t cur = S->cur;
-        const uint32_t sweep = S->step + 1u;
-        const bool upd = force_update || S->field_rule == 1 || (sweep % 10u) != 0u;
-        const int n = S->n_types;
+        const int n = S->n_types, rule = S->field_rule;
         const int64_t NC = S->n_cells;
         const float scale = S->scale;
         const bool lit = S->hamiltonian == 1;
         const bool c16 = S->count16 != 0;
-        const uint32_t* src32 = S->field_counts ? S->field_counts : S->counts[cur];
+        const uint32_t* src32 = S->field_counts ? S->field_counts : S->counts[S->cur];
         float* W = S->omega;
+        unsigned long long* avg = FUSED && S->avg_every ? S->avg : nullptr;
+        const uint32_t avg_every = S->avg_every, stop = S->stop_step;
+        // all that a sweep leaves as it is has been read; a launch beside the move kernel's
+        // last blocks (LaunchShape::chained) waits for the rest of it here
+        if (FUSED && ti == (int)blockIdx.x) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        }
+        __syncthreads();
+        const uint32_t sweep = S->step + 1u;
+        if (FUSED && sweep > stop) continue;  // block-uniform: the system's sweeps are done
+        const bool upd = force_update || rule == 1 || (sweep % 10u) != 0u;
         // the fused sweep samples the time-averaged density at every avg_every-th sweep
-        unsigned long long* avg = FUSED && S->avg && S->avg_every && (sweep % S->avg_every) == 0u ? S->avg : nullptr;
+        if (avg && sweep % avg_every != 0u) avg = nullptr;
+        // the energy of a sweep that another one follows in the same call is not asked for
+        const int mode = FUSED && sweep == stop ? close_mode | kCloseField : close_mode;
+        const bool energy = !FUSED || (mode & kCloseField) != 0;
         double ef = 0.0;
         float wmax = -INFINITY, wmin = INFINITY;  // omega of the tile's cells (new or kept)
         const int64_t end = t.cell0 + t.n_cells;
         if (NT > 0 && !c16 && (NC & 3) == 0 && (t.cell0 & 3) == 0 && (t.n_cells & 3) == 0) {
             for (int64_t cell = t.cell0 + 4 * tid; cell < end; cell += 4 * T)
-                ef += field_cells4<(NT > 0 ? NT : 1), false>(cell, NC, scale, lit, upd, src32, W, cf, avg, wmax, wmin);
+                ef += field_cells4<(NT > 0 ? NT : 1), false>(cell, NC, scale, lit, upd, src32, W, cf, avg, wmax, wmin, energy);
         } else {
             for (int64_t cell = t.cell0 + tid; cell < end; cell += T)
-                ef += field_cell<NT, false>(n, cell, NC, scale, lit, upd, c16, src32, W, cf, avg, wmax, wmin);
+                ef += field_cell<NT, false>(n, cell, NC, scale, lit, upd, c16, src32, W, cf, avg, wmax, wmin, energy);
         }
-        ef = warp_sum(ef);
+        if (energy) ef = warp_sum(ef);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
@@ -679,11 +689,11 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
         if (tid == 0) {
             double e = 0.0;
             for (int w = 0; w < (T + 31) / 32; ++w) {
-                e += s_ef[w];
+                if (energy) e += s_ef[w];
                 wmax = fmaxf(wmax, s_mx[w]);
                 wmin = fminf(wmin, s_mn[w]);
             }
-            ef_part[ti] = e;
+            if (energy) ef_part[ti] = e;
             if (wmax >= wmin) {  // the tile held a non-NaN omega
                 atomicMax(&S->om_max_key, ord_key(wmax));
                 atomicMin(&S->om_min_key, ord_key(wmin));
@@ -699,7 +709,7 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
         __syncthreads();
         if (close_mode && s_last) {
             __threadfence();
-            if (tid == 0) {
+            if (tid == T - 1) {
                 // every tile of the system has folded its omega in: publish the
                 // span (+inf when no bound is known) and reset the keys
                 const uint32_t kx = atomicExch(&S->om_max_key, 0u);
@@ -707,7 +717,7 @@ __global__ void __launch_bounds__(256) k_field(const FieldTile* __restrict__ til
                 const float span = kx >= kn ? __fsub_rn(ord_val(kx), ord_val(kn)) : INFINITY;
                 S->omega_span = span >= 0.0f ? span : INFINITY;  // NaN (inf - inf): no bound
             }
-            close_system(S, ef_part + t.first_tile, t.n_tiles_sys, close_mode, s_acc, s_ef);
+            close_system(S, ef_part + t.first_tile, t.n_tiles_sys, mode, s_acc, s_ef);
             if (tid == 0) S->field_done = 0u;
         }
         __syncthreads();
@@ -1090,17 +1100,32 @@ static void launch_general(const MoveTile* tiles, int n_tiles, int blocks, int m
         k_sweep<MODE, kKeysNone><<<blocks, sh.threads, smem, st>>>(tiles, n_tiles, mtb, ml, sh.keys);
 }
 
+// A launch that may begin (set up its shared memory, wait) beside the last blocks of
+// the kernel before, where `chained`.
+template <typename... Args>
+static cudaError_t launch_chained(void (*kernel)(Args...), int blocks, int threads, int smem, bool chained, cudaStream_t st,
+                                  typename std::common_type<Args>::type... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // The launch of a plan's warp tiles: k_sweep_warp, or k_run when `run` is given.
 template <bool ONE, int FORM, int KEYS>
-static cudaError_t launch_form(const SweepArgs& a, const RunArgs* run, cudaStream_t st) {
+static cudaError_t launch_form(const SweepArgs& a, const RunArgs* run, bool chained, cudaStream_t st) {
     using Lay = SweepLayout<FORM>;
     const int sms = sm_count(), grid = a.n_tiles < sms ? a.n_tiles : sms;
     const int per_sm = (a.n_tiles + grid - 1) / grid, nw = per_sm < Lay::kWarps ? per_sm : Lay::kWarps;
     const int smem = Lay::kTabBytes + nw * (int)sizeof(typename Lay::Warp) + kSlack;
-    if (!run) {
-        k_sweep_warp<ONE, FORM, KEYS><<<grid, 32 * nw, smem, st>>>(a);
-        return cudaGetLastError();
-    }
+    if (!run) return launch_chained(k_sweep_warp<ONE, FORM, KEYS>, grid, 32 * nw, smem, chained, st, a);
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeCooperative;  // the blocks wait for one another
     at.val.cooperative = 1;
@@ -1115,11 +1140,11 @@ static cudaError_t launch_form(const SweepArgs& a, const RunArgs* run, cudaStrea
 }
 
 template <bool ONE, int KEYS>
-static cudaError_t launch_warp(const SweepArgs& a, int form, const RunArgs* run, cudaStream_t st) {
-    if (form == kFormLong) return launch_form<ONE, kFormLong, KEYS>(a, run, st);
-    if (form == kFormUnscreened) return launch_form<ONE, kFormUnscreened, KEYS>(a, run, st);
-    if (form == kFormGraph) return launch_form<ONE, kFormGraph, KEYS>(a, run, st);
-    return launch_form<ONE, kFormScreened, KEYS>(a, run, st);
+static cudaError_t launch_warp(const SweepArgs& a, int form, const RunArgs* run, bool chained, cudaStream_t st) {
+    if (form == kFormLong) return launch_form<ONE, kFormLong, KEYS>(a, run, chained, st);
+    if (form == kFormUnscreened) return launch_form<ONE, kFormUnscreened, KEYS>(a, run, chained, st);
+    if (form == kFormGraph) return launch_form<ONE, kFormGraph, KEYS>(a, run, chained, st);
+    return launch_form<ONE, kFormScreened, KEYS>(a, run, chained, st);
 }
 
 static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const RunArgs* run, cudaStream_t st) {
@@ -1133,9 +1158,9 @@ static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const Ru
     a.sys = sh.sweep;
     a.n_arch = sh.n_arch;
     for (int i = 0; i < sh.n_arch; ++i) a.arch[i] = sh.arch[i];
-    if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.form, run, st);
-    if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.form, run, st);
-    return launch_warp<false, kKeysNone>(a, sh.form, run, st);
+    if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.form, run, sh.chained != 0, st);
+    if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.form, run, sh.chained != 0, st);
+    return launch_warp<false, kKeysNone>(a, sh.form, run, sh.chained != 0, st);
 }
 
 int launch_run(const LaunchShape& sh, const RunArgs& run, void* stream) {
@@ -1161,15 +1186,9 @@ int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int mtb, int ml, 
 
 template <bool FUSED>
 static void launch_field_t(int nt, const FieldTile* tiles, int n_tiles, int force_update, int blocks, int threads,
-                           double* ef, int close_mode, cudaStream_t st) {
-    if (nt == 2)
-        k_field<FUSED, 2><<<blocks, threads, 0, st>>>(tiles, n_tiles, force_update, ef, close_mode);
-    else if (nt == 3)
-        k_field<FUSED, 3><<<blocks, threads, 0, st>>>(tiles, n_tiles, force_update, ef, close_mode);
-    else if (nt == 1)
-        k_field<FUSED, 1><<<blocks, threads, 0, st>>>(tiles, n_tiles, force_update, ef, close_mode);
-    else
-        k_field<FUSED, 0><<<blocks, threads, 0, st>>>(tiles, n_tiles, force_update, ef, close_mode);
+                           double* ef, int close_mode, bool chained, cudaStream_t st) {
+    const auto k = nt == 2 ? k_field<FUSED, 2> : nt == 3 ? k_field<FUSED, 3> : nt == 1 ? k_field<FUSED, 1> : k_field<FUSED, 0>;
+    launch_chained(k, blocks, threads, 0, chained, st, tiles, n_tiles, force_update, ef, close_mode);
 }
 
 int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_tiles, LaunchShape sh, double* ef_part,
@@ -1179,9 +1198,9 @@ int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_til
     const int blocks = sh.blocks > 0 ? sh.blocks : n_tiles;
     const int threads = sh.threads > 256 ? 256 : sh.threads;
     if (fused)
-        launch_field_t<true>(sh.n_types, tiles, n_tiles, force_update, blocks, threads, ef_part, close_mode, st);
+        launch_field_t<true>(sh.n_types, tiles, n_tiles, force_update, blocks, threads, ef_part, close_mode, sh.chained != 0, st);
     else
-        launch_field_t<false>(sh.n_types, tiles, n_tiles, force_update, blocks, threads, ef_part, close_mode, st);
+        launch_field_t<false>(sh.n_types, tiles, n_tiles, force_update, blocks, threads, ef_part, close_mode, false, st);
     return (int)cudaGetLastError();
 }
 

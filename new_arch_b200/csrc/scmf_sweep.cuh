@@ -715,7 +715,7 @@ struct Mover {
     SysDev* S = nullptr;
     const ArchDev* A = nullptr;
     const uint8_t* types = nullptr;
-    uint32_t rng_base = 0u, parity = 0u;
+    uint32_t rng_base = 0u, h_magic = 0u, parity = 0u;
     float span = 0.0f;
     int mode = 0;  // 0: the system's sweeps are done; 1: resolve every trial; 2: screen
 
@@ -739,13 +739,12 @@ struct Mover {
         bulk_load(dst + 8u * Lay::kStride, c.z + g, bytes, bar, a.once != 0);
     }
 
-    // All threads of the block: the tables, the warp's barrier, and its first tile on the way.
+    // All threads of the block: the tables, the warp's barrier, and its first tile on
+    // the way (as soon as the kernel before, if this one may begin beside it, is done).
     __device__ __forceinline__ void start(unsigned char* smem, const WarpTile& t, bool any) {
         if (lane == 0) {
             mbar_init(smem_addr(&wp->full));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            fence_async();
-            if (any) load(t);
         }
         wp->moved[lane] = 0u;
         float4* tab = reinterpret_cast<float4*>(smem);
@@ -754,12 +753,17 @@ struct Mover {
         if (FORM != kFormUnscreened)
             for (int i = threadIdx.x; i < SCMF_SCREEN_SEGS * kScreenCopies; i += blockDim.x)
                 screen[i] = __ldg(screen_table() + i / kScreenCopies);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (lane == 0) {
+            fence_async();
+            if (any) load(t);
+        }
         __syncthreads();
     }
 
-    // Turns to a tile's architecture.  `done`: sweeps of its system made before
-    // this one; omega_span: its omega's.
-    __device__ __forceinline__ void turn_to(const WarpTile& t, uint32_t done, bool active, float omega_span) {
+    // Turns to a tile's architecture (what no sweep changes of it); set() has the rest.
+    __device__ __forceinline__ void turn_to(const WarpTile& t) {
         if (!ONE && t.sys != S) {
             __syncwarp();
             const uint32_t* src = reinterpret_cast<const uint32_t*>(&t.sys->sweep);
@@ -775,11 +779,12 @@ struct Mover {
         A = t.arch;
         types = A->types;
         rng_base = (uint32_t)A->rng_base;
-        set(A->length, A->tpc_magic, done, active, omega_span);
+        h_magic = A->tpc_magic;
     }
 
-    // The constants of a sweep of chains of L beads.
-    __device__ __forceinline__ void set(int L, uint32_t h_magic, uint32_t done, bool active, float omega_span) {
+    // The constants of a sweep of chains of L beads.  `done`: sweeps of the system made
+    // before this one; omega_span: its omega's.
+    __device__ __forceinline__ void set(int L, uint32_t done, bool active, float omega_span) {
         const SweepSys& c = sys();
         span = omega_span;
         s.L = L;
@@ -878,6 +883,9 @@ __device__ __forceinline__ WarpTile tile_at(const SweepArgs& a, int i) {
 // with a quarter, a half, three quarters or all of its first one (by its place
 // among the four warps of its SM sub-partition) and ends with the rest: 0.322 ->
 // 0.313 ms on the large system.
+//
+// A chained launch (LaunchShape::chained) reads only what no sweep changes before
+// griddepcontrol.wait in start().
 template <bool ONE, int FORM, int KEYS>
 __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_warp(const __grid_constant__ SweepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -893,6 +901,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_war
     const int parts = turns + (begin < whole.n_chains ? 1 : 0);
     t.n_chains = begin;
     t.n_beads = begin * t.length;
+    if (turns > 0) m.turn_to(t);  // may run beside the field step before (start)
     m.start(smem_raw, t, turns > 0);
 #pragma unroll 1
     for (int q = 0; q < parts; ++q) {
@@ -905,7 +914,12 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_war
             next.n_chains -= begin;
             next.n_beads -= begin * next.length;
         }
-        if (t.arch != m.A) m.turn_to(t, t.sys->step, t.sys->step < t.sys->stop_step, t.sys->omega_span);
+        if (q == 0 || t.arch != m.A) {
+            const uint32_t step = t.sys->step, stop = t.sys->stop_step;
+            const float omega_span = t.sys->omega_span;
+            if (q) m.turn_to(t);
+            m.set(t.length, step, step < stop, omega_span);
+        }
         if (!m.arrived()) return;
         unsigned nacc = m.move(t, true);
         fence_async();  // this lane's reads and writes of the buffer, before the next copies land
@@ -1105,13 +1119,13 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
         m.start(smem_raw, t, any);
         if (any) {
             const uint32_t base = t.sys->step, stop = t.sys->stop_step;
-            m.turn_to(t, base, base < stop, 0.0f);
+            m.turn_to(t);
             const bool here = m.arrived();
             if (lane == 0) {
                 wp->run.tile = t;
                 wp->run.types = m.types;
                 wp->run.rng_base = m.rng_base;
-                wp->run.h_magic = m.s.h_magic;
+                wp->run.h_magic = m.h_magic;
                 wp->run.base = base;
                 wp->run.stop = stop;
                 wp->run.rule = t.sys->field_rule;
@@ -1164,7 +1178,8 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 span = __fmul_rn(span_now, kSpanAhead);
                 if (FORM == kFormUnscreened || !(span < INFINITY)) continue;
             }
-            m.set(t.length, wp->run.h_magic, done, true, span);
+            m.h_magic = wp->run.h_magic;
+            m.set(t.length, done, true, span);
             const bool ahead = m.mode == 2 && !m.graph();  // a system whose screen may run ahead
             if (pass == 0 ? !m.graph() && !(span <= screened_to) : ahead) m.screen(t, even, odd);
             if (pass == 0) {

@@ -312,11 +312,11 @@ void fill_sweep_constants(SysDev* d) {
     w.seed_hi = d->seed_hi;
     w.count16 = d->count16;
     w.screen = screen_constants(*d);
-    d->by_deg[0] = make_float4(0.0f, INFINITY, 0.0f, 0.0f);  // no bond, nothing to screen by
+    d->by_deg[0] = BondConsts{0.0f, INFINITY, 0.0f, 0.0f};  // no bond, nothing to screen by
     for (int g = 1; g <= kGraphDeg; ++g) {
         float a, b;
         if (!screen_of(*d, g, &a, &b)) w.screen.on = 0;
-        d->by_deg[g] = make_float4(a, b, d->cdeg[g], d->ac4deg[g]);
+        d->by_deg[g] = BondConsts{a, b, d->cdeg[g], d->ac4deg[g]};
     }
     FieldSys& f = d->field;
     f.counts = d->counts[0];

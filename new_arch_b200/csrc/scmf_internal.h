@@ -9,7 +9,7 @@
 //   chain_id     uint32[n_chains]     storage slot -> global chain id (the first
 //                                      Philox counter word).  Storage order is the id
 //                                      order within each architecture (chain_id[chain_base
-//                                      + c] = rng_base + c), which the lean kernels use to
+//                                      + c] = rng_base + c), which the kernels of warp tiles use to
 //                                      compute the id instead of loading it; the other
 //                                      kernels read this table.
 //   counts[2]    uint32[n_types*n_cells] (or uint16 pairs)  per-type cell counts,
@@ -51,6 +51,11 @@ struct alignas(16) GraphBead {
     uint16_t bead;
     uint8_t deg, type;
     uint16_t nbr[kGraphDeg];
+};
+
+// Of the beads of some number of bonds: ScreenDev's a and b, c = 2k deg, A c / 4.
+struct alignas(16) BondConsts {
+    float a, b, c, ac4;
 };
 
 // One polymer architecture of one system.
@@ -192,7 +197,7 @@ struct SysDev {
     uint32_t om_keys[3][2];
     unsigned long long slot_last[kSlots];  // k_run: accepted moves of its last sweep
     SweepSys sweep;
-    float4 by_deg[kGraphDeg + 1];  // of a bead with that many bonds: ScreenDev's a and b, c = 2k deg, A c / 4
+    BondConsts by_deg[kGraphDeg + 1];  // of a bead with that many bonds
     FieldSys field;
     // the statistics of the last sweep in the public layout, written by
     // k_stats_out for asynchronous reads (scmf_step_stats_async)

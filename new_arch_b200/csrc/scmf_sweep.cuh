@@ -138,7 +138,7 @@ struct SweepLayout {
         uint32_t moved[32];    // odd beads next to an even bead that moved: a bit for each row, a word for each lane
         uint16_t list[kListLen];
         SweepSys sys;          // of the tile's system, where a launch has several
-        float4 by_deg[FORM == kFormGraph ? kGraphDeg + 1 : 1];  // SysDev's
+        BondConsts by_deg[FORM == kFormGraph ? kGraphDeg + 1 : 1];  // SysDev's
         // k_run, which has registers for one phase of a sweep at a time: the warp's
         // tile and its architecture, the sweeps that its system has made and makes
         // in all, and the warp's field tile and its system

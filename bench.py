@@ -224,15 +224,15 @@ def run_ours(args):
         return reduce_max(v, dist, "cuda")
 
     # ---- plain large system: the headline step (one replica per rank).  The K
-    # sweeps are timed as the library runs them (scmf_step_async: one CUDA
-    # graph replay per sweep) between CUDA events on the system's stream; a
+    # sweeps are timed as the library runs them (scmf_step_async: two chained
+    # launches per sweep) between CUDA events on the system's stream; a
     # second pass of K sweeps launch by launch, each launch between events,
     # gives the per-kernel times of the roofline and the phases.
     stream = torch.cuda.Stream()
     spec = large_system(seed=replica_seed(7, rank))
     s = nb.System(spec, stream=stream.cuda_stream)
     s.init_coords()
-    s.step(args.warmup)  # also captures the sweep's graph
+    s.step(args.warmup)
     sampler = ClockSampler(local)
     barrier()
     torch.cuda.synchronize()
@@ -253,9 +253,9 @@ def run_ours(args):
     beads_all = gather_ints(spec.n_beads, dist, "cuda")
     value = whole_job_rate(beads_all, args.steps, ms_total / 1e3)
     peak, peak_kind = measured_peaks()
-    # move+grid kernel per launch: read and write x, y, z (counts change only for
-    # accepted moves that leave their cell, ~1 % of beads here: not counted)
-    alg_bytes = 24 * spec.n_beads
+    # move+grid kernel per launch: read x, y, z, write those of the beads that move
+    # (counts change only for accepted moves that leave their cell: not counted)
+    alg_bytes = 12 * (spec.n_beads + st["last_accepts"])
     achieved = alg_bytes / (ms_move / args.steps / 1e3) / 1e9
     traffic = profiled_traffic("sweep_large_system")
     field_bytes = 8 * spec.n_types * spec.n_cells                           # read counts, write omega
@@ -298,12 +298,12 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind, "kernel": "k_sweep_warp (move+grid)",
                          "alg_bytes_per_launch": alg_bytes,
-                         "traffic": traffic.get("dram_bytes_per_launch") if traffic else None,
+                         "traffic": traffic["dram_bytes_per_bead"] * spec.n_beads if traffic else None,
                          "ms_per_launch": ms_move / args.steps},
             "phases": {"move_grid_ms": ms_move / args.steps, "field_ms": ms_field / args.steps,
                        "field_gbs": field_gbs, "field_frac": field_gbs / peak,
                        "profiled_ms_per_step": ms_profiled / args.steps,
-                       "timing": "value: K graph-replayed sweeps between CUDA events on the system's stream; "
+                       "timing": "value: K sweeps as the library launches them between CUDA events on the system's stream; "
                                  "phases: K more sweeps launch by launch, each launch between events"}}
 
     # ---- the blend (largest single-GPU configuration), batched vs plain on the
@@ -345,13 +345,13 @@ def run_blend(nb, args, peak):
         s.step(args.warmup)
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         ev0.record(stream)
-        s.step_async(K)  # graph replay, as for the large system
+        s.step_async(K)  # as the large system
         ev1.record(stream)
         ev1.synchronize()
         ms_total = ev0.elapsed_time(ev1)
         ms_move, ms_field, _ = s.step_profiled(K)
         st = s.stats()
-    move_gbs = 24 * spec.n_beads / (ms_move / K / 1e3) / 1e9
+    move_gbs = 12 * (spec.n_beads + st["last_accepts"]) / (ms_move / K / 1e3) / 1e9
     field_gbs = 8 * spec.n_types * spec.n_cells / (ms_field / K / 1e3) / 1e9
     return {"workload": "blend: 50% A-homopolymer N=64, 40% B-homopolymer N=64, 10% AB diblock N=32; 2M chains "
                         "(121.6M beads), 256x256x64 cells, chiN=15 (N_ref=64), kappaN=40, seed 11",
@@ -371,7 +371,7 @@ def run_batched(nb, batched_mix, args, torch, peak):
     beads = sum(sp.n_beads for sp in specs)
     K = args.batched_sweeps
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    # plain engine: one system at a time, each with its own graph-launched sweeps
+    # plain engine: one system at a time, each with its own sweeps
     for x in systems:
         x.step_async(1)
     torch.cuda.synchronize()
@@ -391,7 +391,7 @@ def run_batched(nb, batched_mix, args, torch, peak):
     e1.record(st)
     e1.synchronize()
     batched_ms = e0.elapsed_time(e1)
-    # per-phase device time of the batched sweeps (launch by launch, no graph)
+    # per-phase device time of the batched sweeps (launch by launch)
     pm, pf, _ = b.step_profiled(10)
     cells_all = sum(sp.n_cells * sp.n_types for sp in specs)
     b.close()
@@ -400,17 +400,11 @@ def run_batched(nb, batched_mix, args, torch, peak):
     plain = beads * K / (plain_ms / 1e3)
     batched = beads * K / (batched_ms / 1e3)
 
-    def move_launches(lengths):
-        # one register-kernel launch per tile kind: chains filling warps exactly, chains across warps
-        kinds = {32 % ((n + 1) // 2) != 0 for n in lengths}
-        return len(kinds)
-    per_sys = sum(1 + move_launches([a.length for a in sp.archs]) for sp in specs)
-    per_batch = 1 + move_launches([a.length for sp in specs for a in sp.archs])
     return {"workload": "256 diblock systems, edges {16..64}^3, N {16..64}, 100 sweeps each", "beads": beads,
             "sweeps": K, "plain_bead_moves_per_s": plain, "batched_bead_moves_per_s": batched,
-            "batched_over_plain": batched / plain, "tune": tune, "gpu_launches_batched": per_batch * K,
-            "gpu_launches_plain": per_sys * K,
-            "move_frac": 24 * beads / (pm / 10 / 1e3) / 1e9 / peak,
+            "batched_over_plain": batched / plain, "tune": tune, "gpu_launches_batched": 2 * K,
+            "gpu_launches_plain": len(specs),  # each on the chip: all its sweeps in one launch
+            "move_frac": 12 * beads / (pm / 10 / 1e3) / 1e9 / peak,
             "field_frac": 8 * cells_all / (pf / 10 / 1e3) / 1e9 / peak,
             "phase_ms": {"move": pm / 10, "field": pf / 10},
             "tune_trials": [{"beads_per_tile": t["beads_per_tile"], "threads_move": t["threads_move"],

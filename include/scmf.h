@@ -357,9 +357,9 @@ scmf_status scmf_analysis_reference(scmf_system* sys);
 scmf_status scmf_analyze(const scmf_system* sys, scmf_observables* out, int32_t n_arch);
 
 /* -------------------------------------------------------------- batched */
-/* Many independent systems advanced together: one persistent kernel per
- * phase over a work list of (system, chain tile) and (system, cell tile),
- * captured once in a CUDA graph.  No reference counterpart (the reference runs
+/* Many independent systems advanced together: one launch per phase and sweep,
+ * or one for many sweeps, over a work list of (system, chain tile) and (system,
+ * cell tile).  No reference counterpart (the reference runs
  * one system per process). */
 typedef struct scmf_batch scmf_batch;
 
@@ -369,7 +369,8 @@ typedef struct scmf_tune {
     int32_t cells_per_tile;    /* 0 = default */
     int32_t threads_field;     /* 0 = default */
     int32_t persistent_ctas;   /* 0 = one CTA per tile (no persistence) */
-    int32_t use_graph;         /* 1 = capture one sweep in a CUDA graph */
+    int32_t use_graph;         /* 1 = a sweep that takes launches of its own may be replayed from a
+                                  CUDA graph */
     int32_t beads_per_tile;    /* > 0: chains per tile = max(1, beads_per_tile / length) for each
                                   architecture (takes precedence over chains_per_tile) */
     int32_t reserved;

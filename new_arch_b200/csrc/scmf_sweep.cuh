@@ -1043,6 +1043,12 @@ __device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r,
     __syncthreads();
 }
 
+// The error word of every system of a launch whose blocks did not come to a barrier.
+__device__ __forceinline__ void flag_run(const RunArgs& r) {
+    if (threadIdx.x == 0)
+        for (int i = 0; i < r.n_sys; ++i) atomicOr(&r.systems[i].sys->error_word, 8u);
+}
+
 // A warp's field step over one tile of cells of N types (0: any number): omega
 // of the new counts, and the averaging sample where the sweep takes one.  Returns
 // the lane's field energy, where it is asked for.
@@ -1191,7 +1197,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 screened_to = span;
             }
         }
-        if (!barrier.wait(&s_ok, [] {})) return;
+        if (!barrier.wait(&s_ok, [] {})) return flag_run(r);
         float wmax = -INFINITY, wmin = INFINITY;
 #pragma unroll 1
         for (int fi = first; fi < r.n_field; fi += stride) {
@@ -1253,7 +1259,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
         const bool ok = barrier.wait(&s_ok, [&] {
             if (ONE) s_span = span_after(a.system, wp->run.rule, wp->run.base + (uint32_t)sweep + 1u, wp->run.base);
         });
-        if (!ok) return;
+        if (!ok) return flag_run(r);
     }
     if (any && wp->run.active) {  // the positions
         const SweepSys& c = ONE ? a.sys : wp->sys;

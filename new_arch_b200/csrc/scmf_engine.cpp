@@ -375,8 +375,9 @@ void DevPlan::release() {
 // The tiles of k_sweep_warp: whole chains of one architecture, as many chains in
 // each (SweepArch::per).  Every warp of the GPU gets the same number of tiles, of
 // sizes up to what its buffer holds and no smaller than a row of 32 bead pairs.
-// Empty for a plan that the kernel does not take.
-static std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
+// A tile of linear chains also has no more than kTilePairs bead pairs.  Empty for a plan
+// that the kernel does not take.
+std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     std::vector<SweepArch> out;
     if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return out;
     *form = !p.linear ? kFormGraph : p.screened ? kFormScreened : kFormUnscreened;
@@ -385,14 +386,17 @@ static std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     const int cap = kSweepForms[*form].beads;
     const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
     int64_t beads = 0;
+    const auto chains_at_most = [&](const Plan::Chains& c) {
+        return c.linear ? std::min(cap / c.length, kTilePairs / ((c.length + 1) / 2)) : cap / c.length;
+    };
     int most = cap;  // what a tile of every architecture can reach
     for (const auto& c : p.chains) {
         beads += (int64_t)c.length * c.n_chains;
-        most = std::min(most, cap / c.length * c.length);
+        most = std::min(most, chains_at_most(c) * c.length);
     }
     const int64_t turns = std::max<int64_t>(1, (beads + warps * most - 1) / (warps * most));  // tiles of a warp
     const auto per_tile = [&](const Plan::Chains& c, int64_t target) {
-        return (int)std::min<int64_t>(cap / c.length, std::max<int64_t>(1, (target + c.length - 1) / c.length));
+        return (int)std::min<int64_t>(chains_at_most(c), std::max<int64_t>(1, (target + c.length - 1) / c.length));
     };
     int64_t target = std::max<int64_t>(64, (beads + warps * turns - 1) / (warps * turns));
     for (; target < cap; target += std::max<int64_t>(1, target / 64)) {  // the last tile of each architecture is a part
@@ -663,7 +667,7 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
             p->max_tile_beads = std::max(p->max_tile_beads, mt.n_chains * A.length);
         }
         p->max_length = std::max(p->max_length, A.length);
-        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.chain_base, (int)a, A.bead_base});
+        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.linear, A.bead_base});
         p->max_deg = std::max(p->max_deg, A.max_deg);
         p->linear = p->linear && A.linear;
     }

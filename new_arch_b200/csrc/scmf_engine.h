@@ -86,7 +86,8 @@ struct Plan {
     struct Chains {
         SysDev* sys;
         const ArchDev* arch;
-        int length, n_chains, chain_base, arch_index;
+        int length, n_chains;
+        bool linear;
         int64_t bead_base;
     };
     std::vector<Chains> chains;
@@ -95,6 +96,10 @@ struct Plan {
     bool one_seed = true;   // every system appended so far has `seed`
     bool one_seed_hi = true;  // ... or at least its upper 32 bits
 };
+
+// The warp tiles of a plan, an entry for each of its `chains`, and the kernels' form
+// (SweepFormId); empty for a plan that k_sweep_warp does not take.
+std::vector<SweepArch> tile_ranges(const Plan& p, int* form);
 
 struct DevPlan {
     MoveTile* d_move = nullptr;

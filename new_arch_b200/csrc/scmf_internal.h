@@ -366,6 +366,11 @@ struct SweepForm {
     int warps, beads;
 };
 constexpr SweepForm kSweepForms[4] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280}};
+// Bead pairs of a tile of linear chains at most: a lane names the tile's pairs by the
+// bits of a word, one for each row of 32.  A chain has half as many pairs as beads,
+// rounded up: tiles of single beads, of trimers and of other short odd chains come to
+// this before they come to the beads of a long form.
+constexpr int kTilePairs = 32 * 32;
 constexpr size_t kL2Bytes = 126u << 20;
 constexpr float kScreenFromAc = 2.0f;  // A 4k from which the screen runs
 

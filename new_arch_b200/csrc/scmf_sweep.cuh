@@ -157,7 +157,7 @@ struct SweepLayout {
     };
     static constexpr int kTabBytes = sweep_tab_bytes(FORM);
     static constexpr int kBytes = kTabBytes + kWarps * (int)sizeof(Warp) + kSlack;
-    static_assert(kBeads <= 2048, "a row of 32 bead pairs is a bit of a lane's mask");
+    static_assert(kTilePairs <= 32 * 32, "a row of 32 bead pairs is a bit of a lane's mask");
     static_assert(kTabBytes % 16 == 0 && sizeof(Warp) % 16 == 0 && offsetof(Warp, pos) % 16 == 0 && kStride % 4 == 0,
                   "16-byte copies");
     static_assert(kBytes <= 227 * 1024, "shared memory of an SM");
@@ -268,7 +268,7 @@ __device__ __forceinline__ PairConsts pair_consts(const SweepConsts& s, bool fir
     return c;
 }
 
-// The lane's pairs of a tile of `items` pairs: bit i for pair 32 i + lane.
+// The lane's pairs of a tile of `items` pairs (kTilePairs at most): bit i for pair 32 i + lane.
 __device__ __forceinline__ uint32_t row_mask(int items) {
     const int n = max(0, (items - (int)(threadIdx.x & 31) + 31) >> 5);
     return n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u;

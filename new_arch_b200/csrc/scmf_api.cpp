@@ -844,8 +844,7 @@ scmf_status scmf_batch_step_async(scmf_batch* b, int32_t n) {
 
 scmf_status scmf_batch_step(scmf_batch* b, int32_t n) {
     RET(scmf_batch_step_async(b, n));
-    CK(cudaStreamSynchronize(b->stream));
-    return SCMF_OK;
+    return b->plan.check(b->stream);
 }
 
 scmf_status scmf_batch_step_profiled(scmf_batch* b, int32_t n, float* ms_move, float* ms_field, float* ms_total) {
@@ -855,8 +854,7 @@ scmf_status scmf_batch_step_profiled(scmf_batch* b, int32_t n, float* ms_move, f
         if (s->stream != b->stream) CK(cudaStreamSynchronize(s->stream));
     }
     RET(profile_sweeps(b->plan, b->stream, n, ms_move, ms_field, ms_total));
-    for (auto* s : b->systems) RET(check_error_word(s));
-    return SCMF_OK;
+    return b->plan.check(b->stream);
 }
 
 scmf_status scmf_batch_tune_trials(const scmf_batch* b, scmf_tune_trial* out, int32_t max, int32_t* n) {
@@ -972,8 +970,12 @@ scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
         }
         if (!r && cudaEventSynchronize(e1) != cudaSuccess) r = fail(SCMF_E_CUDA, "trial failed");
         if (!r) cudaEventElapsedTime(ms, e0, e1);
+        if (!r) r = dp.check(b->stream);  // before the snapshots cover the error words
         dp.release();
-        for (size_t i = 0; i < b->systems.size() && !r; ++i) r = snap_restore(b->systems[i], &snaps[i], b->stream);
+        for (size_t i = 0; i < b->systems.size(); ++i) {
+            const scmf_status back = snap_restore(b->systems[i], &snaps[i], b->stream);
+            if (!r) r = back;
+        }
         return r;
     };
     scmf_tune best = b->plan.tune;

@@ -502,7 +502,7 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     scmf_status rc;
     if ((rc = dev_alloc((void**)&d_move, nm * sizeof(MoveTile), st)) ||
         (rc = dev_alloc((void**)&d_field, nf * sizeof(FieldTile), st)) ||
-        (rc = dev_alloc((void**)&d_close, std::max<size_t>(1, p.close.size()) * sizeof(SysClose), st)) ||
+        (rc = dev_alloc((void**)&d_close, (p.close.size() + 1) * sizeof(SysClose), st)) ||  // and the word of check()
         (rc = dev_alloc((void**)&d_warp, std::max<size_t>(1, wt.size()) * sizeof(WarpTile), st)) ||
         (rc = dev_alloc((void**)&d_ef, nf * sizeof(double), st)) || (rc = dev_alloc((void**)&d_eb, nm * sizeof(double), st)))
         return rc;
@@ -555,6 +555,15 @@ LaunchShape DevPlan::field_shape() const {
 
 scmf_status DevPlan::enqueue_close(int mode, cudaStream_t st) const {
     CKL(launch_close(d_close, n_sys, d_ef, d_eb, mode, st));
+    return SCMF_OK;
+}
+
+scmf_status DevPlan::check(cudaStream_t st) const {
+    uint32_t any = 0, *const d_any = reinterpret_cast<uint32_t*>(d_close + n_sys);
+    CKL(launch_error_words(d_close, n_sys, d_any, st));
+    CK(cudaMemcpyAsync(&any, d_any, sizeof any, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (any) return fail(SCMF_E_DEVICE, "kernel error word 0x%x", any);
     return SCMF_OK;
 }
 

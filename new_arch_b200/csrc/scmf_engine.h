@@ -139,6 +139,8 @@ struct DevPlan {
     scmf_status enqueue_field(cudaStream_t st) const;
     scmf_status enqueue_close(int mode, cudaStream_t st) const;
     scmf_status run_sweeps(cudaStream_t st, int n);
+    // waits for the stream; SCMF_E_DEVICE if a kernel has set a system's error word
+    scmf_status check(cudaStream_t st) const;
 };
 
 scmf_tune default_tune();

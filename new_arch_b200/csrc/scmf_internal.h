@@ -396,6 +396,8 @@ int launch_run(const LaunchShape& shape, const RunArgs& run, void* stream);
 int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_tiles, LaunchShape shape,
                  double* ef_part, int close_mode, void* stream);
 int launch_bond_energy(const MoveTile* tiles, int n_tiles, LaunchShape shape, double* eb_part, void* stream);
+// The systems' error words of a launch list, or'ed into *out.
+int launch_error_words(const SysClose* list, int n_sys, uint32_t* out, void* stream);
 int launch_close(const SysClose* list, int n_sys, const double* ef_part, const double* eb_part, int mode, void* stream);
 int launch_aos_to_soa(const float* aos, SysDev* sys, const ArchDev* arch, int n_arch, int64_t n_beads,
                       void* stream);

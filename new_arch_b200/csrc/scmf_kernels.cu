@@ -740,6 +740,20 @@ __global__ void __launch_bounds__(256) k_close(const SysClose* __restrict__ list
     }
 }
 
+// The error words of the plan's systems in one word (one block).
+__global__ void __launch_bounds__(256) k_error_words(const SysClose* __restrict__ list, int n_sys, uint32_t* out) {
+    uint32_t any = 0u;
+    for (int i = threadIdx.x; i < n_sys; i += blockDim.x) any |= list[i].sys->error_word;
+    __shared__ uint32_t s_any[8];
+    any = __reduce_or_sync(0xffffffffu, any);
+    if ((threadIdx.x & 31) == 0) s_any[threadIdx.x >> 5] = any;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) any |= s_any[w];
+        *out = any;
+    }
+}
+
 // Bond energy sum_bonds k |r_i - r_j|^2 of the current positions, each bond
 // once, one partial per tile (closed by k_close with kCloseBond).
 __global__ void __launch_bounds__(256) k_bond_energy(const MoveTile* __restrict__ tiles, int n_tiles,
@@ -1213,6 +1227,11 @@ int launch_bond_energy(const MoveTile* tiles, int n_tiles, LaunchShape sh, doubl
 int launch_close(const SysClose* list, int n_sys, const double* ef_part, const double* eb_part, int mode, void* stream) {
     if (n_sys <= 0) return 0;
     k_close<<<n_sys < 1024 ? n_sys : 1024, 256, 0, (cudaStream_t)stream>>>(list, n_sys, ef_part, eb_part, mode);
+    return (int)cudaGetLastError();
+}
+
+int launch_error_words(const SysClose* list, int n_sys, uint32_t* out, void* stream) {
+    k_error_words<<<1, 256, 0, (cudaStream_t)stream>>>(list, n_sys, out);
     return (int)cudaGetLastError();
 }
 

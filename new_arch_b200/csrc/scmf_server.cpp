@@ -102,6 +102,8 @@ static void finish(scmf_server* s, Active& a) {
     if (a.sys && a.status == SCMF_OK) {
         scmf_stats stats{};
         scmf_status rc = scmf_get_stats(a.sys, &stats);
+        // a kernel gave up on the system: its state is no result
+        if (!rc && stats.error_word) rc = fail(SCMF_E_DEVICE, "kernel error word 0x%x", stats.error_word);
         if (!rc && a.req.counts_out)
             rc = scmf_get_counts(a.sys, a.req.counts_out, (size_t)a.sys->n_cells * a.sys->spec.n_types);
         r.status = rc;

@@ -63,7 +63,7 @@ int main() {
 
 
 def test_tiles_fit_a_lanes_mask(tmp_path):
-    lib = build.build()
+    lib = build.LIB
     src, exe = tmp_path / "tiles.cpp", tmp_path / "tiles"
     src.write_text(PROGRAM)
     subprocess.run(["g++", "-O1", "-std=c++17", "-I", build.INC, "-I", build.CSRC, "-I",

@@ -178,7 +178,7 @@ struct SysDev {
     // served form gives each request its own sweep count inside a shared
     // round); 0xFFFFFFFF everywhere else
     uint32_t stop_step;
-    uint32_t pad2;
+    uint32_t run_stop;  // stop_step as a launch of many sweeps found it, 0 for a system with an error word
     // counts the field step reads: NULL means counts[cur] (the grid of this
     // system's own beads); a chain shard points it at the sum over all shards
     const uint32_t* field_counts;
@@ -233,6 +233,11 @@ struct FieldTile {
     int32_t first_tile;   // index of this system's first field tile in the launch
     int32_t pad;
 };
+
+// Bits of SysDev::error_word: a tile larger than k_sweep's shared memory; a warp's tile
+// that did not arrive; blocks of a launch that did not come to a barrier.
+constexpr uint32_t kErrorSize = 1u, kErrorTile = 4u, kErrorBarrier = 8u;
+constexpr long long kWaitClocks = 4000000000ll;  // a wait in a kernel gives up after about two seconds
 
 enum SweepMode : int { kMoveOnly = 0, kMoveGrid = 1, kGridOnly = 2 };
 
@@ -333,8 +338,9 @@ struct RunArgs {
     const RunSystem* systems;
     const FieldTile* field;       // a warp's work each
     double* ef_part;              // field energy of every field tile after the last sweep
-    unsigned long long* barrier;  // the grid barrier's count
+    unsigned long long* barrier;  // the grid barrier's count, and after it whether it is broken
     int n_sys, n_field, n_sweeps, pad;
+    long long wait_clocks;        // how long a block waits for the others (kWaitClocks)
 };
 
 // Parameters of k_sweep_warp.

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep(const MoveTile* __restrict__ t
         const int L = Ap->length;
         const int nb = t.n_chains * L;
         if (nb > max_tile_beads || L > max_length) {
-            if (tid == 0) atomicOr(&S->error_word, 1u);
+            if (tid == 0) atomicOr(&S->error_word, kErrorSize);
             continue;
         }
         MoveConsts c;

@@ -85,9 +85,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "memory");
     return done != 0u;
 }
-// Waits for a phase of a barrier of this CTA; false after about two seconds
-// (never in a sound run).
-constexpr long long kWaitClocks = 4000000000ll;
+// Waits for a phase of a barrier of this CTA; false after kWaitClocks (never in a sound
+// run).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
@@ -810,7 +809,7 @@ struct Mover {
     // Waits for the tile asked for; false (and the error word) if it does not come.
     __device__ __forceinline__ bool arrived() {
         const bool ok = mbar_wait(smem_addr(&wp->full), parity);
-        if (!ok && lane == 0) atomicOr(&S->error_word, 4u);
+        if (!ok && lane == 0) atomicOr(&S->error_word, kErrorTile);
         parity ^= 1u;
         return ok;
     }
@@ -935,13 +934,20 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_war
 
 // ------------------------------------------------------ many sweeps a launch
 // A barrier of all CTAs of a (cooperative) launch, on a count in global memory
-// that only grows, by one a CTA and barrier.
+// that only grows, by one a CTA and barrier.  CTAs that give up do so after different
+// numbers of barriers: from then on the barrier is broken, and no launch uses it again.
 struct GridBarrier {
-    unsigned long long* count;
+    unsigned long long* count;  // and after it a word that is set when the barrier breaks
+    long long clocks;           // how long to wait
     unsigned long long target;  // thread 0's
+    bool broken;                // thread 0's
     // The count is a whole number of barriers until the last CTA comes to the first one.
-    __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {
-        if (threadIdx.x == 0) target = __ldcg(c) / gridDim.x * gridDim.x;
+    __device__ __forceinline__ GridBarrier(unsigned long long* c, long long limit)
+        : count(c), clocks(limit), target(0), broken(false) {
+        if (threadIdx.x == 0) {
+            target = __ldcg(c) / gridDim.x * gridDim.x;
+            broken = __ldcg(c + 1) != 0ull;
+        }
     }
     __device__ __forceinline__ void arrive() {
         __syncthreads();
@@ -950,20 +956,20 @@ struct GridBarrier {
             asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
         }
     }
-    // False (to all threads of the CTA) after about two seconds.  Thread 0 calls
-    // `then` before the others go on.
+    // False (to all threads of the CTA) after `clocks`, or where the barrier is broken.
+    // Thread 0 calls `then` before the others go on.
     template <typename Then>
     __device__ __forceinline__ bool wait(int* s_ok, const Then& then) {
         if (threadIdx.x == 0) {
             unsigned long long now;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
-            if (now < target) {
+            if (now < target && !broken) {
                 const long long t0 = clock64();
                 do {
                     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
-                } while (now < target && clock64() - t0 < kWaitClocks);
+                } while (now < target && clock64() - t0 < clocks);
             }
-            *s_ok = now >= target;
+            *s_ok = now >= target && !broken;
             then();
         }
         __syncthreads();
@@ -999,11 +1005,18 @@ __device__ __forceinline__ void fold_span(uint32_t* keys, float wmax, float wmin
     }
 }
 
+// The step at which a system stops: it goes no further once a wait has run out on it,
+// when its counts have moved and its positions may not have been written.
+__device__ __forceinline__ uint32_t stop_of(const SysDev* S) {
+    const uint32_t word = S->error_word, stop = S->stop_step;
+    return word & (kErrorTile | kErrorBarrier) ? 0u : stop;
+}
+
 // Closes a system after its sweeps of a launch (one block).
 __device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r, unsigned long long* s_acc, double* s_ef) {
     SysDev* S = rs.sys;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const uint32_t base = S->step, left = S->stop_step > base ? S->stop_step - base : 0u;
+    const uint32_t base = S->step, left = S->run_stop > base ? S->run_stop - base : 0u;
     const uint32_t made = min((uint32_t)r.n_sweeps, left);
     if (made) {  // block-uniform
         unsigned long long all = 0, last = 0;
@@ -1043,10 +1056,12 @@ __device__ __forceinline__ void close_run(const RunSystem& rs, const RunArgs& r,
     __syncthreads();
 }
 
-// The error word of every system of a launch whose blocks did not come to a barrier.
-__device__ __forceinline__ void flag_run(const RunArgs& r) {
-    if (threadIdx.x == 0)
-        for (int i = 0; i < r.n_sys; ++i) atomicOr(&r.systems[i].sys->error_word, 8u);
+// A launch whose blocks did not come to a barrier: the error word of every system.
+__device__ __forceinline__ void give_up(const RunArgs& r) {
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < r.n_sys; ++i) atomicOr(&r.systems[i].sys->error_word, kErrorBarrier);
+        atomicExch(r.barrier + 1, 1ull);
+    }
 }
 
 // A warp's field step over one tile of cells of N types (0: any number): omega
@@ -1111,12 +1126,14 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     const int lane = threadIdx.x & 31;
     const int first = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x, stride = (int)(blockDim.x >> 5) * (int)gridDim.x;
     const bool any = first < a.n_tiles;
-    GridBarrier barrier(r.barrier);
+    GridBarrier barrier(r.barrier, r.wait_clocks);
     if (ONE && threadIdx.x == 0) s_span = a.system->omega_span;
     if (threadIdx.x < 2) s_keys[threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
     for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {  // the slot of the launch's first field step
         SysDev* S = r.systems[i].sys;
-        if (threadIdx.x < 2) S->om_keys[(S->step + 1u) % 3u][threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
+        const uint32_t step = S->step, stop = stop_of(S);
+        if (threadIdx.x < 2) S->om_keys[(step + 1u) % 3u][threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
+        if (threadIdx.x == 0) S->run_stop = stop;  // for this block's close_run: other blocks may set the word meanwhile
     }
     {
         Mover<ONE, FORM, KEYS> m(a, smem_raw);
@@ -1124,7 +1141,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
         if (any) t = tile_at<ONE>(a, first);
         m.start(smem_raw, t, any);
         if (any) {
-            const uint32_t base = t.sys->step, stop = t.sys->stop_step;
+            const uint32_t base = t.sys->step, stop = stop_of(t.sys);
             m.turn_to(t);
             const bool here = m.arrived();
             if (lane == 0) {
@@ -1153,7 +1170,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
             wp->run.cell0 = t.cell0;
             wp->run.n_cells = t.n_cells;
             wp->run.f_base = t.sys->step;
-            wp->run.f_stop = t.sys->stop_step;
+            wp->run.f_stop = stop_of(t.sys);
         }
         __syncwarp();
     };
@@ -1197,7 +1214,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
                 screened_to = span;
             }
         }
-        if (!barrier.wait(&s_ok, [] {})) return flag_run(r);
+        if (!barrier.wait(&s_ok, [] {})) return give_up(r);
         float wmax = -INFINITY, wmin = INFINITY;
 #pragma unroll 1
         for (int fi = first; fi < r.n_field; fi += stride) {
@@ -1259,7 +1276,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
         const bool ok = barrier.wait(&s_ok, [&] {
             if (ONE) s_span = span_after(a.system, wp->run.rule, wp->run.base + (uint32_t)sweep + 1u, wp->run.base);
         });
-        if (!ok) return flag_run(r);
+        if (!ok) return give_up(r);
     }
     if (any && wp->run.active) {  // the positions
         const SweepSys& c = ONE ? a.sys : wp->sys;

@@ -1,7 +1,10 @@
 """Error words that kernels set on a system reach the caller: from the blocking calls of a
 batch, which has many systems, and from the server, which hands out no counts of such a
 system.  The words are set from the host, by programs built against the library's own
-headers: into a member's record, and by a stand-in for the launch of many sweeps."""
+headers: into a member's record, and by a stand-in for the launch of many sweeps.  And a
+launch of many sweeps whose blocks do not wait for one another sets the word, no launch
+uses its barrier again, and the system stays where it is while the others of a batch go
+on."""
 import os
 import subprocess
 
@@ -84,6 +87,48 @@ int main() {
 }
 """
 
+WAITS = COMMON + r"""
+static SysDev record(const scmf_system* s) {
+    SysDev d;
+    WANT(cudaMemcpy(&d, s->d_sys, sizeof d, cudaMemcpyDeviceToHost), 0);
+    return d;
+}
+static std::vector<uint32_t> counts(const scmf_system* s) {
+    std::vector<uint32_t> c((size_t)s->n_cells * 2);
+    WANT(scmf_get_counts(s, c.data(), c.size()), SCMF_OK);
+    return c;
+}
+int main() {
+    scmf_system* s = started(melt(60000, 32, 64, 5));
+    WANT(s->plan.d_run != nullptr, true);  // many sweeps a launch
+    s->plan.run.wait_clocks = 0;           // a look or two at the count, and no more
+    WANT(scmf_step(s, 20), SCMF_E_DEVICE);
+    WANT(record(s).error_word, kErrorBarrier);
+    WANT(record(s).step, 0);
+    s->plan.run.wait_clocks = kWaitClocks;
+    set_word(s->d_sys, 0);  // as if nothing had been: the plan's barrier stays broken
+    WANT(scmf_step(s, 1100), SCMF_E_DEVICE);
+    WANT(record(s).error_word, kErrorBarrier);
+    WANT(record(s).step, 0);
+    const auto at = counts(s);
+    scmf_system* other = started(melt(400, 32, 12, 6));
+    scmf_system* pair[2] = {s, other};
+    scmf_batch* b = nullptr;
+    WANT(scmf_batch_create(pair, 2, nullptr, nullptr, &b), SCMF_OK);
+    WANT(b->plan.d_run != nullptr, true);
+    WANT(scmf_batch_step(b, 3), SCMF_E_DEVICE);
+    WANT(record(s).step, 0);
+    WANT(counts(s) == at, true);
+    WANT(record(other).step, 3);
+    WANT(record(other).error_word, 0);
+    scmf_batch_destroy(b);
+    scmf_system* same = started(melt(400, 32, 12, 6));
+    WANT(scmf_step(same, 3), SCMF_OK);
+    WANT(counts(other) == counts(same), true);
+    return 0;
+}
+"""
+
 SERVER = COMMON + r"""
 // in place of the library's: no sweep, the error word of every system
 int scmf::launch_run(const LaunchShape&, const RunArgs& run, void* stream) {
@@ -129,6 +174,10 @@ def _run(tmp_path, program):
 
 def test_batch(tmp_path):
     _run(tmp_path, BATCH)
+
+
+def test_blocks_that_do_not_wait(tmp_path):
+    _run(tmp_path, WAITS)
 
 
 def test_server(tmp_path):

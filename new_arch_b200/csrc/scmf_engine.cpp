@@ -588,7 +588,10 @@ scmf_status DevPlan::enqueue_field(cudaStream_t st) const {
 
 scmf_status DevPlan::run_sweeps(cudaStream_t st, int n) {
     if (n <= 0) return SCMF_OK;
-    if (d_run) {
+    // A single sweep is two launches, of which the second begins beside the first: a cooperative launch, its barriers
+    // and the positions' way back cost more than they save (enqueued one by one: 32,000 beads 13.4 us against 17.4,
+    // 2.0M beads 22.4 against 32.8; two sweeps a call are the same either way, three faster in one launch).
+    if (d_run && n > 1) {
         // some milliseconds a launch, so that other work on the GPU gets its turn
         const LaunchShape sh = move_shape();
         for (RunArgs r = run; n > 0; n -= r.n_sweeps) {

@@ -430,17 +430,38 @@ static std::vector<WarpTile> tile_list(const Plan& p, const std::vector<SweepArc
     return out;
 }
 
+// The warps of a launch of n_warp tiles that are made at once.
+static int launched_warps(int n_warp, int form) {
+    const int grid = std::min(n_warp, sm_count());
+    return grid * std::min(kSweepForms[form].warps, (n_warp + grid - 1) / grid);
+}
+
+// Whether a plan's sweeps go many to a launch (k_run): a tile a warp, and no more cells
+// than these warps can make omega of in the time that the launches of two kernels take.
+// A step of a warp over its cells takes 0.6 us where few warps run, so up to 12 steps are
+// as fast as k_field's launch over the whole GPU, and up to 27 where most of the GPU's
+// warps run.  A sweep in one launch against two: 300 chains of 32 on 64^3 cells (7 steps)
+// 10.8 and 12.0 us, on 80^3 (14) 14.8 and 12.7, on 128^3 (55) 40.8 and 16.0; 40 chains on
+// 64^3 (102) 67 and 12; 1,000 on 96^3 (12) 14.0 and 14.0; 60,000 on 200^3 (26) 55.8 and
+// 58.5; 10,000 on 256^3 (55) 90.7 and 77.2; 1,000 with four types on 96^3 (47) 98.6 and 39.4.
+static bool runs_at_once(const Plan& p, int n_warp, int form) {
+    const int all = sm_count() * kSweepForms[form].warps;
+    if (n_warp < 1 || n_warp > all) return false;
+    const int warps = launched_warps(n_warp, form);
+    int64_t cells = 0;
+    for (const auto& c : p.cells) cells += c.second;
+    return cells <= (int64_t)warps * (p.cells4 ? 128 : 32) * (4 * (int64_t)warps >= 3 * (int64_t)all ? 27 : 12);
+}
+
 // The tables of k_run as one buffer, its pointers still offsets: field tiles of a
 // warp each, so that the warps of the launch share the cells evenly.
 static std::vector<char> run_tables(const Plan& p, int n_warp, int form, RunArgs* run) {
-    const int sms = sm_count(), most = kSweepForms[form].warps;
-    const int grid = std::min(n_warp, sms), warps = grid * std::min(most, (n_warp + grid - 1) / grid);  // as launched
+    const int warps = launched_warps(n_warp, form);
     int64_t cells = 0;
     for (const auto& c : p.cells) cells += c.second;
     // whole rows of four cells a lane, or of one where that leaves warps idle
     const int64_t row = cells >= 128 * (int64_t)warps ? 128 : 32;
-    const int64_t turns = std::max<int64_t>(1, (cells + 4096 * (int64_t)warps - 1) / (4096 * (int64_t)warps));
-    const int64_t per = ((cells + warps * turns - 1) / (warps * turns) + row - 1) / row * row;
+    const int64_t per = ((cells + warps - 1) / warps + row - 1) / row * row;
     std::vector<RunSystem> systems;
     std::vector<FieldTile> field;
     for (const auto& c : p.cells) {
@@ -512,7 +533,7 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     CK(cudaMemcpyAsync(d_field, p.field.data(), p.field.size() * sizeof(FieldTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_close, p.close.data(), p.close.size() * sizeof(SysClose), cudaMemcpyHostToDevice, st));
     std::vector<char> run_image;
-    if (n_warp > 0 && n_warp <= sm_count() * kSweepForms[form].warps) {  // a tile a warp
+    if (runs_at_once(p, n_warp, form)) {
         run_image = run_tables(p, n_warp, form, &run);
         if ((rc = dev_alloc(&d_run, run_image.size(), st))) return rc;
         CK(cudaMemcpyAsync(d_run, run_image.data(), run_image.size(), cudaMemcpyHostToDevice, st));
@@ -648,6 +669,7 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     p->cells32 = p->cells32 && n_cells * spec.n_types < (1ll << 31);
     p->position_bytes += (size_t)n_beads * 12;
     p->cells.push_back({d_sys, n_cells});
+    p->cells4 = p->cells4 && spec.n_types <= 3 && spec.p.count_bits == 32 && n_cells % 4 == 0;
     p->screened = p->screened || sweep.screen.on;
     if (p->close.empty()) {
         p->seed = spec.p.seed;

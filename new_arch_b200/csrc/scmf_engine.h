@@ -92,6 +92,7 @@ struct Plan {
     };
     std::vector<Chains> chains;
     std::vector<std::pair<SysDev*, int64_t>> cells;  // of every system, for the field tiles of k_run
+    bool cells4 = true;     // k_run's field step takes the cells of every system four at a time
     uint64_t seed = 0;      // the systems' seed when they all share one
     bool one_seed = true;   // every system appended so far has `seed`
     bool one_seed_hi = true;  // ... or at least its upper 32 bits

@@ -661,9 +661,13 @@ using namespace scmf;
 // Work tiles of this system appended to a plan.
 scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     // systems below ~2.4M beads: four tiles per SM (measured best over the 256-system mix
-    // against two and six per SM with 4-warp CTAs)
+    // against two and six per SM with 4-warp CTAs), the last of each architecture a part:
+    // one tile more than that is a second round of blocks
     const int sms = sm_count();
-    const int64_t target_small = std::max<int64_t>(1, n_beads / (4 * sms));
+    int64_t n_used = 0;
+    for (const ArchHost& A : archs) n_used += A.n_chains > 0;
+    const int64_t rounds = std::max<int64_t>(1, 4 * sms - n_used);
+    const int64_t target_small = (n_beads + rounds - 1) / rounds;
     const size_t first_tile = p->move.size();
     const size_t first_field = p->field.size();
     p->cells32 = p->cells32 && n_cells * spec.n_types < (1ll << 31);
@@ -685,6 +689,7 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
         if (cpt <= 0) {
             const int64_t target = std::min<int64_t>(4096, std::max<int64_t>(A.length, target_small));
             cpt = (int)std::max<int64_t>(1, target / A.length);
+            if (cpt >= 8 && cpt * A.length < target) ++cpt;  // of a few long chains a tile more would be too large
             // a few hundred beads at least, so that small systems do not fall into tiles of single chains
             if (A.linear && A.length <= 64) cpt = std::max(cpt, 256 / A.length);
         }

@@ -377,14 +377,10 @@ void DevPlan::release() {
 // sizes up to what its buffer holds and no smaller than a row of 32 bead pairs.
 // A tile of linear chains also has no more than kTilePairs bead pairs.  Empty for a plan
 // that the kernel does not take.
-std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
+static std::vector<SweepArch> form_ranges(const Plan& p, int form) {
     std::vector<SweepArch> out;
-    if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return out;
-    *form = !p.linear ? kFormGraph : p.screened ? kFormScreened : kFormUnscreened;
-    if (p.linear && p.max_length > kSweepForms[*form].beads) *form = kFormLong;
-    if (p.max_length > kSweepForms[*form].beads) return out;
-    const int cap = kSweepForms[*form].beads;
-    const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
+    const int cap = kSweepForms[form].beads;
+    const int64_t warps = (int64_t)sm_count() * kSweepForms[form].warps;
     int64_t beads = 0;
     const auto chains_at_most = [&](const Plan::Chains& c) {
         return c.linear ? std::min(cap / c.length, kTilePairs / ((c.length + 1) / 2)) : cap / c.length;
@@ -417,6 +413,41 @@ static int tiles_of(const std::vector<SweepArch>& ranges) {
     return ranges.empty() ? 0 : ranges.back().first + (ranges.back().n_chains + ranges.back().per - 1) / ranges.back().per;
 }
 
+std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
+    if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return {};
+    int64_t beads = 0, exact = 0;  // all, and those of chains that are not screened
+    for (const auto& c : p.chains) {
+        beads += (int64_t)c.length * c.n_chains;
+        exact += c.screened ? 0 : (int64_t)c.length * c.n_chains;
+    }
+    *form = !p.linear ? kFormGraph : exact < beads ? kFormScreened : kFormUnscreened;
+    if (p.linear && p.max_length > kSweepForms[*form].beads) *form = kFormLong;
+    if (p.max_length > kSweepForms[*form].beads) return {};
+    std::vector<SweepArch> out = form_ranges(p, *form);
+    // Trials that are all made exactly are made faster in registers (k_sweep_pairs) than in tiles, from 352 beads a warp
+    // on also than in k_run: a sweep of 0.4M beads 12.4 us in k_run and 16.0 so, 0.8M 21.3 and 18.9 (in chains of 48 or 64
+    // 19.4 and 20.3, 19.0 and 19.7), 2.0M 46.1 and 33.5, 20.5M 379 (in tiles) and 223.  So are many systems of which a
+    // quarter of the beads is not screened: 32M beads, 25 % 467 us in tiles and 432 so, 50 % 634 and 452, 10 % 350 and
+    // 399.  At least three lanes of four must have a pair.
+    const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
+    if (p.linear && (exact == beads ? beads > 352 * warps : tiles_of(out) > warps && 4 * exact >= beads)) {
+        int64_t pairs = 0, lanes = 0;
+        bool even = p.cells.size() == 1 && p.chains.size() <= kSweepMaxArch;
+        for (const auto& c : p.chains) {
+            if (c.length > 64) return out;
+            const int h = (c.length + 1) / 2, per = 32 / h;
+            pairs += (int64_t)h * c.n_chains;
+            lanes += (int64_t)32 * ((c.n_chains + per - 1) / per);
+            even = even && (c.length | c.bead_base) % 2 == 0;
+        }
+        if (4 * pairs >= 3 * lanes) {
+            *form = even ? kFormPairs : kFormPairsList;
+            out = form_ranges(p, *form);
+        }
+    }
+    return out;
+}
+
 static std::vector<WarpTile> tile_list(const Plan& p, const std::vector<SweepArch>& ranges) {
     std::vector<WarpTile> out;
     out.reserve((size_t)tiles_of(ranges));
@@ -446,7 +477,7 @@ static int launched_warps(int n_warp, int form) {
 // 58.5; 10,000 on 256^3 (55) 90.7 and 77.2; 1,000 with four types on 96^3 (47) 98.6 and 39.4.
 static bool runs_at_once(const Plan& p, int n_warp, int form) {
     const int all = sm_count() * kSweepForms[form].warps;
-    if (n_warp < 1 || n_warp > all) return false;
+    if (n_warp < 1 || n_warp > all || form == kFormPairs || form == kFormPairsList) return false;
     const int warps = launched_warps(n_warp, form);
     int64_t cells = 0;
     for (const auto& c : p.cells) cells += c.second;
@@ -508,7 +539,7 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     form = kFormScreened;
     const std::vector<SweepArch> ranges = tile_ranges(p, &form);
     n_warp = tiles_of(ranges);
-    one = n_sys == 1 && ranges.size() <= kSweepMaxArch;
+    one = n_sys == 1 && ranges.size() <= kSweepMaxArch && form != kFormPairsList;
     std::vector<WarpTile> wt;
     if (one) {
         system = p.close[0].sys;
@@ -674,7 +705,6 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
     p->position_bytes += (size_t)n_beads * 12;
     p->cells.push_back({d_sys, n_cells});
     p->cells4 = p->cells4 && spec.n_types <= 3 && spec.p.count_bits == 32 && n_cells % 4 == 0;
-    p->screened = p->screened || sweep.screen.on;
     if (p->close.empty()) {
         p->seed = spec.p.seed;
         p->sweep = sweep;
@@ -707,7 +737,8 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
             p->max_tile_beads = std::max(p->max_tile_beads, mt.n_chains * A.length);
         }
         p->max_length = std::max(p->max_length, A.length);
-        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.linear, A.bead_base});
+        // a bead without bonds has no energy to screen by
+        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.linear, A.bead_base, sweep.screen.on && A.max_deg > 0});
         p->max_deg = std::max(p->max_deg, A.max_deg);
         p->linear = p->linear && A.linear;
     }

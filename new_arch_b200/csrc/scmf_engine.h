@@ -81,7 +81,6 @@ struct Plan {
     SweepSys sweep{};           // of the first system
     bool linear = true;   // every architecture is a linear chain
     bool cells32 = true;  // cells times types below 2^31 in every system
-    bool screened = false;  // some system's moves are screened
     // the chains of every architecture, for the warp tiles of k_sweep_warp
     struct Chains {
         SysDev* sys;
@@ -89,6 +88,7 @@ struct Plan {
         int length, n_chains;
         bool linear;
         int64_t bead_base;
+        bool screened;
     };
     std::vector<Chains> chains;
     std::vector<std::pair<SysDev*, int64_t>> cells;  // of every system, for the field tiles of k_run

@@ -367,11 +367,15 @@ struct SweepArgs {
 // both, screened or not, and twelve warps: 2.0M beads in combs 25.1 us a sweep; with
 // sixteen 28.5 (the screen of arbitrary neighbours does not fit 128 registers beside
 // the exact trials), with eight 26.6.
-enum SweepFormId { kFormScreened = 0, kFormLong = 1, kFormUnscreened = 2, kFormGraph = 3 };
+// k_sweep_pairs has forms of its own, for one system of even chains and for any others:
+// no buffers, as many warps as its registers leave, and tiles that only share out the work.
+// 28 warps spill, 16 and 20 are too few (20.5M beads 222 us with 24 or 28, 245 with 20; in
+// the second form 60 systems of 14M beads 308 us with 20, 352 with 16).
+enum SweepFormId { kFormScreened = 0, kFormLong = 1, kFormUnscreened = 2, kFormGraph = 3, kFormPairs = 4, kFormPairsList = 5 };
 struct SweepForm {
     int warps, beads;
 };
-constexpr SweepForm kSweepForms[4] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280}};
+constexpr SweepForm kSweepForms[6] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280}, {24, 1024}, {20, 1024}};
 // Bead pairs of a tile of linear chains at most: a lane names the tile's pairs by the
 // bits of a word, one for each row of 32.  A chain has half as many pairs as beads,
 // rounded up: tiles of single beads, of trimers and of other short odd chains come to

@@ -1072,6 +1072,12 @@ static cudaError_t opt_in_warp() {
     return e;
 }
 
+template <bool ONE, int FOLD, int KEYS>
+static cudaError_t opt_in_pairs() {
+    return cudaFuncSetAttribute((const void*)k_sweep_pairs<ONE, FOLD, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                pairs_smem<ONE>());
+}
+
 int configure_kernels() {
     // once per device, with that device current
     static std::mutex mu;
@@ -1096,6 +1102,11 @@ int configure_kernels() {
     cudaError_t e = opt_in_warp<true, kKeysBoth>();
     if (e == cudaSuccess) e = opt_in_warp<false, kKeysHigh>();
     if (e == cudaSuccess) e = opt_in_warp<false, kKeysNone>();
+    if (e == cudaSuccess) e = opt_in_pairs<true, 0, kKeysBoth>();
+    if (e == cudaSuccess) e = opt_in_pairs<true, 1, kKeysBoth>();
+    if (e == cudaSuccess) e = opt_in_pairs<true, 2, kKeysBoth>();
+    if (e == cudaSuccess) e = opt_in_pairs<false, 3, kKeysHigh>();
+    if (e == cudaSuccess) e = opt_in_pairs<false, 3, kKeysNone>();
     for (const void* f : general)
         if (e == cudaSuccess) e = opt_in(f, bytes);
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
@@ -1161,6 +1172,12 @@ static cudaError_t launch_warp(const SweepArgs& a, int form, const RunArgs* run,
     return launch_form<ONE, kFormScreened, KEYS>(a, run, chained, st);
 }
 
+template <bool ONE, int FOLD, int KEYS>
+static cudaError_t launch_pairs(const SweepArgs& a, int warps, bool chained, cudaStream_t st) {
+    const int sms = sm_count(), grid = a.n_tiles < sms ? a.n_tiles : sms;
+    return launch_chained(k_sweep_pairs<ONE, FOLD, KEYS>, grid, 32 * warps, pairs_smem<ONE>(), chained, st, a);
+}
+
 static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const RunArgs* run, cudaStream_t st) {
     SweepArgs a{};
     a.tiles = sh.warp_tiles;
@@ -1172,6 +1189,16 @@ static cudaError_t launch_warp(const LaunchShape& sh, bool move_counts, const Ru
     a.sys = sh.sweep;
     a.n_arch = sh.n_arch;
     for (int i = 0; i < sh.n_arch; ++i) a.arch[i] = sh.arch[i];
+    const int warps = kSweepForms[sh.form].warps;
+    if (sh.form == kFormPairs) {
+        if (a.sys.fold == 0) return launch_pairs<true, 0, kKeysBoth>(a, warps, sh.chained != 0, st);
+        if (a.sys.fold == 1) return launch_pairs<true, 1, kKeysBoth>(a, warps, sh.chained != 0, st);
+        return launch_pairs<true, 2, kKeysBoth>(a, warps, sh.chained != 0, st);
+    }
+    if (sh.form == kFormPairsList) {
+        if (sh.keyed != kKeysNone) return launch_pairs<false, 3, kKeysHigh>(a, warps, sh.chained != 0, st);
+        return launch_pairs<false, 3, kKeysNone>(a, warps, sh.chained != 0, st);
+    }
     if (sh.one) return launch_warp<true, kKeysBoth>(a, sh.form, run, sh.chained != 0, st);
     if (sh.keyed != kKeysNone) return launch_warp<false, kKeysHigh>(a, sh.form, run, sh.chained != 0, st);
     return launch_warp<false, kKeysNone>(a, sh.form, run, sh.chained != 0, st);

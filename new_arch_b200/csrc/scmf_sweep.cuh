@@ -932,6 +932,212 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1) k_sweep_war
     }
 }
 
+// ------------------------------------------------- every trial, in registers
+// One move of systems that are not screened, of linear chains of up to 64 beads: a row of
+// lanes has whole chains, each lane a bead pair in registers.  It makes the even bead and
+// then the odd one, with neighbours by shuffles, and loads the next row's pair meanwhile.
+// Nothing of a trial is left out, so there is nothing to gather and no reason to keep a
+// tile: without its buffers an SM has 24 warps, and room for copies of the normal table
+// (lane l reads copy l mod 8, so the eight lanes of a 16-byte phase never meet in a bank).
+// Bound by instruction issue, with the latency of omega's
+// reads behind it.  These may go through L1: omega does not change while the kernel
+// runs, and the old and the new cell of a small step share a line.
+//
+// A sweep of 20.5M beads in chains of 32, nine trials in ten accepted: 223 us on 128^3
+// cells and 229 on 96^3, where tiles in shared memory took 379 and 392 (four warps a
+// scheduler do not cover the latency of an exact trial, and each move was three
+// scattered words to memory); 20M single beads 349 and 527; 20 systems of 4.7M beads 77
+// and 117.  With 28 warps and one copy of the normal table in tiles of 640 beads 318.
+// Without the prefetch of the next row 249, the Philox blocks of a pair made apart 237.
+//
+// ONE: one system of chains of even lengths, whose pairs lie on 8-byte boundaries.
+// FOLD: SweepSys::fold of the one system, or 3: each system's own.
+constexpr int kPairCopies = 8;
+template <bool ONE>
+constexpr int pairs_smem() {
+    return SCMF_NORMAL_SEGS * kPairCopies * (int)sizeof(float4) + (ONE ? 0 : kSweepForms[kFormPairsList].warps * (int)sizeof(SweepSys));
+}
+
+template <int FOLD>
+__device__ __forceinline__ int cell_of_fold(const SweepSys& c, float x, float y, float z) {
+    if (FOLD == 0)
+        return fold_pow2(x, c.inv_d[0], c.n[0] - 1) +
+               c.n[0] * (fold_pow2(y, c.inv_d[1], c.n[1] - 1) + c.n[1] * fold_pow2(z, c.inv_d[2], c.n[2] - 1));
+    if (FOLD == 1)
+        return fold_magic(x, c.inv_d[0], c.n[0], c.fold_off[0], c.fold_mag[0]) +
+               c.n[0] * (fold_magic(y, c.inv_d[1], c.n[1], c.fold_off[1], c.fold_mag[1]) +
+                         c.n[1] * fold_magic(z, c.inv_d[2], c.n[2], c.fold_off[2], c.fold_mag[2]));
+    if (FOLD == 2)
+        return fold(x, c.inv_d[0], c.n[0]) +
+               c.n[0] * (fold(y, c.inv_d[1], c.n[1]) + c.n[1] * fold(z, c.inv_d[2], c.n[2]));
+    return cell_index(c, x, y, z);
+}
+
+// A lane's trial (where act) with trial_f's expressions, under branches that the warp
+// takes as one; a bead that moves has its new position afterwards.
+template <int FOLD>
+__device__ __forceinline__ bool trial_pair(const SweepSys& c, float& x, float& y, float& z, float fx, float fy, float fz,
+                                           float cc, float ac4, float n0, float n1, float n2, uint32_t aw, float span,
+                                           bool act, uint32_t typ, int& c_old, int& c_new) {
+    const float dx = __fmaf_rn(c.A, fx, __fmul_rn(c.R, n0));
+    const float dy = __fmaf_rn(c.A, fy, __fmul_rn(c.R, n1));
+    const float dz = __fmaf_rn(c.A, fz, __fmul_rn(c.R, n2));
+    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+    const float fd = __fmaf_rn(fx, dx, __fmaf_rn(fy, dy, __fmul_rn(fz, dz)));
+    const float deb = __fmul_rn(ac4, __fmaf_rn(cc, d2, __fmul_rn(-2.0f, fd)));
+    const float u = u01(aw);
+    c_old = c_new = 0;
+    bool acc = false;
+    if (__any_sync(0xffffffffu, act && maybe_accepted(deb, span, log_lower(u)))) {
+        const float px = __fadd_rn(x, dx), py = __fadd_rn(y, dy), pz = __fadd_rn(z, dz);
+        c_old = cell_of_fold<FOLD>(c, x, y, z);
+        c_new = cell_of_fold<FOLD>(c, px, py, pz);
+        const float dE = __fadd_rn(__fsub_rn(c.omega[typ + c_new], c.omega[typ + c_old]), deb);
+        // log_lower decides without the logarithm for the rejected ones (trial_f)
+        acc = dE < 0.0f;
+        const bool near = !acc && -dE > log_lower(u);
+        if (__any_sync(0xffffffffu, near)) acc = acc || (near && log_f(u) < -dE);
+        acc = acc && act;
+        if (acc) {
+            x = px;
+            y = py;
+            z = pz;
+        }
+    }
+    return acc;
+}
+
+template <bool ONE, int FOLD, int KEYS>
+__global__ void __launch_bounds__(kSweepForms[ONE ? kFormPairs : kFormPairsList].warps * 32, 1)
+    k_sweep_pairs(const __grid_constant__ SweepArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    float4* const table = reinterpret_cast<float4*>(smem_raw);
+    for (int i = threadIdx.x; i < SCMF_NORMAL_SEGS * kPairCopies; i += blockDim.x) table[i] = __ldg(normal_table() + i / kPairCopies);
+    const float4* const ntab = table + (lane & (kPairCopies - 1));
+    SweepSys* const own = reinterpret_cast<SweepSys*>(table + SCMF_NORMAL_SEGS * kPairCopies) + warp;  // !ONE
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __syncthreads();
+    const int first = warp * (int)gridDim.x + (int)blockIdx.x, stride = nwarps * (int)gridDim.x;
+    const SweepSys& c = ONE ? a.sys : *own;
+    SysDev* S = nullptr;
+    const ArchDev* A = nullptr;
+    uint32_t step = 0u, stop = 0u, rng0 = 0u, typ_e = 0u, typ_o = 0u;
+    float span = 0.0f, cc_e = 0.0f, ac_e = 0.0f, cc_o = 0.0f, ac_o = 0.0f, k2l = 0.0f, k2o = 0.0f, k2r = 0.0f;
+    int slot = 0, k = 0, per = 1;
+    PairHead head{};
+    unsigned nacc = 0;
+    const auto flush = [&](int at) {  // the system's accepted moves so far
+        nacc = warp_sum(nacc);
+        if (lane == 0 && nacc) atomicAdd(&S->slot_acc[at % kSlots], (unsigned long long)nacc);
+        nacc = 0u;
+    };
+#pragma unroll 1
+    for (int i = first; i < a.n_tiles; i += stride) {
+        const WarpTile t = tile_at<ONE>(a, i);
+        const int L = t.length;
+        if (t.arch != A) {
+            if (t.sys != S) {
+                if (!ONE && S) flush(i);
+                S = t.sys;
+                if (!ONE) {
+                    __syncwarp();
+                    const uint32_t* src = reinterpret_cast<const uint32_t*>(&S->sweep);
+                    for (int w = lane; w < (int)(sizeof(SweepSys) / 4); w += 32) reinterpret_cast<uint32_t*>(own)[w] = src[w];
+                    __syncwarp();
+                }
+                step = S->step + 1u;
+                stop = S->stop_step;
+                span = S->omega_span;
+            }
+            A = t.arch;
+            const int h = (L + 1) >> 1;
+            per = 32 / h;
+            slot = (int)div_magic((uint32_t)lane, A->tpc_magic, h);
+            k = lane - slot * h;
+            rng0 = (uint32_t)A->rng_base;
+            const bool has_l = k > 0, has_o = ONE || 2 * k + 1 < L, has_r = 2 * k + 2 < L;
+            k2l = has_l ? c.k2 : 0.0f;
+            k2o = has_o ? c.k2 : 0.0f;
+            k2r = has_r ? c.k2 : 0.0f;
+            const int deg = (has_l ? 1 : 0) + (has_o ? 1 : 0);
+            cc_e = deg == 2 ? c.cdeg[2] : deg == 1 ? c.cdeg[1] : 0.0f;
+            ac_e = deg == 2 ? c.ac4[2] : deg == 1 ? c.ac4[1] : 0.0f;
+            cc_o = has_r ? c.cdeg[2] : c.cdeg[1];
+            ac_o = has_r ? c.ac4[2] : c.ac4[1];
+            typ_e = (uint32_t)__ldg(A->types + 2 * k) * c.n_cells;
+            typ_o = has_o ? (uint32_t)__ldg(A->types + 2 * k + 1) * c.n_cells : 0u;
+            head = pair_head<KEYS>(2u * (uint32_t)k, step, c.seed_lo, a.keys);
+        }
+        if (step > stop) continue;  // the system's sweeps are done
+        const bool has_o = ONE || 2 * k + 1 < L, aligned = ONE || ((L | (int)t.bead0) & 1) == 0;
+        float* const X = c.x + t.bead0;
+        float* const Y = c.y + t.bead0;
+        float* const Z = c.z + t.bead0;
+        float nx[2], ny[2], nz[2];  // the next row's pair
+        const auto fetch = [&](int c0) {
+            const int p = min(c0 + slot, t.n_chains - 1) * L + 2 * k;
+            if (aligned) {
+                const float2 x = __ldcs(reinterpret_cast<const float2*>(X + p)), y = __ldcs(reinterpret_cast<const float2*>(Y + p)),
+                             z = __ldcs(reinterpret_cast<const float2*>(Z + p));
+                nx[0] = x.x, nx[1] = x.y, ny[0] = y.x, ny[1] = y.y, nz[0] = z.x, nz[1] = z.y;
+            } else {
+                const int q = p + (has_o ? 1 : 0);
+                nx[0] = __ldcs(X + p), ny[0] = __ldcs(Y + p), nz[0] = __ldcs(Z + p);
+                nx[1] = __ldcs(X + q), ny[1] = __ldcs(Y + q), nz[1] = __ldcs(Z + q);
+            }
+        };
+        fetch(0);
+#pragma unroll 1
+        for (int c0 = 0; c0 < t.n_chains; c0 += per) {
+            const int cl = min(c0 + slot, t.n_chains - 1), p = cl * L + 2 * k;
+            const bool act = slot < per && c0 + slot < t.n_chains;
+            float xe = nx[0], xo = nx[1], ye = ny[0], yo = ny[1], ze = nz[0], zo = nz[1];
+            if (c0 + per < t.n_chains) fetch(c0 + per);
+            // the odd bead before, or where there is none the bead itself, and no spring
+            float lx = __shfl_up_sync(0xffffffffu, xo, 1), ly = __shfl_up_sync(0xffffffffu, yo, 1), lz = __shfl_up_sync(0xffffffffu, zo, 1);
+            if (k == 0) lx = xe, ly = ye, lz = ze;
+            uint4 we, wo;
+            pair_blocks<KEYS>(rng0 + t.chain + (uint32_t)cl, head, c.seed_lo, c.seed_hi, a.keys, we, wo);
+            float n0, n1, n2, fx = 0.0f, fy = 0.0f, fz = 0.0f;
+            int old_e, new_e, old_o = 0, new_o = 0;
+            normals3<kPairCopies>(we, ntab, n0, n1, n2);
+            add_bond(k2l, xe, ye, ze, lx, ly, lz, fx, fy, fz);
+            add_bond(k2o, xe, ye, ze, xo, yo, zo, fx, fy, fz);
+            const bool me = trial_pair<FOLD>(c, xe, ye, ze, fx, fy, fz, cc_e, ac_e, n0, n1, n2, accept_word(we), span, act, typ_e, old_e, new_e);
+            bool mo = false;
+            if (ONE || L > 1) {
+                // the even bead after, moved
+                float rx = __shfl_down_sync(0xffffffffu, xe, 1), ry = __shfl_down_sync(0xffffffffu, ye, 1), rz = __shfl_down_sync(0xffffffffu, ze, 1);
+                if (2 * k + 2 >= L) rx = xo, ry = yo, rz = zo;
+                normals3<kPairCopies>(wo, ntab, n0, n1, n2);
+                fx = fy = fz = 0.0f;
+                add_bond(c.k2, xo, yo, zo, xe, ye, ze, fx, fy, fz);
+                add_bond(k2r, xo, yo, zo, rx, ry, rz, fx, fy, fz);
+                mo = trial_pair<FOLD>(c, xo, yo, zo, fx, fy, fz, cc_o, ac_o, n0, n1, n2, accept_word(wo), span, act && has_o, typ_o, old_o, new_o);
+            }
+            nacc += (me ? 1u : 0u) + (mo ? 1u : 0u);
+            const bool count_e = me && new_e != old_e, count_o = mo && new_o != old_o;
+            if (a.move_counts && __any_sync(0xffffffffu, count_e || count_o)) {
+                if (count_e) count_move(c.counts, c.count16 != 0, typ_e, old_e, new_e);
+                if (count_o) count_move(c.counts, c.count16 != 0, typ_o, old_o, new_o);
+            }
+            if (aligned) {
+                if (act) {
+                    __stcs(reinterpret_cast<float2*>(X + p), make_float2(xe, xo));
+                    __stcs(reinterpret_cast<float2*>(Y + p), make_float2(ye, yo));
+                    __stcs(reinterpret_cast<float2*>(Z + p), make_float2(ze, zo));
+                }
+            } else {
+                if (me) X[p] = xe, Y[p] = ye, Z[p] = ze;
+                if (mo) X[p + 1] = xo, Y[p + 1] = yo, Z[p + 1] = zo;
+            }
+        }
+    }
+    if (S) flush(first);
+}
+
 // ------------------------------------------------------ many sweeps a launch
 // A barrier of all CTAs of a (cooperative) launch, on a count in global memory
 // that only grows, by one a CTA and barrier.  CTAs that give up do so after different

@@ -239,11 +239,12 @@ static bool screen_of(const SysDev& d, int g, float* a, float* b) {
 static ScreenDev screen_constants(const SysDev& d) {
     ScreenDev s{};
     const double delta = SCMF_SCREEN_DELTA, A = d.A;
-    s.on = A > 0.0 && A * (double)d.cdeg[2] >= kScreenFromAc;
+    for (int level = kScreenGraphs; level <= kScreenAll; ++level)
+        if (A > 0.0 && A * (double)d.cdeg[2] >= kScreenFromAc[level]) s.on = level;
     s.add = rounded_up((1.0 + 1.0 / kScreenEta) * 3.0 * delta * delta * kScreenUnit * kScreenUnit);
     s.u = rounded_up(4.0 / A);
     for (int g = 1; g <= 2; ++g)
-        if (!screen_of(d, g, &s.a[g], &s.b[g])) s.on = 0;
+        if (!screen_of(d, g, &s.a[g], &s.b[g])) s.on = kScreenOff;
     return s;
 }
 
@@ -315,7 +316,7 @@ void fill_sweep_constants(SysDev* d) {
     d->by_deg[0] = BondConsts{0.0f, INFINITY, 0.0f, 0.0f};  // no bond, nothing to screen by
     for (int g = 1; g <= kGraphDeg; ++g) {
         float a, b;
-        if (!screen_of(*d, g, &a, &b)) w.screen.on = 0;
+        if (!screen_of(*d, g, &a, &b)) w.screen.on = kScreenOff;
         d->by_deg[g] = BondConsts{a, b, d->cdeg[g], d->ac4deg[g]};
     }
     FieldSys& f = d->field;
@@ -415,19 +416,21 @@ static int tiles_of(const std::vector<SweepArch>& ranges) {
 
 std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return {};
-    int64_t beads = 0, exact = 0;  // all, and those of chains that are not screened
+    int64_t beads = 0, exact = 0;  // all, and those of chains whose trials k_sweep_pairs makes as fast as a screen does
+    bool screened = false;
     for (const auto& c : p.chains) {
         beads += (int64_t)c.length * c.n_chains;
-        exact += c.screened ? 0 : (int64_t)c.length * c.n_chains;
+        exact += c.screen < kScreenAll ? (int64_t)c.length * c.n_chains : 0;
+        screened = screened || c.screen >= kScreenTiles;
     }
-    *form = !p.linear ? kFormGraph : exact < beads ? kFormScreened : kFormUnscreened;
+    *form = !p.linear ? kFormGraph : screened ? kFormScreened : kFormUnscreened;
     if (p.linear && p.max_length > kSweepForms[*form].beads) *form = kFormLong;
     if (p.max_length > kSweepForms[*form].beads) return {};
     std::vector<SweepArch> out = form_ranges(p, *form);
     // Trials that are all made exactly are made faster in registers (k_sweep_pairs) than in tiles, from 352 beads a warp
     // on also than in k_run: a sweep of 0.4M beads 12.4 us in k_run and 16.0 so, 0.8M 21.3 and 18.9 (in chains of 48 or 64
-    // 19.4 and 20.3, 19.0 and 19.7), 2.0M 46.1 and 33.5, 20.5M 379 (in tiles) and 223.  So are many systems of which a
-    // quarter of the beads is not screened: 32M beads, 25 % 467 us in tiles and 432 so, 50 % 634 and 452, 10 % 350 and
+    // 19.4 and 20.3, 19.0 and 19.7), 2.0M 46.1 and 33.5, 20.5M 379 (in tiles) and 223.  So are those of many systems of
+    // which a quarter of the beads is not screened: 32M beads, 25 % 467 us in tiles and 432 so, 50 % 634 and 452, 10 % 350 and
     // 399.  At least three lanes of four must have a pair.
     const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
     if (p.linear && (exact == beads ? beads > 352 * warps : tiles_of(out) > warps && 4 * exact >= beads)) {
@@ -738,7 +741,7 @@ scmf_status scmf_system::append_plan(const scmf_tune& t, Plan* p) {
         }
         p->max_length = std::max(p->max_length, A.length);
         // a bead without bonds has no energy to screen by
-        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.linear, A.bead_base, sweep.screen.on && A.max_deg > 0});
+        p->chains.push_back({d_sys, d_arch + a, A.length, A.n_chains, A.linear, A.bead_base, A.max_deg ? sweep.screen.on : kScreenOff});
         p->max_deg = std::max(p->max_deg, A.max_deg);
         p->linear = p->linear && A.linear;
     }

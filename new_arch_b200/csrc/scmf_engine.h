@@ -88,7 +88,7 @@ struct Plan {
         int length, n_chains;
         bool linear;
         int64_t bead_base;
-        bool screened;
+        int screen;  // ScreenLevel
     };
     std::vector<Chains> chains;
     std::vector<std::pair<SysDev*, int64_t>> cells;  // of every system, for the field tiles of k_run

@@ -105,7 +105,7 @@ struct ScreenDev {
     float a[3], b[3];  // a = (A - 1/c) / R
     float u;           // 4 / A
     float add;
-    int32_t on;  // 0: every trial is resolved (see screen_constants)
+    int32_t on;  // ScreenLevel (see screen_constants)
     int32_t pad;
 };
 
@@ -382,7 +382,14 @@ constexpr SweepForm kSweepForms[6] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280
 // this before they come to the beads of a long form.
 constexpr int kTilePairs = 32 * 32;
 constexpr size_t kL2Bytes = 126u << 20;
-constexpr float kScreenFromAc = 2.0f;  // A 4k from which the screen runs
+// The screen of a system by x = A 4k: from which x it runs for branched chains, for linear
+// ones, and for linear ones even where k_sweep_pairs could make every trial.  Below a line
+// so many trials pass that making all of them is faster.  10M beads in chains of 33, x 2.4:
+// screened 226 us a sweep, not 185; x 3.1: 137 and 174.  20.5M beads in chains of 32, x 3.1:
+// screened 298, in k_sweep_pairs 216; x 3.7: 191 and 209.  10M beads in combs, x 1.96: 255 and
+// 235; x 2.4: 210 and 229.
+enum ScreenLevel : int { kScreenOff = 0, kScreenGraphs = 1, kScreenTiles = 2, kScreenAll = 3 };
+constexpr float kScreenFromAc[4] = {0.0f, 2.0f, 2.8f, 3.4f};
 
 // Streaming multiprocessors of the current device (read once per device; 148
 // on a B200), for grid and tile sizing.

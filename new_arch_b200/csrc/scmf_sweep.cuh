@@ -800,7 +800,8 @@ struct Mover {
         s.add = c.screen.add;
         s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
         s.u1 = __fmul_rn(c.screen.u, -0x1.62e7p-1f);  // a little over ln 2
-        mode = !active ? 0 : FORM != kFormUnscreened && c.screen.on && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
+        const bool screened = FORM != kFormUnscreened && c.screen.on >= (graph() ? kScreenGraphs : kScreenTiles);
+        mode = !active ? 0 : screened && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
         const int k = lane & (s.h - 1);
         s.pc = pair_consts(s, k == 0, false, k == s.h - 1);
         s.head = pair_head<KEYS>(2u * (uint32_t)k, s.step, s.k0, a.keys);

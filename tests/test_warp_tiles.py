@@ -18,7 +18,7 @@ using namespace scmf;
 static int check(std::initializer_list<Plan::Chains> chains, bool screened) {
     Plan p;
     for (Plan::Chains c : chains) {
-        c.screened = screened && c.length > 1;
+        c.screen = screened && c.length > 1 ? kScreenAll : kScreenOff;
         p.chains.push_back(c);
         p.linear = p.linear && c.linear;
         p.max_length = c.length > p.max_length ? c.length : p.max_length;
@@ -46,7 +46,7 @@ static int check(std::initializer_list<Plan::Chains> chains, bool screened) {
 int main() {
     int bad = 0;
     const auto of = [](int length, long long beads, bool linear) {
-        return Plan::Chains{nullptr, nullptr, length, (int)(beads / length), linear, 0, false};
+        return Plan::Chains{nullptr, nullptr, length, (int)(beads / length), linear, 0, kScreenOff};
     };
     for (int screened = 0; screened < 2; ++screened)
         for (int length = 1; length <= 64; ++length)

@@ -517,7 +517,7 @@ static std::vector<char> run_tables(const Plan& p, int n_warp, int form, RunArgs
     std::memcpy(image.data() + at_field, field.data(), field.size() * sizeof(FieldTile));
     *run = RunArgs{};
     run->barrier = nullptr;
-    run->wait_clocks = kWaitClocks;
+    run->wait = (uint32_t)(kWaitClocks >> kWaitShift);
     run->systems = (const RunSystem*)(size_t)64;
     run->field = (const FieldTile*)at_field;
     run->ef_part = (double*)at_ef;

@@ -238,6 +238,7 @@ struct FieldTile {
 // that did not arrive; blocks of a launch that did not come to a barrier.
 constexpr uint32_t kErrorSize = 1u, kErrorTile = 4u, kErrorBarrier = 8u;
 constexpr long long kWaitClocks = 4000000000ll;  // a wait in a kernel gives up after about two seconds
+constexpr int kWaitShift = 10;
 
 enum SweepMode : int { kMoveOnly = 0, kMoveGrid = 1, kGridOnly = 2 };
 
@@ -339,8 +340,8 @@ struct RunArgs {
     const FieldTile* field;       // a warp's work each
     double* ef_part;              // field energy of every field tile after the last sweep
     unsigned long long* barrier;  // the grid barrier's count, and after it whether it is broken
-    int n_sys, n_field, n_sweeps, pad;
-    long long wait_clocks;        // how long a block waits for the others (kWaitClocks)
+    int n_sys, n_field, n_sweeps;
+    uint32_t wait;                // how long a block waits for the others, in 2^kWaitShift clocks
 };
 
 // Parameters of k_sweep_warp.
@@ -382,8 +383,8 @@ constexpr SweepForm kSweepForms[6] = {{16, 960}, {8, 1984}, {16, 960}, {12, 1280
 // this before they come to the beads of a long form.
 constexpr int kTilePairs = 32 * 32;
 constexpr size_t kL2Bytes = 126u << 20;
-// The screen of a system by x = A 4k: from which x it runs for branched chains, for linear
-// ones, and for linear ones even where k_sweep_pairs could make every trial.  Below a line
+// The screen of a system by x = A 4k: from which x it runs in plans with branched chains, in
+// those of linear ones, and in these even where k_sweep_pairs could make every trial.  Below a line
 // so many trials pass that making all of them is faster.  10M beads in chains of 33, x 2.4:
 // screened 226 us a sweep, not 185; x 3.1: 137 and 174.  20.5M beads in chains of 32, x 3.1:
 // screened 298, in k_sweep_pairs 216; x 3.7: 191 and 209.  10M beads in combs, x 1.96: 255 and

@@ -800,7 +800,7 @@ struct Mover {
         s.add = c.screen.add;
         s.u0 = __fmul_rn(c.screen.u, __fadd_rn(span, 0x1p-18f));
         s.u1 = __fmul_rn(c.screen.u, -0x1.62e7p-1f);  // a little over ln 2
-        const bool screened = FORM != kFormUnscreened && c.screen.on >= (graph() ? kScreenGraphs : kScreenTiles);
+        const bool screened = FORM != kFormUnscreened && c.screen.on >= (FORM == kFormGraph ? kScreenGraphs : kScreenTiles);
         mode = !active ? 0 : screened && s.L > 1 ? 2 : 1;  // one bead has no energy to screen by
         const int k = lane & (s.h - 1);
         s.pc = pair_consts(s, k == 0, false, k == s.h - 1);
@@ -1144,39 +1144,37 @@ __global__ void __launch_bounds__(kSweepForms[ONE ? kFormPairs : kFormPairsList]
 // that only grows, by one a CTA and barrier.  CTAs that give up do so after different
 // numbers of barriers: from then on the barrier is broken, and no launch uses it again.
 struct GridBarrier {
-    unsigned long long* count;  // and after it a word that is set when the barrier breaks
-    long long clocks;           // how long to wait
+    const RunArgs& r;           // barrier: the count, and after it a word that is set when the barrier breaks
     unsigned long long target;  // thread 0's
-    bool broken;                // thread 0's
     // The count is a whole number of barriers until the last CTA comes to the first one.
-    __device__ __forceinline__ GridBarrier(unsigned long long* c, long long limit)
-        : count(c), clocks(limit), target(0), broken(false) {
+    // Thread 0 says in *s_ok whether the barrier is whole.
+    __device__ __forceinline__ GridBarrier(const RunArgs& run, int* s_ok) : r(run), target(0) {
         if (threadIdx.x == 0) {
-            target = __ldcg(c) / gridDim.x * gridDim.x;
-            broken = __ldcg(c + 1) != 0ull;
+            target = __ldcg(r.barrier) / gridDim.x * gridDim.x;
+            *s_ok = __ldcg(r.barrier + 1) == 0ull;
         }
     }
     __device__ __forceinline__ void arrive() {
         __syncthreads();
         if (threadIdx.x == 0) {
             target += gridDim.x;
-            asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+            asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(r.barrier) : "memory");
         }
     }
-    // False (to all threads of the CTA) after `clocks`, or where the barrier is broken.
-    // Thread 0 calls `then` before the others go on.
+    // False (to all threads of the CTA) after r.wait.  Thread 0 calls `then` before the
+    // others go on.
     template <typename Then>
     __device__ __forceinline__ bool wait(int* s_ok, const Then& then) {
         if (threadIdx.x == 0) {
             unsigned long long now;
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
-            if (now < target && !broken) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(r.barrier) : "memory");
+            if (now < target) {
                 const long long t0 = clock64();
                 do {
-                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(count) : "memory");
-                } while (now < target && clock64() - t0 < clocks);
+                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(r.barrier) : "memory");
+                } while (now < target && (uint32_t)((clock64() - t0) >> kWaitShift) < r.wait);
             }
-            *s_ok = now >= target && !broken;
+            *s_ok = now >= target;
             then();
         }
         __syncthreads();
@@ -1333,7 +1331,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
     const int lane = threadIdx.x & 31;
     const int first = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x, stride = (int)(blockDim.x >> 5) * (int)gridDim.x;
     const bool any = first < a.n_tiles;
-    GridBarrier barrier(r.barrier, r.wait_clocks);
+    GridBarrier barrier(r, &s_ok);
     if (ONE && threadIdx.x == 0) s_span = a.system->omega_span;
     if (threadIdx.x < 2) s_keys[threadIdx.x] = threadIdx.x ? 0xFFFFFFFFu : 0u;
     for (int i = blockIdx.x; i < r.n_sys; i += gridDim.x) {  // the slot of the launch's first field step
@@ -1364,6 +1362,7 @@ __global__ void __launch_bounds__(SweepLayout<FORM>::kWarps * 32, 1)
             __syncwarp();
         }
     }
+    if (!s_ok) return give_up(r);  // to be seen since the block's barrier in start()
     // the warp's field tile (its first, where it has several) and that one's system
     FieldSys* const fs = &wp->field;
     const auto at_field = [&](const FieldTile& t) {

@@ -101,11 +101,11 @@ static std::vector<uint32_t> counts(const scmf_system* s) {
 int main() {
     scmf_system* s = started(melt(60000, 32, 64, 5));
     WANT(s->plan.d_run != nullptr, true);  // many sweeps a launch
-    s->plan.run.wait_clocks = 0;           // a look or two at the count, and no more
+    s->plan.run.wait = 0;                  // a look or two at the count, and no more
     WANT(scmf_step(s, 20), SCMF_E_DEVICE);
     WANT(record(s).error_word, kErrorBarrier);
     WANT(record(s).step, 0);
-    s->plan.run.wait_clocks = kWaitClocks;
+    s->plan.run.wait = (uint32_t)(kWaitClocks >> kWaitShift);
     set_word(s->d_sys, 0);  // as if nothing had been: the plan's barrier stays broken
     WANT(scmf_step(s, 1100), SCMF_E_DEVICE);
     WANT(record(s).error_word, kErrorBarrier);

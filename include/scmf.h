@@ -363,15 +363,20 @@ scmf_status scmf_analyze(const scmf_system* sys, scmf_observables* out, int32_t 
  * one system per process). */
 typedef struct scmf_batch scmf_batch;
 
+/* Launch options; results do not depend on them.  The move options apply where the general
+ * move kernel runs: in plans with a bead of more than six bonds, a linear chain of more than
+ * 1,984 beads (1,280 beside branched ones), a branched one of more than 1,280, or 2^31 cells
+ * times types.  The other move kernels share out the chains by themselves.  The field options
+ * apply to sweeps that are launched one by one: those of plans that do not stay on the chip,
+ * and single ones. */
 typedef struct scmf_tune {
-    int32_t chains_per_tile;   /* 0 = per-architecture default */
-    int32_t threads_move;      /* 0 = default */
-    int32_t cells_per_tile;    /* 0 = default */
-    int32_t threads_field;     /* 0 = default */
-    int32_t persistent_ctas;   /* 0 = one CTA per tile (no persistence) */
-    int32_t use_graph;         /* 1 = a sweep that takes launches of its own may be replayed from a
-                                  CUDA graph */
-    int32_t beads_per_tile;    /* > 0: chains per tile = max(1, beads_per_tile / length) for each
+    int32_t chains_per_tile;   /* move: 0 = per-architecture default */
+    int32_t threads_move;      /* move: 0 = default */
+    int32_t cells_per_tile;    /* field: 0 = default */
+    int32_t threads_field;     /* field: 0 = default */
+    int32_t persistent_ctas;   /* both: 0 = one CTA per tile (no persistence) */
+    int32_t use_graph;         /* move: 1 = a sweep is replayed from a CUDA graph */
+    int32_t beads_per_tile;    /* move: > 0: chains per tile = max(1, beads_per_tile / length) for each
                                   architecture (takes precedence over chains_per_tile) */
     int32_t reserved;
 } scmf_tune;
@@ -387,7 +392,8 @@ scmf_status scmf_batch_step_async(scmf_batch* b, int32_t n_sweeps);
 scmf_status scmf_batch_step_profiled(scmf_batch* b, int32_t n_sweeps, float* ms_move, float* ms_field,
                                      float* ms_total);
 /* Times candidate tunings on snapshots of the batch's systems (their state is
- * restored afterwards) and installs the fastest; *out receives it. */
+ * restored afterwards) and installs the fastest; *out receives it.  Options that
+ * do not apply to the batch (see scmf_tune) are not tried. */
 scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps_per_trial, scmf_tune* out);
 /* One tuning the last scmf_batch_autotune timed, with the device time of its
  * timed sweeps (milliseconds). */

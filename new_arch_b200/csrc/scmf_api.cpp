@@ -945,8 +945,8 @@ static void snap_free(Snapshot* sn, cudaStream_t st) {
 
 // Project-written autotuner: times a small grid of (threads per move CTA,
 // chains per tile, persistent CTAs), where the general move kernel runs, and
-// then (cells per field tile) on the batch's own systems, restoring their state
-// after every trial.
+// then (cells per field tile), where sweeps are launched one by one, on the
+// batch's own systems, restoring their state after every trial.
 scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
     if (!b || sweeps < 1) return fail(SCMF_E_INVALID, "bad arguments");
     RET(batch_sync_members(b));
@@ -1009,7 +1009,7 @@ scmf_status scmf_batch_autotune(scmf_batch* b, int32_t sweeps, scmf_tune* out) {
         }
         const scmf_tune base = best;
         for (int c : {2048, 8192, 32768}) {
-            if (rc) break;
+            if (rc || b->plan.d_run) break;  // a launch of many sweeps sizes its field tiles too
             scmf_tune t = base;
             t.cells_per_tile = c;
             tried(t);

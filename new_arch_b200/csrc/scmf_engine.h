@@ -49,7 +49,8 @@ struct ArchHost {
 // ones to and from pageable memory through a pinned buffer and several threads.
 // copy_to_host waits for the stream and the copy.  copy_to_device_staged makes
 // the copy if it is one of those (else false), calling `enqueued` after every
-// piece with the bytes that the stream's copies so far cover, and waits for it.
+// piece with the bytes that the stream's copies so far cover, and waits for it, and
+// before it for the stream's earlier work.
 scmf_status copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
 bool copy_to_device_staged(void* dev, const void* host, size_t bytes, cudaStream_t st,
                            const std::function<scmf_status(size_t)>& enqueued, scmf_status* rc);

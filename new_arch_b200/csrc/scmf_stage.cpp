@@ -35,9 +35,9 @@ constexpr size_t kStageFrom = 64u << 20;  // from here the copy gains more than 
 constexpr size_t kPieceBytes = 1u << 20;
 constexpr int kPieces = 12;
 
-std::mutex g_mu;               // the buffer's user, and the two below
+std::mutex g_mu;               // the buffer's user
 char* g_buffer = nullptr;
-int g_systems = 0;             // systems alive
+std::atomic<int> g_systems{0};  // systems alive (making and destroying one waits for no copy)
 
 bool pageable(const void* p) {
     cudaPointerAttributes a{};
@@ -100,7 +100,8 @@ struct Transfer {
 bool staged(void* dev, void* host, size_t bytes, bool to_host, cudaStream_t st,
             const std::function<scmf_status(size_t)>& enqueued, scmf_status* rc) {
     if (bytes < kStageFrom || !pageable(host)) return false;
-    if (to_host && cudaStreamSynchronize(st) != cudaSuccess) return false;  // no thread spins on earlier work
+    // nobody waits for earlier work of the stream with the buffer in hand, and no thread spins on it
+    if (cudaStreamSynchronize(st) != cudaSuccess) return false;
     std::unique_lock<std::mutex> lock(g_mu, std::try_to_lock);
     if (!lock.owns_lock()) return false;
     if (!g_buffer && cudaHostAlloc((void**)&g_buffer, kPieces * kPieceBytes, cudaHostAllocPortable) != cudaSuccess) {
@@ -173,14 +174,12 @@ bool copy_to_device_staged(void* dev, const void* host, size_t bytes, cudaStream
     return staged(dev, const_cast<void*>(host), bytes, false, st, enqueued, rc);
 }
 
-void stage_system_made() {
-    std::lock_guard<std::mutex> g(g_mu);
-    ++g_systems;
-}
+void stage_system_made() { ++g_systems; }
 
 void stage_system_gone() {
+    if (--g_systems) return;
     std::lock_guard<std::mutex> g(g_mu);
-    if (--g_systems == 0 && g_buffer) {
+    if (g_systems == 0 && g_buffer) {  // another may have been made meanwhile
         cudaFreeHost(g_buffer);
         g_buffer = nullptr;
     }

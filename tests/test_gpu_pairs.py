@@ -82,6 +82,26 @@ def test_moves_without_counts():
         compare_state(s, orc, "smc_move", energies=False)
 
 
+@pytest.mark.parametrize("length", [32, 3])
+def test_any_omega(length):
+    """The caller's omega with NaN, infinite and very large cells among ordinary ones."""
+    import numpy as np
+    import new_arch_b200 as nb
+    spec = _spec([(length, BEADS // length + 1)], (64, 64, 64))
+    with nb.System(spec) as s:
+        s.init_coords()
+        orc = oracle_for(spec)
+        rng = np.random.default_rng(5)
+        w = rng.normal(0.0, 2.0, 2 * 64 ** 3).astype(np.float32)
+        odd = rng.integers(0, w.size, w.size // 20)
+        w[odd] = rng.choice(np.float32([np.nan, np.inf, -np.inf, 3e38, -3e38, 1e-40, -0.0]), odd.size)
+        s.set_omega(w)
+        orc.set_omega(w)
+        s.smc_move(2)
+        orc.smc_move(2)
+        assert_coords_equal(s.coords(), orc.coords(), "any omega")
+
+
 @pytest.mark.parametrize("seeds", ["one", "upper half", "any"])
 def test_batch(seeds):
     import new_arch_b200 as nb

@@ -180,7 +180,8 @@ scmf_status scmf_step(scmf_system* sys, int32_t n_sweeps);
 /* The same, enqueued on the system's stream without waiting (for graphs of
  * the caller's own work and for timing with events on that stream). */
 scmf_status scmf_step_async(scmf_system* sys, int32_t n_sweeps);
-/* n_sweeps full MC steps enqueued kernel by kernel (no graph) with CUDA
+/* n_sweeps full MC steps enqueued kernel by kernel (no graph, no launch of many
+ * sweeps, which scmf_step may use) with CUDA
  * events around every launch on the system's stream; returns after the last
  * sweep with the summed device time of the fused move+grid kernel, of the
  * field kernel, and the device time from the first launch to the end of the
@@ -387,8 +388,7 @@ scmf_status scmf_batch_step(scmf_batch* b, int32_t n_sweeps);
 /* The same, enqueued on the batch's stream without waiting. */
 scmf_status scmf_batch_step_async(scmf_batch* b, int32_t n_sweeps);
 /* scmf_step_profiled for a batch: its sweeps launch by launch with CUDA events
- * on the batch's stream; the move time covers both move launches of a plan
- * that runs them side by side.  Same results as scmf_batch_step. */
+ * on the batch's stream.  Same results as scmf_batch_step. */
 scmf_status scmf_batch_step_profiled(scmf_batch* b, int32_t n_sweeps, float* ms_move, float* ms_field,
                                      float* ms_total);
 /* Times candidate tunings on snapshots of the batch's systems (their state is

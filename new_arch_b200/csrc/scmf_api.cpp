@@ -603,9 +603,9 @@ scmf_status scmf_step(scmf_system* s, int32_t n) {
 }
 
 // n fused sweeps of a plan enqueued launch by launch, each bracketed by CUDA
-// events on `st`: the summed device time of the move launches (both tile kinds
-// when the plan forks them), of the field launches, and from the first launch
-// to the end of the last.
+// events on `st`: the summed device time of the move launches, of the field
+// launches, and from the first launch to the end of the last.  Launched so even
+// where run_sweeps makes many sweeps a launch or chains its launches.
 static scmf_status profile_sweeps(const DevPlan& p, cudaStream_t st, int32_t n, float* ms_move, float* ms_field,
                                   float* ms_total) {
     *ms_move = 0.0f;

@@ -5,9 +5,10 @@
 // The reference's host orchestration (smc.cu:3-72, mesh.cu:161-248,
 // mesh_mpi.cpp:4-27, test.cpp:37-43) launches one kernel at a time with a
 // cudaDeviceSynchronize after each and a P2P/MPI density reduction.  Here a
-// sweep is two launches on one stream (fused move+grid, then field) with no
-// host round trip, optionally replayed from a CUDA graph; the step counter,
-// the counts double buffer and the statistics live on the device.
+// sweep is a share of one launch of many sweeps, two launches chained on one
+// stream (fused move+grid, then field) or a replayed CUDA graph of these
+// (DevPlan::run_sweeps), with no host round trip; the step counter, the counts
+// and the statistics live on the device.
 #include "scmf_engine.h"
 #include "scmf_screen_table.h"
 
@@ -373,7 +374,7 @@ void DevPlan::release() {
     n_move = n_field = n_sys = n_warp = 0;
 }
 
-// The tiles of k_sweep_warp: whole chains of one architecture, as many chains in
+// The tiles of the move kernels of warp tiles: whole chains of one architecture, as many chains in
 // each (SweepArch::per).  Every warp of the GPU gets the same number of tiles, of
 // sizes up to what its buffer holds and no smaller than a row of 32 bead pairs.
 // A tile of linear chains also has no more than kTilePairs bead pairs.  Empty for a plan
@@ -553,7 +554,6 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     }
     sweep = p.sweep;
     once = p.position_bytes > kL2Bytes / 2;
-    beads = (int64_t)(p.position_bytes / 12);
     const size_t nm = std::max<size_t>(1, p.move.size()), nf = std::max<size_t>(1, p.field.size());
     scmf_status rc;
     if ((rc = dev_alloc((void**)&d_move, nm * sizeof(MoveTile), st)) ||

@@ -82,7 +82,7 @@ struct Plan {
     SweepSys sweep{};           // of the first system
     bool linear = true;   // every architecture is a linear chain
     bool cells32 = true;  // cells times types below 2^31 in every system
-    // the chains of every architecture, for the warp tiles of k_sweep_warp
+    // the chains of every architecture, for the warp tiles
     struct Chains {
         SysDev* sys;
         const ArchDev* arch;
@@ -100,7 +100,7 @@ struct Plan {
 };
 
 // The warp tiles of a plan, an entry for each of its `chains`, and the kernels' form
-// (SweepFormId); empty for a plan that k_sweep_warp does not take.
+// (SweepFormId); empty for a plan that takes the general move kernel.
 std::vector<SweepArch> tile_ranges(const Plan& p, int* form);
 
 struct DevPlan {
@@ -110,7 +110,6 @@ struct DevPlan {
     // k_run: its systems, field tiles, partial energies and barrier, in one buffer
     void* d_run = nullptr;
     RunArgs run{};
-    int64_t beads = 0;           // of all systems
     // one system of few architectures: its constants and tile ranges (no list)
     bool one = false;
     SysDev* system = nullptr;
@@ -118,7 +117,7 @@ struct DevPlan {
     int n_arch = 0;
     SweepArch arch[kSweepMaxArch] = {};
     bool once = false;           // the positions are more than L2 holds
-    WarpTile* d_warp = nullptr;  // tiles of k_sweep_warp (see tile_ranges)
+    WarpTile* d_warp = nullptr;  // warp tiles, where the launch has a list (see tile_ranges)
     double* d_ef = nullptr;      // field energy per field tile
     double* d_eb = nullptr;      // bond energy per move tile
     int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;

@@ -82,7 +82,7 @@ struct ArchDev {
     float init_sigma;
 };
 
-// The screen of k_sweep_warp: constants of the test that proves a trial
+// The screen of k_sweep_warp and k_run: constants of the test that proves a trial
 // rejected before its exact normals, energy and omega are formed.
 //
 // With d = A f + R n the displacement and c = 2k deg, the energy that the trial
@@ -109,7 +109,7 @@ struct ScreenDev {
     int32_t pad;
 };
 
-// What the move kernel of warp tiles reads of a system, fixed for its life.
+// What the move kernels of warp tiles read of a system, fixed for its life.
 struct SweepSys {
     float *x, *y, *z;
     const float* omega;
@@ -215,7 +215,7 @@ struct MoveTile {
     int32_t arch_index;   // architecture of the tile within its system
 };
 
-// Work item of k_sweep_warp: a run of whole chains of one architecture.
+// Work item of the move kernels of warp tiles: a run of whole chains of one architecture.
 struct WarpTile {
     SysDev* sys;
     const ArchDev* arch;
@@ -315,7 +315,7 @@ struct LaunchShape {
     // `keys`, kKeysHigh when they share its upper 32 bits, else kKeysNone
     int keyed;
     PhiloxKeys keys;
-    // every architecture of the launch fits a warp's tile: the tiles of k_sweep_warp
+    // every architecture of the launch fits a warp's tile (see tile_ranges)
     const WarpTile* warp_tiles;
     int n_warp_tiles;
     int form;           // SweepFormId
@@ -344,7 +344,7 @@ struct RunArgs {
     uint32_t wait;                // how long a block waits for the others, in 2^kWaitShift clocks
 };
 
-// Parameters of k_sweep_warp.
+// Parameters of the move kernels of warp tiles.
 struct SweepArgs {
     const WarpTile* tiles;
     int n_tiles, move_counts, once, pad;
@@ -406,11 +406,11 @@ int launch_copy_counts(const SysDev* d_sys, uint32_t* dst, int64_t n_words, void
 // kernel one per move tile into eb_part; k_close sums and publishes them.
 int launch_sweep(int mode, const MoveTile* tiles, int n_tiles, int max_tile_beads, int max_length,
                  const LaunchShape& shape, void* stream);
-// close_mode != 0: the last field tile of every system closes it in the same
-// launch (what k_close does with that mode), so a sweep is two launches.
 // n_sweeps whole sweeps of a plan with warp tiles (shape.warp_tiles)
 // in one cooperative launch.
 int launch_run(const LaunchShape& shape, const RunArgs& run, void* stream);
+// close_mode != 0: the last field tile of every system closes it in the same
+// launch (what k_close does with that mode), so a sweep is two launches.
 int launch_field(bool fused, int force_update, const FieldTile* tiles, int n_tiles, LaunchShape shape,
                  double* ef_part, int close_mode, void* stream);
 int launch_bond_energy(const MoveTile* tiles, int n_tiles, LaunchShape shape, double* eb_part, void* stream);

@@ -1,12 +1,15 @@
 // sm_100a kernels of the SCMF engine.
 //
 //   k_init_coords   random-walk chains (device_function.cu:140-207)
-//   k_sweep_warp    one MC sweep of linear chains (scmf_sweep.cuh): odd/even
-//                   half-sweeps of smart-MC trials (device_function.cu:444-454,
+//   k_sweep_warp    one MC sweep on warp tiles, of linear chains and other bond
+//                   graphs of up to six bonds a bead (scmf_sweep.cuh): odd/even or
+//                   colour by colour, smart-MC trials (device_function.cu:444-454,
 //                   509-799), moving one cell count for each accepted move that
 //                   leaves its cell, so counts stay the grid of the positions
 //                   (device_function.cu:471-508)
-//   k_sweep         the same for any bond graph (graph-colour half-sweeps)
+//   k_sweep_pairs   the same in registers, where no trial is screened
+//   k_run           many whole sweeps, where the positions fit on the chip
+//   k_sweep         a sweep of what these do not take (longer chains, more bonds)
 //   k_grid          counts of the current positions from scratch
 //   k_field<fused>  counts -> omega (SCMF0, device_function.cu:373-412) with the
 //                   field-energy reduction; in the fused step the block that
@@ -260,7 +263,7 @@ size_t sweep_smem_bytes(int max_tile_beads, int max_length) {
 }
 
 // One MC sweep over tiles of whole chains staged in shared memory: of plans that
-// k_sweep_warp does not take (a bead of more than six bonds, a chain longer than a
+// the kernels of warp tiles do not take (a bead of more than six bonds, a chain longer than a
 // warp's tile, 2^31 cells times types), every trial made exactly.
 //   MODE kMoveOnly / kMoveGrid: moves; moves keeping counts[cur] the grid of
 //   the positions (accepted moves that change cell move a count).
@@ -1143,7 +1146,7 @@ static cudaError_t launch_chained(void (*kernel)(Args...), int blocks, int threa
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// The launch of a plan's warp tiles: k_sweep_warp, or k_run when `run` is given.
+// A launch over warp tiles in shared memory: k_sweep_warp, or k_run when `run` is given.
 template <bool ONE, int FORM, int KEYS>
 static cudaError_t launch_form(const SweepArgs& a, const RunArgs* run, bool chained, cudaStream_t st) {
     using Lay = SweepLayout<FORM>;

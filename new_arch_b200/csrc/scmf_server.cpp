@@ -9,8 +9,8 @@
 //   rounds      at each round boundary adds the ready systems, drops the
 //               finished and cancelled ones, rebuilds the batched plan if the
 //               set changed, and runs a fixed number of sweeps over every
-//               active system on the server stream (one move and one field
-//               launch per sweep for all of them).  A system stops at its own
+//               active system on the server stream (one launch for all of them
+//               and the round's sweeps, or two for each sweep).  A system stops at its own
 //               sweep count inside the round: its SysDev stop_step makes the
 //               kernels skip its tiles, so rounds are not cut short by the
 //               request with the fewest sweeps left.

@@ -1,6 +1,6 @@
-// The move on warp tiles: k_sweep_warp (one sweep's move of any systems) and
-// k_run (many whole sweeps of systems that fit on the chip); included by
-// scmf_kernels.cu.
+// The move on warp tiles: k_sweep_warp (one sweep's move of any systems),
+// k_sweep_pairs (of systems that are not screened) and k_run (many whole sweeps of
+// systems that fit on the chip); included by scmf_kernels.cu.
 //
 // What a sweep costs is arithmetic: every trial needs its Philox block (twenty
 // 32 x 32 -> 64 bit products, four cycles of a scheduler's multiplier each),
@@ -24,11 +24,11 @@
 //    Even beads first; every odd neighbour of an even bead that moved, whose
 //    screen saw the old position, is added to the odd beads' list.
 //
-// A system whose proposals mostly pass (ScreenDev::on 0: the reference's own
-// units) skips the screen and resolves every trial.  Either way positions and
+// A system whose proposals mostly pass (ScreenLevel: the reference's own units)
+// skips the screen and resolves every trial, here or in k_sweep_pairs.  Either way positions and
 // counts are the ones that the oracle gives, bit for bit.
 //
-// Each warp has tiles of its own (up to kSweepBeads beads in its part of shared
+// Each warp has tiles of its own (up to SweepLayout::kBeads beads in its part of shared
 // memory) and waits for no other warp.  Measured against this on the large system
 // (51.2M beads, 0.326 ms): warps that only screen beside warps that only resolve
 // 0.375 ms (an exact trial waits for positions, table and omega, but mostly it
@@ -874,7 +874,7 @@ __device__ __forceinline__ WarpTile tile_at(const SweepArgs& a, int i) {
 }
 
 // One move of the systems of a launch.  One CTA per SM; each warp strides over
-// the tiles (whole chains of one architecture, up to kSweepBeads beads), whose
+// the tiles (whole chains of one architecture, up to SweepLayout::kBeads beads), whose
 // positions come by bulk copies, the next tile's from the moment the current one
 // is done.  Beads that move are written back, and nothing else.
 //

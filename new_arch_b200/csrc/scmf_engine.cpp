@@ -651,9 +651,14 @@ scmf_status DevPlan::run_sweeps(cudaStream_t st, int n) {
         const LaunchShape sh = move_shape();
         for (RunArgs r = run; n > 0; n -= r.n_sweeps) {
             r.n_sweeps = std::min(n, 1024);
-            CKL(launch_run(sh, r, st));
+            const int e = launch_run(sh, r, st);
+            if (e == (int)cudaErrorCooperativeLaunchTooLarge) {  // a context that has not all of the GPU's SMs
+                cudaGetLastError();
+                break;
+            }
+            CKL(e);
         }
-        return SCMF_OK;
+        if (n <= 0) return SCMF_OK;
     }
     // A sweep of warp tiles that do not all fit on the chip takes 50 us and more, so launching its two kernels one by one
     // keeps ahead of the GPU, and each may begin (tables, descriptors) beside the last blocks of the one before, which

@@ -4,7 +4,8 @@ system.  The words are set from the host, by programs built against the library'
 headers: into a member's record, and by a stand-in for the launch of many sweeps.  And a
 launch of many sweeps whose blocks do not wait for one another sets the word, no launch
 uses its barrier again, and the system stays where it is while the others of a batch go
-on."""
+on.  Where a context cannot hold the launch's blocks all at once (again a stand-in says so),
+sweeps are launched one by one."""
 import os
 import subprocess
 
@@ -160,6 +161,35 @@ int main() {
 """
 
 
+SMALL = COMMON + r"""
+// as in a context with a part of the GPU's SMs
+static int asked = 0;
+int scmf::launch_run(const LaunchShape&, const RunArgs&, void*) {
+    ++asked;
+    return (int)cudaErrorCooperativeLaunchTooLarge;
+}
+int main() {
+    scmf_system* s[2] = {started(melt(300, 32, 12, 5)), started(melt(300, 32, 12, 5))};
+    WANT(s[0]->plan.d_run != nullptr, true);
+    WANT(scmf_step(s[0], 7), SCMF_OK);
+    WANT(asked, 1);
+    for (int i = 0; i < 7; ++i) WANT(scmf_step(s[1], 1), SCMF_OK);
+    WANT(asked, 1);
+    std::vector<float> x[2];
+    scmf_stats st[2];
+    for (int i = 0; i < 2; ++i) {
+        x[i].resize(s[i]->n_beads * 3);
+        WANT(scmf_get_coords(s[i], x[i].data(), x[i].size()), SCMF_OK);
+        WANT(scmf_get_sweep_stats(s[i], &st[i]), SCMF_OK);
+        WANT(st[i].step, 7);
+    }
+    WANT(x[0] == x[1], true);
+    WANT(st[0].total_accepts, st[1].total_accepts);
+    return 0;
+}
+"""
+
+
 def _run(tmp_path, program):
     lib = build.LIB
     src, exe = tmp_path / "p.cpp", tmp_path / "p"
@@ -178,6 +208,10 @@ def test_batch(tmp_path):
 
 def test_blocks_that_do_not_wait(tmp_path):
     _run(tmp_path, WAITS)
+
+
+def test_blocks_that_do_not_fit(tmp_path):
+    _run(tmp_path, SMALL)
 
 
 def test_server(tmp_path):

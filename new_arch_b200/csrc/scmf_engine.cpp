@@ -360,14 +360,14 @@ scmf_tune resolve_tune(const scmf_tune* t) {
 void DevPlan::release() {
     if (graph) cudaGraphExecDestroy(graph);
     if (graph_src) cudaGraphDestroy(graph_src);
-    void* ptrs[] = {d_move, d_field, d_close, d_warp, d_ef, d_eb, d_run};
+    void* ptrs[] = {d_move, d_field, d_close, tiles.list, single.list == tiles.list ? nullptr : single.list, d_ef, d_eb, d_run};
     for (void* p : ptrs) dev_free(p, stream);
     graph = nullptr;
     graph_src = nullptr;
     d_move = nullptr;
     d_field = nullptr;
     d_close = nullptr;
-    d_warp = nullptr;
+    tiles = single = WarpTiles{};
     d_run = nullptr;
     d_ef = nullptr;
     d_eb = nullptr;
@@ -415,6 +415,22 @@ static int tiles_of(const std::vector<SweepArch>& ranges) {
     return ranges.empty() ? 0 : ranges.back().first + (ranges.back().n_chains + ranges.back().per - 1) / ranges.back().per;
 }
 
+// The tiles of k_sweep_pairs, where at least three lanes of four have a pair; empty otherwise.
+static std::vector<SweepArch> pairs_ranges(const Plan& p, int* form) {
+    int64_t pairs = 0, lanes = 0;
+    bool even = p.cells.size() == 1 && p.chains.size() <= kSweepMaxArch;
+    for (const auto& c : p.chains) {
+        if (!c.linear || c.length > 64) return {};
+        const int h = (c.length + 1) / 2, per = 32 / h;
+        pairs += (int64_t)h * c.n_chains;
+        lanes += (int64_t)32 * ((c.n_chains + per - 1) / per);
+        even = even && (c.length | c.bead_base) % 2 == 0;
+    }
+    if (4 * pairs < 3 * lanes) return {};
+    *form = even ? kFormPairs : kFormPairsList;
+    return form_ranges(p, *form);
+}
+
 std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     if (p.chains.empty() || !p.cells32 || p.max_deg > kGraphDeg) return {};
     int64_t beads = 0, exact = 0;  // all, and those of chains whose trials k_sweep_pairs makes as fast as a screen does
@@ -432,22 +448,11 @@ std::vector<SweepArch> tile_ranges(const Plan& p, int* form) {
     // on also than in k_run: a sweep of 0.4M beads 12.4 us in k_run and 16.0 so, 0.8M 21.3 and 18.9 (in chains of 48 or 64
     // 19.4 and 20.3, 19.0 and 19.7), 2.0M 46.1 and 33.5, 20.5M 379 (in tiles) and 223.  So are those of many systems of
     // which a quarter of the beads is not screened: 32M beads, 25 % 467 us in tiles and 432 so, 50 % 634 and 452, 10 % 350 and
-    // 399.  At least three lanes of four must have a pair.
+    // 399.
     const int64_t warps = (int64_t)sm_count() * kSweepForms[*form].warps;
-    if (p.linear && (exact == beads ? beads > 352 * warps : tiles_of(out) > warps && 4 * exact >= beads)) {
-        int64_t pairs = 0, lanes = 0;
-        bool even = p.cells.size() == 1 && p.chains.size() <= kSweepMaxArch;
-        for (const auto& c : p.chains) {
-            if (c.length > 64) return out;
-            const int h = (c.length + 1) / 2, per = 32 / h;
-            pairs += (int64_t)h * c.n_chains;
-            lanes += (int64_t)32 * ((c.n_chains + per - 1) / per);
-            even = even && (c.length | c.bead_base) % 2 == 0;
-        }
-        if (4 * pairs >= 3 * lanes) {
-            *form = even ? kFormPairs : kFormPairsList;
-            out = form_ranges(p, *form);
-        }
+    if (exact == beads ? beads > 352 * warps : tiles_of(out) > warps && 4 * exact >= beads) {
+        std::vector<SweepArch> in_pairs = pairs_ranges(p, form);
+        if (!in_pairs.empty()) return in_pairs;
     }
     return out;
 }
@@ -540,35 +545,52 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     one_seed_hi = p.one_seed_hi && !p.close.empty();
     seed = p.seed;
     n_sys = (int)p.close.size();
-    form = kFormScreened;
+    system = n_sys == 1 ? p.close[0].sys : nullptr;
+    std::vector<WarpTile> lists[2];
+    const auto place = [&](const std::vector<SweepArch>& ranges, int form, WarpTiles* w, std::vector<WarpTile>* list) -> scmf_status {
+        w->form = form;
+        w->n = tiles_of(ranges);
+        w->one = n_sys == 1 && ranges.size() <= kSweepMaxArch && form != kFormPairsList;
+        if (w->one) {
+            w->n_arch = (int)ranges.size();
+            std::copy(ranges.begin(), ranges.end(), w->arch);
+            return SCMF_OK;
+        }
+        *list = tile_list(p, ranges);
+        scmf_status e = dev_alloc((void**)&w->list, std::max<size_t>(1, list->size()) * sizeof(WarpTile), st);
+        if (!e && !list->empty())
+            CK(cudaMemcpyAsync(w->list, list->data(), list->size() * sizeof(WarpTile), cudaMemcpyHostToDevice, st));
+        return e;
+    };
+    int form = kFormScreened;
     const std::vector<SweepArch> ranges = tile_ranges(p, &form);
-    n_warp = tiles_of(ranges);
-    one = n_sys == 1 && ranges.size() <= kSweepMaxArch && form != kFormPairsList;
-    std::vector<WarpTile> wt;
-    if (one) {
-        system = p.close[0].sys;
-        n_arch = (int)ranges.size();
-        std::copy(ranges.begin(), ranges.end(), arch);
-    } else {
-        wt = tile_list(p, ranges);
+    scmf_status rc = place(ranges, form, &tiles, &lists[0]);
+    if (rc) return rc;
+    // A launch of one sweep has none of what makes k_run the faster of the two for few unscreened beads: 0.4M beads 18.9 us
+    // a sweep in tiles and 16.1 in pairs, 0.8M 25.5 and 19.4, 10,000 11.2 and 10.4.
+    single = tiles;
+    if (form == kFormUnscreened) {
+        const std::vector<SweepArch> in_pairs = pairs_ranges(p, &form);
+        if (!in_pairs.empty()) {
+            single = WarpTiles{};
+            if ((rc = place(in_pairs, form, &single, &lists[1]))) return rc;
+        }
     }
+    n_warp = single.n;
     sweep = p.sweep;
     once = p.position_bytes > kL2Bytes / 2;
     const size_t nm = std::max<size_t>(1, p.move.size()), nf = std::max<size_t>(1, p.field.size());
-    scmf_status rc;
     if ((rc = dev_alloc((void**)&d_move, nm * sizeof(MoveTile), st)) ||
         (rc = dev_alloc((void**)&d_field, nf * sizeof(FieldTile), st)) ||
         (rc = dev_alloc((void**)&d_close, (p.close.size() + 1) * sizeof(SysClose), st)) ||  // and the word of check()
-        (rc = dev_alloc((void**)&d_warp, std::max<size_t>(1, wt.size()) * sizeof(WarpTile), st)) ||
         (rc = dev_alloc((void**)&d_ef, nf * sizeof(double), st)) || (rc = dev_alloc((void**)&d_eb, nm * sizeof(double), st)))
         return rc;
-    if (!wt.empty()) CK(cudaMemcpyAsync(d_warp, wt.data(), wt.size() * sizeof(WarpTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_move, p.move.data(), p.move.size() * sizeof(MoveTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_field, p.field.data(), p.field.size() * sizeof(FieldTile), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_close, p.close.data(), p.close.size() * sizeof(SysClose), cudaMemcpyHostToDevice, st));
     std::vector<char> run_image;
-    if (runs_at_once(p, n_warp, form)) {
-        run_image = run_tables(p, n_warp, form, &run);
+    if (runs_at_once(p, tiles.n, tiles.form)) {
+        run_image = run_tables(p, tiles.n, tiles.form, &run);
         if ((rc = dev_alloc(&d_run, run_image.size(), st))) return rc;
         CK(cudaMemcpyAsync(d_run, run_image.data(), run_image.size(), cudaMemcpyHostToDevice, st));
         const auto at = [&](const void* offset) { return (char*)d_run + (size_t)offset; };
@@ -582,20 +604,21 @@ scmf_status DevPlan::upload(const Plan& p, const scmf_tune& t, cudaStream_t st) 
     return SCMF_OK;
 }
 
-LaunchShape DevPlan::move_shape() const {
+LaunchShape DevPlan::move_shape(bool many) const {
+    const WarpTiles& w = many ? tiles : single;
     LaunchShape sh{};
     sh.blocks = tune.persistent_ctas > 0 ? std::min(tune.persistent_ctas, n_move) : 0;
     sh.threads = tune.threads_move;
     sh.n_types = n_types_uniform;
     sh.keyed = one_seed ? kKeysBoth : (one_seed_hi ? kKeysHigh : kKeysNone);
     sh.keys = philox_schedule((uint32_t)seed, (uint32_t)(seed >> 32));
-    sh.warp_tiles = d_warp;
-    sh.n_warp_tiles = n_warp;
-    sh.form = form;
-    sh.one = one ? 1 : 0;
+    sh.warp_tiles = w.list;
+    sh.n_warp_tiles = w.n;
+    sh.form = w.form;
+    sh.one = w.one ? 1 : 0;
     sh.system = system;
-    sh.n_arch = one ? n_arch : 0;
-    for (int i = 0; i < sh.n_arch; ++i) sh.arch[i] = arch[i];
+    sh.n_arch = w.n_arch;
+    for (int i = 0; i < sh.n_arch; ++i) sh.arch[i] = w.arch[i];
     sh.once = once ? 1 : 0;
     sh.sweep = sweep;
     return sh;
@@ -648,7 +671,7 @@ scmf_status DevPlan::run_sweeps(cudaStream_t st, int n) {
     // 2.0M beads 22.4 against 32.8; two sweeps a call are the same either way, three faster in one launch).
     if (d_run && n > 1) {
         // some milliseconds a launch, so that other work on the GPU gets its turn
-        const LaunchShape sh = move_shape();
+        const LaunchShape sh = move_shape(true);
         for (RunArgs r = run; n > 0; n -= r.n_sweeps) {
             r.n_sweeps = std::min(n, 1024);
             const int e = launch_run(sh, r, st);

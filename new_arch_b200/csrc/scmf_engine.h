@@ -103,6 +103,14 @@ struct Plan {
 // (SweepFormId); empty for a plan that takes the general move kernel.
 std::vector<SweepArch> tile_ranges(const Plan& p, int* form);
 
+// The warp tiles of a launch: a list, or for one system of few architectures their ranges.
+struct WarpTiles {
+    WarpTile* list = nullptr;
+    int n = 0, form = kFormScreened, n_arch = 0;
+    bool one = false;
+    SweepArch arch[kSweepMaxArch] = {};
+};
+
 struct DevPlan {
     MoveTile* d_move = nullptr;
     FieldTile* d_field = nullptr;
@@ -110,18 +118,14 @@ struct DevPlan {
     // k_run: its systems, field tiles, partial energies and barrier, in one buffer
     void* d_run = nullptr;
     RunArgs run{};
-    // one system of few architectures: its constants and tile ranges (no list)
-    bool one = false;
-    SysDev* system = nullptr;
+    SysDev* system = nullptr;  // of a plan of one: itself and its constants
     SweepSys sweep{};
-    int n_arch = 0;
-    SweepArch arch[kSweepMaxArch] = {};
+    WarpTiles tiles, single;   // of many sweeps a launch; of one (the same, or those of k_sweep_pairs)
     bool once = false;           // the positions are more than L2 holds
-    WarpTile* d_warp = nullptr;  // warp tiles, where the launch has a list (see tile_ranges)
     double* d_ef = nullptr;      // field energy per field tile
     double* d_eb = nullptr;      // bond energy per move tile
-    int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;
-    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0, form = 0;
+    int n_move = 0, n_field = 0, n_sys = 0, n_warp = 0;  // n_warp: of `single`, 0 for the general move kernel
+    int max_tile_beads = 0, max_length = 0, n_types_uniform = 0;
     bool one_seed = false;     // every system of the plan has `seed`: move launches take its key schedule
     bool one_seed_hi = false;  // they share its upper 32 bits: the second key word's schedule
     uint64_t seed = 0;
@@ -131,7 +135,7 @@ struct DevPlan {
     cudaStream_t stream = nullptr;  // allocations of the plan are ordered on it
     void release();
     scmf_status upload(const Plan& p, const scmf_tune& t, cudaStream_t st);
-    LaunchShape move_shape() const;
+    LaunchShape move_shape(bool many = false) const;  // of a launch of one sweep, or of many
     LaunchShape field_shape() const;
     // one fused sweep enqueued on `st`: the move launch, then the field launch
     // whose last tile per system closes the sweep
